@@ -234,6 +234,26 @@ def test_rmsnorm_and_mlp_block(M, with_weight, residual):
         assert np.array_equal(plain.numpy(), out.numpy())
 
 
+@pytest.mark.parametrize("M,K,pad", [(1, 64, 0), (3, 4096, 0), (2, 4104, 8), (2, 16384, 0), (1, 16392, 0), (5, 250, 0), (4, 1000, 4)])
+@pytest.mark.parametrize("with_weight", [False, True])
+def test_rmsnorm_edges(M, K, pad, with_weight):
+    """both forms of the kernel at the edges of their ranges: whole 16-byte units in registers (up to K = 16384, rows with a
+    padded pitch), and the element-wise form (K beyond that, K or the pitch no multiple of 8); within one bf16 ulp of the oracle, two
+    with a weight (rsqrt against 1 / sqrt, one more rounding)"""
+    rng = np.random.default_rng(K + M)
+    ld = K + pad
+    x = H.normal_bf16(rng, (M, ld), 1.5)
+    wn = H.normal_bf16(rng, (K,), 1.0) if with_weight else None
+    dx, dw = H.Dev(x), H.Dev(wn) if with_weight else None
+    dn = H.Dev(shape=(M, ld), dtype=np.uint16, fill=0xCD)
+    capi.rmsnorm(dx.ptr, ld * 2, M, K, 1e-6, dn.ptr, ld * 2, dw.ptr if dw else None)
+    capi.sync_check()
+    got = dn.numpy()
+    want = port.rmsnorm(np.ascontiguousarray(x[:, :K]), 1e-6, wn)
+    assert np.abs(got[:, :K].astype(np.int32) - want.astype(np.int32)).max() <= (2 if with_weight else 1)
+    assert (got[:, K:] == 0xCDCD).all()
+
+
 def test_decode_mlp_in_one_launch_subprocess():
     """B200FC_MLP_FUSED=1 (read once per process, hence the child process): gate/up and down of a decode-shaped MLP run
     as two jobs of ONE launch with a bounded grid-wide barrier between them.  Off by default (measured slower than two
