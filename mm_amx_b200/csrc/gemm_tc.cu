@@ -17,26 +17,15 @@
 //   stores are predicated.
 // Every mbarrier wait is bounded: when one runs out, the CTA raises an abort flag, all roles fall through to the
 // common exit (TMEM is freed there) and the kernel stores an error code for the host.
-#include <cuda.h>
 #include <cstdlib>
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace b200fc {
 
 namespace {
 
-constexpr int BM = 128;
-constexpr int SLAB_BYTES = 128;          // K extent of one pipeline stage, in bytes of operand elements
-constexpr int MMA_K_BYTES = 32;          // K extent of one tcgen05.mma (16 bf16 / 32 int8)
 constexpr int NUM_THREADS = 192;
 constexpr int EPI_WARP0 = 2;
-#ifndef B200FC_EPI_SLEEP_NS
-#define B200FC_EPI_SLEEP_NS 256
-#endif
-constexpr int EPI_SLEEP_NS = B200FC_EPI_SLEEP_NS;
-
-// staging tiles of the four epilogue warps: 32 rows x 32 four-byte columns each, rows padded to 33 words
-constexpr int EPI_TILE_WORDS = 32 * 33;
 constexpr int EPI_TILE_BYTES = 4 * EPI_TILE_WORDS * 4;
 
 template <int BN> struct Cfg {
@@ -80,351 +69,6 @@ struct GemmParams {
     char* ar_out_mc;            // multicast address of all replicas of the output buffer
     unsigned long long wait_limit_ns;  // every bounded wait gives up after this long
 };
-
-// ---- PTX wrappers ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned long long globaltimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait.  Returns false when the CTA is aborting (this wait or another role's ran out of time).
-// SLEEP_NS > 0: back off between polls (for waits that are long and not latency critical: the epilogue warps wait most
-// of a tile's main loop, and five spinning warps cost issue slots and power that the tensor pipe could use).
-template <int SLEEP_NS = 0>
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int* abort_flag, unsigned long long limit) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = globaltimer();
-    while (true) {
-        if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (globaltimer() - t0 > limit) {
-            *abort_flag = 1;
-            return false;
-        }
-    }
-}
-__device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, unsigned bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
-        : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-template <bool I8>
-__device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc,
-                                       unsigned idesc, unsigned accumulate) {
-    if constexpr (I8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    }
-}
-__device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Shared-memory operand descriptor: K-major tile, rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes
-// apart (stride-dimension byte offset); descriptor version 1 (Blackwell).
-__device__ __forceinline__ unsigned long long make_smem_desc(unsigned smem_addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (unsigned long long)1 << 16;            // leading-dimension byte offset (unused for swizzled K-major)
-    d |= (unsigned long long)(1024 >> 4) << 32;  // stride-dimension byte offset
-    d |= (unsigned long long)1 << 46;            // descriptor version
-    d |= (unsigned long long)2 << 61;            // SWIZZLE_128B
-    return d;
-}
-
-// ---- epilogue on 32 consecutive columns of one output row ------------------------------------------------------------
-struct EpiArgs {       // what the epilogue of one 32-column chunk needs to know
-    const Epilogue* ep;
-    int vec_ok, acc_is_int, n1;
-    int M;             // rows of the output
-    unsigned* tile;    // this warp's staging tile in shared memory (EPI_TILE_WORDS words)
-    // the chunk's 32 per-column values, staged in shared memory ahead of the tile (16-byte aligned), or null: read
-    // them from global memory
-    const float* cv_deq = nullptr;
-    const float* cv_bias = nullptr;
-    const float* cv_q = nullptr;
-};
-// 32 rows x 32 four-byte values, one row per lane in registers -> global memory with full-line stores: the tile goes
-// through shared memory and comes back with eight lanes per row (16 bytes each), so that one store instruction writes
-// four whole 128-byte row segments instead of 32 scattered 16-byte pieces.  Both passes use 16-byte accesses: row r
-// keeps its 16-byte piece j at position j ^ (r & 7), which makes the eight lanes of every shared-memory wavefront hit
-// eight different bank groups on the way in (lanes = rows) and on the way out (lanes = pieces of one row).
-// Called by all lanes of the warp; `tile` is 16-byte aligned.
-__device__ __forceinline__ void store_tile_4b(const unsigned (&val)[32], unsigned* tile, char* C, long long ldc, int m, int n,
-                                              int M) {
-    const int lane = threadIdx.x & 31, m0 = m - lane;
-    uint4* t4 = (uint4*)tile;
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-        t4[lane * 8 + (j ^ (lane & 7))] = make_uint4(val[4 * j], val[4 * j + 1], val[4 * j + 2], val[4 * j + 3]);
-    __syncwarp();
-    const int piece = lane & 7;
-#pragma unroll
-    for (int it = 0; it < 8; it++) {
-        const int rr = it * 4 + (lane >> 3);
-        const uint4 q = t4[rr * 8 + (piece ^ (rr & 7))];
-        if (m0 + rr < M) *(uint4*)(C + (long long)(m0 + rr) * ldc + (long long)(n + piece * 4) * 4) = q;
-    }
-    __syncwarp();
-}
-// the 32 per-column values vec[n .. n + 32) of a chunk (every lane needs all of them): eight 16-byte loads when the
-// chunk is whole and the vector 16-byte aligned, else 32 scalar loads clamped to the last valid column
-__device__ __forceinline__ void load_col_vec(const float* __restrict__ vec, int n, int n1, float (&out)[32]) {
-    if (n + 32 <= n1 && (((uintptr_t)(vec + n)) & 15) == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float4 t = __ldg((const float4*)(vec + n) + j);
-            out[4 * j] = t.x; out[4 * j + 1] = t.y; out[4 * j + 2] = t.z; out[4 * j + 3] = t.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; j++) out[j] = __ldg(vec + min(n + j, n1 - 1));
-    }
-}
-// the same 32 values from the warp's staged copy (every lane reads the same addresses: broadcasts)
-__device__ __forceinline__ void load_col_vec(const float* staged, const float* __restrict__ vec, int n, int n1, float (&out)[32]) {
-    if (staged) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float4 t = ((const float4*)staged)[j];
-            out[4 * j] = t.x; out[4 * j + 1] = t.y; out[4 * j + 2] = t.z; out[4 * j + 3] = t.w;
-        }
-    } else {
-        load_col_vec(vec, n, n1, out);
-    }
-}
-__device__ __forceinline__ void epilogue_chunk(const unsigned (&r)[32], int m, int n, const EpiArgs p, bool row_ok,
-                                               long long c_offset = 0) {
-    const Epilogue& ep = *p.ep;
-    const bool staged = p.vec_ok && n + 32 <= p.n1 && !ep.mc_reduce;   // warp-uniform
-    if (ep.out_dtype == B200FC_S32 && staged) {
-        store_tile_4b(r, p.tile, (char*)ep.C + c_offset, ep.ldc, m, n, p.M);
-        return;
-    }
-    const bool staged_f32 = ep.out_dtype == B200FC_F32 && staged && !(ep.steps & B200FC_STEP_SILU_MUL);   // warp-uniform
-    if (!row_ok && !staged_f32) return;   // (rows beyond M take part in the staged store's shuffle through shared memory)
-    char* crow = (char*)ep.C + c_offset + (long long)m * ep.ldc;
-    if (ep.out_dtype == B200FC_S32) {  // raw accumulators
-        if (p.vec_ok && n + 32 <= p.n1) {
-            int4* dst = (int4*)(crow + (long long)n * 4);
-#pragma unroll
-            for (int j = 0; j < 8; j++) dst[j] = make_int4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((int*)crow)[n + j] = (int)r[j];
-        }
-        return;
-    }
-    float v[32];
-#pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = p.acc_is_int ? (float)(int)r[j] : __uint_as_float(r[j]);
-
-    if (ep.mc_reduce) {
-        // Fused all-reduce: C is a multicast mapping of the output on every GPU of the tensor-parallel group; the
-        // NVSwitch adds this rank's contribution into all replicas (multimem.red), so no separate collective runs.
-        const bool full = p.vec_ok && n + 32 <= p.n1;
-        if (ep.out_dtype == B200FC_F32) {
-            float* dst = (float*)(crow + (long long)n * 4);
-            if (full) {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    asm volatile("multimem.red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
-                                 "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
-                                 : "memory");
-            } else {
-                for (int j = 0; j < 32; j++)
-                    if (n + j < p.n1) asm volatile("multimem.red.relaxed.sys.global.add.f32 [%0], %1;" ::"l"(dst + j), "f"(v[j]) : "memory");
-            }
-        } else {
-            unsigned short* dst = (unsigned short*)(crow + (long long)n * 2);
-            if (full) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    unsigned o[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
-                        o[q] = *(unsigned*)&h;
-                    }
-                    asm volatile("multimem.red.relaxed.sys.global.add.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dst + 8 * j),
-                                 "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3])
-                                 : "memory");
-                }
-            } else {
-                for (int j = 0; j < 32; j += 2)   // the launcher guarantees an even column range for this mode
-                    if (n + j + 1 < p.n1) {
-                        __nv_bfloat162 h = __floats2bfloat162_rn(v[j], v[j + 1]);
-                        asm volatile("multimem.red.relaxed.sys.global.add.bf16x2 [%0], %1;" ::"l"(dst + j), "r"(*(unsigned*)&h) : "memory");
-                    }
-            }
-        }
-        return;
-    }
-
-    if (ep.steps & B200FC_STEP_SILU_MUL) {
-        // columns [0,16) gate, [16,32) up of the same 16 channels -> 16 bf16 outputs at column n/2
-        __align__(16) unsigned short o[16];
-#pragma unroll
-        for (int j = 0; j < 16; j++) o[j] = f32_to_bf16_bits(silu_f(v[j]) * v[16 + j]);
-        int nc = n >> 1;
-        unsigned short* dst = (unsigned short*)crow + nc;
-        if (p.vec_ok && n + 32 <= p.n1) {
-            ((int4*)dst)[0] = *(int4*)&o[0];
-            ((int4*)dst)[1] = *(int4*)&o[8];
-        } else {
-            for (int j = 0; j < 16; j++)
-                if (n + 16 + j < p.n1) dst[j] = o[j];
-        }
-        return;
-    }
-
-    if (ep.steps & B200FC_STEP_DEQUANT) {
-        if (ep.deq_per_oc) {
-            float sc[32];
-            load_col_vec(p.cv_deq, ep.deq_per_oc, n, p.n1, sc);
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] *= ep.deq_scale * sc[j];
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] *= ep.deq_scale;
-        }
-    }
-    if (ep.steps & B200FC_STEP_BIAS) {
-        float bs[32];
-        load_col_vec(p.cv_bias, ep.bias, n, p.n1, bs);
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] += bs[j];
-    }
-    if (ep.steps & B200FC_STEP_GELU) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = gelu_erf_poly(v[j]);
-    }
-    if (ep.steps & B200FC_STEP_QUANT) {
-        if (ep.q_per_oc) {
-            float qs[32];
-            load_col_vec(p.cv_q, ep.q_per_oc, n, p.n1, qs);
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] *= qs[j];
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] *= ep.q_scale;
-        }
-    }
-    const bool full = p.vec_ok && n + 32 <= p.n1;
-    if (ep.residual && row_ok) {
-        // residual added in fp32, before the one rounding of the output
-        const char* rrow = (const char*)ep.residual + (long long)m * ep.ld_res;
-        if (full && (((uintptr_t)rrow + (size_t)n * 2) & 15) == 0) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int4 t = __ldg((const int4*)(rrow + (long long)n * 2) + q);
-                const unsigned w4[4] = {(unsigned)t.x, (unsigned)t.y, (unsigned)t.z, (unsigned)t.w};
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    v[8 * q + 2 * e] += __uint_as_float(w4[e] << 16);
-                    v[8 * q + 2 * e + 1] += __uint_as_float(w4[e] & 0xffff0000u);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++)
-                v[j] += __uint_as_float((unsigned)((const unsigned short*)rrow)[min(n + j, p.n1 - 1)] << 16);
-        }
-    }
-    if (staged_f32) {
-        unsigned u[32];
-#pragma unroll
-        for (int j = 0; j < 32; j++) u[j] = __float_as_uint(v[j]);
-        store_tile_4b(u, p.tile, (char*)ep.C + c_offset, ep.ldc, m, n, p.M);
-    } else if (ep.out_dtype == B200FC_F32) {
-        if (full) {
-            float4* dst = (float4*)(crow + (long long)n * 4);
-#pragma unroll
-            for (int j = 0; j < 8; j++) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((float*)crow)[n + j] = v[j];
-        }
-    } else if (ep.out_dtype == B200FC_BF16) {
-        if (full) {
-            __align__(16) unsigned o[16];
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                o[j] = *(unsigned*)&h;
-            }
-            int4* dst = (int4*)(crow + (long long)n * 2);
-#pragma unroll
-            for (int j = 0; j < 4; j++) dst[j] = *(int4*)&o[4 * j];
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((unsigned short*)crow)[n + j] = f32_to_bf16_bits(v[j]);
-        }
-    } else {  // int8
-        if (full) {
-            __align__(16) unsigned o[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                unsigned b0 = f32_to_s8(v[4 * j]) & 0xff, b1 = f32_to_s8(v[4 * j + 1]) & 0xff;
-                unsigned b2 = f32_to_s8(v[4 * j + 2]) & 0xff, b3 = f32_to_s8(v[4 * j + 3]) & 0xff;
-                o[j] = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
-            }
-            int4* dst = (int4*)(crow + n);
-            dst[0] = *(int4*)&o[0];
-            dst[1] = *(int4*)&o[4];
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((signed char*)crow)[n + j] = (signed char)f32_to_s8(v[j]);
-        }
-    }
-}
 
 // ---- the kernel --------------------------------------------------------------------------------------------------------
 template <int BN, bool I8>
@@ -473,7 +117,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        {
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -481,19 +125,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
                 const int row_a = tm * BM, row_w = p.n0 + tn * BN;
                 for (int ks = 0; ks < p.k_slabs; ks++) {
-                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns));
+                    if (!ok) break;
                     const unsigned full = bar_full + 8 * stage;
-                    mbar_expect_tx(full, C::STAGE_BYTES);
                     const unsigned sa = smem_u32(smem + stage * C::STAGE_BYTES);
                     const int kx = ks * (I8 ? SLAB_BYTES : SLAB_BYTES / 2);  // element coordinate along K
-                    tma_load_2d(sa, &map_a, full, kx, row_a);
-                    tma_load_2d(sa + C::A_BYTES, &map_w, full, kx, row_w);
+                    if (elect_one()) {
+                        mbar_expect_tx(full, C::STAGE_BYTES);
+                        tma_load_2d(sa, &map_a, full, kx, row_a);
+                        tma_load_2d(sa + C::A_BYTES, &map_w, full, kx, row_w);
+                    }
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
+        // ---------------- MMA issuer (the whole warp; see elect_one) ----------------
         int stage = 0;
         unsigned phase = 0;
         int it = 0;
@@ -501,16 +148,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, it++) {
             const int ab = it & 1;
             const unsigned acc_phase = (unsigned)(it >> 1) & 1;
-            if (!mbar_wait(bar_acc_empty + 8 * ab, acc_phase ^ 1, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty + 8 * ab, acc_phase ^ 1, abort_flag, p.wait_limit_ns));
+            if (!ok) break;
             tc_fence_after();
             const unsigned d_tmem = tmem_base + (unsigned)(ab * BN);
             for (int ks = 0; ks < p.k_slabs; ks++) {
-                if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.wait_limit_ns));
+                if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) {
-                    const unsigned sa = smem_u32(smem + stage * C::STAGE_BYTES);
-                    const unsigned long long adesc = make_smem_desc(sa);
-                    const unsigned long long bdesc = make_smem_desc(sa + C::A_BYTES);
+                const unsigned sa = smem_u32(smem + stage * C::STAGE_BYTES);
+                const unsigned long long adesc = make_smem_desc(sa);
+                const unsigned long long bdesc = make_smem_desc(sa + C::A_BYTES);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++) {
                         // advancing K inside the swizzle atom = advancing the start address (units of 16 bytes)
@@ -521,7 +170,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     tc_commit(bar_empty + 8 * stage);  // frees the stage once these MMAs have read it
                     if (ks == p.k_slabs - 1) tc_commit(bar_acc_full + 8 * ab);
                 }
-                __syncwarp();
                 if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
             }
         }
@@ -598,38 +246,6 @@ template <int BN> struct Cfg2 {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + EPI_TILE_BYTES + COLVEC_BYTES;
 };
 
-__device__ __forceinline__ unsigned cluster_ctarank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of the same shared-memory offset in CTA `rank` of the cluster
-__device__ __forceinline__ unsigned mapa_rank(unsigned addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_arrive_remote(unsigned cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(unsigned dst, const CUtensorMap* map, unsigned leader_bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(leader_bar), "r"(x), "r"(y)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair_keep(unsigned dst, const CUtensorMap* map, unsigned leader_bar, int x, int y,
-                                                      unsigned long long policy) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-        " [%0], [%1, {%3, %4}], [%2], %5;"
-        ::"r"(dst), "l"(map), "r"(leader_bar), "r"(x), "r"(y), "l"(policy)
-        : "memory");
-}
 // tile index (the order in which the CTA pairs take tiles) -> row tile tm and column tile tn
 __device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& tm, int& tn) {
     if (p.panel_rows <= 0 || p.panel_rows >= p.tiles_m) {
@@ -641,29 +257,6 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& 
         tm = pi * p.panel_rows + r % ph; tn = r / ph;
     }
 }
-__device__ __forceinline__ void tc_commit_pair(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"((unsigned short)3)
-                 : "memory");
-}
-template <bool I8>
-__device__ __forceinline__ void tc_mma_pair(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc,
-                                            unsigned idesc, unsigned accumulate) {
-    if constexpr (I8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    }
-}
-
 constexpr int AR_UNROLL = 22;  // 192 threads x 22 pieces cover the 4096 pieces of a 128 x 256 bf16 unit
 
 // All-reduce work of the fused tensor-parallel down projection, run by whole CTAs: the pairs reserved for it from the
@@ -793,7 +386,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     } else if (p.ar_world && !(p.ar_phases & 1)) {
     } else if (warp == 0) {
         // ---------------- TMA producer (one per CTA) ----------------
-        if (lane == 0) {
+        {
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -808,20 +401,23 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 const int row_a = tm * (2 * BM) + (int)rank * BM;
                 const int row_w = p.n0 + tn * BN + (int)rank * (BN / 2);
                 for (int ks = ks0; ks < ks1; ks++) {
-                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) { ok = false; break; }
-                    if (leader) mbar_expect_tx(bar_full + 8 * stage, 2 * C::STAGE_BYTES);
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns));
+                    if (!ok) break;
                     const unsigned sa = smem_u32(smem + stage * C::STAGE_BYTES);
                     const int kx = ks * (I8 ? SLAB_BYTES : SLAB_BYTES / 2);
-                    if (p.panel_rows > 0) tma_load_2d_pair_keep(sa, &map_a, leader_full + 8 * stage, kx, row_a, keep_policy);
-                    else tma_load_2d_pair(sa, &map_a, leader_full + 8 * stage, kx, row_a);
-                    tma_load_2d_pair(sa + C::A_BYTES, &map_w, leader_full + 8 * stage, kx, row_w);
+                    if (elect_one()) {
+                        if (leader) mbar_expect_tx(bar_full + 8 * stage, 2 * C::STAGE_BYTES);
+                        if (p.panel_rows > 0) tma_load_2d_pair_keep(sa, &map_a, leader_full + 8 * stage, kx, row_a, keep_policy);
+                        else tma_load_2d_pair(sa, &map_a, leader_full + 8 * stage, kx, row_a);
+                        tma_load_2d_pair(sa + C::A_BYTES, &map_w, leader_full + 8 * stage, kx, row_w);
+                    }
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer (leader CTA only; one thread waits and issues, its warp mates park) ----------------
-        if (leader && lane == 0) {
+        // ---------------- MMA issuer (leader CTA only; the whole warp, see elect_one) ----------------
+        if (leader) {
             int stage = 0;
             unsigned phase = 0;
             int it = 0;
@@ -831,22 +427,26 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 const int ks0 = p.k_slabs * split / p.splits, ks1 = p.k_slabs * (split + 1) / p.splits;
                 const int ab = it & 1;
                 const unsigned acc_phase = (unsigned)(it >> 1) & 1;
-                if (!mbar_wait(bar_acc_empty + 8 * ab, acc_phase ^ 1, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty + 8 * ab, acc_phase ^ 1, abort_flag, p.wait_limit_ns));
+                if (!ok) break;
                 tc_fence_after();
                 const unsigned d_tmem = tmem_base + (unsigned)(ab * BN);
                 for (int ks = ks0; ks < ks1; ks++) {
-                    if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.wait_limit_ns));
+                    if (!ok) break;
                     tc_fence_after();
                     const unsigned sa = smem_u32(smem + stage * C::STAGE_BYTES);
                     const unsigned long long adesc = make_smem_desc(sa);
                     const unsigned long long bdesc = make_smem_desc(sa + C::A_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++)
-                        tc_mma_pair<I8>(d_tmem, adesc + (unsigned long long)(k * (MMA_K_BYTES >> 4)),
-                                        bdesc + (unsigned long long)(k * (MMA_K_BYTES >> 4)), p.idesc,
-                                        (unsigned)(((ks - ks0) | k) != 0));
-                    tc_commit_pair(bar_empty + 8 * stage);
-                    if (ks == ks1 - 1) tc_commit_pair(bar_acc_full + 8 * ab);
+                        for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++)
+                            tc_mma_pair<I8>(d_tmem, adesc + (unsigned long long)(k * (MMA_K_BYTES >> 4)),
+                                            bdesc + (unsigned long long)(k * (MMA_K_BYTES >> 4)), p.idesc,
+                                            (unsigned)(((ks - ks0) | k) != 0));
+                        tc_commit_pair(bar_empty + 8 * stage);
+                        if (ks == ks1 - 1) tc_commit_pair(bar_acc_full + 8 * ab);
+                    }
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -1008,71 +608,6 @@ __global__ void splitk_reduce_kernel(const unsigned* __restrict__ ws, long long 
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)sym;
-    }
-    return fn;
-}
-
-// 2-D K-major tensor map: inner dimension = K elements, outer = rows; box = {128 bytes of K, box_rows}.
-int make_map(CUtensorMap* map, const void* base, bool i8, uint64_t k_elems, uint64_t rows, uint64_t ld_bytes,
-             uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) { set_error("cuTensorMapEncodeTiled entry point not available"); return B200FC_ERR_CUDA; }
-    cuuint64_t dims[2] = {k_elems, rows};
-    cuuint64_t strides[1] = {ld_bytes};
-    cuuint32_t box[2] = {(cuuint32_t)(i8 ? SLAB_BYTES : SLAB_BYTES / 2), box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, i8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims,
-                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (%d)", (int)r); return B200FC_ERR_CUDA; }
-    return B200FC_OK;
-}
-
-// tcgen05 instruction descriptor (dense, K-major A and B, M = 128): accumulator format bits [4,6), A format [7,10),
-// B format [10,13), N >> 3 at [17,23), M >> 4 at [24,29).
-unsigned make_idesc(bool i8, bool a_signed, bool b_signed, int bn, int mma_m = BM) {
-    unsigned d = 0;
-    if (i8) {
-        d |= 2u << 4;                       // int32 accumulator
-        d |= (a_signed ? 1u : 0u) << 7;     // 8-bit integer: 1 = signed, 0 = unsigned
-        d |= (b_signed ? 1u : 0u) << 10;
-    } else {
-        d |= 1u << 4;                       // fp32 accumulator
-        d |= 1u << 7;                       // bf16
-        d |= 1u << 10;
-    }
-    d |= (unsigned)(bn >> 3) << 17;
-    d |= (unsigned)(mma_m >> 4) << 24;
-    return d;
-}
-
-int num_sms() {
-    static std::atomic<int> cache[64];   // SM count per device ordinal (0 = not asked yet)
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int n = cache[dev & 63].load(std::memory_order_relaxed);
-    if (!n) {
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-        cache[dev & 63].store(n, std::memory_order_relaxed);
-    }
-    // the persistent GEMM grids take one CTA per SM; a caller that overlaps a collective with them leaves it a few SMs
-    const int lim = sm_limit();
-    return (lim >= 2 && lim < n) ? (lim & ~1) : n;
-}
-
 template <int BN, bool I8>
 int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mw, const GemmParams& p, cudaStream_t s) {
     using C = Cfg<BN>;
