@@ -275,6 +275,8 @@ int matmul_device(const Weight& w, Weight* w_mut, const void* A, int dtypeA, int
         if (rc) return rc;
         A_use = buf; lda_use = ld2;
     }
+    rc = launch_gemm_wave(w, A_use, dtypeA, M, K, lda_use, n0, n1, ep, s);
+    if (rc != B200FC_ERR_UNSUPPORTED) return rc;
     if (w.compressed) {
         // M > 16 with compressed weights.  The reference decompresses 16 weight rows at a time into a reused
         // buffer right before the tile product (kernels_amx.hpp:1443-1514); here a block of weight rows is widened to

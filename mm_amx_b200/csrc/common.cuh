@@ -158,6 +158,10 @@ int launch_mlp_decode_fused(const Weight& gate_up, const Weight& down, const voi
 // gemm_tc.cu: tcgen05 GEMM, bf16 x bf16 -> fp32 or 8-bit x 8-bit -> int32
 int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, const void* A, int dtypeA, int M, int K,
                    int64_t lda, int n0, int n1, const Epilogue& ep, cudaStream_t s);
+// gemm_wave.cu: the same layer, any weight type, for calls whose output fits one wave of tiles; B200FC_ERR_UNSUPPORTED
+// without a message = it does not, take launch_gemm_tc
+int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,
+                     cudaStream_t s);
 // gemm_tc.cu: bf16 GEMM whose output is all-reduced over a tensor-parallel group inside the kernel
 struct AllReduceDesc {
     int world, rank;

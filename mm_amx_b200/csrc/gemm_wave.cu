@@ -1,0 +1,617 @@
+// Fully-connected layer whose output fits the GPU as ONE wave of tiles: small and medium prefill calls (17 rows and more).
+//
+// Replaces the same M > 16 branches as gemm_tc.cu (include/kernels_amx.hpp:1255-1313), and those of the compressed-weight
+// specialisation (kernels_amx.hpp:1443-1514).  gemm_tc.cu's kernel is persistent over tiles of a fixed width, which pays
+// for its double-buffered accumulators once every SM has several tiles; a call with about as many tiles as SMs loses most of
+// its time to a ragged second round, to a split of K that goes through global memory, and (quantised weights) to a pass
+// that widens the weights to bf16 before anything is multiplied.  Here:
+//   - every CTA, or pair of CTAs (more than 128 rows), gets exactly one tile of 128 / 256 rows x W columns, W any multiple
+//     of 32 / 64 up to 256 / 512 (all of TMEM): the launcher picks W and the split of K so that one wave fills the SMs;
+//   - the S parts of a split K form one cluster and add their accumulators in rank order through distributed shared memory;
+//   - int8-compressed and 4-bit weights cross HBM and L2 as they are stored: eight warps widen each slab to bf16 in shared
+//     memory between the TMA load and the MMA.
+// int8 values are exact in bf16; a 4-bit value is multiplied by its group scale in fp32 and rounded to bf16.
+//
+// Warps: 0 = TMA loads of activations (and of plain weights), 1 = MMA issue (one lane) and TMEM owner, 2 = TMA loads of
+// quantised weights, 3 idle, 4-11 = widening, then epilogue (two warps per TMEM quarter).
+// Barriers of ring slot s: full[s] in the pair's leader: one arrive.expect_tx for the TMA bytes of both CTAs, plus one
+// arrival of every widening warp of both; empty[s] in each CTA, released by the leader's tcgen05.commit.
+// raw_full / raw_empty: the ring of weights as stored.  Every wait is bounded as in gemm_tc.cu.
+#include <cstdlib>
+#include "tc_common.cuh"
+
+namespace b200fc {
+
+namespace {
+
+enum WaveMode { W_BF16 = 0, W_I8 = 1, W_U8C = 2, W_U4C = 3 };   // weights: bf16, 8-bit (8-bit MMA), int8 compressed, 4-bit
+
+constexpr int WAVE_THREADS = 384;
+constexpr int WORKERS = 8;
+constexpr int MAX_SLOTS = 12, MAX_RAW = 8, MAX_W = 512;
+constexpr int WAVE_BAR_BYTES = 512;
+constexpr int COLVEC_FLOATS = 3 * MAX_W;
+constexpr int WAVE_SMEM = 232448;                                                  // all an SM gives to one CTA
+constexpr int RING_BYTES = (WAVE_SMEM - 1024 - WAVE_BAR_BYTES - COLVEC_FLOATS * 4) / 1024 * 1024;
+constexpr int CHUNK_BYTES = 32 * BM * 4;                                           // 32 columns of fp32 / int32 partial sums
+constexpr int WARP_TILE_BYTES = 4096;                                              // store_tile_4b's staging tile
+
+struct WaveParams {
+    int M, n0, n1, n_pad;
+    int R, R0;              // weight rows (= output columns) per CTA; of the first MMA of a K step
+    int tiles_m, S;
+    int slabs, units;       // K in 128-byte slabs of the MMA operands / in 128-byte pieces of the stored weight rows
+    int slots, raw_slots;
+    unsigned idesc0, idesc1;
+    int vec_ok;
+    Epilogue ep;
+    const float* scale_grp;
+    int* status;
+    unsigned long long wait_limit_ns;
+};
+
+// Arrival of a widening warp on the leader's barrier.  No cluster-scope release: the data was handed to the async proxy by a
+// proxy fence before, which is what the MMA reads through, and a release at cluster scope (a full memory barrier of the
+// warp) cost about a microsecond per slab.
+__device__ __forceinline__ void mbar_arrive_leader(unsigned cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void st_cluster_v4(unsigned cluster_addr, unsigned a, unsigned b, unsigned c, unsigned d) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ unsigned bf16x2_sub(unsigned a, unsigned b) {
+    const __nv_bfloat162 r = __hsub2(*(const __nv_bfloat162*)&a, *(const __nv_bfloat162*)&b);
+    return *(const unsigned*)&r;
+}
+// two offset-binary weights u = v + 128 (bytes selected by sel, zero-extended) -> bf16x2 of v, exactly: 0x4300 | low 7 bits
+// is 128 + low; 128 is taken off where bit 7 of u is set and 256 where it is not
+__device__ __forceinline__ unsigned u8x2_to_bf16x2(unsigned w, unsigned sel) {
+    const unsigned p = __byte_perm(w, 0u, sel);
+    unsigned a, c;
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(a) : "r"(p), "r"(0x007f007fu), "r"(0x43004300u));   // (p & m) | k
+    asm("lop3.b32 %0, %1, %2, %3, 0xae;" : "=r"(c) : "r"(p), "r"(0x00800080u), "r"(0x43004300u));   // (~p & m) | k
+    return bf16x2_sub(a, c);
+}
+// nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of (n - 8) * scale, each product rounded once from fp32
+__device__ __forceinline__ unsigned nib2_to_bf16x2(unsigned w, float scale) {
+    unsigned a;
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(a) : "r"(w), "r"(0x000f000fu), "r"(0x43004300u));   // 128 + n
+    a = bf16x2_sub(a, 0x43084308u);                                                                 // - 136, exact
+    const __nv_bfloat162 r = __floats2bfloat162_rn(__uint_as_float(a << 16) * scale, __uint_as_float(a & 0xffff0000u) * scale);
+    return *(const unsigned*)&r;
+}
+
+template <int CG, int MODE>
+__global__ void __launch_bounds__(WAVE_THREADS, 1)
+gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const WaveParams p) {
+    constexpr bool I8 = MODE == W_I8, WQ = MODE == W_U8C || MODE == W_U4C;
+    constexpr int SPU = MODE == W_U8C ? 2 : (MODE == W_U4C ? 4 : 1);   // slabs per stored 128-byte piece
+    constexpr int A_BYTES = BM * SLAB_BYTES;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + (((smem_u32(smem_raw) + 1023u) & ~1023u) - smem_u32(smem_raw));
+    const unsigned bars = smem_u32(smem + RING_BYTES);
+    const unsigned bar_full = bars, bar_empty = bars + 8 * MAX_SLOTS;
+    const unsigned bar_raw_full = bars + 16 * MAX_SLOTS, bar_raw_empty = bar_raw_full + 8 * MAX_RAW;
+    const unsigned bar_acc = bar_raw_empty + 8 * MAX_RAW;
+    unsigned* tmem_holder = (unsigned*)(smem + RING_BYTES + 16 * MAX_SLOTS + 16 * MAX_RAW + 8);
+    volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
+    float* colvec = (float*)(smem + RING_BYTES + WAVE_BAR_BYTES);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned crank = cluster_ctarank();
+    const int rank = CG == 2 ? (int)(crank & 1) : 0;        // CTA of the pair
+    const unsigned leader_rank = CG == 2 ? (crank & ~1u) : crank;
+    const int split = CG == 2 ? (int)(crank >> 1) : (int)crank;
+    const bool leader = rank == 0;
+    const int tile = (int)(blockIdx.x / (unsigned)(CG * p.S));
+    const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+    const int W = CG * p.R, nb = p.n0 + tn * W;
+    const int stage_bytes = A_BYTES + p.R * SLAB_BYTES, raw_bytes = p.R * SLAB_BYTES;
+    unsigned char* raw_ring = smem + p.slots * stage_bytes;
+    const int u0 = (int)((long long)p.units * split / p.S), u1 = (int)((long long)p.units * (split + 1) / p.S);
+    const int n_units = u1 - u0, n_slabs = min(u1 * SPU, p.slabs) - u0 * SPU;
+    const unsigned tmem_cols = W <= 32 ? 32 : (W <= 64 ? 64 : (W <= 128 ? 128 : (W <= 256 ? 256 : 512)));
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < p.slots; i++) {
+            mbar_init(bar_full + 8 * i, 1 + (WQ ? CG * WORKERS : 0));
+            mbar_init(bar_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < p.raw_slots; i++) {
+            mbar_init(bar_raw_full + 8 * i, 1);
+            mbar_init(bar_raw_empty + 8 * i, WORKERS);
+        }
+        mbar_init(bar_acc, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        if constexpr (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // the pair's barriers exist before anyone signals them
+    tc_fence_after();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const unsigned tmem_base = *tmem_holder;
+
+    if (warp == 0) {
+        // ---------------- TMA: activations, and weights that need no widening ----------------
+        const unsigned leader_full = CG == 2 ? mapa_rank(bar_full, leader_rank) : bar_full;
+        const int row_a = (tm * CG + rank) * BM, row_w = nb + rank * p.R;
+        const unsigned tx = (unsigned)(CG * (A_BYTES + (WQ ? 0 : p.R * SLAB_BYTES)));
+        const unsigned ring = smem_u32(smem);
+        auto load_a = [&](int ks, int slot) {
+            const int kx = ks * (I8 ? SLAB_BYTES : SLAB_BYTES / 2);
+            const unsigned dst = ring + (unsigned)(slot * stage_bytes);
+            if constexpr (CG == 2) tma_load_2d_pair(dst, &map_a, leader_full + 8 * slot, kx, row_a);
+            else tma_load_2d(dst, &map_a, leader_full + 8 * slot, kx, row_a);
+        };
+        auto load_w = [&](int ks, int slot) {
+            const int kx = ks * (I8 ? SLAB_BYTES : SLAB_BYTES / 2);
+            const unsigned dst = ring + (unsigned)(slot * stage_bytes) + A_BYTES;
+            if constexpr (CG == 2) tma_load_2d_pair(dst, &map_w, leader_full + 8 * slot, kx, row_w);
+            else tma_load_2d(dst, &map_w, leader_full + 8 * slot, kx, row_w);
+        };
+        // plain weights do not depend on the previous kernel of the stream: the first ring of them travels while it ends
+        const int pre = WQ ? 0 : min(p.slots, n_units);
+        for (int j = 0; j < pre; j++)
+            if (elect_one()) {
+                if (leader) mbar_expect_tx(bar_full + 8 * j, tx);
+                load_w(u0 + j, j);
+            }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        int slot = 0;
+        unsigned phase = 0;
+        bool alive = true;
+        for (int j = 0; j < n_units && alive; j++) {
+            const int ks_first = (u0 + j) * SPU;
+            for (int ks = ks_first; ks < min(ks_first + SPU, p.slabs); ks++) {
+                if (j >= pre) {
+                    alive = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * slot, phase ^ 1, abort_flag, p.wait_limit_ns));
+                    if (!alive) break;
+                }
+                if (elect_one()) {
+                    if (j >= pre) {
+                        if (leader) mbar_expect_tx(bar_full + 8 * slot, tx);
+                        if (!WQ) load_w(ks, slot);
+                    }
+                    load_a(ks, slot);
+                }
+                if (++slot == p.slots) { slot = 0; phase ^= 1; }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ---------------- MMA issue ----------------
+        if (leader) {
+            int slot = 0;
+            unsigned phase = 0;
+            const unsigned ring = smem_u32(smem);
+            for (int i = 0; i < n_slabs; i++) {
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * slot, phase, abort_flag, p.wait_limit_ns))) break;
+                tc_fence_after();
+                const unsigned sa = ring + (unsigned)(slot * stage_bytes);
+                const unsigned long long adesc = make_smem_desc(sa);
+                const unsigned long long bdesc = make_smem_desc(sa + A_BYTES);
+                const unsigned long long bdesc1 = make_smem_desc(sa + A_BYTES + p.R0 * SLAB_BYTES);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++) {
+                        const unsigned long long adv = (unsigned long long)(k * (MMA_K_BYTES >> 4));
+                        const unsigned acc = (unsigned)((i | k) != 0);
+                        if constexpr (CG == 2) tc_mma_pair<I8>(tmem_base, adesc + adv, bdesc + adv, p.idesc0, acc);
+                        else tc_mma<I8>(tmem_base, adesc + adv, bdesc + adv, p.idesc0, acc);
+                        if (CG == 2 && p.R0 < p.R) tc_mma_pair<I8>(tmem_base + 2 * p.R0, adesc + adv, bdesc1 + adv, p.idesc1, acc);
+                    }
+                    if constexpr (CG == 2) {
+                        const unsigned short mask = (unsigned short)(3u << leader_rank);
+                        tc_commit_mask(bar_empty + 8 * slot, mask);
+                        if (i == n_slabs - 1) tc_commit_mask(bar_acc, mask);
+                    } else {
+                        tc_commit(bar_empty + 8 * slot);
+                        if (i == n_slabs - 1) tc_commit(bar_acc);
+                    }
+                }
+                if (++slot == p.slots) { slot = 0; phase ^= 1; }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 2) {
+        // ---------------- TMA: quantised weights as stored ----------------
+        if (WQ) {
+            int slot = 0;
+            unsigned phase = 0;
+            for (int j = 0; j < n_units; j++) {
+                const int u = u0 + j;
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.wait_limit_ns))) break;
+                if (elect_one()) {
+                    mbar_expect_tx(bar_raw_full + 8 * slot, (unsigned)raw_bytes);
+                    tma_load_2d(smem_u32(raw_ring + slot * raw_bytes), &map_w, bar_raw_full + 8 * slot, u * SLAB_BYTES, nb + rank * p.R);
+                }
+                if (++slot == p.raw_slots) { slot = 0; phase ^= 1; }
+            }
+        }
+        __syncwarp();
+    } else if (warp >= 4) {
+        const int wi = warp - 4;
+        bool ok = true;
+        // per-column vectors of the tile (they may come from the previous kernel of the stream)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const bool plain_ep = !(p.ep.steps & B200FC_STEP_SILU_MUL) && p.ep.out_dtype != B200FC_S32;
+        const bool use_deq = plain_ep && (p.ep.steps & B200FC_STEP_DEQUANT) && p.ep.deq_per_oc;
+        const bool use_bias = plain_ep && (p.ep.steps & B200FC_STEP_BIAS) && p.ep.bias;
+        const bool use_q = plain_ep && (p.ep.steps & B200FC_STEP_QUANT) && p.ep.q_per_oc;
+        if (use_deq || use_bias || use_q)
+            for (int i = wi * 32 + lane; i < W; i += WORKERS * 32) {
+                const int col = min(nb + i, p.n1 - 1);
+                if (use_deq) colvec[i] = __ldg(p.ep.deq_per_oc + col);
+                if (use_bias) colvec[MAX_W + i] = __ldg(p.ep.bias + col);
+                if (use_q) colvec[2 * MAX_W + i] = __ldg(p.ep.q_per_oc + col);
+            }
+        if constexpr (WQ) {
+            // ---------------- widening: warp wi takes 32 K of every slab for row groups wi / 2 and wi / 2 + 4 ----------------
+            const int kh = wi & 1;
+            int n_grp = 0;
+            for (int g = wi >> 1; g * 32 < p.R; g += 4) n_grp++;
+            const unsigned leader_full = CG == 2 ? mapa_rank(bar_full, leader_rank) : bar_full;
+            // 4-bit weights: the scales of this thread's rows for the two groups of 128 K of a piece, one piece ahead
+            float sc[2][2] = {}, sc_next[2][2] = {};
+            auto load_scales = [&](int u) {
+#pragma unroll
+                for (int gi = 0; gi < 2; gi++) {
+                    const int row = min(nb + rank * p.R + ((wi >> 1) + 4 * gi) * 32 + lane, p.n_pad - 1);   // (rows past the matrix are never stored)
+                    const float* s = p.scale_grp + ((size_t)(row >> 7) * p.units + u) * 256 + (row & 127);
+                    sc_next[gi][0] = __ldg(s);
+                    sc_next[gi][1] = __ldg(s + 128);
+                }
+            };
+            if constexpr (MODE == W_U4C) load_scales(u0);
+            int slot = 0, rslot = 0;
+            unsigned phase = 0, rphase = 0;
+            for (int j = 0; j < n_units && ok; j++) {
+                const int u = u0 + j;
+                if constexpr (MODE == W_U4C) {
+#pragma unroll
+                    for (int gi = 0; gi < 2; gi++) { sc[gi][0] = sc_next[gi][0]; sc[gi][1] = sc_next[gi][1]; }
+                    if (j + 1 < n_units) load_scales(u0 + j + 1);
+                }
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_raw_full + 8 * rslot, rphase, abort_flag, p.wait_limit_ns));
+                if (!ok) break;
+                const unsigned char* raw = raw_ring + rslot * raw_bytes;
+#pragma unroll
+                for (int s = 0; s < SPU; s++) {
+                    if (u * SPU + s >= p.slabs) break;          // warp-uniform: the last piece may reach past K
+                    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * slot, phase ^ 1, abort_flag, p.wait_limit_ns));
+                    if (!ok) break;
+                    unsigned char* dst = smem + slot * stage_bytes + A_BYTES;
+#pragma unroll
+                    for (int gi = 0; gi < 2; gi++) {
+                        if (gi >= n_grp) break;
+                        const int row = ((wi >> 1) + 4 * gi) * 32 + lane, sw = row & 7;
+                        const unsigned char* src = raw + row * SLAB_BYTES;
+                        unsigned char* d = dst + row * SLAB_BYTES;
+                        if constexpr (MODE == W_U8C) {
+#pragma unroll
+                            for (int q = 0; q < 2; q++) {
+                                const uint4 v = *(const uint4*)(src + (((4 * s + 2 * kh + q) ^ sw) << 4));
+                                const uint4 lo = make_uint4(u8x2_to_bf16x2(v.x, 0x4140), u8x2_to_bf16x2(v.x, 0x4342),
+                                                            u8x2_to_bf16x2(v.y, 0x4140), u8x2_to_bf16x2(v.y, 0x4342));
+                                const uint4 hi = make_uint4(u8x2_to_bf16x2(v.z, 0x4140), u8x2_to_bf16x2(v.z, 0x4342),
+                                                            u8x2_to_bf16x2(v.w, 0x4140), u8x2_to_bf16x2(v.w, 0x4342));
+                                *(uint4*)(d + (((4 * kh + 2 * q) ^ sw) << 4)) = lo;
+                                *(uint4*)(d + (((4 * kh + 2 * q + 1) ^ sw) << 4)) = hi;
+                            }
+                        } else {
+                            // the 16-byte unit that holds K [64 s + 32 kh, +32) of the piece (see quant4_kernel in pack.cu)
+                            const uint4 v = *(const uint4*)(src + (((4 * (s & 1) + 2 * kh + (s >> 1)) ^ sw) << 4));
+                            const unsigned w4[4] = {v.x, v.y, v.z, v.w};
+                            const float f = sc[gi][s >> 1];
+#pragma unroll
+                            for (int q = 0; q < 4; q++)
+                                *(uint4*)(d + (((4 * kh + q) ^ sw) << 4)) =
+                                    make_uint4(nib2_to_bf16x2(w4[q], f), nib2_to_bf16x2(w4[q] >> 4, f),
+                                               nib2_to_bf16x2(w4[q] >> 8, f), nib2_to_bf16x2(w4[q] >> 12, f));
+                        }
+                    }
+                    // the widened bytes must be visible to the tensor core (async proxy) before the slot counts as full
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (CG == 1 || leader) mbar_arrive(bar_full + 8 * slot);
+                        else mbar_arrive_leader(leader_full + 8 * slot);
+                    }
+                    if (++slot == p.slots) { slot = 0; phase ^= 1; }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_raw_empty + 8 * rslot);
+                if (++rslot == p.raw_slots) { rslot = 0; rphase ^= 1; }
+            }
+        }
+        // ---------------- epilogue ----------------
+        asm volatile("bar.sync 1, %0;" ::"n"(WORKERS * 32) : "memory");
+        ok = __all_sync(0xffffffffu, ok && mbar_wait<32>(bar_acc, 0, abort_flag, p.wait_limit_ns));
+        tc_fence_after();
+        const int quarter = warp & 3, half = wi >> 2;
+        const int chunks = W / 32;
+        const int m = (tm * CG + rank) * BM + quarter * 32 + lane;
+        const bool row_ok = m < p.M;
+        const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16);
+        // accumulator column of a chunk -> output column: with a pair, MMA 0 holds the first R0 columns of CTA 0's R and of
+        // CTA 1's R side by side, MMA 1 the other R - R0 of both
+        auto chunk_col = [&](int c) -> int {
+            if constexpr (CG == 1) return c * 32;
+            const int h = c * 32 >= 2 * p.R0, rows = h ? p.R - p.R0 : p.R0, cc = c * 32 - (h ? 2 * p.R0 : 0);
+            const int r = cc >= rows;
+            return r * p.R + (h ? p.R0 : 0) + cc - (r ? rows : 0);
+        };
+        // every load of the ring has landed and every MMA has read it: the ring is free
+        unsigned* stage_tile = (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES);
+        auto finish_chunk = [&](const unsigned (&r)[32], int c) {
+            const int col = chunk_col(c), n = nb + col;
+            EpiArgs ea{&p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, stage_tile};
+            if (use_deq) ea.cv_deq = colvec + col;
+            if (use_bias) ea.cv_bias = colvec + MAX_W + col;
+            if (use_q) ea.cv_q = colvec + 2 * MAX_W + col;
+            epilogue_chunk(r, m, n, ea, row_ok);
+        };
+        if (p.S == 1) {
+            if (ok) {
+#pragma unroll 1
+                for (int c = half; c < chunks; c += 2) {
+                    if (nb + chunk_col(c) >= p.n1) continue;
+                    unsigned r[32];
+                    tc_ld32(taddr + (unsigned)(c * 32), r);
+                    tc_wait_ld();
+                    finish_chunk(r, c);
+                }
+            }
+        } else {
+            // Part `q` of K hands chunk c of its accumulators to CTA (c mod S) of the cluster: 16 KB at slot (c / S) * S + q of
+            // that CTA's ring, as [4-column piece][row] 16-byte units.  Remote stores are posted, so nothing waits for a
+            // round trip (reading the other CTAs' sums took 3 us per chunk); the ring has to be free in every CTA first.
+            const unsigned mine = smem_u32(smem) + (unsigned)((quarter * 32 + lane) * 16);
+            __syncwarp();
+            cluster_sync_all();
+            if (ok) {
+#pragma unroll 1
+                for (int c = half; c < chunks; c += 2) {
+                    unsigned r[32];
+                    tc_ld32(taddr + (unsigned)(c * 32), r);
+                    const int owner = c % p.S;
+                    const unsigned dst = mapa_rank(mine + (unsigned)(((c / p.S) * p.S + split) * CHUNK_BYTES), (unsigned)(owner * CG + rank));
+                    tc_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        st_cluster_v4(dst + (unsigned)(j * BM * 16), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                }
+            }
+            __syncwarp();
+            cluster_sync_all();
+            // every CTA finishes the chunks it owns, adding the parts in the order of K
+            if (ok) {
+                int turn = 0;
+#pragma unroll 1
+                for (int c = split; c < chunks; c += p.S, turn++) {
+                    if ((turn & 1) != half || nb + chunk_col(c) >= p.n1) continue;
+                    const uint4* src = (const uint4*)(smem + turn * p.S * CHUNK_BYTES) + quarter * 32 + lane;
+                    unsigned r[32];
+#pragma unroll
+                    for (int j = 0; j < 32; j++) r[j] = 0;      // (0 + x = x, and a part of -0 ends as +0 like any sum with it)
+#pragma unroll 2
+                    for (int q = 0; q < p.S; q++) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const uint4 v = src[q * (CHUNK_BYTES / 16) + j * BM];
+                            const unsigned x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                if (I8) r[4 * j + e] += x[e];
+                                else r[4 * j + e] = __float_as_uint(__uint_as_float(r[4 * j + e]) + __uint_as_float(x[e]));
+                            }
+                        }
+                    }
+                    finish_chunk(r, c);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    if (warp < 4 && p.S > 1) {
+        __syncwarp();
+        cluster_sync_all();   // (the workers' barriers around the exchange of partial sums)
+        cluster_sync_all();
+    }
+
+    // ---------------- common exit ----------------
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        if (threadIdx.x == 0) {
+            atomicExch(p.status, 2);
+            const unsigned long long t0 = globaltimer();
+            while (globaltimer() - t0 < 200000ull) { }   // copies still in flight land before shared memory is released
+        }
+        __syncthreads();
+    }
+    cluster_sync_all();   // a peer may still signal this CTA's barriers or read its partial sums until here
+    if (warp == 1) {
+        tc_fence_after();
+        if constexpr (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    }
+}
+
+// ---- host side ----------------------------------------------------------------------------------------------------------
+struct WaveShape { int cg, R, S, tiles_m, tiles_n; };
+
+// Largest number of clusters of `size` CTAs (one CTA per SM) that are resident together; asked once per device.
+template <int CG, int MODE>
+int max_clusters(int size, int* out) {
+    static std::atomic<int> cache[64][9];
+    static std::atomic<unsigned long long> attr_devices{0};
+    const int arc = once_per_device(attr_devices, [] {
+        B200FC_CUDA(cudaFuncSetAttribute(gemm_wave_kernel<CG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, WAVE_SMEM));
+        return (int)B200FC_OK;
+    });
+    if (arc) return arc;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int n = cache[dev & 63][size].load(std::memory_order_relaxed);
+    if (!n) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(size * 148), 1, 1);
+        cfg.blockDim = dim3(WAVE_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = WAVE_SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        B200FC_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_wave_kernel<CG, MODE>, &cfg));
+        if (n < 1) n = -1;
+        cache[dev & 63][size].store(n, std::memory_order_relaxed);
+    }
+    *out = n < 0 ? 0 : n;
+    return B200FC_OK;
+}
+
+template <int CG, int MODE>
+int max_tiles(int S, int* out) {
+    int n = 0;
+    const int rc = max_clusters<CG, MODE>(CG * S, &n);
+    if (rc) return rc;
+    const int by_sms = num_sms() / (CG * S);
+    *out = n < by_sms ? n : by_sms;
+    return B200FC_OK;
+}
+
+// Picks the columns per CTA and the split of K of a call that fits one wave; false = it does not.  The model counts SM
+// clocks of one CTA: per 128-byte slab the slowest of operand loads (about 48 bytes per clock and SM reach shared memory from
+// L2), MMAs (the 256-wide one takes 128 clocks per 32 bytes of K) and widening; plus the reduction and the epilogue.
+template <int CG, int MODE>
+int pick_shape(int M, int nspan, int slabs, int units, WaveShape* best, bool* found) {
+    const int tiles_m = (M + BM * CG - 1) / (BM * CG);
+    const int rows_a = M < BM ? M : BM;
+    const int wbytes = MODE == W_U4C ? 34 : (MODE == W_U8C ? 64 : 128);
+    double best_cost = 0;
+    *found = false;
+    for (int S = 1; S * CG <= 8 && S <= units; S++) {
+        int cap = 0;
+        const int rc = max_tiles<CG, MODE>(S, &cap);
+        if (rc) return rc;
+        for (int R = 32; R <= 256; R += 32) {
+            const int W = R * CG, tiles_n = (nspan + W - 1) / W;
+            if ((long long)tiles_m * tiles_n > cap) continue;
+            if (S > 1 && S * ((W / 32 + S - 1) / S) * CHUNK_BYTES + WORKERS * WARP_TILE_BYTES > RING_BYTES) continue;
+            const double load = (rows_a * 128.0 + R * (double)wbytes) / 48.0, mma = 2.0 * W;
+            const double cvt = MODE == W_U4C ? 2.2 * R : (MODE == W_U8C ? 1.4 * R : 0.0);
+            double slab = load > mma ? load : mma;
+            if (cvt > slab) slab = cvt;
+            const double hbm = (double)nspan * slabs * wbytes / 3400.0;
+            double loop = slab * ((slabs + S - 1) / S);
+            if (loop < hbm) loop = hbm;
+            const double red = S > 1 ? 1500.0 + W * 4.0 + W * 512.0 * (S - 1) / S / 30.0 : 0.0;
+            const double cost = loop + red + 400.0 * ((W / 32 + 2 * S - 1) / (2 * S));
+            if (!*found || cost < best_cost) {
+                *found = true;
+                best_cost = cost;
+                *best = WaveShape{CG, R, S, tiles_m, tiles_n};
+            }
+        }
+    }
+    return B200FC_OK;
+}
+
+template <int CG, int MODE>
+int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const float* scale_grp, const void* A, int M, int K,
+             int64_t lda, int n0, int n1, unsigned a_signed, unsigned w_signed, const Epilogue& ep, cudaStream_t s) {
+    constexpr bool I8 = MODE == W_I8, WQ = MODE == W_U8C || MODE == W_U4C;
+    constexpr int SPU = MODE == W_U8C ? 2 : (MODE == W_U4C ? 4 : 1);
+    WaveParams p = {};
+    const int slab_elems = I8 ? SLAB_BYTES : SLAB_BYTES / 2;
+    p.slabs = (K + slab_elems - 1) / slab_elems;
+    p.units = (p.slabs + SPU - 1) / SPU;
+    if (MODE == W_U4C) p.units = (int)(w_ld / SLAB_BYTES);     // (the group scales are laid out by it)
+    WaveShape sh;
+    bool found = false;
+    int rc = pick_shape<CG, MODE>(M, n1 - n0, p.slabs, p.units, &sh, &found);
+    if (rc) return rc;
+    if (!found) return B200FC_ERR_UNSUPPORTED;
+    p.M = M; p.n0 = n0; p.n1 = n1; p.n_pad = W_N_pad;
+    p.R = sh.R; p.S = sh.S; p.tiles_m = sh.tiles_m;
+    p.R0 = CG == 2 && sh.R > 128 ? (sh.R / 2 + 31) / 32 * 32 : sh.R;
+    p.idesc0 = make_idesc(I8, a_signed, w_signed, CG * p.R0, CG * BM);
+    p.idesc1 = make_idesc(I8, a_signed, w_signed, CG * (p.R - p.R0), CG * BM);
+    const int stage = BM * SLAB_BYTES + sh.R * SLAB_BYTES, raw = sh.R * SLAB_BYTES;
+    if (WQ) {
+        p.slots = 3;
+        p.raw_slots = (RING_BYTES - p.slots * stage) / raw;
+        if (p.raw_slots > 6) p.raw_slots = 6;
+        p.slots = (RING_BYTES - p.raw_slots * raw) / stage;
+    } else {
+        p.slots = RING_BYTES / stage;
+    }
+    if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
+    p.ep = ep;
+    p.scale_grp = scale_grp;
+    p.status = kernel_status_word();
+    if (!p.status) { set_error("gemm: no kernel status word on this device"); return B200FC_ERR_CUDA; }
+    p.wait_limit_ns = wait_limit_ns();
+    const int es = ep.out_dtype == B200FC_F32 || ep.out_dtype == B200FC_S32 ? 4 : (ep.out_dtype == B200FC_BF16 ? 2 : 1);
+    const bool c_aligned = ((uintptr_t)ep.C & 15) == 0 && (ep.ldc & 15) == 0;
+    p.vec_ok = c_aligned && ((ep.steps & B200FC_STEP_SILU_MUL) ? (n0 % 32) == 0 : ((n0 * es) & 15) == 0) ? 1 : 0;
+
+    CUtensorMap ma, mw;
+    rc = make_map(&ma, A, I8, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BM);
+    if (rc) return rc;
+    if (WQ) rc = make_map(&mw, W_data, true, (uint64_t)w_ld, (uint64_t)W_N_pad, (uint64_t)w_ld, (uint32_t)p.R);
+    else rc = make_map(&mw, W_data, I8, (uint64_t)W_K_pad, (uint64_t)W_N_pad, (uint64_t)w_ld, (uint32_t)p.R);
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(CG * sh.S * sh.tiles_m * sh.tiles_n), 1, 1);
+    cfg.blockDim = dim3(WAVE_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = WAVE_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)(CG * sh.S);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_wave_kernel<CG, MODE>, ma, mw, p));
+    count_launch();
+    return B200FC_OK;
+}
+
+}  // namespace
+
+int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,
+                     cudaStream_t s) {
+    if (M <= 0 || n1 <= n0) return B200FC_OK;
+    if (ep.mc_reduce || (((uintptr_t)A | (uintptr_t)lda) & 15)) return B200FC_ERR_UNSUPPORTED;
+    static int enabled = -1;                       // B200FC_GEMM_WAVE=0: never (for measurements)
+    if (enabled < 0) { const char* e = getenv("B200FC_GEMM_WAVE"); enabled = e ? atoi(e) : 1; }
+    if (!enabled) return B200FC_ERR_UNSUPPORTED;
+    const bool a8 = dtypeA != B200FC_BF16;
+    const unsigned as = dtypeA == B200FC_S8, ws = w.dtype == B200FC_S8;
+#define B200FC_WAVE(CG, MODE) run_wave<CG, MODE>(w.data, w.ld_bytes(), w.K_pad, w.N_pad, w.scale_grp, A, M, K, lda, n0, n1, as, ws, ep, s)
+    if (w.compressed) {
+        if (w.dtype == B200FC_S4) return M <= BM ? B200FC_WAVE(1, W_U4C) : B200FC_WAVE(2, W_U4C);
+        return M <= BM ? B200FC_WAVE(1, W_U8C) : B200FC_WAVE(2, W_U8C);
+    }
+    if (a8) return M <= BM ? B200FC_WAVE(1, W_I8) : B200FC_WAVE(2, W_I8);
+    return M <= BM ? B200FC_WAVE(1, W_BF16) : B200FC_WAVE(2, W_BF16);
+#undef B200FC_WAVE
+}
+
+}  // namespace b200fc

@@ -1,0 +1,75 @@
+"""GPU: the one-wave GEMM (gemm_wave.cu) at the edges of its tiles, for every weight type, against the CPU oracle.
+
+Inputs on which every partial sum is exact in fp32 (two-valued activations, integer or power-of-two weights), so the result
+must equal the oracle bit for bit whatever the tile width, the split of K and the order of summation.
+"""
+import numpy as np
+import pytest
+
+import helpers as H
+from mm_amx_b200 import capi
+from oracle import port
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (17, 64, 32),        # one slab of K, one 32-column tile
+    (33, 72, 40),        # K and N tails inside one tile
+    (17, 8192, 256),     # K split over a whole cluster
+    (128, 2080, 1000),   # the last row count of the single-CTA form; a K part that ends inside a stored piece
+    (129, 2080, 1000),   # the first one of the pair form, its second CTA nearly without rows
+    (100, 4096, 2750),   # several columns tiles, split K, ragged last tile
+    (256, 1536, 4104),   # pair form with a split of K
+    (300, 200, 9000),    # two row tiles, wide tiles whose columns come from two MMAs
+    (2048, 128, 4096),   # 512-column tiles: all of tensor memory
+    (2100, 136, 5000),   # more tiles than one wave: the persistent kernel, with widened blocks for quantised weights
+]
+
+
+def check(w, x, acc, steps, bias):
+    got = H.run_matmul(w, x, capi.F32, steps=steps)
+    assert np.array_equal(got, acc)
+    got = H.run_matmul(w, x, capi.BF16, steps=steps | capi.STEP_BIAS, bias=bias)
+    assert np.array_equal(got, port.postops(acc, port.BIAS, port.BF16, bias=bias))
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+@pytest.mark.parametrize("kind", ["bf16", "s8", "int8_compressed", "int4"])
+def test_every_weight_type_exact(kind, M, K, N):
+    rng = np.random.default_rng(M + 3 * K + 7 * N)
+    bias = rng.integers(-8, 9, N).astype(np.float32)
+    if kind == "s8":
+        x, B = rng.integers(-128, 128, (M, K), dtype=np.int8), rng.integers(-128, 128, (N, K), dtype=np.int8)
+        acc = port.gemm_i8(x, B, transposeB=True)
+        w = H.pack(B, True)
+        assert np.array_equal(H.run_matmul(w, x, capi.S32), acc)
+        q = np.float32(2.0 ** -9)
+        got = H.run_matmul(w, x, capi.S8, steps=capi.STEP_BIAS | capi.STEP_QUANT, bias=bias, q_scale=q)
+        assert np.array_equal(got, port.postops(acc, port.BIAS | port.QUANT, port.S8, bias=bias, q_scale=q))
+        return
+    x = H.two_valued_bf16(rng, (M, K))
+    if kind == "bf16":
+        B = H.two_valued_bf16(rng, (N, K))
+        check(H.pack(B, True), x, port.gemm_bf16(x, B, transposeB=True), 0, bias)
+    elif kind == "int8_compressed":
+        B = rng.integers(-128, 128, (N, K), dtype=np.int8)
+        w = H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=np.ones(N, np.float32))
+        check(w, x, port.gemm_bf16_w8(x, B, transposeB=True), capi.STEP_DEQUANT, bias)
+    else:
+        q0 = rng.integers(-7, 8, (N, K)).astype(np.float32)
+        q0[:, ::128] = 7                    # every group reaches the full range, so the scale is 2^-6 exactly
+        B = H.bf16_bits(q0 * np.float32(2.0 ** -6))
+        q, d = port.quantize_weight_int4(B)
+        check(H.pack(B, True, capi.PACK_INT4_GROUP), x, port.gemm_bf16_w4(x, q, d), capi.STEP_DEQUANT, bias)
+
+
+@pytest.mark.parametrize("M,K,N,n0,n1", [(40, 512, 900, 128, 777), (200, 512, 900, 128, 900), (200, 512, 900, 0, 129)])
+def test_column_range_leaves_the_rest_alone(M, K, N, n0, n1):
+    rng = np.random.default_rng(M + n1)
+    x = H.two_valued_bf16(rng, (M, K))
+    B = rng.integers(-128, 128, (N, K), dtype=np.int8)
+    w = H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=np.ones(N, np.float32))
+    got = H.run_matmul(w, x, capi.F32, steps=capi.STEP_DEQUANT, n0=n0, n1=n1)
+    assert np.array_equal(got[:, n0:n1], port.gemm_bf16_w8(x, B, transposeB=True)[:, n0:n1])
+    rest = np.delete(got, np.s_[n0:n1], axis=1).view(np.uint32)
+    assert (rest == 0xCDCDCDCD).all()
