@@ -188,14 +188,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int m = tm * BM + quarter * 32 + lane;
             const bool row_ok = m < p.M;
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(ab * BN);
+            const EpiArgs ea{p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, epi_tile};
+            const int kind = epilogue_kind(p.ep, p.vec_ok), n_first = p.n0 + tn * BN;
+            const int whole = kind == EPI_GENERAL ? 0 : min(BN, p.n1 - n_first) / 32;
+            for_epilogue_kind(kind, I8, [&](auto k) {
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; c++) {
-                const int n = p.n0 + tn * BN + c * 32;
-                if (n >= p.n1) break;  // warp-uniform
+                for (int c = 0; c < whole; c++) {
+                    unsigned r[32];
+                    tc_ld32(taddr + (unsigned)(c * 32), r);
+                    tc_wait_ld();
+                    epilogue_whole<decltype(k)::value>(r, m, n_first + c * 32, ea);
+                }
+            });
+#pragma unroll 1
+            for (int c = whole; c < BN / 32 && n_first + c * 32 < p.n1; c++) {   // (warp-uniform)
                 unsigned r[32];
                 tc_ld32(taddr + (unsigned)(c * 32), r);
                 tc_wait_ld();
-                epilogue_chunk(r, m, n, EpiArgs{&p.ep, p.vec_ok, p.acc_is_int, p.n1, p.M, epi_tile}, row_ok);
+                epilogue_chunk(r, m, n_first + c * 32, ea, row_ok);
             }
             tc_fence_before();
             __syncwarp();
@@ -490,18 +500,31 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const int m = tm * (2 * BM) + (int)rank * BM + quarter * 32 + lane;
             const bool row_ok = m < p.M;
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(ab * BN);
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; c++) {
-                const int n = p.n0 + tn * BN + c * 32;
-                if (n >= p.n1) break;
-                unsigned r[32];
-                tc_ld32(taddr + (unsigned)(c * 32), r);
-                tc_wait_ld();
-                EpiArgs ea{&p.ep, p.vec_ok, p.acc_is_int, p.n1, p.M, epi_tile};
+            EpiArgs ea{p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, epi_tile};
+            auto set_vecs = [&](int c) {
                 if (use_deq) ea.cv_deq = colvec + c * 32;
                 if (use_bias) ea.cv_bias = colvec + BN + c * 32;
                 if (use_q) ea.cv_q = colvec + 2 * BN + c * 32;
-                epilogue_chunk(r, m, n, ea, row_ok, c_offset);
+            };
+            const int kind = epilogue_kind(p.ep, p.vec_ok), n_first = p.n0 + tn * BN;
+            const int whole = kind == EPI_GENERAL ? 0 : min(BN, p.n1 - n_first) / 32;
+            for_epilogue_kind(kind, I8, [&](auto k) {
+#pragma unroll 1
+                for (int c = 0; c < whole; c++) {
+                    unsigned r[32];
+                    tc_ld32(taddr + (unsigned)(c * 32), r);
+                    tc_wait_ld();
+                    set_vecs(c);
+                    epilogue_whole<decltype(k)::value>(r, m, n_first + c * 32, ea, c_offset);
+                }
+            });
+#pragma unroll 1
+            for (int c = whole; c < BN / 32 && n_first + c * 32 < p.n1; c++) {   // (warp-uniform)
+                unsigned r[32];
+                tc_ld32(taddr + (unsigned)(c * 32), r);
+                tc_wait_ld();
+                set_vecs(c);
+                epilogue_chunk(r, m, n_first + c * 32, ea, row_ok, c_offset);
             }
             tc_fence_before();
             if (p.ar_world) __threadfence_system();  // this warp's part of the tile is visible to every GPU ...

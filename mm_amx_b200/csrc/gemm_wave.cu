@@ -8,15 +8,16 @@
 //   - every CTA, or pair of CTAs (more than 128 rows), gets exactly one tile of 128 / 256 rows x W columns, W any multiple
 //     of 32 / 64 up to 256 / 512 (all of TMEM): the launcher picks W and the split of K so that one wave fills the SMs;
 //   - the S parts of a split K form one cluster and add their accumulators in rank order through distributed shared memory;
-//   - int8-compressed and 4-bit weights cross HBM and L2 as they are stored: eight warps widen each slab to bf16 in shared
+//   - int8-compressed and 4-bit weights cross HBM and L2 as they are stored: twelve warps widen each slab to bf16 in shared
 //     memory between the TMA load and the MMA.
 // int8 values are exact in bf16; a 4-bit value is multiplied by its group scale in fp32 and rounded to bf16.
 //
 // Warps: 0 = TMA loads of activations (and of plain weights), 1 = MMA issue (one lane) and TMEM owner, 2 = TMA loads of
-// quantised weights, 3 idle, 4-11 = widening, then epilogue (two warps per TMEM quarter).
-// Barriers of ring slot s: full[s] in the pair's leader: one arrive.expect_tx for the TMA bytes of both CTAs, plus one
-// arrival of every widening warp of both; empty[s] in each CTA, released by the leader's tcgen05.commit.
-// raw_full / raw_empty: the ring of weights as stored.  Every wait is bounded as in gemm_tc.cu.
+// quantised weights, 3 idle, 4-15 = widening, then epilogue (three warps per TMEM quarter).
+// Rings: slots of activations and plain weights (full[s] in the pair's leader: one arrive.expect_tx for the bytes of both CTAs;
+// empty[s] in each CTA, released by the leader's tcgen05.commit); quantised weights have a ring of their own for the widened
+// slabs (wide_full: the arrivals of the widening warps of both CTAs that take the slab), so that the activations' ring can
+// be deep enough for their latency, and a third one for the pieces as stored (raw).  Every wait is bounded as in gemm_tc.cu.
 #include <cstdlib>
 #include "tc_common.cuh"
 
@@ -26,22 +27,23 @@ namespace {
 
 enum WaveMode { W_BF16 = 0, W_I8 = 1, W_U8C = 2, W_U4C = 3 };   // weights: bf16, 8-bit (8-bit MMA), int8 compressed, 4-bit
 
-constexpr int WAVE_THREADS = 384;
-constexpr int WORKERS = 8;
-constexpr int MAX_SLOTS = 12, MAX_RAW = 8, MAX_W = 512;
+constexpr int SETS = 3;                               // sets of four worker warps, one warp of a set per TMEM quarter
+constexpr int WORKERS = 4 * SETS;
+constexpr int WAVE_THREADS = 128 + 32 * WORKERS;
+constexpr int MAX_SLOTS = 12, MAX_RAW = 8, MAX_WIDE = 8, MAX_W = 512;
 constexpr int WAVE_BAR_BYTES = 512;
 constexpr int COLVEC_FLOATS = 3 * MAX_W;
 constexpr int WAVE_SMEM = 232448;                                                  // all an SM gives to one CTA
 constexpr int RING_BYTES = (WAVE_SMEM - 1024 - WAVE_BAR_BYTES - COLVEC_FLOATS * 4) / 1024 * 1024;
 constexpr int CHUNK_BYTES = 32 * BM * 4;                                           // 32 columns of fp32 / int32 partial sums
-constexpr int WARP_TILE_BYTES = 4096;                                              // store_tile_4b's staging tile
+constexpr int WARP_TILE_BYTES = 4096;                                              // staging tile of an epilogue warp
 
 struct WaveParams {
     int M, n0, n1, n_pad;
     int R, R0;              // weight rows (= output columns) per CTA; of the first MMA of a K step
     int tiles_m, S;
     int slabs, units;       // K in 128-byte slabs of the MMA operands / in 128-byte pieces of the stored weight rows
-    int slots, raw_slots;
+    int slots, raw_slots, wide_slots;
     unsigned idesc0, idesc1;
     int vec_ok;
     Epilogue ep;
@@ -92,8 +94,9 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const unsigned bars = smem_u32(smem + RING_BYTES);
     const unsigned bar_full = bars, bar_empty = bars + 8 * MAX_SLOTS;
     const unsigned bar_raw_full = bars + 16 * MAX_SLOTS, bar_raw_empty = bar_raw_full + 8 * MAX_RAW;
-    const unsigned bar_acc = bar_raw_empty + 8 * MAX_RAW;
-    unsigned* tmem_holder = (unsigned*)(smem + RING_BYTES + 16 * MAX_SLOTS + 16 * MAX_RAW + 8);
+    const unsigned bar_wide_full = bar_raw_empty + 8 * MAX_RAW, bar_wide_empty = bar_wide_full + 8 * MAX_WIDE;
+    const unsigned bar_acc = bar_wide_empty + 8 * MAX_WIDE;
+    unsigned* tmem_holder = (unsigned*)(smem + RING_BYTES + 16 * (MAX_SLOTS + MAX_RAW + MAX_WIDE) + 8);
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
     float* colvec = (float*)(smem + RING_BYTES + WAVE_BAR_BYTES);
 
@@ -106,20 +109,26 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int tile = (int)(blockIdx.x / (unsigned)(CG * p.S));
     const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
     const int W = CG * p.R, nb = p.n0 + tn * W;
-    const int stage_bytes = A_BYTES + p.R * SLAB_BYTES, raw_bytes = p.R * SLAB_BYTES;
-    unsigned char* raw_ring = smem + p.slots * stage_bytes;
+    const int w_bytes = p.R * SLAB_BYTES;                          // a slab of weights as MMA operand; a stored piece of as many rows
+    const int stage_bytes = A_BYTES + (WQ ? 0 : w_bytes);
+    unsigned char* wide_ring = smem + p.slots * stage_bytes;
+    unsigned char* raw_ring = wide_ring + p.wide_slots * w_bytes;
     const int u0 = (int)((long long)p.units * split / p.S), u1 = (int)((long long)p.units * (split + 1) / p.S);
     const int n_units = u1 - u0, n_slabs = min(u1 * SPU, p.slabs) - u0 * SPU;
     const unsigned tmem_cols = W <= 32 ? 32 : (W <= 64 ? 64 : (W <= 128 ? 128 : (W <= 256 ? 256 : 512)));
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.slots; i++) {
-            mbar_init(bar_full + 8 * i, 1 + (WQ ? CG * WORKERS : 0));
+            mbar_init(bar_full + 8 * i, 1);
             mbar_init(bar_empty + 8 * i, 1);
         }
         for (int i = 0; i < p.raw_slots; i++) {
             mbar_init(bar_raw_full + 8 * i, 1);
             mbar_init(bar_raw_empty + 8 * i, WORKERS);
+        }
+        for (int i = 0; i < p.wide_slots; i++) {
+            mbar_init(bar_wide_full + 8 * i, CG * 4);
+            mbar_init(bar_wide_empty + 8 * i, 1);
         }
         mbar_init(bar_acc, 1);
         *abort_flag = 0;
@@ -145,7 +154,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // ---------------- TMA: activations, and weights that need no widening ----------------
         const unsigned leader_full = CG == 2 ? mapa_rank(bar_full, leader_rank) : bar_full;
         const int row_a = (tm * CG + rank) * BM, row_w = nb + rank * p.R;
-        const unsigned tx = (unsigned)(CG * (A_BYTES + (WQ ? 0 : p.R * SLAB_BYTES)));
+        const unsigned tx = (unsigned)(CG * stage_bytes);
         const unsigned ring = smem_u32(smem);
         auto load_a = [&](int ks, int slot) {
             const int kx = ks * (I8 ? SLAB_BYTES : SLAB_BYTES / 2);
@@ -191,16 +200,18 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else if (warp == 1) {
         // ---------------- MMA issue ----------------
         if (leader) {
-            int slot = 0;
-            unsigned phase = 0;
-            const unsigned ring = smem_u32(smem);
+            int slot = 0, wslot = 0;
+            unsigned phase = 0, wphase = 0;
+            const unsigned ring = smem_u32(smem), wring = smem_u32(wide_ring);
             for (int i = 0; i < n_slabs; i++) {
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * slot, phase, abort_flag, p.wait_limit_ns))) break;
+                if (WQ && !__all_sync(0xffffffffu, mbar_wait(bar_wide_full + 8 * wslot, wphase, abort_flag, p.wait_limit_ns))) break;
                 tc_fence_after();
                 const unsigned sa = ring + (unsigned)(slot * stage_bytes);
+                const unsigned sb = WQ ? wring + (unsigned)(wslot * w_bytes) : sa + A_BYTES;
                 const unsigned long long adesc = make_smem_desc(sa);
-                const unsigned long long bdesc = make_smem_desc(sa + A_BYTES);
-                const unsigned long long bdesc1 = make_smem_desc(sa + A_BYTES + p.R0 * SLAB_BYTES);
+                const unsigned long long bdesc = make_smem_desc(sb);
+                const unsigned long long bdesc1 = make_smem_desc(sb + p.R0 * SLAB_BYTES);
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++) {
@@ -213,13 +224,16 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if constexpr (CG == 2) {
                         const unsigned short mask = (unsigned short)(3u << leader_rank);
                         tc_commit_mask(bar_empty + 8 * slot, mask);
+                        if (WQ) tc_commit_mask(bar_wide_empty + 8 * wslot, mask);
                         if (i == n_slabs - 1) tc_commit_mask(bar_acc, mask);
                     } else {
                         tc_commit(bar_empty + 8 * slot);
+                        if (WQ) tc_commit(bar_wide_empty + 8 * wslot);
                         if (i == n_slabs - 1) tc_commit(bar_acc);
                     }
                 }
                 if (++slot == p.slots) { slot = 0; phase ^= 1; }
+                if (WQ && ++wslot == p.wide_slots) { wslot = 0; wphase ^= 1; }
             }
         }
         __syncwarp();
@@ -232,8 +246,8 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const int u = u0 + j;
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.wait_limit_ns))) break;
                 if (elect_one()) {
-                    mbar_expect_tx(bar_raw_full + 8 * slot, (unsigned)raw_bytes);
-                    tma_load_2d(smem_u32(raw_ring + slot * raw_bytes), &map_w, bar_raw_full + 8 * slot, u * SLAB_BYTES, nb + rank * p.R);
+                    mbar_expect_tx(bar_raw_full + 8 * slot, (unsigned)w_bytes);
+                    tma_load_2d(smem_u32(raw_ring + slot * w_bytes), &map_w, bar_raw_full + 8 * slot, u * SLAB_BYTES, nb + rank * p.R);
                 }
                 if (++slot == p.raw_slots) { slot = 0; phase ^= 1; }
             }
@@ -256,78 +270,93 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (use_q) colvec[2 * MAX_W + i] = __ldg(p.ep.q_per_oc + col);
             }
         if constexpr (WQ) {
-            // ---------------- widening: warp wi takes 32 K of every slab for row groups wi / 2 and wi / 2 + 4 ----------------
-            const int kh = wi & 1;
-            int n_grp = 0;
-            for (int g = wi >> 1; g * 32 < p.R; g += 4) n_grp++;
-            const unsigned leader_full = CG == 2 ? mapa_rank(bar_full, leader_rank) : bar_full;
+            // ---------------- widening ----------------
+            // The sets of four warps take the slabs in turn, so that a warp's waits, its proxy fence and its arrival (about
+            // a thousand clocks, mostly latency) come once per SETS slabs.  Inside a slab a warp takes every fourth item; an
+            // item is 32 rows (one per lane) x 32 K, read before the slot is waited for.
+            const int set = wi >> 2, w_in_set = wi & 3, n_items = p.R / 16;
+            const unsigned leader_full = CG == 2 ? mapa_rank(bar_wide_full, leader_rank) : bar_wide_full;
             // 4-bit weights: the scales of this thread's rows for the two groups of 128 K of a piece, one piece ahead
-            float sc[2][2] = {}, sc_next[2][2] = {};
+            float sc[4][2] = {}, sc_next[4][2] = {};
             auto load_scales = [&](int u) {
 #pragma unroll
-                for (int gi = 0; gi < 2; gi++) {
-                    const int row = min(nb + rank * p.R + ((wi >> 1) + 4 * gi) * 32 + lane, p.n_pad - 1);   // (rows past the matrix are never stored)
+                for (int e = 0; e < 4; e++) {
+                    const int row = min(nb + rank * p.R + ((w_in_set + 4 * e) >> 1) * 32 + lane, p.n_pad - 1);   // (rows past the matrix are never stored)
                     const float* s = p.scale_grp + ((size_t)(row >> 7) * p.units + u) * 256 + (row & 127);
-                    sc_next[gi][0] = __ldg(s);
-                    sc_next[gi][1] = __ldg(s + 128);
+                    sc_next[e][0] = __ldg(s);
+                    sc_next[e][1] = __ldg(s + 128);
                 }
             };
             if constexpr (MODE == W_U4C) load_scales(u0);
-            int slot = 0, rslot = 0;
+            int slot = 0, rslot = 0, turn = 0;
             unsigned phase = 0, rphase = 0;
             for (int j = 0; j < n_units && ok; j++) {
                 const int u = u0 + j;
                 if constexpr (MODE == W_U4C) {
 #pragma unroll
-                    for (int gi = 0; gi < 2; gi++) { sc[gi][0] = sc_next[gi][0]; sc[gi][1] = sc_next[gi][1]; }
+                    for (int e = 0; e < 4; e++) { sc[e][0] = sc_next[e][0]; sc[e][1] = sc_next[e][1]; }
                     if (j + 1 < n_units) load_scales(u0 + j + 1);
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(bar_raw_full + 8 * rslot, rphase, abort_flag, p.wait_limit_ns));
                 if (!ok) break;
-                const unsigned char* raw = raw_ring + rslot * raw_bytes;
-#pragma unroll
+                const unsigned char* raw = raw_ring + rslot * w_bytes;
+                // (not unrolled: the warps are at different places of this code, and four copies of it outgrow the
+                // instruction cache)
+#pragma unroll 1
                 for (int s = 0; s < SPU; s++) {
                     if (u * SPU + s >= p.slabs) break;          // warp-uniform: the last piece may reach past K
-                    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * slot, phase ^ 1, abort_flag, p.wait_limit_ns));
-                    if (!ok) break;
-                    unsigned char* dst = smem + slot * stage_bytes + A_BYTES;
+                    if (turn == set) {
+                        constexpr int UNITS = MODE == W_U8C ? 2 : 1;     // 16-byte units of an item's row
+                        uint4 v[4][UNITS];
 #pragma unroll
-                    for (int gi = 0; gi < 2; gi++) {
-                        if (gi >= n_grp) break;
-                        const int row = ((wi >> 1) + 4 * gi) * 32 + lane, sw = row & 7;
-                        const unsigned char* src = raw + row * SLAB_BYTES;
-                        unsigned char* d = dst + row * SLAB_BYTES;
-                        if constexpr (MODE == W_U8C) {
+                        for (int e = 0; e < 4; e++) {
+                            const int item = w_in_set + 4 * e, row = (item >> 1) * 32 + lane, kh = item & 1;
+                            if (item >= n_items) break;
+                            // 4 bits: the unit that holds K [64 s + 32 kh, +32) of the piece (see quant4_kernel in pack.cu)
 #pragma unroll
-                            for (int q = 0; q < 2; q++) {
-                                const uint4 v = *(const uint4*)(src + (((4 * s + 2 * kh + q) ^ sw) << 4));
-                                const uint4 lo = make_uint4(u8x2_to_bf16x2(v.x, 0x4140), u8x2_to_bf16x2(v.x, 0x4342),
-                                                            u8x2_to_bf16x2(v.y, 0x4140), u8x2_to_bf16x2(v.y, 0x4342));
-                                const uint4 hi = make_uint4(u8x2_to_bf16x2(v.z, 0x4140), u8x2_to_bf16x2(v.z, 0x4342),
-                                                            u8x2_to_bf16x2(v.w, 0x4140), u8x2_to_bf16x2(v.w, 0x4342));
-                                *(uint4*)(d + (((4 * kh + 2 * q) ^ sw) << 4)) = lo;
-                                *(uint4*)(d + (((4 * kh + 2 * q + 1) ^ sw) << 4)) = hi;
+                            for (int q = 0; q < UNITS; q++)
+                                v[e][q] = *(const uint4*)(raw + row * SLAB_BYTES +
+                                                          (((MODE == W_U8C ? 4 * s + 2 * kh + q : 4 * (s & 1) + 2 * kh + (s >> 1)) ^ (row & 7)) << 4));
+                        }
+                        ok = __all_sync(0xffffffffu, mbar_wait(bar_wide_empty + 8 * slot, phase ^ 1, abort_flag, p.wait_limit_ns));
+                        if (!ok) break;
+                        unsigned char* dst = wide_ring + slot * w_bytes;
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int item = w_in_set + 4 * e, row = (item >> 1) * 32 + lane, kh = item & 1, sw = row & 7;
+                            if (item >= n_items) break;
+                            unsigned char* d = dst + row * SLAB_BYTES;
+                            if constexpr (MODE == W_U8C) {
+#pragma unroll
+                                for (int q = 0; q < 2; q++) {
+                                    const uint4 b = v[e][q];
+                                    *(uint4*)(d + (((4 * kh + 2 * q) ^ sw) << 4)) =
+                                        make_uint4(u8x2_to_bf16x2(b.x, 0x4140), u8x2_to_bf16x2(b.x, 0x4342),
+                                                   u8x2_to_bf16x2(b.y, 0x4140), u8x2_to_bf16x2(b.y, 0x4342));
+                                    *(uint4*)(d + (((4 * kh + 2 * q + 1) ^ sw) << 4)) =
+                                        make_uint4(u8x2_to_bf16x2(b.z, 0x4140), u8x2_to_bf16x2(b.z, 0x4342),
+                                                   u8x2_to_bf16x2(b.w, 0x4140), u8x2_to_bf16x2(b.w, 0x4342));
+                                }
+                            } else {
+                                const unsigned w4[4] = {v[e][0].x, v[e][0].y, v[e][0].z, v[e][0].w};
+                                const float f = s < 2 ? sc[e][0] : sc[e][1];
+#pragma unroll
+                                for (int q = 0; q < 4; q++)
+                                    *(uint4*)(d + (((4 * kh + q) ^ sw) << 4)) =
+                                        make_uint4(nib2_to_bf16x2(w4[q], f), nib2_to_bf16x2(w4[q] >> 4, f),
+                                                   nib2_to_bf16x2(w4[q] >> 8, f), nib2_to_bf16x2(w4[q] >> 12, f));
                             }
-                        } else {
-                            // the 16-byte unit that holds K [64 s + 32 kh, +32) of the piece (see quant4_kernel in pack.cu)
-                            const uint4 v = *(const uint4*)(src + (((4 * (s & 1) + 2 * kh + (s >> 1)) ^ sw) << 4));
-                            const unsigned w4[4] = {v.x, v.y, v.z, v.w};
-                            const float f = sc[gi][s >> 1];
-#pragma unroll
-                            for (int q = 0; q < 4; q++)
-                                *(uint4*)(d + (((4 * kh + q) ^ sw) << 4)) =
-                                    make_uint4(nib2_to_bf16x2(w4[q], f), nib2_to_bf16x2(w4[q] >> 4, f),
-                                               nib2_to_bf16x2(w4[q] >> 8, f), nib2_to_bf16x2(w4[q] >> 12, f));
+                        }
+                        // the widened bytes must be visible to the tensor core (async proxy) before the slot counts as full
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (CG == 1 || leader) mbar_arrive(bar_wide_full + 8 * slot);
+                            else mbar_arrive_leader(leader_full + 8 * slot);
                         }
                     }
-                    // the widened bytes must be visible to the tensor core (async proxy) before the slot counts as full
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (CG == 1 || leader) mbar_arrive(bar_full + 8 * slot);
-                        else mbar_arrive_leader(leader_full + 8 * slot);
-                    }
-                    if (++slot == p.slots) { slot = 0; phase ^= 1; }
+                    if (++turn == SETS) turn = 0;
+                    if (++slot == p.wide_slots) { slot = 0; phase ^= 1; }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_raw_empty + 8 * rslot);
@@ -338,7 +367,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         asm volatile("bar.sync 1, %0;" ::"n"(WORKERS * 32) : "memory");
         ok = __all_sync(0xffffffffu, ok && mbar_wait<32>(bar_acc, 0, abort_flag, p.wait_limit_ns));
         tc_fence_after();
-        const int quarter = warp & 3, half = wi >> 2;
+        const int quarter = warp & 3, third = wi >> 2;
         const int chunks = W / 32;
         const int m = (tm * CG + rank) * BM + quarter * 32 + lane;
         const bool row_ok = m < p.M;
@@ -353,26 +382,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         };
         // every load of the ring has landed and every MMA has read it: the ring is free
         unsigned* stage_tile = (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES);
-        auto finish_chunk = [&](const unsigned (&r)[32], int c) {
-            const int col = chunk_col(c), n = nb + col;
-            EpiArgs ea{&p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, stage_tile};
-            if (use_deq) ea.cv_deq = colvec + col;
-            if (use_bias) ea.cv_bias = colvec + MAX_W + col;
-            if (use_q) ea.cv_q = colvec + 2 * MAX_W + col;
-            epilogue_chunk(r, m, n, ea, row_ok);
-        };
-        if (p.S == 1) {
-            if (ok) {
-#pragma unroll 1
-                for (int c = half; c < chunks; c += 2) {
-                    if (nb + chunk_col(c) >= p.n1) continue;
-                    unsigned r[32];
-                    tc_ld32(taddr + (unsigned)(c * 32), r);
-                    tc_wait_ld();
-                    finish_chunk(r, c);
-                }
-            }
-        } else {
+        if (p.S > 1) {
             // Part `q` of K hands chunk c of its accumulators to CTA (c mod S) of the cluster: 16 KB at slot (c / S) * S + q of
             // that CTA's ring, as [4-column piece][row] 16-byte units.  Remote stores are posted, so nothing waits for a
             // round trip (reading the other CTAs' sums took 3 us per chunk); the ring has to be free in every CTA first.
@@ -381,7 +391,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             cluster_sync_all();
             if (ok) {
 #pragma unroll 1
-                for (int c = half; c < chunks; c += 2) {
+                for (int c = third; c < chunks; c += SETS) {
                     unsigned r[32];
                     tc_ld32(taddr + (unsigned)(c * 32), r);
                     const int owner = c % p.S;
@@ -394,34 +404,62 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             }
             __syncwarp();
             cluster_sync_all();
-            // every CTA finishes the chunks it owns, adding the parts in the order of K
-            if (ok) {
-                int turn = 0;
-#pragma unroll 1
-                for (int c = split; c < chunks; c += p.S, turn++) {
-                    if ((turn & 1) != half || nb + chunk_col(c) >= p.n1) continue;
-                    const uint4* src = (const uint4*)(smem + turn * p.S * CHUNK_BYTES) + quarter * 32 + lane;
-                    unsigned r[32];
+        }
+        // accumulators of the t-th chunk this CTA finishes: its own, or the sum of the parts in the order of K
+        auto fetch = [&](int t, int c, unsigned (&r)[32]) {
+            if (p.S == 1) {
+                tc_ld32(taddr + (unsigned)(c * 32), r);
+                tc_wait_ld();
+                return;
+            }
+            const uint4* src = (const uint4*)(smem + t * p.S * CHUNK_BYTES) + quarter * 32 + lane;
 #pragma unroll
-                    for (int j = 0; j < 32; j++) r[j] = 0;      // (0 + x = x, and a part of -0 ends as +0 like any sum with it)
+            for (int j = 0; j < 32; j++) r[j] = 0;      // (0 + x = x, and a part of -0 ends as +0 like any sum with it)
 #pragma unroll 2
-                    for (int q = 0; q < p.S; q++) {
+            for (int q = 0; q < p.S; q++) {
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            const uint4 v = src[q * (CHUNK_BYTES / 16) + j * BM];
-                            const unsigned x[4] = {v.x, v.y, v.z, v.w};
+                for (int j = 0; j < 8; j++) {
+                    const uint4 v = src[q * (CHUNK_BYTES / 16) + j * BM];
+                    const unsigned x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                if (I8) r[4 * j + e] += x[e];
-                                else r[4 * j + e] = __float_as_uint(__uint_as_float(r[4 * j + e]) + __uint_as_float(x[e]));
-                            }
-                        }
+                    for (int e = 0; e < 4; e++) {
+                        if (I8) r[4 * j + e] += x[e];
+                        else r[4 * j + e] = __float_as_uint(__uint_as_float(r[4 * j + e]) + __uint_as_float(x[e]));
                     }
-                    finish_chunk(r, c);
                 }
             }
-            __syncwarp();
+        };
+        // every load of the ring has landed and every MMA has read it: the staging tiles lie at its end
+        EpiArgs ea{p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES)};
+        auto set_vecs = [&](int col) {
+            if (use_deq) ea.cv_deq = colvec + col;
+            if (use_bias) ea.cv_bias = colvec + MAX_W + col;
+            if (use_q) ea.cv_q = colvec + 2 * MAX_W + col;
+        };
+        const int kind = epilogue_kind(p.ep, p.vec_ok);
+        if (ok) {
+            for_epilogue_kind(kind, I8, [&](auto k) {
+#pragma unroll 1
+                for (int t = third, c = split + third * p.S; c < chunks; t += SETS, c += SETS * p.S) {
+                    const int col = chunk_col(c);
+                    if (nb + col + 32 > p.n1) continue;      // (warp-uniform)
+                    unsigned r[32];
+                    fetch(t, c, r);
+                    set_vecs(col);
+                    epilogue_whole<decltype(k)::value>(r, m, nb + col, ea);
+                }
+            });
+#pragma unroll 1
+            for (int t = third, c = split + third * p.S; c < chunks; t += SETS, c += SETS * p.S) {
+                const int col = chunk_col(c);
+                if (nb + col >= p.n1 || (kind != EPI_GENERAL && nb + col + 32 <= p.n1)) continue;
+                unsigned r[32];
+                fetch(t, c, r);
+                set_vecs(col);
+                epilogue_chunk(r, m, nb + col, ea, row_ok);
+            }
         }
+        __syncwarp();
     }
     if (warp < 4 && p.S > 1) {
         __syncwarp();
@@ -550,14 +588,17 @@ int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const f
     p.R0 = CG == 2 && sh.R > 128 ? (sh.R / 2 + 31) / 32 * 32 : sh.R;
     p.idesc0 = make_idesc(I8, a_signed, w_signed, CG * p.R0, CG * BM);
     p.idesc1 = make_idesc(I8, a_signed, w_signed, CG * (p.R - p.R0), CG * BM);
-    const int stage = BM * SLAB_BYTES + sh.R * SLAB_BYTES, raw = sh.R * SLAB_BYTES;
+    const int a_bytes = BM * SLAB_BYTES, w_bytes = sh.R * SLAB_BYTES;
     if (WQ) {
-        p.slots = 3;
-        p.raw_slots = (RING_BYTES - p.slots * stage) / raw;
-        if (p.raw_slots > 6) p.raw_slots = 6;
-        p.slots = (RING_BYTES - p.raw_slots * raw) / stage;
+        // three widened slabs (more measured no faster); stored pieces for six slabs and more ahead (HBM latency); the rest
+        // for activations
+        p.wide_slots = 3;
+        p.slots = sh.R <= 192 ? 4 : 3;
+        p.raw_slots = (RING_BYTES - p.wide_slots * w_bytes - p.slots * a_bytes) / w_bytes;
+        if (p.raw_slots > (SPU == 4 ? 3 : 5)) p.raw_slots = SPU == 4 ? 3 : 5;
+        p.slots = (RING_BYTES - (p.wide_slots + p.raw_slots) * w_bytes) / a_bytes;
     } else {
-        p.slots = RING_BYTES / stage;
+        p.slots = RING_BYTES / (a_bytes + w_bytes);
     }
     if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
     p.ep = ep;

@@ -17,8 +17,8 @@ constexpr int MMA_K_BYTES = 32;          // K extent of one tcgen05.mma (16 bf16
 #endif
 constexpr int EPI_SLEEP_NS = B200FC_EPI_SLEEP_NS;
 
-// staging tiles of the four epilogue warps: 32 rows x 32 four-byte columns each, rows padded to 33 words
-constexpr int EPI_TILE_WORDS = 32 * 33;
+// staging tile of an epilogue warp: 32 rows x 32 four-byte columns
+constexpr int EPI_TILE_WORDS = 32 * 32;
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -136,7 +136,7 @@ __device__ __forceinline__ unsigned long long make_smem_desc(unsigned smem_addr)
 
 // ---- epilogue on 32 consecutive columns of one output row ------------------------------------------------------------
 struct EpiArgs {       // what the epilogue of one 32-column chunk needs to know
-    const Epilogue* ep;
+    Epilogue ep;       // (by value: the fields then live in registers)
     int vec_ok, acc_is_int, n1;
     int M;             // rows of the output
     unsigned* tile;    // this warp's staging tile in shared memory (EPI_TILE_WORDS words)
@@ -146,61 +146,25 @@ struct EpiArgs {       // what the epilogue of one 32-column chunk needs to know
     const float* cv_bias = nullptr;
     const float* cv_q = nullptr;
 };
-// 32 rows x 32 four-byte values, one row per lane in registers -> global memory with full-line stores: the tile goes
-// through shared memory and comes back with eight lanes per row (16 bytes each), so that one store instruction writes
-// four whole 128-byte row segments instead of 32 scattered 16-byte pieces.  Both passes use 16-byte accesses: row r
-// keeps its 16-byte piece j at position j ^ (r & 7), which makes the eight lanes of every shared-memory wavefront hit
-// eight different bank groups on the way in (lanes = rows) and on the way out (lanes = pieces of one row).
-// Called by all lanes of the warp; `tile` is 16-byte aligned.
-__device__ __forceinline__ void store_tile_4b(const unsigned (&val)[32], unsigned* tile, char* C, long long ldc, int m, int n,
-                                              int M) {
-    const int lane = threadIdx.x & 31, m0 = m - lane;
-    uint4* t4 = (uint4*)tile;
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-        t4[lane * 8 + (j ^ (lane & 7))] = make_uint4(val[4 * j], val[4 * j + 1], val[4 * j + 2], val[4 * j + 3]);
-    __syncwarp();
-    const int piece = lane & 7;
-#pragma unroll
-    for (int it = 0; it < 8; it++) {
-        const int rr = it * 4 + (lane >> 3);
-        const uint4 q = t4[rr * 8 + (piece ^ (rr & 7))];
-        if (m0 + rr < M) *(uint4*)(C + (long long)(m0 + rr) * ldc + (long long)(n + piece * 4) * 4) = q;
-    }
-    __syncwarp();
+// Output rows leave through shared memory: the lanes of a warp hold one row each, and their direct stores would write 32
+// scattered pieces of 16 bytes.  A warp's staging tile keeps UNITS 16-byte units per row (8: 32 four-byte values; 4: 32 bf16;
+// 2: 32 int8 or 16 bf16); unit j of row r sits at position j ^ swizzle(r), so that neither pass has bank conflicts.
+template <int UNITS>
+__device__ __forceinline__ int tile_pos(int row, int unit) {
+    return row * UNITS + (unit ^ (UNITS == 8 ? (row & 7) : (UNITS == 4 ? ((row >> 1) & 3) : ((row >> 2) & 1))));
 }
-// The same for rows of 64 bytes (32 bf16; val[j] = 4-byte words of the lane's row) and of 32 bytes (32 int8, or 16 bf16):
-// one store instruction writes 8 / 16 whole row segments, where direct stores wrote 32 half sectors.  `c0` = the row
-// segment's byte offset inside an output row.  Piece j of row r sits at j ^ ((r >> 1) & 3) / j ^ ((r >> 2) & 1): no conflicts.
-__device__ __forceinline__ void store_tile_64(const unsigned (&val)[16], unsigned* tile, char* C, long long ldc, int m, long long c0, int M) {
-    const int lane = threadIdx.x & 31, m0 = m - lane;
-    uint4* t4 = (uint4*)tile;
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-        t4[lane * 4 + (j ^ ((lane >> 1) & 3))] = make_uint4(val[4 * j], val[4 * j + 1], val[4 * j + 2], val[4 * j + 3]);
+// the tile -> rows [m0, m0 + 32) of C, byte columns [c0, c0 + 16 UNITS): every store instruction writes whole row segments
+template <int UNITS>
+__device__ __forceinline__ void flush_tile(const unsigned* tile, char* C, long long ldc, int m0, long long c0, int M) {
+    constexpr int ROWS = 32 / UNITS;                 // rows per store instruction
+    const int lane = threadIdx.x & 31, unit = lane % UNITS;
     __syncwarp();
-    const int piece = lane & 3;
+    char* dst = C + (long long)(m0 + lane / UNITS) * ldc + c0 + unit * 16;
 #pragma unroll
-    for (int it = 0; it < 4; it++) {
-        const int rr = it * 8 + (lane >> 2);
-        const uint4 q = t4[rr * 4 + (piece ^ ((rr >> 1) & 3))];
-        if (m0 + rr < M) *(uint4*)(C + (long long)(m0 + rr) * ldc + c0 + piece * 16) = q;
-    }
-    __syncwarp();
-}
-__device__ __forceinline__ void store_tile_32(const unsigned (&val)[8], unsigned* tile, char* C, long long ldc, int m, long long c0, int M) {
-    const int lane = threadIdx.x & 31, m0 = m - lane;
-    uint4* t4 = (uint4*)tile;
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-        t4[lane * 2 + (j ^ ((lane >> 2) & 1))] = make_uint4(val[4 * j], val[4 * j + 1], val[4 * j + 2], val[4 * j + 3]);
-    __syncwarp();
-    const int piece = lane & 1;
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const int rr = it * 16 + (lane >> 1);
-        const uint4 q = t4[rr * 2 + (piece ^ ((rr >> 2) & 1))];
-        if (m0 + rr < M) *(uint4*)(C + (long long)(m0 + rr) * ldc + c0 + piece * 16) = q;
+    for (int it = 0; it < UNITS; it++) {
+        const int row = it * ROWS + lane / UNITS;
+        const uint4 q = ((const uint4*)tile)[tile_pos<UNITS>(row, unit)];
+        if (m0 + row < M) *(uint4*)(dst + (long long)(it * ROWS) * ldc) = q;
     }
     __syncwarp();
 }
@@ -227,29 +191,40 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// gelu_erf_poly (common.cuh) on two values: the same operations in the same order, the polynomial two values at a time
-__device__ __forceinline__ f32x2 gelu_erf_poly2(f32x2 v) {
+// gelu_erf_poly (common.cuh) on eight values: the same operations in the same order for each, four chains of pairs side by side
+__device__ __forceinline__ void gelu_erf_poly8(f32x2 (&v)[4]) {
     constexpr unsigned coef[15] = {0x1f1c83fdu, 0xa3198977u, 0x268a7927u, 0xa998c963u, 0x2c67ddb2u, 0xaf013b2cu, 0x315d4a4fu,
                                    0xb3969b11u, 0x35a776e9u, 0xb79b0914u, 0x3970b255u, 0xbb1b7399u, 0x3ca3621fu, 0xbe082bc7u,
                                    0x3f4c4228u};
-    const f32x2 x2 = mul2(v, v), xh = mul2(v, pack2(0.5f, 0.5f));
-    f32x2 q = pack2(__uint_as_float(coef[0]), __uint_as_float(coef[0]));
+    f32x2 x2[4], q[4];
 #pragma unroll
-    for (int i = 1; i < 15; i++) q = fma2(q, x2, pack2(__uint_as_float(coef[i]), __uint_as_float(coef[i])));
-    q = mul2(fma2(q, v, pack2(1.0f, 1.0f)), xh);
-    float x[2], h[2], y[2];
-    unpack2(v, x[0], x[1]);
-    unpack2(xh, h[0], h[1]);
-    unpack2(q, y[0], y[1]);
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-        float far;      // x < -5 -> 0, x > 5 -> x, NaN -> NaN
-        asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(far) : "f"(x[e]));
-        const float ax = fabsf(x[e]);
-        if (!(ax <= 5.0f)) y[e] = far;
-        if (ax <= __uint_as_float(0x33800000u)) y[e] = h[e];
+    for (int j = 0; j < 4; j++) {
+        x2[j] = mul2(v[j], v[j]);
+        q[j] = pack2(__uint_as_float(coef[0]), __uint_as_float(coef[0]));
     }
-    return pack2(y[0], y[1]);
+#pragma unroll
+    for (int i = 1; i < 15; i++) {
+        const f32x2 c = pack2(__uint_as_float(coef[i]), __uint_as_float(coef[i]));
+#pragma unroll
+        for (int j = 0; j < 4; j++) q[j] = fma2(q[j], x2[j], c);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const f32x2 xh = mul2(v[j], pack2(0.5f, 0.5f));
+        float x[2], h[2], y[2];
+        unpack2(v[j], x[0], x[1]);
+        unpack2(xh, h[0], h[1]);
+        unpack2(mul2(fma2(q[j], v[j], pack2(1.0f, 1.0f)), xh), y[0], y[1]);
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            float far;      // x < -5 -> 0, x > 5 -> x, NaN -> NaN
+            asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(far) : "f"(x[e]));
+            const float ax = fabsf(x[e]);
+            if (!(ax <= 5.0f)) y[e] = far;
+            if (ax <= __uint_as_float(0x33800000u)) y[e] = h[e];
+        }
+        v[j] = pack2(y[0], y[1]);
+    }
 }
 // four fp32 -> four int8, as f32_to_s8 (round to nearest even, saturate, NaN -> -128) but off the conversion unit, whose 16
 // values per clock and SM bound an int8 epilogue: clamp, then the rounding of adding 1.5 * 2^23 leaves the integer in the
@@ -260,200 +235,290 @@ __device__ __forceinline__ unsigned f32x4_to_s8x4(float a, float b, float c, flo
     const unsigned uc = __float_as_uint(fminf(fmaxf(c, -128.0f), 127.0f) + magic), ud = __float_as_uint(fminf(fmaxf(d, -128.0f), 127.0f) + magic);
     return __byte_perm(__byte_perm(ua, ub, 0x0040), __byte_perm(uc, ud, 0x0040), 0x5410);
 }
-// the 32 per-column values vec[n .. n + 32) of a chunk (every lane needs all of them): eight 16-byte loads when the
-// chunk is whole and the vector 16-byte aligned, else 32 scalar loads clamped to the last valid column
-__device__ __forceinline__ void load_col_vec(const float* __restrict__ vec, int n, int n1, float (&out)[32]) {
-    if (n + 32 <= n1 && (((uintptr_t)(vec + n)) & 15) == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float4 t = __ldg((const float4*)(vec + n) + j);
-            out[4 * j] = t.x; out[4 * j + 1] = t.y; out[4 * j + 2] = t.z; out[4 * j + 3] = t.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; j++) out[j] = __ldg(vec + min(n + j, n1 - 1));
-    }
-}
-// the same 32 values from the warp's staged copy (every lane reads the same addresses: broadcasts)
-__device__ __forceinline__ void load_col_vec(const float* staged, const float* __restrict__ vec, int n, int n1, float (&out)[32]) {
+// the per-column values vec[n .. n + 8) (every lane needs all of them): from the copy staged for the chunk, as two 16-byte loads
+// where they are whole and aligned, else as scalar loads clamped to the last valid column
+__device__ __forceinline__ void load_col_vec(const float* staged, const float* __restrict__ vec, int n, int n1, f32x2 (&out)[4]) {
+    float4 t[2];
     if (staged) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float4 t = ((const float4*)staged)[j];
-            out[4 * j] = t.x; out[4 * j + 1] = t.y; out[4 * j + 2] = t.z; out[4 * j + 3] = t.w;
-        }
+        t[0] = ((const float4*)staged)[0];
+        t[1] = ((const float4*)staged)[1];
+    } else if (n + 8 <= n1 && (((uintptr_t)(vec + n)) & 15) == 0) {
+        t[0] = __ldg((const float4*)(vec + n));
+        t[1] = __ldg((const float4*)(vec + n) + 1);
     } else {
-        load_col_vec(vec, n, n1, out);
+        float* f = (float*)t;
+#pragma unroll
+        for (int j = 0; j < 8; j++) f[j] = __ldg(vec + min(n + j, n1 - 1));
     }
+#pragma unroll
+    for (int h = 0; h < 2; h++) { out[2 * h] = pack2(t[h].x, t[h].y); out[2 * h + 1] = pack2(t[h].z, t[h].w); }
 }
-__device__ __forceinline__ void epilogue_chunk(const unsigned (&r)[32], int m, int n, const EpiArgs p, bool row_ok,
-                                               long long c_offset = 0) {
-    const Epilogue& ep = *p.ep;
+__device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *(const unsigned*)&h;
+}
+// Post-ops and store of 32 consecutive columns [n, n + 32) of one output row per lane, whose accumulators are in `acc`.  Called by
+// all lanes of the warp.  This is the form for everything: chunks at the ragged end, unaligned outputs, residuals, multicast.
+__device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m, int n, const EpiArgs& p, bool row_ok, long long c_offset = 0) {
+    const Epilogue& ep = p.ep;
     const bool staged = p.vec_ok && n + 32 <= p.n1 && !ep.mc_reduce;   // warp-uniform
+    const int lane = threadIdx.x & 31, m0 = m - lane;
     char* Cb = (char*)ep.C + c_offset;
-    if (ep.out_dtype == B200FC_S32 && staged) {
-        store_tile_4b(r, p.tile, Cb, ep.ldc, m, n, p.M);
-        return;
-    }
-    if (!row_ok && !staged) return;   // (rows beyond M take part in the staged stores' shuffle through shared memory)
-    char* crow = (char*)ep.C + c_offset + (long long)m * ep.ldc;
-    if (ep.out_dtype == B200FC_S32) {  // raw accumulators
-        for (int j = 0; j < 32; j++)
-            if (n + j < p.n1) ((int*)crow)[n + j] = (int)r[j];
-        return;
-    }
-    float v[32];
-#pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = p.acc_is_int ? (float)(int)r[j] : __uint_as_float(r[j]);
-
-    if (ep.mc_reduce) {
-        // Fused all-reduce: C is a multicast mapping of the output on every GPU of the tensor-parallel group; the
-        // NVSwitch adds this rank's contribution into all replicas (multimem.red), so no separate collective runs.
-        const bool full = p.vec_ok && n + 32 <= p.n1;
-        if (ep.out_dtype == B200FC_F32) {
-            float* dst = (float*)(crow + (long long)n * 4);
-            if (full) {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    asm volatile("multimem.red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
-                                 "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
-                                 : "memory");
-            } else {
-                for (int j = 0; j < 32; j++)
-                    if (n + j < p.n1) asm volatile("multimem.red.relaxed.sys.global.add.f32 [%0], %1;" ::"l"(dst + j), "f"(v[j]) : "memory");
-            }
-        } else {
-            unsigned short* dst = (unsigned short*)(crow + (long long)n * 2);
-            if (full) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    unsigned o[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
-                        o[q] = *(unsigned*)&h;
-                    }
-                    asm volatile("multimem.red.relaxed.sys.global.add.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dst + 8 * j),
-                                 "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3])
-                                 : "memory");
-                }
-            } else {
-                for (int j = 0; j < 32; j += 2)   // the launcher guarantees an even column range for this mode
-                    if (n + j + 1 < p.n1) {
-                        __nv_bfloat162 h = __floats2bfloat162_rn(v[j], v[j + 1]);
-                        asm volatile("multimem.red.relaxed.sys.global.add.bf16x2 [%0], %1;" ::"l"(dst + j), "r"(*(unsigned*)&h) : "memory");
-                    }
-            }
-        }
-        return;
-    }
+    char* crow = Cb + (long long)m * ep.ldc;
+    uint4* tile = (uint4*)p.tile;
 
     if (ep.steps & B200FC_STEP_SILU_MUL) {
-        // columns [0,16) gate, [16,32) up of the same 16 channels -> 16 bf16 outputs at column n/2
-        float y[16];
+        // columns [0,16) gate, [16,32) up of the same 16 channels -> 16 bf16 outputs at column n / 2
 #pragma unroll
-        for (int j = 0; j < 16; j++) y[j] = silu_f(v[j]) * v[16 + j];
-        if (staged) {
-            unsigned o[8];
+        for (int h = 0; h < 2; h++) {
+            float y[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
-                o[j] = *(unsigned*)&h;
+            for (int j = 0; j < 8; j++) y[j] = silu_f(__uint_as_float(acc[8 * h + j])) * __uint_as_float(acc[16 + 8 * h + j]);
+            if (staged) {
+                tile[tile_pos<2>(lane, h)] = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]), pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
+            } else if (row_ok) {
+                unsigned short* dst = (unsigned short*)crow + (n >> 1) + 8 * h;
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (n + 16 + 8 * h + j < p.n1) dst[j] = f32_to_bf16_bits(y[j]);
             }
-            store_tile_32(o, p.tile, Cb, ep.ldc, m, n, p.M);      // column n / 2, two bytes each
-        } else {
-            unsigned short* dst = (unsigned short*)crow + (n >> 1);
-            for (int j = 0; j < 16; j++)
-                if (n + 16 + j < p.n1) dst[j] = f32_to_bf16_bits(y[j]);
         }
+        if (staged) flush_tile<2>(p.tile, Cb, ep.ldc, m0, n, p.M);
         return;
     }
 
-    {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        unsigned r[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = acc[8 * q + j];
+        const int nq = n + 8 * q;
+        if (ep.out_dtype != B200FC_S32) {
+            f32x2 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                w[j] = p.acc_is_int ? pack2((float)(int)r[2 * j], (float)(int)r[2 * j + 1])
+                                    : pack2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            f32x2 cv[4];
+            if (ep.steps & B200FC_STEP_DEQUANT) {
+                const f32x2 one = pack2(ep.deq_scale, ep.deq_scale);
+                if (ep.deq_per_oc) load_col_vec(p.cv_deq ? p.cv_deq + 8 * q : nullptr, ep.deq_per_oc, nq, p.n1, cv);
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = mul2(w[j], ep.deq_per_oc ? mul2(one, cv[j]) : one);
+            }
+            if (ep.steps & B200FC_STEP_BIAS) {
+                load_col_vec(p.cv_bias ? p.cv_bias + 8 * q : nullptr, ep.bias, nq, p.n1, cv);
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = add2(w[j], cv[j]);
+            }
+            if (ep.steps & B200FC_STEP_GELU) gelu_erf_poly8(w);
+            if (ep.steps & B200FC_STEP_QUANT) {
+                const f32x2 one = pack2(ep.q_scale, ep.q_scale);
+                if (ep.q_per_oc) load_col_vec(p.cv_q ? p.cv_q + 8 * q : nullptr, ep.q_per_oc, nq, p.n1, cv);
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = mul2(w[j], ep.q_per_oc ? cv[j] : one);
+            }
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 4; j++) unpack2(w[j], v[2 * j], v[2 * j + 1]);
+            if (ep.residual && row_ok) {
+                // residual added in fp32, before the one rounding of the output
+                const char* rrow = (const char*)ep.residual + (long long)m * ep.ld_res;
+                if (staged && (((uintptr_t)rrow + (size_t)nq * 2) & 15) == 0) {
+                    const int4 t = __ldg((const int4*)(rrow + (long long)nq * 2));
+                    const unsigned w4[4] = {(unsigned)t.x, (unsigned)t.y, (unsigned)t.z, (unsigned)t.w};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        v[2 * e] += __uint_as_float(w4[e] << 16);
+                        v[2 * e + 1] += __uint_as_float(w4[e] & 0xffff0000u);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        v[j] += __uint_as_float((unsigned)((const unsigned short*)rrow)[min(nq + j, p.n1 - 1)] << 16);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) r[j] = __float_as_uint(v[j]);
+        }
+        auto f = [&](int j) { return __uint_as_float(r[j]); };
+        if (staged) {
+            if (ep.out_dtype == B200FC_BF16) {
+                tile[tile_pos<4>(lane, q)] = make_uint4(pack_bf16x2(f(0), f(1)), pack_bf16x2(f(2), f(3)), pack_bf16x2(f(4), f(5)), pack_bf16x2(f(6), f(7)));
+            } else if (ep.out_dtype == B200FC_S8) {
+                ((uint2*)tile)[2 * tile_pos<2>(lane, q >> 1) + (q & 1)] = make_uint2(f32x4_to_s8x4(f(0), f(1), f(2), f(3)), f32x4_to_s8x4(f(4), f(5), f(6), f(7)));
+            } else {
+                tile[tile_pos<8>(lane, 2 * q)] = make_uint4(r[0], r[1], r[2], r[3]);
+                tile[tile_pos<8>(lane, 2 * q + 1)] = make_uint4(r[4], r[5], r[6], r[7]);
+            }
+        } else if (!row_ok) {
+        } else if (ep.mc_reduce) {
+            // Fused all-reduce: C is a multicast mapping of the output on every GPU of the tensor-parallel group; the NVSwitch
+            // adds this rank's contribution into all replicas (multimem.red), so no separate collective runs.
+            const bool full = p.vec_ok && n + 32 <= p.n1;
+            if (ep.out_dtype == B200FC_F32) {
+                float* dst = (float*)(crow + (long long)nq * 4);
+                if (full) {
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+                        asm volatile("multimem.red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
+                                     "f"(f(4 * j)), "f"(f(4 * j + 1)), "f"(f(4 * j + 2)), "f"(f(4 * j + 3))
+                                     : "memory");
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (nq + j < p.n1) asm volatile("multimem.red.relaxed.sys.global.add.f32 [%0], %1;" ::"l"(dst + j), "f"(f(j)) : "memory");
+                }
+            } else {
+                unsigned short* dst = (unsigned short*)(crow + (long long)nq * 2);
+                const unsigned o[4] = {pack_bf16x2(f(0), f(1)), pack_bf16x2(f(2), f(3)), pack_bf16x2(f(4), f(5)), pack_bf16x2(f(6), f(7))};
+                if (full) {
+                    asm volatile("multimem.red.relaxed.sys.global.add.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(o[0]), "r"(o[1]),
+                                 "r"(o[2]), "r"(o[3])
+                                 : "memory");
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)   // the launcher guarantees an even column range for this mode
+                        if (nq + 2 * j + 1 < p.n1)
+                            asm volatile("multimem.red.relaxed.sys.global.add.bf16x2 [%0], %1;" ::"l"(dst + 2 * j), "r"(o[j]) : "memory");
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                if (nq + j >= p.n1) break;
+                if (ep.out_dtype == B200FC_BF16) ((unsigned short*)crow)[nq + j] = f32_to_bf16_bits(f(j));
+                else if (ep.out_dtype == B200FC_S8) ((signed char*)crow)[nq + j] = (signed char)f32_to_s8(f(j));
+                else ((unsigned*)crow)[nq + j] = r[j];
+            }
+        }
+    }
+    if (staged) {
+        if (ep.out_dtype == B200FC_BF16) flush_tile<4>(p.tile, Cb, ep.ldc, m0, (long long)n * 2, p.M);
+        else if (ep.out_dtype == B200FC_S8) flush_tile<2>(p.tile, Cb, ep.ldc, m0, n, p.M);
+        else flush_tile<8>(p.tile, Cb, ep.ldc, m0, (long long)n * 4, p.M);
+    }
+}
+// The same for whole aligned chunks without residual and multicast, i.e. nearly all of them: one output kind per
+// instantiation, and one branch per post-op and chunk.  (With the choice made inside, per eight columns, a chunk took 2400
+// clocks of a warp for a plain bf16 store.)
+template <int V> struct IntConst { static constexpr int value = V; };
+enum EpiKind { EPI_F32 = 0, EPI_BF16, EPI_S8, EPI_S32, EPI_SILU, EPI_GENERAL };
+__device__ __forceinline__ int epilogue_kind(const Epilogue& ep, int vec_ok) {
+    if (!vec_ok || ep.mc_reduce || ep.residual) return EPI_GENERAL;
+    if (ep.steps & B200FC_STEP_SILU_MUL) return EPI_SILU;
+    return ep.out_dtype == B200FC_F32 ? EPI_F32 : (ep.out_dtype == B200FC_BF16 ? EPI_BF16 : (ep.out_dtype == B200FC_S8 ? EPI_S8 : EPI_S32));
+}
+template <int KIND>
+__device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m, int n, const EpiArgs& p, long long c_offset = 0) {
+    const Epilogue& ep = p.ep;
+    const int lane = threadIdx.x & 31, m0 = m - lane;
+    char* C = (char*)ep.C + c_offset;
+    uint4* tile = (uint4*)p.tile;
+    if constexpr (KIND == EPI_SILU) {
+        float y[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) y[j] = silu_f(__uint_as_float(acc[j])) * __uint_as_float(acc[16 + j]);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            tile[tile_pos<2>(lane, h)] = make_uint4(pack_bf16x2(y[8 * h], y[8 * h + 1]), pack_bf16x2(y[8 * h + 2], y[8 * h + 3]),
+                                                    pack_bf16x2(y[8 * h + 4], y[8 * h + 5]), pack_bf16x2(y[8 * h + 6], y[8 * h + 7]));
+        flush_tile<2>(p.tile, C, ep.ldc, m0, n, p.M);
+        return;
+    } else if constexpr (KIND == EPI_S32) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) tile[tile_pos<8>(lane, j)] = make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+        flush_tile<8>(p.tile, C, ep.ldc, m0, (long long)n * 4, p.M);
+        return;
+    } else {
         f32x2 w[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) w[j] = pack2(v[2 * j], v[2 * j + 1]);
-        // v = v * cv[j] (or * one scale), v + cv[j]
-        auto scale_by = [&](const float* staged_cv, const float* vec, float one) {
-            if (vec) {
-                float sc[32];
-                load_col_vec(staged_cv, vec, n, p.n1, sc);
+        for (int j = 0; j < 16; j++)
+            w[j] = p.acc_is_int ? pack2((float)(int)acc[2 * j], (float)(int)acc[2 * j + 1])
+                                : pack2(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+        if (ep.steps & B200FC_STEP_DEQUANT) {
+            const f32x2 one = pack2(ep.deq_scale, ep.deq_scale);
+            if (ep.deq_per_oc) {
 #pragma unroll
-                for (int j = 0; j < 16; j++) w[j] = mul2(w[j], mul2(pack2(one, one), pack2(sc[2 * j], sc[2 * j + 1])));
+                for (int q = 0; q < 4; q++) {
+                    f32x2 cv[4];
+                    load_col_vec(p.cv_deq ? p.cv_deq + 8 * q : nullptr, ep.deq_per_oc, n + 8 * q, p.n1, cv);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) w[4 * q + j] = mul2(w[4 * q + j], mul2(one, cv[j]));
+                }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; j++) w[j] = mul2(w[j], pack2(one, one));
+                for (int j = 0; j < 16; j++) w[j] = mul2(w[j], one);
             }
-        };
-        if (ep.steps & B200FC_STEP_DEQUANT) scale_by(p.cv_deq, ep.deq_per_oc, ep.deq_scale);
+        }
         if (ep.steps & B200FC_STEP_BIAS) {
-            float bs[32];
-            load_col_vec(p.cv_bias, ep.bias, n, p.n1, bs);
 #pragma unroll
-            for (int j = 0; j < 16; j++) w[j] = add2(w[j], pack2(bs[2 * j], bs[2 * j + 1]));
+            for (int q = 0; q < 4; q++) {
+                f32x2 cv[4];
+                load_col_vec(p.cv_bias ? p.cv_bias + 8 * q : nullptr, ep.bias, n + 8 * q, p.n1, cv);
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[4 * q + j] = add2(w[4 * q + j], cv[j]);
+            }
         }
         if (ep.steps & B200FC_STEP_GELU) {
 #pragma unroll
-            for (int j = 0; j < 16; j++) w[j] = gelu_erf_poly2(w[j]);
+            for (int q = 0; q < 4; q++) {
+                f32x2 t[4] = {w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]};
+                gelu_erf_poly8(t);
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[4 * q + j] = t[j];
+            }
         }
-        if (ep.steps & B200FC_STEP_QUANT) scale_by(p.cv_q, ep.q_per_oc, ep.q_per_oc ? 1.0f : ep.q_scale);
+        if (ep.steps & B200FC_STEP_QUANT) {
+            const f32x2 one = pack2(ep.q_scale, ep.q_scale);
+            if (ep.q_per_oc) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    f32x2 cv[4];
+                    load_col_vec(p.cv_q ? p.cv_q + 8 * q : nullptr, ep.q_per_oc, n + 8 * q, p.n1, cv);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) w[4 * q + j] = mul2(w[4 * q + j], cv[j]);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; j++) w[j] = mul2(w[j], one);
+            }
+        }
+        float v[32];
 #pragma unroll
         for (int j = 0; j < 16; j++) unpack2(w[j], v[2 * j], v[2 * j + 1]);
-    }
-    const bool full = p.vec_ok && n + 32 <= p.n1;
-    if (ep.residual && row_ok) {
-        // residual added in fp32, before the one rounding of the output
-        const char* rrow = (const char*)ep.residual + (long long)m * ep.ld_res;
-        if (full && (((uintptr_t)rrow + (size_t)n * 2) & 15) == 0) {
+        if constexpr (KIND == EPI_F32) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int4 t = __ldg((const int4*)(rrow + (long long)n * 2) + q);
-                const unsigned w4[4] = {(unsigned)t.x, (unsigned)t.y, (unsigned)t.z, (unsigned)t.w};
+            for (int j = 0; j < 8; j++)
+                tile[tile_pos<8>(lane, j)] = make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3]));
+            flush_tile<8>(p.tile, C, ep.ldc, m0, (long long)n * 4, p.M);
+        } else if constexpr (KIND == EPI_BF16) {
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    v[8 * q + 2 * e] += __uint_as_float(w4[e] << 16);
-                    v[8 * q + 2 * e + 1] += __uint_as_float(w4[e] & 0xffff0000u);
-                }
-            }
+            for (int j = 0; j < 4; j++)
+                tile[tile_pos<4>(lane, j)] = make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]),
+                                                        pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
+            flush_tile<4>(p.tile, C, ep.ldc, m0, (long long)n * 2, p.M);
         } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++)
-                v[j] += __uint_as_float((unsigned)((const unsigned short*)rrow)[min(n + j, p.n1 - 1)] << 16);
-        }
-    }
-    if (ep.out_dtype == B200FC_F32) {
-        if (staged) {
-            unsigned u[32];
-#pragma unroll
-            for (int j = 0; j < 32; j++) u[j] = __float_as_uint(v[j]);
-            store_tile_4b(u, p.tile, Cb, ep.ldc, m, n, p.M);
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((float*)crow)[n + j] = v[j];
-        }
-    } else if (ep.out_dtype == B200FC_BF16) {
-        if (staged) {
-            unsigned o[16];
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                o[j] = *(unsigned*)&h;
-            }
-            store_tile_64(o, p.tile, Cb, ep.ldc, m, (long long)n * 2, p.M);
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((unsigned short*)crow)[n + j] = f32_to_bf16_bits(v[j]);
-        }
-    } else {  // int8
-        if (staged) {
             unsigned o[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) o[j] = f32x4_to_s8x4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            store_tile_32(o, p.tile, Cb, ep.ldc, m, n, p.M);
-        } else {
-            for (int j = 0; j < 32; j++)
-                if (n + j < p.n1) ((signed char*)crow)[n + j] = (signed char)f32_to_s8(v[j]);
+#pragma unroll
+            for (int h = 0; h < 2; h++) tile[tile_pos<2>(lane, h)] = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
+            flush_tile<2>(p.tile, C, ep.ldc, m0, n, p.M);
         }
+    }
+}
+// Runs body(IntConst<KIND>) for the call's output kind: the loop over a tile's whole chunks is instantiated per kind.  The chunks
+// that are not whole (all of them for EPI_GENERAL) are left to the caller, who has one loop of epilogue_chunk for them.
+template <class Body>
+__device__ __forceinline__ void for_epilogue_kind(int kind, bool i8, const Body& body) {
+    switch (kind) {
+        case EPI_F32: body(IntConst<EPI_F32>()); break;
+        case EPI_BF16: body(IntConst<EPI_BF16>()); break;
+        case EPI_S8: body(IntConst<EPI_S8>()); break;
+        case EPI_S32: if (i8) body(IntConst<EPI_S32>()); break;
+        case EPI_SILU: if (!i8) body(IntConst<EPI_SILU>()); break;
+        default: break;
     }
 }
 
