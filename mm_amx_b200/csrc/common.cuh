@@ -151,6 +151,10 @@ size_t gemv_scratch_bytes();
 void set_decode_ctas_per_sm(int n);
 int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,
                     cudaStream_t s, void* scratch);
+// gemv_tq.cu: the same for int8-compressed and 4-bit weights on the tensor cores; B200FC_ERR_UNSUPPORTED without a message = not
+// these weights or not this alignment
+int launch_gemv_tq(const Weight& w, const void* A, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep, int max_ctas,
+                   cudaStream_t s);
 // gemv_tma.cu: gate/up + down of a decode-shaped MLP (bf16 weights, M <= 16) in one launch; B200FC_ERR_UNSUPPORTED
 // without a message = not possible for this shape / device, launch the two matrices one after the other
 int launch_mlp_decode_fused(const Weight& gate_up, const Weight& down, const void* x, int64_t ldx, int M, int K, int ns,

@@ -61,24 +61,9 @@ __device__ __forceinline__ void mbar_arrive_leader(unsigned cluster_addr) {
 __device__ __forceinline__ void st_cluster_v4(unsigned cluster_addr, unsigned a, unsigned b, unsigned c, unsigned d) {
     asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
-__device__ __forceinline__ unsigned bf16x2_sub(unsigned a, unsigned b) {
-    const __nv_bfloat162 r = __hsub2(*(const __nv_bfloat162*)&a, *(const __nv_bfloat162*)&b);
-    return *(const unsigned*)&r;
-}
-// two offset-binary weights u = v + 128 (bytes selected by sel, zero-extended) -> bf16x2 of v, exactly: 0x4300 | low 7 bits
-// is 128 + low; 128 is taken off where bit 7 of u is set and 256 where it is not
-__device__ __forceinline__ unsigned u8x2_to_bf16x2(unsigned w, unsigned sel) {
-    const unsigned p = __byte_perm(w, 0u, sel);
-    unsigned a, c;
-    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(a) : "r"(p), "r"(0x007f007fu), "r"(0x43004300u));   // (p & m) | k
-    asm("lop3.b32 %0, %1, %2, %3, 0xae;" : "=r"(c) : "r"(p), "r"(0x00800080u), "r"(0x43004300u));   // (~p & m) | k
-    return bf16x2_sub(a, c);
-}
 // nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of (n - 8) * scale, each product rounded once from fp32
-__device__ __forceinline__ unsigned nib2_to_bf16x2(unsigned w, float scale) {
-    unsigned a;
-    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(a) : "r"(w), "r"(0x000f000fu), "r"(0x43004300u));   // 128 + n
-    a = bf16x2_sub(a, 0x43084308u);                                                                 // - 136, exact
+__device__ __forceinline__ unsigned nib2_to_bf16x2_scaled(unsigned w, float scale) {
+    const unsigned a = nib2_to_bf16x2(w);
     const __nv_bfloat162 r = __floats2bfloat162_rn(__uint_as_float(a << 16) * scale, __uint_as_float(a & 0xffff0000u) * scale);
     return *(const unsigned*)&r;
 }
@@ -343,8 +328,8 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                                 for (int q = 0; q < 4; q++)
                                     *(uint4*)(d + (((4 * kh + q) ^ sw) << 4)) =
-                                        make_uint4(nib2_to_bf16x2(w4[q], f), nib2_to_bf16x2(w4[q] >> 4, f),
-                                                   nib2_to_bf16x2(w4[q] >> 8, f), nib2_to_bf16x2(w4[q] >> 12, f));
+                                        make_uint4(nib2_to_bf16x2_scaled(w4[q], f), nib2_to_bf16x2_scaled(w4[q] >> 4, f),
+                                                   nib2_to_bf16x2_scaled(w4[q] >> 8, f), nib2_to_bf16x2_scaled(w4[q] >> 12, f));
                             }
                         }
                         // the widened bytes must be visible to the tensor core (async proxy) before the slot counts as full

@@ -1540,12 +1540,18 @@ static int launch_tc(const CUtensorMap& map_w, const Params& p, const void* A, i
 int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,
                     cudaStream_t s, void* scratch) {
     if (n1 <= n0 && M >= 1 && M <= 16) return B200FC_OK;
+    read_switches();
+    static int use_tq = -1;
+    if (use_tq < 0) { const char* e = getenv("B200FC_GEMV_TQ"); use_tq = e ? atoi(e) : 1; }   // 0: never (for measurements)
+    if (use_tq) {
+        const int rq = launch_gemv_tq(w, A, M, K, lda, n0, n1, ep, (int)max_ctas(), s);
+        if (rq != B200FC_ERR_UNSUPPORTED) return rq;
+    }
     CUtensorMap map;
     Params p;
     int row_blocks = 0;
     int rc = prepare_job(w, A, M, K, lda, n0, n1, ep, s, scratch, map, p, row_blocks);
     if (rc) return rc;
-    read_switches();
     p.pf_cap = g_pf_cap;
     const long long gmax = max_ctas();
     // Three ways to cut the work; the cost model counts the stages of the longest CTA plus the time of the reduction

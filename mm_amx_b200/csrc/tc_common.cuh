@@ -579,6 +579,26 @@ __device__ __forceinline__ void tc_mma_pair(unsigned d_tmem, unsigned long long 
     }
 }
 
+__device__ __forceinline__ unsigned bf16x2_sub(unsigned a, unsigned b) {
+    const __nv_bfloat162 r = __hsub2(*(const __nv_bfloat162*)&a, *(const __nv_bfloat162*)&b);
+    return *(const unsigned*)&r;
+}
+// two offset-binary weights u = v + 128 (bytes selected by sel, zero-extended) -> bf16x2 of v, exactly: 0x4300 | low 7 bits
+// is 128 + low; 128 is taken off where bit 7 of u is set and 256 where it is not
+__device__ __forceinline__ unsigned u8x2_to_bf16x2(unsigned w, unsigned sel) {
+    const unsigned p = __byte_perm(w, 0u, sel);
+    unsigned a, c;
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(a) : "r"(p), "r"(0x007f007fu), "r"(0x43004300u));   // (p & m) | k
+    asm("lop3.b32 %0, %1, %2, %3, 0xae;" : "=r"(c) : "r"(p), "r"(0x00800080u), "r"(0x43004300u));   // (~p & m) | k
+    return bf16x2_sub(a, c);
+}
+// nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of n - 8, exactly: (128 + n) - 136
+__device__ __forceinline__ unsigned nib2_to_bf16x2(unsigned w) {
+    unsigned a;
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(a) : "r"(w), "r"(0x000f000fu), "r"(0x43004300u));
+    return bf16x2_sub(a, 0x43084308u);
+}
+
 // ---- host side -----------------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
