@@ -394,6 +394,11 @@ int launch_gemv_tq(const Weight& w, const void* A, int M, int K, int64_t lda, in
     TqParams p = {};
     p.spr = (int)(w.ld_bytes() / SLAB_BYTES);
     const int row_blocks = (n1 - n0 + TQ_ROWS - 1) / TQ_ROWS;
+    // More row blocks than SMs, so that a CTA has one to itself and some SMs have two CTAs, others one: with long rows that
+    // imbalance costs more than the faster product gains, and gemv_tma.cu cuts the stream into equal pieces (us, there / here:
+    // int8 1 x 8192 x 20480 36.9 / 47.0, x 28672 46.0 / 47.7; 4 bits 8 x 8192 x 25088 35.6 / 40.6; 16 rows int8 x 20480 45.4 / 48.6,
+    // x 25088 51.5 / 49.4; K = 3328 is level at 1 row and 1.2 to 1.3 times faster here at 16).
+    if (2 * row_blocks > max_ctas && (M <= 8 ? K >= 4096 : K >= 8192 && 7 * row_blocks < 4 * max_ctas)) return B200FC_ERR_UNSUPPORTED;
     // as many parts of K per row block as keep all CTAs resident, of two stages and more each
     int S = max_ctas / row_blocks;
     if (S > 8) S = 8;
