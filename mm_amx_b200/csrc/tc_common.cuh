@@ -48,8 +48,7 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
     return ok != 0;
 }
 // Bounded wait.  Returns false when the CTA is aborting (this wait or another role's ran out of time).
-// The clock is read after a batch of failed attempts only: a read of %globaltimer takes most of a microsecond, and one in front of
-// the second attempt put that on every slab of a main loop whose loads are not always early (0.46 us per slab whatever its size).
+// The clock and the abort flag are looked at after a batch of failed attempts only (try_wait itself suspends the thread for a while).
 // SLEEP_NS > 0: back off between polls (for waits that are long and not latency critical: the epilogue warps wait most
 // of a tile's main loop, and five spinning warps cost issue slots and power that the tensor pipe could use).
 template <int SLEEP_NS = 0>
@@ -109,6 +108,7 @@ __device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long adesc
     }
 }
 __device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned (&r)[32]) {
+    __syncwarp();      // (lanes of rows past M may have left the previous chunk early; the load is a warp-wide instruction)
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -409,15 +409,17 @@ __device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m,
         // A lane's 16 values are one 32-byte sector: stored directly, the way through shared memory only adds latency.  Rows past M
         // stay out of the arithmetic as well: their accumulators are zeros, and a division of zero takes the slow path of
         // the division (94 us instead of 58 for 436 x 3072 x 20096).
-        if (m >= p.M) return;
-        float y[16];
+        if (m < p.M) {
+            float y[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) y[j] = silu_f(__uint_as_float(acc[j])) * __uint_as_float(acc[16 + j]);
-        uint4* dst = (uint4*)(C + (long long)m * ep.ldc + n);       // column n / 2, two bytes each
+            for (int j = 0; j < 16; j++) y[j] = silu_f(__uint_as_float(acc[j])) * __uint_as_float(acc[16 + j]);
+            uint4* dst = (uint4*)(C + (long long)m * ep.ldc + n);       // column n / 2, two bytes each
 #pragma unroll
-        for (int h = 0; h < 2; h++)
-            dst[h] = make_uint4(pack_bf16x2(y[8 * h], y[8 * h + 1]), pack_bf16x2(y[8 * h + 2], y[8 * h + 3]),
-                                pack_bf16x2(y[8 * h + 4], y[8 * h + 5]), pack_bf16x2(y[8 * h + 6], y[8 * h + 7]));
+            for (int h = 0; h < 2; h++)
+                dst[h] = make_uint4(pack_bf16x2(y[8 * h], y[8 * h + 1]), pack_bf16x2(y[8 * h + 2], y[8 * h + 3]),
+                                    pack_bf16x2(y[8 * h + 4], y[8 * h + 5]), pack_bf16x2(y[8 * h + 6], y[8 * h + 7]));
+        }
+        __syncwarp();
         return;
     } else if constexpr (KIND == EPI_S32) {
 #pragma unroll
