@@ -150,6 +150,17 @@ __device__ __forceinline__ float ld_peer_f32(unsigned addr, unsigned rank) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
     return v;
 }
+// the fp32 values at shared-memory address `addr` of all S <= 8 CTAs of the cluster, added in rank order; the loads travel together
+// (Llama-7B MLP block at M = 1: 54.64 -> 54.56 us)
+__device__ __forceinline__ float cluster_sum(unsigned addr, int S) {
+    float t[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) t[q] = q < S ? ld_peer_f32(addr, (unsigned)q) : 0.0f;
+    float sum = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) sum += t[q];
+    return sum;
+}
 // strong (coherent at GPU scope) 16-byte load: partial sums written by other SMs during this launch
 __device__ __forceinline__ float4 ld_gpu_f4(const float4* p) {
     float4 v;
@@ -899,18 +910,14 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
             const int tok = e / out_rows, orow = e % out_rows;
             if (silu) {
                 const int grow = 32 * (orow >> 4) + (orow & 15);
-                float gsum = 0.0f, usum = 0.0f;
-                for (int q = 0; q < S; q++) {
-                    gsum += ld_peer_f32(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow), (unsigned)q);
-                    usum += ld_peer_f32(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow + 16), (unsigned)q);
-                }
+                const float gsum = cluster_sum(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow), S);
+                const float usum = cluster_sum(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow + 16), S);
                 if (blk_row0 + grow + 16 < p.n1) {
                     unsigned short* crow = (unsigned short*)((char*)ep.C + (long long)tok * ep.ldc);
                     crow[(blk_row0 >> 1) + orow] = f32_to_bf16_bits(silu_f(gsum) * usum);
                 }
             } else {
-                float sum = 0.0f;
-                for (int q = 0; q < S; q++) sum += ld_peer_f32(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + orow), (unsigned)q);
+                const float sum = cluster_sum(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + orow), S);
                 const int n = blk_row0 + orow;
                 if (n < p.n1) store_scalar(postop_staged(sum, orow, ep.steps, s_ep), tok, n, ep);
             }
@@ -1307,18 +1314,14 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
             const int tok = e / out_rows, orow = e % out_rows;
             if (silu) {
                 const int grow = 32 * (orow >> 4) + (orow & 15);
-                float gsum = 0.0f, usum = 0.0f;
-                for (int q = 0; q < S; q++) {
-                    gsum += ld_peer_f32(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow), (unsigned)q);
-                    usum += ld_peer_f32(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow + 16), (unsigned)q);
-                }
+                const float gsum = cluster_sum(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow), S);
+                const float usum = cluster_sum(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + grow + 16), S);
                 if (blk_row0 + grow + 16 < p.n1) {
                     unsigned short* crow = (unsigned short*)((char*)ep.C + (long long)tok * ep.ldc);
                     crow[(blk_row0 >> 1) + orow] = f32_to_bf16_bits(silu_f(gsum) * usum);
                 }
             } else {
-                float sum = 0.0f;
-                for (int q = 0; q < S; q++) sum += ld_peer_f32(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + orow), (unsigned)q);
+                const float sum = cluster_sum(part_addr + 4u * (unsigned)(tok * ROWS_PER_CTA + orow), S);
                 const int n = blk_row0 + orow;
                 if (n < p.n1) store_scalar(postop_staged(sum, orow, ep.steps, s_ep), tok, n, ep);
             }
