@@ -42,6 +42,7 @@ struct WaveParams {
     int M, n0, n1, n_pad;
     int R, R0;              // weight rows (= output columns) per CTA; of the first MMA of a K step
     int tiles_m, S;
+    int sets;               // accumulators that the slabs take in turn (sets x W columns of tensor memory)
     int slabs, units;       // K in 128-byte slabs of the MMA operands / in 128-byte pieces of the stored weight rows
     int slots, raw_slots, wide_slots;
     unsigned idesc0, idesc1;
@@ -100,7 +101,8 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     unsigned char* raw_ring = wide_ring + p.wide_slots * w_bytes;
     const int u0 = (int)((long long)p.units * split / p.S), u1 = (int)((long long)p.units * (split + 1) / p.S);
     const int n_units = u1 - u0, n_slabs = min(u1 * SPU, p.slabs) - u0 * SPU;
-    const unsigned tmem_cols = W <= 32 ? 32 : (W <= 64 ? 64 : (W <= 128 ? 128 : (W <= 256 ? 256 : 512)));
+    const int n_sets = min(p.sets, n_slabs), cols = p.sets * W;
+    const unsigned tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.slots; i++) {
@@ -185,7 +187,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else if (warp == 1) {
         // ---------------- MMA issue ----------------
         if (leader) {
-            int slot = 0, wslot = 0;
+            int slot = 0, wslot = 0, set = 0;
             unsigned phase = 0, wphase = 0;
             const unsigned ring = smem_u32(smem), wring = smem_u32(wide_ring);
             for (int i = 0; i < n_slabs; i++) {
@@ -201,10 +203,10 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                     for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++) {
                         const unsigned long long adv = (unsigned long long)(k * (MMA_K_BYTES >> 4));
-                        const unsigned acc = (unsigned)((i | k) != 0);
-                        if constexpr (CG == 2) tc_mma_pair<I8>(tmem_base, adesc + adv, bdesc + adv, p.idesc0, acc);
-                        else tc_mma<I8>(tmem_base, adesc + adv, bdesc + adv, p.idesc0, acc);
-                        if (CG == 2 && p.R0 < p.R) tc_mma_pair<I8>(tmem_base + 2 * p.R0, adesc + adv, bdesc1 + adv, p.idesc1, acc);
+                        const unsigned acc = (unsigned)(i >= p.sets || k != 0);
+                        if constexpr (CG == 2) tc_mma_pair<I8>(tmem_base + set * W, adesc + adv, bdesc + adv, p.idesc0, acc);
+                        else tc_mma<I8>(tmem_base + set * W, adesc + adv, bdesc + adv, p.idesc0, acc);
+                        if (CG == 2 && p.R0 < p.R) tc_mma_pair<I8>(tmem_base + set * W + 2 * p.R0, adesc + adv, bdesc1 + adv, p.idesc1, acc);
                     }
                     if constexpr (CG == 2) {
                         const unsigned short mask = (unsigned short)(3u << leader_rank);
@@ -217,6 +219,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         if (i == n_slabs - 1) tc_commit(bar_acc);
                     }
                 }
+                if (++set == p.sets) set = 0;
                 if (++slot == p.slots) { slot = 0; phase ^= 1; }
                 if (WQ && ++wslot == p.wide_slots) { wslot = 0; wphase ^= 1; }
             }
@@ -367,6 +370,21 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         };
         // every load of the ring has landed and every MMA has read it: the ring is free
         unsigned* stage_tile = (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES);
+        // columns [32 c, +32) of this CTA's accumulators, the sets added in order
+        auto load_acc = [&](int c, unsigned (&r)[32]) {
+            tc_ld32(taddr + (unsigned)(c * 32), r);
+            tc_wait_ld();
+            if constexpr (!I8) {
+#pragma unroll 1
+                for (int t = 1; t < n_sets; t++) {
+                    unsigned x[32];
+                    tc_ld32(taddr + (unsigned)(t * W + c * 32), x);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
+                }
+            }
+        };
         if (p.S > 1) {
             // Part `q` of K hands chunk c of its accumulators to CTA (c mod S) of the cluster: 16 KB at slot (c / S) * S + q of
             // that CTA's ring, as [4-column piece][row] 16-byte units.  Remote stores are posted, so nothing waits for a
@@ -378,10 +396,9 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll 1
                 for (int c = third; c < chunks; c += SETS) {
                     unsigned r[32];
-                    tc_ld32(taddr + (unsigned)(c * 32), r);
+                    load_acc(c, r);
                     const int owner = c % p.S;
                     const unsigned dst = mapa_rank(mine + (unsigned)(((c / p.S) * p.S + split) * CHUNK_BYTES), (unsigned)(owner * CG + rank));
-                    tc_wait_ld();
 #pragma unroll
                     for (int j = 0; j < 8; j++)
                         st_cluster_v4(dst + (unsigned)(j * BM * 16), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
@@ -393,8 +410,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // accumulators of the t-th chunk this CTA finishes: its own, or the sum of the parts in the order of K
         auto fetch = [&](int t, int c, unsigned (&r)[32]) {
             if (p.S == 1) {
-                tc_ld32(taddr + (unsigned)(c * 32), r);
-                tc_wait_ld();
+                load_acc(c, r);
                 return;
             }
             const uint4* src = (const uint4*)(smem + t * p.S * CHUNK_BYTES) + quarter * 32 + lane;
@@ -516,11 +532,14 @@ int max_tiles(int S, int* out) {
     return B200FC_OK;
 }
 
+int max_sets(int W) { return W <= 64 ? 8 : (W <= 128 ? 4 : (W <= 256 ? 2 : 1)); }   // accumulators of W columns in tensor memory
+
 // Picks the columns per CTA and the split of K of a call that fits one wave; false = it does not.  The model counts SM
 // clocks of one CTA: per 128-byte slab the slowest of operand loads (about 48 bytes per clock and SM reach shared memory from
 // L2), MMAs (the 256-wide one takes 128 clocks per 32 bytes of K) and widening; plus the reduction and the epilogue.
+// `chains`: the number of chains that K is to be summed in, see run_wave.
 template <int CG, int MODE>
-int pick_shape(int M, int nspan, int slabs, int units, WaveShape* best, bool* found) {
+int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* best, bool* found) {
     const int tiles_m = (M + BM * CG - 1) / (BM * CG);
     const int rows_a = M < BM ? M : BM;
     const int wbytes = MODE == W_U4C ? 34 : (MODE == W_U8C ? 64 : 128);
@@ -533,6 +552,7 @@ int pick_shape(int M, int nspan, int slabs, int units, WaveShape* best, bool* fo
         for (int R = 32; R <= 256; R += 32) {
             const int W = R * CG, tiles_n = (nspan + W - 1) / W;
             if ((long long)tiles_m * tiles_n > cap) continue;
+            if (S * max_sets(W) < chains) continue;
             if (S > 1 && S * ((W / 32 + S - 1) / S) * CHUNK_BYTES + WORKERS * WARP_TILE_BYTES > RING_BYTES) continue;
             const double load = (rows_a * 128.0 + R * (double)wbytes) / 48.0, mma = 2.0 * W;
             const double cvt = MODE == W_U4C ? 2.2 * R : (MODE == W_U8C ? 1.4 * R : 0.0);
@@ -565,7 +585,21 @@ int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const f
     if (MODE == W_U4C) p.units = (int)(w_ld / SLAB_BYTES);     // (the group scales are laid out by it)
     WaveShape sh;
     bool found = false;
-    int rc = pick_shape<CG, MODE>(M, n1 - n0, p.slabs, p.units, &sh, &found);
+    // The tensor core's error grows with the length of a chain of fp32 sums (256 x 4096 x 4096, relative to float64: 1.08e-6 in three
+    // chains, 7.9e-7 in four, 5.1e-7 in six).  K is cut into as many chains as gemm_tc.cu's split of the same call has, counting the parts of the
+    // cluster and, inside a CTA, accumulators that the slabs take in turn.
+    int chains = 1;
+    if (!I8) {
+        int span = n1 - n0;
+        const int blk = (int)(((size_t)32 << 20) / ((size_t)W_K_pad * 2)) / kRowPad * kRowPad;    // columns of a widened block there
+        if (WQ && span > blk) span = blk < kRowPad ? kRowPad : blk;
+        const int tiles = (M + 2 * BM - 1) / (2 * BM) * ((span + 255) / 256), pairs = num_sms() / 2;
+        if (tiles * 2 <= pairs && p.slabs >= 16) {
+            chains = pairs / tiles < 8 ? pairs / tiles : 8;
+            if (chains > p.slabs / 8) chains = p.slabs / 8;
+        }
+    }
+    int rc = pick_shape<CG, MODE>(M, n1 - n0, p.slabs, p.units, chains, &sh, &found);
     if (rc) return rc;
     if (!found) return B200FC_ERR_UNSUPPORTED;
     // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256
@@ -573,6 +607,8 @@ int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const f
     if (!WQ && CG == 2 && sh.S == 1 && sh.R == 128 && 4 * sh.tiles_m * sh.tiles_n > num_sms()) return B200FC_ERR_UNSUPPORTED;
     p.M = M; p.n0 = n0; p.n1 = n1; p.n_pad = W_N_pad;
     p.R = sh.R; p.S = sh.S; p.tiles_m = sh.tiles_m;
+    p.sets = 1;
+    while (p.sets * sh.S < chains) p.sets *= 2;
     p.R0 = CG == 2 && sh.R > 128 ? (sh.R / 2 + 31) / 32 * 32 : sh.R;
     p.idesc0 = make_idesc(I8, a_signed, w_signed, CG * p.R0, CG * BM);
     p.idesc1 = make_idesc(I8, a_signed, w_signed, CG * (p.R - p.R0), CG * BM);
