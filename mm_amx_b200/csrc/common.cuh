@@ -162,6 +162,8 @@ int launch_mlp_decode_fused(const Weight& gate_up, const Weight& down, const voi
 // gemm_tc.cu: tcgen05 GEMM, bf16 x bf16 -> fp32 or 8-bit x 8-bit -> int32
 int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, const void* A, int dtypeA, int M, int K,
                    int64_t lda, int n0, int n1, const Epilogue& ep, cudaStream_t s);
+// 0 = choose by shape, 1 = force the 1-CTA kernel, 2 = force the 2-CTA kernel (B200FC_GEMM_CTAS, for experiments)
+int gemm_forced_ctas();
 // gemm_wave.cu: the same layer, any weight type, for calls whose output fits one wave of tiles; B200FC_ERR_UNSUPPORTED
 // without a message = it does not, take launch_gemm_tc
 int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,

@@ -743,8 +743,9 @@ bool tail_split_enabled() {
     return v != 0;
 }
 
-// 0 = choose by shape, 1 = force the 1-CTA kernel, 2 = force the 2-CTA kernel (B200FC_GEMM_CTAS, for experiments)
-int forced_ctas() {
+}  // namespace
+
+int gemm_forced_ctas() {
     static int v = -1;
     if (v < 0) {
         const char* e = getenv("B200FC_GEMM_CTAS");
@@ -752,8 +753,6 @@ int forced_ctas() {
     }
     return v;
 }
-
-}  // namespace
 
 int launch_gemm_tc_allreduce(const void* W_data, int W_K_pad, int W_N_pad, const void* A, int M, int K, int64_t lda,
                              int N, const AllReduceDesc& ar, cudaStream_t s) {
@@ -867,7 +866,7 @@ int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, co
     // 2-CTA tiles (256 x 256 per CTA pair) when there are at least two 128-row blocks of M and enough tiles
     // ... or when the 1-CTA kernel would leave most SMs without a tile while K is long (the 2-CTA launcher splits K)
     const bool few_tiles = tiles_m * ((nspan + 255) / 256) * 2 <= num_sms() / 2 && K >= 2048;
-    const bool pair_ok = (forced_ctas() == 2) || (forced_ctas() == 0 && nspan > 128 && (M > BM || few_tiles));
+    const bool pair_ok = (gemm_forced_ctas() == 2) || (gemm_forced_ctas() == 0 && nspan > 128 && (M > BM || few_tiles));
     if (pair_ok) {
         const int bn2 = 256;
         p.tiles_m = (M + 2 * BM - 1) / (2 * BM);

@@ -667,8 +667,8 @@ int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, i
                      cudaStream_t s) {
     if (M <= 0 || n1 <= n0) return B200FC_OK;
     if (ep.mc_reduce || (((uintptr_t)A | (uintptr_t)lda) & 15)) return B200FC_ERR_UNSUPPORTED;
-    static int enabled = -1;                       // B200FC_GEMM_WAVE=0: never (for measurements)
-    if (enabled < 0) { const char* e = getenv("B200FC_GEMM_WAVE"); enabled = e ? atoi(e) : 1; }
+    static int enabled = -1;                       // B200FC_GEMM_WAVE=0, or a GEMM forced by its own switch: never
+    if (enabled < 0) { const char* e = getenv("B200FC_GEMM_WAVE"); enabled = (e ? atoi(e) : 1) && !gemm_forced_ctas(); }
     if (!enabled) return B200FC_ERR_UNSUPPORTED;
     const bool a8 = dtypeA != B200FC_BF16;
     const unsigned as = dtypeA == B200FC_S8, ws = w.dtype == B200FC_S8;

@@ -1478,7 +1478,7 @@ static int prepare_job(const Weight& w, const void* A, int M, int K, int64_t lda
 }
 
 // environment switches, for experiments
-static int g_pf_cap = -1, g_per_sm = 2, g_force_stream = 0, g_force_aligned = 0;
+static int g_pf_cap = -1, g_per_sm = 2, g_force_stream = 0, g_force_aligned = 0, g_use_tq = 1;
 static void read_switches() {
     if (g_pf_cap >= 0) return;
     const char* e = getenv("B200FC_GEMV_CTAS_PER_SM");   // 1 leaves the second resident place to the next kernel
@@ -1486,6 +1486,8 @@ static void read_switches() {
     e = getenv("B200FC_GEMV_STREAMK");                   // 1: never align pieces with row blocks
     g_force_stream = (e && atoi(e) == 1) ? 1 : 0;
     g_force_aligned = (e && atoi(e) == 2) ? 1 : 0;       // 2: align whenever the row blocks fit the grid
+    e = getenv("B200FC_GEMV_TQ");                        // 0: never gemv_tq.cu, nor under a switch about how this file's kernels work
+    g_use_tq = (e ? atoi(e) : 1) && !getenv("B200FC_GEMV_XIMG") && !getenv("B200FC_GEMV_STREAMK") && !getenv("B200FC_GEMV_PREFETCH");
     e = getenv("B200FC_GEMV_PREFETCH");                  // stages prefetched into L2 at CTA start (0 = none)
     int v = e ? atoi(e) : 0;
     g_pf_cap = v < 0 ? 0 : (v > 64 ? 64 : v);
@@ -1544,9 +1546,7 @@ int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, i
                     cudaStream_t s, void* scratch) {
     if (n1 <= n0 && M >= 1 && M <= 16) return B200FC_OK;
     read_switches();
-    static int use_tq = -1;
-    if (use_tq < 0) { const char* e = getenv("B200FC_GEMV_TQ"); use_tq = e ? atoi(e) : 1; }   // 0: never (for measurements)
-    if (use_tq) {
+    if (g_use_tq) {
         const int rq = launch_gemv_tq(w, A, M, K, lda, n0, n1, ep, (int)max_ctas(), s);
         if (rq != B200FC_ERR_UNSUPPORTED) return rq;
     }
