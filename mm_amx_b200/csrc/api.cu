@@ -286,8 +286,7 @@ int matmul_device(const Weight& w, Weight* w_mut, const void* A, int dtypeA, int
         // copy of the matrix is kept.
         (void)w_mut;
         const size_t row_bytes = (size_t)w.K_pad * 2;
-        int blk = (int)(((size_t)32 << 20) / row_bytes) / kRowPad * kRowPad;
-        if (blk < kRowPad) blk = kRowPad;
+        const int blk = widened_block_rows(w.K_pad);
         const int r_lo = n0 / kRowPad * kRowPad;                  // packed rows are padded to kRowPad
         void* wide = nullptr;
         rc = get_stream_scratch((size_t)blk * row_bytes, s, 3, &wide);

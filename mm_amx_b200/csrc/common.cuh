@@ -164,6 +164,13 @@ int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, co
                    int64_t lda, int n0, int n1, const Epilogue& ep, cudaStream_t s);
 // 0 = choose by shape, 1 = force the 1-CTA kernel, 2 = force the 2-CTA kernel (B200FC_GEMM_CTAS, for experiments)
 int gemm_forced_ctas();
+// parts of K that launch_gemm_tc sums one after the other for a bf16 call of nspan columns: chains of fp32 sums
+int gemm_tc_chains(int M, int K, int nspan);
+// rows of compressed weights that are widened to bf16 at a time in front of launch_gemm_tc: 32 MB of them
+inline int widened_block_rows(int K_pad) {
+    const int blk = (int)(((size_t)32 << 20) / ((size_t)K_pad * 2)) / kRowPad * kRowPad;
+    return blk < kRowPad ? kRowPad : blk;
+}
 // gemm_wave.cu: the same layer, any weight type, for calls whose output fits one wave of tiles; B200FC_ERR_UNSUPPORTED
 // without a message = it does not, take launch_gemm_tc
 int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,

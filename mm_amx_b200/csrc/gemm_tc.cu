@@ -651,6 +651,22 @@ int launch_cfg(const CUtensorMap& ma, const CUtensorMap& mw, const GemmParams& p
     return B200FC_OK;
 }
 
+// Whether a call goes to the 2-CTA kernel: 256 x 256 tiles per CTA pair when there are at least two 128-row blocks of M and enough
+// tiles, or when the 1-CTA kernel would leave most SMs without a tile while K is long (the 2-CTA launcher splits K).
+bool takes_pairs(int M, int K, int nspan) {
+    const bool few_tiles = (M + BM - 1) / BM * ((nspan + 255) / 256) * 2 <= num_sms() / 2 && K >= 2048;
+    return gemm_forced_ctas() == 2 || (gemm_forced_ctas() == 0 && nspan > 128 && (M > BM || few_tiles));
+}
+// Too few tiles to occupy the GPU (small M): parts of K, so that every pair has work.
+int pair_splits(int tiles, int k_slabs) {
+    const int max_pairs = num_sms() / 2;
+    if (tiles * 2 > max_pairs || k_slabs < 16) return 1;
+    int splits = max_pairs / tiles;
+    if (splits > 8) splits = 8;
+    if (splits > k_slabs / 8) splits = k_slabs / 8;
+    return splits < 1 ? 1 : splits;
+}
+
 template <int BN, bool I8>
 int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cudaStream_t s) {
     using C = Cfg2<BN>;
@@ -665,15 +681,9 @@ int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cuda
     }
     const int tiles = p.tiles_m * p.tiles_n;
     const int max_pairs = num_sms() / 2;
-    // Too few tiles to occupy the GPU (small M): split K so that every pair has work; the raw partial accumulators go
-    // through a workspace of this stream and a second kernel sums them in order and runs the post-ops.
-    int splits = 1;
-    if (tiles * 2 <= max_pairs && p.k_slabs >= 16 && !p.ep.mc_reduce) {
-        splits = max_pairs / tiles;
-        if (splits > 8) splits = 8;
-        if (splits > p.k_slabs / 8) splits = p.k_slabs / 8;
-        if (splits < 1) splits = 1;
-    }
+    // K in parts: the raw partial accumulators go through a workspace of this stream and a second kernel sums them in order and
+    // runs the post-ops.
+    const int splits = p.ep.mc_reduce ? 1 : pair_splits(tiles, p.k_slabs);
     p.splits = splits;
     p.split_stride = 0;
     const Epilogue final_ep = p.ep;
@@ -752,6 +762,11 @@ int gemm_forced_ctas() {
         v = e ? atoi(e) : 0;
     }
     return v;
+}
+
+int gemm_tc_chains(int M, int K, int nspan) {
+    if (!takes_pairs(M, K, nspan)) return 1;
+    return pair_splits((M + 2 * BM - 1) / (2 * BM) * ((nspan + 255) / 256), (K + SLAB_BYTES / 2 - 1) / (SLAB_BYTES / 2));
 }
 
 int launch_gemm_tc_allreduce(const void* W_data, int W_K_pad, int W_N_pad, const void* A, int M, int K, int64_t lda,
@@ -863,11 +878,7 @@ int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, co
     CUtensorMap ma, mw;
     int rc = make_map(&ma, A, i8, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BM);
     if (rc) return rc;
-    // 2-CTA tiles (256 x 256 per CTA pair) when there are at least two 128-row blocks of M and enough tiles
-    // ... or when the 1-CTA kernel would leave most SMs without a tile while K is long (the 2-CTA launcher splits K)
-    const bool few_tiles = tiles_m * ((nspan + 255) / 256) * 2 <= num_sms() / 2 && K >= 2048;
-    const bool pair_ok = (gemm_forced_ctas() == 2) || (gemm_forced_ctas() == 0 && nspan > 128 && (M > BM || few_tiles));
-    if (pair_ok) {
+    if (takes_pairs(M, K, nspan)) {
         const int bn2 = 256;
         p.tiles_m = (M + 2 * BM - 1) / (2 * BM);
         p.tiles_n = (nspan + bn2 - 1) / bn2;

@@ -30,7 +30,7 @@ enum WaveMode { W_BF16 = 0, W_I8 = 1, W_U8C = 2, W_U4C = 3 };   // weights: bf16
 constexpr int SETS = 3;                               // sets of four worker warps, one warp of a set per TMEM quarter
 constexpr int WORKERS = 4 * SETS;
 constexpr int WAVE_THREADS = 128 + 32 * WORKERS;
-constexpr int MAX_SLOTS = 12, MAX_RAW = 8, MAX_WIDE = 8, MAX_W = 512;
+constexpr int MAX_SLOTS = 12, MAX_RAW = 8, MAX_WIDE = 4, MAX_W = 512;
 constexpr int WAVE_BAR_BYTES = 512;
 constexpr int COLVEC_FLOATS = 3 * MAX_W;
 constexpr int WAVE_SMEM = 232448;                                                  // all an SM gives to one CTA
@@ -42,7 +42,7 @@ struct WaveParams {
     int M, n0, n1, n_pad;
     int R, R0;              // weight rows (= output columns) per CTA; of the first MMA of a K step
     int tiles_m, S;
-    int sets;               // accumulators that the slabs take in turn (sets x W columns of tensor memory)
+    int parts, sets;        // parts of a CTA's K, and accumulators that the slabs of a part take in turn (W columns of tensor memory each)
     int slabs, units;       // K in 128-byte slabs of the MMA operands / in 128-byte pieces of the stored weight rows
     int slots, raw_slots, wide_slots;
     unsigned idesc0, idesc1;
@@ -69,7 +69,11 @@ __device__ __forceinline__ unsigned nib2_to_bf16x2_scaled(unsigned w, float scal
     return *(const unsigned*)&r;
 }
 
-template <int CG, int MODE>
+// FOLD: K in several parts, see below (quantised weights).  A kernel of its own, because the folding code costs the widening loop
+// registers and instruction cache also where it does not run (int8 705 x 2560 x 10240: 44.8 us with it, 42.3 without).  A fold
+// costs about 2 us, most of it reading tensor memory (500 clocks per 32 columns and accumulator): int8 35 x 6400 x 21104 in three
+// chains 61 us, in eight 74; through widened blocks and a split of K 285.
+template <int CG, int MODE, bool FOLD>
 __global__ void __launch_bounds__(WAVE_THREADS, 1)
 gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const WaveParams p) {
     constexpr bool I8 = MODE == W_I8, WQ = MODE == W_U8C || MODE == W_U4C;
@@ -81,8 +85,8 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const unsigned bar_full = bars, bar_empty = bars + 8 * MAX_SLOTS;
     const unsigned bar_raw_full = bars + 16 * MAX_SLOTS, bar_raw_empty = bar_raw_full + 8 * MAX_RAW;
     const unsigned bar_wide_full = bar_raw_empty + 8 * MAX_RAW, bar_wide_empty = bar_wide_full + 8 * MAX_WIDE;
-    const unsigned bar_acc = bar_wide_empty + 8 * MAX_WIDE;
-    unsigned* tmem_holder = (unsigned*)(smem + RING_BYTES + 16 * (MAX_SLOTS + MAX_RAW + MAX_WIDE) + 8);
+    const unsigned bar_acc = bar_wide_empty + 8 * MAX_WIDE, bar_part = bar_acc + 8, bar_folded = bar_part + 8;
+    unsigned* tmem_holder = (unsigned*)(smem + RING_BYTES + 16 * (MAX_SLOTS + MAX_RAW + MAX_WIDE) + 24);
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
     float* colvec = (float*)(smem + RING_BYTES + WAVE_BAR_BYTES);
 
@@ -101,7 +105,9 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     unsigned char* raw_ring = wide_ring + p.wide_slots * w_bytes;
     const int u0 = (int)((long long)p.units * split / p.S), u1 = (int)((long long)p.units * (split + 1) / p.S);
     const int n_units = u1 - u0, n_slabs = min(u1 * SPU, p.slabs) - u0 * SPU;
-    const int n_sets = min(p.sets, n_slabs), cols = p.sets * W;
+    // K in chains of fp32 sums: the slabs take the accumulators in turn.  Where tensor memory holds too few of them K is cut into parts
+    // as well, after each of which (but the last) the workers fold the accumulators into a sum, behind them in tensor memory.
+    const int parts = FOLD ? min(p.parts, n_slabs) : 1, cols = (p.sets + (parts > 1 ? 1 : 0)) * W;
     const unsigned tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
 
     if (threadIdx.x == 0) {
@@ -118,6 +124,8 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             mbar_init(bar_wide_empty + 8 * i, 1);
         }
         mbar_init(bar_acc, 1);
+        mbar_init(bar_part, 1);
+        mbar_init(bar_folded, CG * WORKERS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -187,10 +195,17 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else if (warp == 1) {
         // ---------------- MMA issue ----------------
         if (leader) {
-            int slot = 0, wslot = 0, set = 0;
+            int slot = 0, wslot = 0, set = 0, part = 0, start = 0, end = n_slabs / parts;      // slabs of the part
             unsigned phase = 0, wphase = 0;
             const unsigned ring = smem_u32(smem), wring = smem_u32(wide_ring);
             for (int i = 0; i < n_slabs; i++) {
+                if (FOLD && i == end) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_folded, (unsigned)part & 1, abort_flag, p.wait_limit_ns))) break;
+                    part++;
+                    start = end;
+                    end = n_slabs * (part + 1) / parts;
+                    set = 0;
+                }
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * slot, phase, abort_flag, p.wait_limit_ns))) break;
                 if (WQ && !__all_sync(0xffffffffu, mbar_wait(bar_wide_full + 8 * wslot, wphase, abort_flag, p.wait_limit_ns))) break;
                 tc_fence_after();
@@ -203,7 +218,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                     for (int k = 0; k < SLAB_BYTES / MMA_K_BYTES; k++) {
                         const unsigned long long adv = (unsigned long long)(k * (MMA_K_BYTES >> 4));
-                        const unsigned acc = (unsigned)(i >= p.sets || k != 0);
+                        const unsigned acc = (unsigned)(i - start >= p.sets || k != 0);
                         if constexpr (CG == 2) tc_mma_pair<I8>(tmem_base + set * W, adesc + adv, bdesc + adv, p.idesc0, acc);
                         else tc_mma<I8>(tmem_base + set * W, adesc + adv, bdesc + adv, p.idesc0, acc);
                         if (CG == 2 && p.R0 < p.R) tc_mma_pair<I8>(tmem_base + set * W + 2 * p.R0, adesc + adv, bdesc1 + adv, p.idesc1, acc);
@@ -212,10 +227,12 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         const unsigned short mask = (unsigned short)(3u << leader_rank);
                         tc_commit_mask(bar_empty + 8 * slot, mask);
                         if (WQ) tc_commit_mask(bar_wide_empty + 8 * wslot, mask);
+                        if (FOLD && i == end - 1 && i != n_slabs - 1) tc_commit_mask(bar_part, mask);
                         if (i == n_slabs - 1) tc_commit_mask(bar_acc, mask);
                     } else {
                         tc_commit(bar_empty + 8 * slot);
                         if (WQ) tc_commit(bar_wide_empty + 8 * wslot);
+                        if (FOLD && i == end - 1 && i != n_slabs - 1) tc_commit(bar_part);
                         if (i == n_slabs - 1) tc_commit(bar_acc);
                     }
                 }
@@ -257,6 +274,40 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (use_bias) colvec[MAX_W + i] = __ldg(p.ep.bias + col);
                 if (use_q) colvec[2 * MAX_W + i] = __ldg(p.ep.q_per_oc + col);
             }
+        const int quarter = warp & 3, third = wi >> 2;
+        const int chunks = W / 32;
+        const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16);
+        // the accumulators of a part, once its MMAs are done, into the sum: fp32 adds in order, the columns shared out as in the epilogue
+        const unsigned folded_leader = CG == 2 ? mapa_rank(bar_folded, leader_rank) : bar_folded;
+        int folds = 0;
+        auto fold_part = [&]() {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_part, (unsigned)folds & 1, abort_flag, p.wait_limit_ns));
+            if (!ok) return;
+            tc_fence_after();
+            const int filled = min(p.sets, n_slabs * (folds + 1) / parts - n_slabs * folds / parts);
+#pragma unroll 1
+            for (int c = third; c < chunks; c += SETS) {
+                unsigned sum[32], x[32];
+                tc_ld32(taddr + (unsigned)((folds ? p.sets * W : 0) + c * 32), sum);
+#pragma unroll 1
+                for (int t = folds ? 0 : 1; t < filled; t++) {
+                    tc_ld32(taddr + (unsigned)(t * W + c * 32), x);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(x[j]));
+                }
+                tc_wait_ld();
+                tc_st32(taddr + (unsigned)(p.sets * W + c * 32), sum);
+            }
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                if (CG == 1 || leader) mbar_arrive(bar_folded);
+                else mbar_arrive_remote(folded_leader);
+            }
+            folds++;
+        };
         if constexpr (WQ) {
             // ---------------- widening ----------------
             // The sets of four warps take the slabs in turn, so that a warp's waits, its proxy fence and its arrival (about
@@ -276,7 +327,10 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 }
             };
             if constexpr (MODE == W_U4C) load_scales(u0);
-            int slot = 0, rslot = 0, turn = 0;
+            int slot = 0, rslot = 0, turn = 0, slab = 0;
+            // A part is folded when the ring of widened slabs has been filled behind it: the MMAs of the next one wait for the fold, and
+            // go on at once with the slabs that are there.
+            int fold_at = parts > 1 ? n_slabs / parts + p.wide_slots : n_slabs;
             unsigned phase = 0, rphase = 0;
             for (int j = 0; j < n_units && ok; j++) {
                 const int u = u0 + j;
@@ -293,6 +347,13 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll 1
                 for (int s = 0; s < SPU; s++) {
                     if (u * SPU + s >= p.slabs) break;          // warp-uniform: the last piece may reach past K
+                    if constexpr (FOLD) {
+                        if (slab++ == fold_at) {
+                            fold_part();
+                            if (!ok) break;
+                            fold_at = folds < parts - 1 ? n_slabs * (folds + 1) / parts + p.wide_slots : n_slabs;
+                        }
+                    }
                     if (turn == set) {
                         constexpr int UNITS = MODE == W_U8C ? 2 : 1;     // 16-byte units of an item's row
                         uint4 v[4][UNITS];
@@ -351,15 +412,14 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (++rslot == p.raw_slots) { rslot = 0; rphase ^= 1; }
             }
         }
+        if constexpr (FOLD)
+            while (folds < parts - 1 && ok) fold_part();        // (a part shorter than the ring)
         // ---------------- epilogue ----------------
         asm volatile("bar.sync 1, %0;" ::"n"(WORKERS * 32) : "memory");
         ok = __all_sync(0xffffffffu, ok && mbar_wait<32>(bar_acc, 0, abort_flag, p.wait_limit_ns));
         tc_fence_after();
-        const int quarter = warp & 3, third = wi >> 2;
-        const int chunks = W / 32;
         const int m = (tm * CG + rank) * BM + quarter * 32 + lane;
         const bool row_ok = m < p.M;
-        const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16);
         // accumulator column of a chunk -> output column: with a pair, MMA 0 holds the first R0 columns of CTA 0's R and of
         // CTA 1's R side by side, MMA 1 the other R - R0 of both
         auto chunk_col = [&](int c) -> int {
@@ -370,13 +430,14 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         };
         // every load of the ring has landed and every MMA has read it: the ring is free
         unsigned* stage_tile = (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES);
-        // columns [32 c, +32) of this CTA's accumulators, the sets added in order
+        // columns [32 c, +32) of this CTA's result: the sum of the folded parts, if any, and the last part's accumulators in order
+        const int filled = min(p.sets, n_slabs - n_slabs * (parts - 1) / parts);
         auto load_acc = [&](int c, unsigned (&r)[32]) {
-            tc_ld32(taddr + (unsigned)(c * 32), r);
+            tc_ld32(taddr + (unsigned)((parts > 1 ? p.sets * W : 0) + c * 32), r);
             tc_wait_ld();
             if constexpr (!I8) {
 #pragma unroll 1
-                for (int t = 1; t < n_sets; t++) {
+                for (int t = parts > 1 ? 0 : 1; t < filled; t++) {
                     unsigned x[32];
                     tc_ld32(taddr + (unsigned)(t * W + c * 32), x);
                     tc_wait_ld();
@@ -490,15 +551,20 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // ---- host side ----------------------------------------------------------------------------------------------------------
 struct WaveShape { int cg, R, S, tiles_m, tiles_n; };
 
+template <int CG, int MODE, bool FOLD>
+int allow_smem() {
+    static std::atomic<unsigned long long> attr_devices{0};
+    return once_per_device(attr_devices, [] {
+        B200FC_CUDA(cudaFuncSetAttribute(gemm_wave_kernel<CG, MODE, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, WAVE_SMEM));
+        return (int)B200FC_OK;
+    });
+}
+
 // Largest number of clusters of `size` CTAs (one CTA per SM) that are resident together; asked once per device.
 template <int CG, int MODE>
 int max_clusters(int size, int* out) {
     static std::atomic<int> cache[64][9];
-    static std::atomic<unsigned long long> attr_devices{0};
-    const int arc = once_per_device(attr_devices, [] {
-        B200FC_CUDA(cudaFuncSetAttribute(gemm_wave_kernel<CG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, WAVE_SMEM));
-        return (int)B200FC_OK;
-    });
+    const int arc = allow_smem<CG, MODE, false>();
     if (arc) return arc;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -514,7 +580,7 @@ int max_clusters(int size, int* out) {
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        B200FC_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_wave_kernel<CG, MODE>, &cfg));
+        B200FC_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_wave_kernel<CG, MODE, false>, &cfg));
         if (n < 1) n = -1;
         cache[dev & 63][size].store(n, std::memory_order_relaxed);
     }
@@ -533,11 +599,16 @@ int max_tiles(int S, int* out) {
 }
 
 int max_sets(int W) { return 512 / W < 8 ? 512 / W : 8; }   // accumulators of W columns in tensor memory
+// parts that `chains` chains of sums in a CTA take (one of the accumulators then holds the sum); 0 = impossible
+int parts_of(int chains, int W) {
+    const int n = max_sets(W);
+    return chains <= n ? 1 : (n < 2 ? 0 : (chains + n - 2) / (n - 1));
+}
 
 // Picks the columns per CTA and the split of K of a call that fits one wave; false = it does not.  The model counts SM
 // clocks of one CTA: per 128-byte slab the slowest of operand loads (about 48 bytes per clock and SM reach shared memory from
 // L2), MMAs (the 256-wide one takes 128 clocks per 32 bytes of K) and widening; plus the reduction and the epilogue.
-// `chains`: the number of chains that K is to be summed in, see run_wave.
+// `chains`: the number of chains that K is to be summed in at least, see k_chains.
 template <int CG, int MODE>
 int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* best, bool* found) {
     const int tiles_m = (M + BM * CG - 1) / (BM * CG);
@@ -552,7 +623,8 @@ int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* be
         for (int R = 32; R <= 256; R += 32) {
             const int W = R * CG, tiles_n = (nspan + W - 1) / W;
             if ((long long)tiles_m * tiles_n > cap) continue;
-            if (S * max_sets(W) < chains) continue;
+            const int parts = parts_of((chains + S - 1) / S, W);
+            if (!parts || (parts > 1 && MODE != W_U8C && MODE != W_U4C)) continue;    // (plain weights never need it: their chains are fewer)
             if (S > 1 && S * ((W / 32 + S - 1) / S) * CHUNK_BYTES + WORKERS * WARP_TILE_BYTES > RING_BYTES) continue;
             const double load = (rows_a * 128.0 + R * (double)wbytes) / 48.0, mma = 2.0 * W;
             const double cvt = MODE == W_U4C ? 2.2 * R : (MODE == W_U8C ? 1.4 * R : 0.0);
@@ -562,7 +634,8 @@ int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* be
             double loop = slab * ((slabs + S - 1) / S);
             if (loop < hbm) loop = hbm;
             const double red = S > 1 ? 1500.0 + W * 4.0 + W * 512.0 * (S - 1) / S / 30.0 : 0.0;
-            const double cost = loop + red + 400.0 * ((W / 32 + 2 * S - 1) / (2 * S));
+            const double fold = (parts - 1) * (300.0 + 2.0 * W);
+            const double cost = loop + red + fold + 400.0 * ((W / 32 + 2 * S - 1) / (2 * S));
             if (!*found || cost < best_cost) {
                 *found = true;
                 best_cost = cost;
@@ -573,48 +646,34 @@ int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* be
     return B200FC_OK;
 }
 
+struct WaveCall {
+    const Weight& w;
+    const void* A;
+    int M, K;
+    int64_t lda;
+    bool a_signed;
+    const Epilogue& ep;
+    cudaStream_t s;
+    int slabs, units, chains;
+};
+
 template <int CG, int MODE>
-int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const float* scale_grp, const void* A, int M, int K,
-             int64_t lda, int n0, int n1, unsigned a_signed, unsigned w_signed, const Epilogue& ep, cudaStream_t s) {
+int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
     constexpr bool I8 = MODE == W_I8, WQ = MODE == W_U8C || MODE == W_U4C;
     constexpr int SPU = MODE == W_U8C ? 2 : (MODE == W_U4C ? 4 : 1);
+    const Epilogue& ep = call.ep;
+    const int64_t w_ld = call.w.ld_bytes();
+    const bool w_signed = call.w.dtype == B200FC_S8;
     WaveParams p = {};
-    const int slab_elems = I8 ? SLAB_BYTES : SLAB_BYTES / 2;
-    p.slabs = (K + slab_elems - 1) / slab_elems;
-    p.units = (p.slabs + SPU - 1) / SPU;
-    if (MODE == W_U4C) p.units = (int)(w_ld / SLAB_BYTES);     // (the group scales are laid out by it)
-    WaveShape sh;
-    bool found = false;
-    // The tensor core's error grows with the length of a chain of fp32 sums (256 x 4096 x 4096, relative to float64: 1.08e-6 in three
-    // chains, 7.9e-7 in four, 5.1e-7 in six).  K is cut into as many chains as gemm_tc.cu's split of the same call has, counting the parts of the
-    // cluster and, inside a CTA, accumulators that the slabs take in turn.
-    int chains = 1;
-    if (!I8) {
-        int span = n1 - n0;
-        const int blk = (int)(((size_t)32 << 20) / ((size_t)W_K_pad * 2)) / kRowPad * kRowPad;    // columns of a widened block there
-        if (WQ && span > blk) span = blk < kRowPad ? kRowPad : blk;
-        const int tiles = (M + 2 * BM - 1) / (2 * BM) * ((span + 255) / 256), pairs = num_sms() / 2;
-        if (tiles * 2 <= pairs && p.slabs >= 16) {
-            chains = pairs / tiles < 8 ? pairs / tiles : 8;
-            if (chains > p.slabs / 8) chains = p.slabs / 8;
-        }
-    }
-    // A shape that cannot have them is out where the difference can be seen: not behind the rounding of bf16 and int8 outputs or of
-    // 4-bit weights (1e-3 and more).
-    const bool seen = ep.out_dtype == B200FC_F32 && MODE != W_U4C;
-    int rc = pick_shape<CG, MODE>(M, n1 - n0, p.slabs, p.units, seen ? chains : 1, &sh, &found);
-    if (rc) return rc;
-    if (!found) return B200FC_ERR_UNSUPPORTED;
-    // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256
-    // 46.8 / 42.7, 250 x 2784 x 14928 27.6 / 26.7)
-    if (!WQ && CG == 2 && sh.S == 1 && sh.R == 128 && 4 * sh.tiles_m * sh.tiles_n > num_sms()) return B200FC_ERR_UNSUPPORTED;
-    p.M = M; p.n0 = n0; p.n1 = n1; p.n_pad = W_N_pad;
+    p.slabs = call.slabs; p.units = call.units;
+    p.M = call.M; p.n0 = n0; p.n1 = n1; p.n_pad = call.w.N_pad;
     p.R = sh.R; p.S = sh.S; p.tiles_m = sh.tiles_m;
-    p.sets = (chains + sh.S - 1) / sh.S;
-    if (p.sets > max_sets(CG * sh.R)) p.sets = max_sets(CG * sh.R);
+    const int chains = (call.chains + sh.S - 1) / sh.S;
+    p.parts = parts_of(chains, CG * sh.R);
+    p.sets = (chains + p.parts - 1) / p.parts;
     p.R0 = CG == 2 && sh.R > 128 ? (sh.R / 2 + 31) / 32 * 32 : sh.R;
-    p.idesc0 = make_idesc(I8, a_signed, w_signed, CG * p.R0, CG * BM);
-    p.idesc1 = make_idesc(I8, a_signed, w_signed, CG * (p.R - p.R0), CG * BM);
+    p.idesc0 = make_idesc(I8, call.a_signed, w_signed, CG * p.R0, CG * BM);
+    p.idesc1 = make_idesc(I8, call.a_signed, w_signed, CG * (p.R - p.R0), CG * BM);
     const int a_bytes = BM * SLAB_BYTES, w_bytes = sh.R * SLAB_BYTES;
     if (WQ) {
         // three widened slabs (more measured no faster); stored pieces for six slabs and more ahead (HBM latency); the rest
@@ -629,7 +688,7 @@ int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const f
     }
     if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
     p.ep = ep;
-    p.scale_grp = scale_grp;
+    p.scale_grp = call.w.scale_grp;
     p.status = kernel_status_word();
     if (!p.status) { set_error("gemm: no kernel status word on this device"); return B200FC_ERR_CUDA; }
     p.wait_limit_ns = wait_limit_ns();
@@ -638,16 +697,16 @@ int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const f
     p.vec_ok = c_aligned && ((ep.steps & B200FC_STEP_SILU_MUL) ? (n0 % 32) == 0 : ((n0 * es) & 15) == 0) ? 1 : 0;
 
     CUtensorMap ma, mw;
-    rc = make_map(&ma, A, I8, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BM);
+    int rc = make_map(&ma, call.A, I8, (uint64_t)call.K, (uint64_t)call.M, (uint64_t)call.lda, BM);
     if (rc) return rc;
-    if (WQ) rc = make_map(&mw, W_data, true, (uint64_t)w_ld, (uint64_t)W_N_pad, (uint64_t)w_ld, (uint32_t)p.R);
-    else rc = make_map(&mw, W_data, I8, (uint64_t)W_K_pad, (uint64_t)W_N_pad, (uint64_t)w_ld, (uint32_t)p.R);
+    rc = WQ ? make_map(&mw, call.w.data, true, (uint64_t)w_ld, (uint64_t)call.w.N_pad, (uint64_t)w_ld, (uint32_t)p.R)
+            : make_map(&mw, call.w.data, I8, (uint64_t)call.w.K_pad, (uint64_t)call.w.N_pad, (uint64_t)w_ld, (uint32_t)p.R);
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CG * sh.S * sh.tiles_m * sh.tiles_n), 1, 1);
     cfg.blockDim = dim3(WAVE_THREADS, 1, 1);
     cfg.dynamicSmemBytes = WAVE_SMEM;
-    cfg.stream = s;
+    cfg.stream = call.s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -656,9 +715,81 @@ int run_wave(const void* W_data, int64_t w_ld, int W_K_pad, int W_N_pad, const f
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_wave_kernel<CG, MODE>, ma, mw, p));
+    if (p.parts == 1) {
+        B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_wave_kernel<CG, MODE, false>, ma, mw, p));
+    } else if constexpr (WQ) {
+        rc = allow_smem<CG, MODE, true>();
+        if (rc) return rc;
+        B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_wave_kernel<CG, MODE, true>, ma, mw, p));
+    }
     count_launch();
     return B200FC_OK;
+}
+
+// The tensor core's error grows with the length of a chain of fp32 sums (256 x 4096 x 4096, relative to float64: 1.08e-6 in three
+// chains, 7.9e-7 in four, 5.1e-7 in six).  K is cut into at least as many chains as launch_gemm_tc cuts it into.  For quantised weights
+// that is a number for each block of rows that would be widened in front of it (fewer columns, more parts): the error
+// of the whole result, as the root mean square of 1 / chains, must not be larger.
+int k_chains(const Weight& w, int M, int K, int n0, int n1) {
+    if (!w.compressed) return gemm_tc_chains(M, K, n1 - n0);
+    const int blk = widened_block_rows(w.K_pad);
+    double sum = 0.0;
+    for (int r0 = n0 / kRowPad * kRowPad; r0 < n1; r0 += blk) {
+        const int cols = (r0 + blk < n1 ? r0 + blk : n1) - (r0 > n0 ? r0 : n0), c = gemm_tc_chains(M, K, cols);
+        sum += (double)cols / (c * c);
+    }
+    int chains = 1;
+    while ((double)(n1 - n0) / (chains * chains) > sum * 1.000001) chains++;
+    return chains;
+}
+
+template <int MODE>
+int plan_wave(const WaveCall& c, int nspan, int chains, WaveShape* sh, bool* found) {
+    *found = false;
+    int rc = B200FC_OK;
+    if (c.M > BM) rc = pick_shape<2, MODE>(c.M, nspan, c.slabs, c.units, chains, sh, found);
+    // One wave of pair tiles wider than 256 columns fills tensor memory and has no place for a second accumulator.  Single-CTA tiles
+    // of half the rows and columns do, where one wave of them suffices; they cost a quantised weight little more, since the
+    // widening of 256 rows bounds either (4 bits 300 x 4096 x 11008 in three chains: 61 us, in two halves of pair tiles 93; 51 in
+    // one chain).
+    if (!rc && !*found && (c.M <= BM || MODE == W_U8C || MODE == W_U4C))
+        rc = pick_shape<1, MODE>(c.M, nspan, c.slabs, c.units, chains, sh, found);
+    return rc;
+}
+
+template <int MODE>
+int run_wave(WaveCall& c, int n0, int n1) {
+    constexpr bool WQ = MODE == W_U8C || MODE == W_U4C;
+    constexpr int SPU = MODE == W_U8C ? 2 : (MODE == W_U4C ? 4 : 1);
+    const int slab_elems = MODE == W_I8 ? SLAB_BYTES : SLAB_BYTES / 2;
+    c.slabs = (c.K + slab_elems - 1) / slab_elems;
+    c.units = MODE == W_U4C ? (int)(c.w.ld_bytes() / SLAB_BYTES) : (c.slabs + SPU - 1) / SPU;     // (the group scales are laid out by it)
+    auto launch = [&](const WaveShape& sh, int a, int b) { return sh.cg == 1 ? run_wave<1, MODE>(c, sh, a, b) : run_wave<2, MODE>(c, sh, a, b); };
+    WaveShape sh;
+    bool found = false;
+    int rc = plan_wave<MODE>(c, n1 - n0, c.chains, &sh, &found);
+    if (rc) return rc;
+    if (found) {
+        // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256
+        // 46.8 / 42.7, 250 x 2784 x 14928 27.6 / 26.7)
+        if (!WQ && sh.cg == 2 && sh.S == 1 && sh.R == 128 && 4 * sh.tiles_m * sh.tiles_n > num_sms()) return B200FC_ERR_UNSUPPORTED;
+        return launch(sh, n0, n1);
+    }
+    if (!WQ || c.chains == 1) return B200FC_ERR_UNSUPPORTED;
+    // One wave but for the number of chains: two halves, each a wave of narrower tiles (4 bits 651 x 7680 x 12160: 159 us in
+    // three chains, 96 in one, 275 through widened blocks)
+    rc = plan_wave<MODE>(c, n1 - n0, 1, &sh, &found);
+    if (rc) return rc;
+    const int mid = (int)(((long long)n0 + n1 + 2 * kRowPad - 1) / (2 * kRowPad)) * kRowPad;
+    if (!found || mid <= n0 || mid >= n1) return B200FC_ERR_UNSUPPORTED;
+    WaveShape half[2];
+    for (int h = 0; h < 2; h++) {
+        rc = plan_wave<MODE>(c, h ? n1 - mid : mid - n0, c.chains, &half[h], &found);
+        if (rc) return rc;
+        if (!found) return B200FC_ERR_UNSUPPORTED;
+    }
+    rc = launch(half[0], n0, mid);
+    return rc ? rc : launch(half[1], mid, n1);
 }
 
 }  // namespace
@@ -671,15 +802,9 @@ int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, i
     if (enabled < 0) { const char* e = getenv("B200FC_GEMM_WAVE"); enabled = (e ? atoi(e) : 1) && !gemm_forced_ctas(); }
     if (!enabled) return B200FC_ERR_UNSUPPORTED;
     const bool a8 = dtypeA != B200FC_BF16;
-    const unsigned as = dtypeA == B200FC_S8, ws = w.dtype == B200FC_S8;
-#define B200FC_WAVE(CG, MODE) run_wave<CG, MODE>(w.data, w.ld_bytes(), w.K_pad, w.N_pad, w.scale_grp, A, M, K, lda, n0, n1, as, ws, ep, s)
-    if (w.compressed) {
-        if (w.dtype == B200FC_S4) return M <= BM ? B200FC_WAVE(1, W_U4C) : B200FC_WAVE(2, W_U4C);
-        return M <= BM ? B200FC_WAVE(1, W_U8C) : B200FC_WAVE(2, W_U8C);
-    }
-    if (a8) return M <= BM ? B200FC_WAVE(1, W_I8) : B200FC_WAVE(2, W_I8);
-    return M <= BM ? B200FC_WAVE(1, W_BF16) : B200FC_WAVE(2, W_BF16);
-#undef B200FC_WAVE
+    WaveCall c{w, A, M, K, lda, dtypeA == B200FC_S8, ep, s, 0, 0, a8 ? 1 : k_chains(w, M, K, n0, n1)};   // (sums of 8-bit products are exact)
+    if (w.compressed) return w.dtype == B200FC_S4 ? run_wave<W_U4C>(c, n0, n1) : run_wave<W_U8C>(c, n0, n1);
+    return a8 ? run_wave<W_I8>(c, n0, n1) : run_wave<W_BF16>(c, n0, n1);
 }
 
 }  // namespace b200fc

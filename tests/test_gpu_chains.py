@@ -1,0 +1,81 @@
+"""GPU: the one-wave GEMM sums K in no longer chains than the persistent kernel with its split of K does for the same call.
+
+The tensor core's error grows with the length of a chain of fp32 sums.  Both are run on the same ordinary values (the persistent
+kernel in a child process with B200FC_GEMM_WAVE=0) and compared with float64, in fp32 and, behind a bias that cancels the result, in
+bf16: there the rounding of the output no longer hides the sums.  4-bit weights have power-of-two scales, so that value x scale is
+exact in bf16.  All values are positive, which makes the error proportional to the length of the chains.
+"""
+import json
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    ("int8", 35, 6400, 21104),    # more chains than accumulators fit beside 160-column tiles
+    ("int8", 153, 6496, 4352),    # pair form; the widened blocks have different numbers of chains
+    ("int8", 256, 4096, 16384),   # 256-column tiles: one accumulator and the sum
+    ("int4", 202, 7360, 8320),
+    ("int4", 300, 4096, 11008),   # single-CTA tiles although there are more than 128 rows
+    ("int4", 651, 7680, 12160),   # two halves
+    ("int4", 60, 11008, 16384),   # the cluster's parts of K have several chains each
+    ("bf16", 256, 4096, 4096),
+]
+
+CODE = textwrap.dedent("""
+    import json, sys
+    import torch
+    from mm_amx_b200 import capi
+    res = []
+    for kind, M, K, N in json.loads(sys.argv[1]):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(K + N)
+        A = torch.randn((M, K), generator=g, device="cuda").abs().to(torch.bfloat16)
+        steps = 0 if kind == "bf16" else capi.STEP_DEQUANT
+        if kind == "int8":
+            B = torch.randint(1, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+            one = torch.ones(N, device="cuda")
+            w = capi.Weight(B.data_ptr(), capi.S8, K, N, K, True, capi.PACK_INT8_CHANNEL, one.data_ptr())
+        else:
+            if kind == "int4":
+                B = torch.randint(1, 8, (N, K), generator=g, device="cuda").float()
+                B[:, ::128] = 7
+                B = (B / 64).to(torch.bfloat16)
+            else:
+                B = torch.randn((N, K), generator=g, device="cuda").abs().to(torch.bfloat16)
+            w = capi.Weight(B.data_ptr(), capi.BF16, K, N, 2 * K, True, capi.PACK_INT4_GROUP if kind == "int4" else capi.PACK_PLAIN)
+        def call(A, out, code, steps, bias=None):
+            ep = capi.make_epilogue(out.data_ptr(), N * out.element_size(), code, steps, bias.data_ptr() if bias is not None else None)
+            w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep)
+            capi.sync_check()
+            return out.double()
+        ref = torch.cat([A.double() @ B[i:i + 2048].double().t() for i in range(0, N, 2048)], 1)
+        c = call(A, torch.empty((M, N), device="cuda"), capi.F32, steps)
+        same = A[:1].expand(M, K).contiguous()                  # all rows alike: one bias per column cancels them
+        bias = -ref[0].float()
+        r = call(same, torch.empty((M, N), dtype=torch.bfloat16, device="cuda"), capi.BF16, steps | capi.STEP_BIAS, bias)
+        r -= ref[0] + bias.double()
+        res.append([float((c - ref).norm() / ref.norm()), float(r.norm() / (ref[0].norm() * M ** 0.5))])
+    print("errors", json.dumps(res))
+""")
+
+
+def errors(**switches):
+    env = dict(os.environ, **switches)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env["PYTHONPATH"] = os.pathsep.join([root, env.get("PYTHONPATH", "")])
+    r = subprocess.run([sys.executable, "-c", CODE, json.dumps(SHAPES)], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return json.loads(r.stdout.split("errors", 1)[1])
+
+
+def test_chains_are_no_longer_than_with_the_split_of_k_subprocess():
+    for shape, wave, split in zip(SHAPES, errors(), errors(B200FC_GEMM_WAVE="0")):
+        for what, e, bound in zip(("fp32", "bf16"), wave, split):
+            # 5 %: the chains end at other slabs of K and are added in another order; one chain fewer of eight is 14 %
+            assert e <= 1.05 * bound, (shape, what, e, bound)
+            assert bound < 4e-6, (shape, what, bound)           # (that is, the persistent kernel did split K)
