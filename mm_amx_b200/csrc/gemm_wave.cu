@@ -53,9 +53,12 @@ struct WaveParams {
     unsigned long long wait_limit_ns;
 };
 
-// Arrival of a widening warp on the leader's barrier.  No cluster-scope release: the data was handed to the async proxy by a
-// proxy fence before, which is what the MMA reads through; a release at cluster scope is a full memory barrier of the warp at
-// every slab (4 bits, 100 x 4096 x 11008: 36.7 us with it, 26.6 without).
+// Arrival of a widening warp of the second CTA on the leader's barrier.  The bytes are handed over by the warp's proxy fence, which orders
+// them before what the async proxy reads from then on, and the MMA that reads them is issued behind the leader's wait, which
+// acquires at cluster scope.  The arrival itself has the default (CTA) scope: the form that CUTLASS has for the same hand-over
+// of transformed operands to a two-CTA MMA (ClusterBarrier::arrive(cta_id) behind fence_view_async_shared).  A release at cluster
+// scope is a full memory barrier at every slab: in each widening warp 36.7 us for 4 bits, 100 x 4096 x 11008 (26.6 without); in one
+// forwarding warp of the second CTA 38.1 us for int8, 705 x 2560 x 10240 (32.1) and 157 us for 300 x 11008 x 8192 (100).
 __device__ __forceinline__ void mbar_arrive_leader(unsigned cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -200,14 +203,14 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const unsigned ring = smem_u32(smem), wring = smem_u32(wide_ring);
             for (int i = 0; i < n_slabs; i++) {
                 if (FOLD && i == end) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_folded, (unsigned)part & 1, abort_flag, p.wait_limit_ns))) break;
+                    if (!__all_sync(0xffffffffu, mbar_wait<0, CG == 2>(bar_folded, (unsigned)part & 1, abort_flag, p.wait_limit_ns))) break;
                     part++;
                     start = end;
                     end = n_slabs * (part + 1) / parts;
                     set = 0;
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * slot, phase, abort_flag, p.wait_limit_ns))) break;
-                if (WQ && !__all_sync(0xffffffffu, mbar_wait(bar_wide_full + 8 * wslot, wphase, abort_flag, p.wait_limit_ns))) break;
+                if (WQ && !__all_sync(0xffffffffu, mbar_wait<0, CG == 2>(bar_wide_full + 8 * wslot, wphase, abort_flag, p.wait_limit_ns))) break;
                 tc_fence_after();
                 const unsigned sa = ring + (unsigned)(slot * stage_bytes);
                 const unsigned sb = WQ ? wring + (unsigned)(wslot * w_bytes) : sa + A_BYTES;

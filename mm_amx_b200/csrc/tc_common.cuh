@@ -36,30 +36,42 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// CLUSTER: acquires at cluster scope, for a phase that arrivals of another CTA of the cluster complete
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
     unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if constexpr (CLUSTER) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    }
     return ok != 0;
 }
 // Bounded wait.  Returns false when the CTA is aborting (this wait or another role's ran out of time).
 // The clock and the abort flag are looked at after a batch of failed attempts only (try_wait itself suspends the thread for a while).
 // SLEEP_NS > 0: back off between polls (for waits that are long and not latency critical: the epilogue warps wait most
 // of a tile's main loop, and five spinning warps cost issue slots and power that the tensor pipe could use).
-template <int SLEEP_NS = 0>
+template <int SLEEP_NS = 0, bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int* abort_flag, unsigned long long limit) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     unsigned long long t0 = 0;
     while (true) {
 #pragma unroll 1
         for (int i = 0; i < 16; i++) {
             if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
-            if (mbar_try_wait(bar, parity)) return true;
+            if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         }
         if (*abort_flag) return false;
         const unsigned long long now = globaltimer();

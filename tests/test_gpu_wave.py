@@ -73,3 +73,31 @@ def test_column_range_leaves_the_rest_alone(M, K, N, n0, n1):
     assert np.array_equal(got[:, n0:n1], port.gemm_bf16_w8(x, B, transposeB=True)[:, n0:n1])
     rest = np.delete(got, np.s_[n0:n1], axis=1).view(np.uint32)
     assert (rest == 0xCDCDCDCD).all()
+
+
+@pytest.mark.parametrize("M,K,N", [(200, 4096, 8192), (705, 2560, 10240), (300, 8192, 4096)])
+@pytest.mark.parametrize("kind", ["int8_compressed", "int4"])
+def test_pair_form_repeats_bit_for_bit(kind, M, K, N):
+    """slabs widened by one CTA of a pair are multiplied by the other: every one of 100 launches gives the same bits, with the weights and
+    activations out of the caches in every other one"""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    A = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    if kind == "int4":
+        B = (torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+        w = capi.Weight(B.data_ptr(), capi.BF16, K, N, 2 * K, True, capi.PACK_INT4_GROUP)
+    else:
+        B = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+        one = torch.ones(N, device="cuda")
+        w = capi.Weight(B.data_ptr(), capi.S8, K, N, K, True, capi.PACK_INT8_CHANNEL, one.data_ptr())
+    flush = torch.empty(64 << 20, dtype=torch.int32, device="cuda")
+    first = None
+    for i in range(100):
+        C = torch.full((M, N), float("nan"), device="cuda")
+        if i & 1:
+            flush.fill_(i)
+        w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, capi.make_epilogue(C.data_ptr(), 4 * N, capi.F32, capi.STEP_DEQUANT))
+        first = C if first is None else first
+        assert torch.equal(C, first), i
+    capi.sync_check()
