@@ -78,12 +78,19 @@ struct ScratchKey {
 };
 static std::map<ScratchKey, Scratch> g_scratch;
 
-int get_stream_scratch(size_t bytes, cudaStream_t s, int slot, void** out) {
+int get_stream_scratch(size_t bytes, cudaStream_t s, int slot, void** out, bool* own) {
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(g_mu);
     Scratch& sc = g_scratch[ScratchKey{dev, s, slot}];
+    if (own) *own = false;
     if (sc.bytes < bytes) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (own && cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive) {
+            B200FC_CUDA(cudaMallocAsync(out, bytes, s));
+            *own = true;
+            return B200FC_OK;
+        }
         if (sc.p) { cudaStreamSynchronize(s); cudaFree(sc.p); sc.p = nullptr; sc.bytes = 0; }
         B200FC_CUDA(cudaMalloc(&sc.p, bytes));
         sc.bytes = bytes;

@@ -43,6 +43,7 @@ struct WaveParams {
     int R, R0;              // weight rows (= output columns) per CTA; of the first MMA of a K step
     int tiles_m, S;
     int parts, sets;        // parts of a CTA's K, and accumulators that the slabs of a part take in turn (W columns of tensor memory each)
+    char* sums;             // what the parts but the last add up to: a tile of 128 rows x W columns per CTA, or null (one part)
     int slabs, units;       // K in 128-byte slabs of the MMA operands / in 128-byte pieces of the stored weight rows
     int slots, raw_slots, wide_slots;
     unsigned idesc0, idesc1;
@@ -73,9 +74,11 @@ __device__ __forceinline__ unsigned nib2_to_bf16x2_scaled(unsigned w, float scal
 }
 
 // FOLD: K in several parts, see below (quantised weights).  A kernel of its own, because the folding code costs the widening loop
-// registers and instruction cache also where it does not run (int8 705 x 2560 x 10240: 44.8 us with it, 42.3 without).  A fold
-// costs about 2 us, most of it reading tensor memory (500 clocks per 32 columns and accumulator): int8 35 x 6400 x 21104 in three
-// chains 61 us, in eight 74; through widened blocks and a split of K 285.
+// registers and instruction cache also where it does not run (int8 705 x 2560 x 10240: 44.8 us with it, 42.3 without).  Calls whose
+// chains do not fit pay for both (us, one chain / as many as asked for / through widened blocks and a split of K): 4 bits
+// 512 x 4096 x 11008 42 / 61 / 127 (two folds), int8 705 x 4096 x 10240 45 / 58 / 126 (one fold, 6.5 of it, of which the workers read
+// tensor memory at 500 clocks per 32 columns), int8 300 x 11008 x 8192 75 / 103 / 249 (13 are the slower loop).  No gain: folding
+// each chain by itself under the next one, adding with red instead of load and store, the fold as a function that is called.
 template <int CG, int MODE, bool FOLD>
 __global__ void __launch_bounds__(WAVE_THREADS, 1)
 gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const WaveParams p) {
@@ -109,8 +112,8 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int u0 = (int)((long long)p.units * split / p.S), u1 = (int)((long long)p.units * (split + 1) / p.S);
     const int n_units = u1 - u0, n_slabs = min(u1 * SPU, p.slabs) - u0 * SPU;
     // K in chains of fp32 sums: the slabs take the accumulators in turn.  Where tensor memory holds too few of them K is cut into parts
-    // as well, after each of which (but the last) the workers fold the accumulators into a sum, behind them in tensor memory.
-    const int parts = FOLD ? min(p.parts, n_slabs) : 1, cols = (p.sets + (parts > 1 ? 1 : 0)) * W;
+    // as well, after each of which (but the last) the workers add the accumulators to a sum in global memory (L2).
+    const int parts = FOLD ? min(p.parts, n_slabs) : 1, cols = p.sets * W;
     const unsigned tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
 
     if (threadIdx.x == 0) {
@@ -280,7 +283,19 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int quarter = warp & 3, third = wi >> 2;
         const int chunks = W / 32;
         const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16);
-        // the accumulators of a part, once its MMAs are done, into the sum: fp32 adds in order, the columns shared out as in the epilogue
+        // this thread's row of a chunk's sums: eight 16-byte units, one per four columns; only this thread reads and writes them
+        auto sums_of = [&](int c) {
+            return (uint4*)(p.sums + ((size_t)blockIdx.x * chunks + c) * CHUNK_BYTES) + quarter * 32 + lane;
+        };
+        auto load_sums = [&](int c, unsigned (&r)[32]) {
+            const uint4* src = sums_of(c);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const uint4 v = __ldcg(src + j * BM);
+                r[4 * j] = v.x; r[4 * j + 1] = v.y; r[4 * j + 2] = v.z; r[4 * j + 3] = v.w;
+            }
+        };
+        // the accumulators of a part, once its MMAs are done, into the sums: fp32 adds in order, the columns shared out as in the epilogue
         const unsigned folded_leader = CG == 2 ? mapa_rank(bar_folded, leader_rank) : bar_folded;
         int folds = 0;
         auto fold_part = [&]() {
@@ -291,7 +306,12 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll 1
             for (int c = third; c < chunks; c += SETS) {
                 unsigned sum[32], x[32];
-                tc_ld32(taddr + (unsigned)((folds ? p.sets * W : 0) + c * 32), sum);
+                if (folds) {
+                    load_sums(c, sum);
+                } else {
+                    tc_ld32(taddr + (unsigned)(c * 32), sum);
+                    tc_wait_ld();
+                }
 #pragma unroll 1
                 for (int t = folds ? 0 : 1; t < filled; t++) {
                     tc_ld32(taddr + (unsigned)(t * W + c * 32), x);
@@ -299,10 +319,10 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < 32; j++) sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(x[j]));
                 }
-                tc_wait_ld();
-                tc_st32(taddr + (unsigned)(p.sets * W + c * 32), sum);
+                uint4* dst = sums_of(c);
+#pragma unroll
+                for (int j = 0; j < 8; j++) __stcg(dst + j * BM, make_uint4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]));
             }
-            tc_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -433,11 +453,15 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         };
         // every load of the ring has landed and every MMA has read it: the ring is free
         unsigned* stage_tile = (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES);
-        // columns [32 c, +32) of this CTA's result: the sum of the folded parts, if any, and the last part's accumulators in order
+        // columns [32 c, +32) of this CTA's result: the sums of the folded parts, if any, and the last part's accumulators in order
         const int filled = min(p.sets, n_slabs - n_slabs * (parts - 1) / parts);
         auto load_acc = [&](int c, unsigned (&r)[32]) {
-            tc_ld32(taddr + (unsigned)((parts > 1 ? p.sets * W : 0) + c * 32), r);
-            tc_wait_ld();
+            if (FOLD && parts > 1) {
+                load_sums(c, r);
+            } else {
+                tc_ld32(taddr + (unsigned)(c * 32), r);
+                tc_wait_ld();
+            }
             if constexpr (!I8) {
 #pragma unroll 1
                 for (int t = parts > 1 ? 0 : 1; t < filled; t++) {
@@ -602,11 +626,8 @@ int max_tiles(int S, int* out) {
 }
 
 int max_sets(int W) { return 512 / W < 8 ? 512 / W : 8; }   // accumulators of W columns in tensor memory
-// parts that `chains` chains of sums in a CTA take (one of the accumulators then holds the sum); 0 = impossible
-int parts_of(int chains, int W) {
-    const int n = max_sets(W);
-    return chains <= n ? 1 : (n < 2 ? 0 : (chains + n - 2) / (n - 1));
-}
+// parts that `chains` chains of sums in a CTA take
+int parts_of(int chains, int W) { return (chains + max_sets(W) - 1) / max_sets(W); }
 
 // Picks the columns per CTA and the split of K of a call that fits one wave; false = it does not.  The model counts SM
 // clocks of one CTA: per 128-byte slab the slowest of operand loads (about 48 bytes per clock and SM reach shared memory from
@@ -627,7 +648,7 @@ int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* be
             const int W = R * CG, tiles_n = (nspan + W - 1) / W;
             if ((long long)tiles_m * tiles_n > cap) continue;
             const int parts = parts_of((chains + S - 1) / S, W);
-            if (!parts || (parts > 1 && MODE != W_U8C && MODE != W_U4C)) continue;    // (plain weights never need it: their chains are fewer)
+            if (parts > 1 && MODE != W_U8C && MODE != W_U4C) continue;    // (plain weights never need it: their chains are fewer)
             if (S > 1 && S * ((W / 32 + S - 1) / S) * CHUNK_BYTES + WORKERS * WARP_TILE_BYTES > RING_BYTES) continue;
             const double load = (rows_a * 128.0 + R * (double)wbytes) / 48.0, mma = 2.0 * W;
             const double cvt = MODE == W_U4C ? 2.2 * R : (MODE == W_U8C ? 1.4 * R : 0.0);
@@ -637,7 +658,7 @@ int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* be
             double loop = slab * ((slabs + S - 1) / S);
             if (loop < hbm) loop = hbm;
             const double red = S > 1 ? 1500.0 + W * 4.0 + W * 512.0 * (S - 1) / S / 30.0 : 0.0;
-            const double fold = (parts - 1) * (300.0 + 2.0 * W);
+            const double fold = (parts - 1) * (600.0 + 4.0 * W);
             const double cost = loop + red + fold + 400.0 * ((W / 32 + 2 * S - 1) / (2 * S));
             if (!*found || cost < best_cost) {
                 *found = true;
@@ -674,6 +695,14 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
     const int chains = (call.chains + sh.S - 1) / sh.S;
     p.parts = parts_of(chains, CG * sh.R);
     p.sets = (chains + p.parts - 1) / p.parts;
+    const int grid = CG * sh.S * sh.tiles_m * sh.tiles_n;
+    bool own_sums = false;
+    if (p.parts > 1) {
+        // the workspace of the split of K in gemm_tc.cu, which this takes the place of; memory of the graph where the stream is being
+        // captured and has none that is large enough
+        int rc = get_stream_scratch((size_t)grid * (CG * sh.R / 32) * CHUNK_BYTES, call.s, 1, (void**)&p.sums, &own_sums);
+        if (rc) return rc;
+    }
     p.R0 = CG == 2 && sh.R > 128 ? (sh.R / 2 + 31) / 32 * 32 : sh.R;
     p.idesc0 = make_idesc(I8, call.a_signed, w_signed, CG * p.R0, CG * BM);
     p.idesc1 = make_idesc(I8, call.a_signed, w_signed, CG * (p.R - p.R0), CG * BM);
@@ -706,7 +735,7 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
             : make_map(&mw, call.w.data, I8, (uint64_t)call.w.K_pad, (uint64_t)call.w.N_pad, (uint64_t)w_ld, (uint32_t)p.R);
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(CG * sh.S * sh.tiles_m * sh.tiles_n), 1, 1);
+    cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(WAVE_THREADS, 1, 1);
     cfg.dynamicSmemBytes = WAVE_SMEM;
     cfg.stream = call.s;
@@ -724,6 +753,7 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
         rc = allow_smem<CG, MODE, true>();
         if (rc) return rc;
         B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_wave_kernel<CG, MODE, true>, ma, mw, p));
+        if (own_sums) B200FC_CUDA(cudaFreeAsync(p.sums, call.s));
     }
     count_launch();
     return B200FC_OK;
@@ -747,52 +777,22 @@ int k_chains(const Weight& w, int M, int K, int n0, int n1) {
 }
 
 template <int MODE>
-int plan_wave(const WaveCall& c, int nspan, int chains, WaveShape* sh, bool* found) {
-    *found = false;
-    int rc = B200FC_OK;
-    if (c.M > BM) rc = pick_shape<2, MODE>(c.M, nspan, c.slabs, c.units, chains, sh, found);
-    // One wave of pair tiles wider than 256 columns fills tensor memory and has no place for a second accumulator.  Single-CTA tiles
-    // of half the rows and columns do, where one wave of them suffices; they cost a quantised weight little more, since the
-    // widening of 256 rows bounds either (4 bits 300 x 4096 x 11008 in three chains: 61 us, in two halves of pair tiles 93; 51 in
-    // one chain).
-    if (!rc && !*found && (c.M <= BM || MODE == W_U8C || MODE == W_U4C))
-        rc = pick_shape<1, MODE>(c.M, nspan, c.slabs, c.units, chains, sh, found);
-    return rc;
-}
-
-template <int MODE>
 int run_wave(WaveCall& c, int n0, int n1) {
     constexpr bool WQ = MODE == W_U8C || MODE == W_U4C;
     constexpr int SPU = MODE == W_U8C ? 2 : (MODE == W_U4C ? 4 : 1);
     const int slab_elems = MODE == W_I8 ? SLAB_BYTES : SLAB_BYTES / 2;
     c.slabs = (c.K + slab_elems - 1) / slab_elems;
     c.units = MODE == W_U4C ? (int)(c.w.ld_bytes() / SLAB_BYTES) : (c.slabs + SPU - 1) / SPU;     // (the group scales are laid out by it)
-    auto launch = [&](const WaveShape& sh, int a, int b) { return sh.cg == 1 ? run_wave<1, MODE>(c, sh, a, b) : run_wave<2, MODE>(c, sh, a, b); };
     WaveShape sh;
     bool found = false;
-    int rc = plan_wave<MODE>(c, n1 - n0, c.chains, &sh, &found);
+    const int rc = c.M <= BM ? pick_shape<1, MODE>(c.M, n1 - n0, c.slabs, c.units, c.chains, &sh, &found)
+                             : pick_shape<2, MODE>(c.M, n1 - n0, c.slabs, c.units, c.chains, &sh, &found);
     if (rc) return rc;
-    if (found) {
-        // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256
-        // 46.8 / 42.7, 250 x 2784 x 14928 27.6 / 26.7)
-        if (!WQ && sh.cg == 2 && sh.S == 1 && sh.R == 128 && 4 * sh.tiles_m * sh.tiles_n > num_sms()) return B200FC_ERR_UNSUPPORTED;
-        return launch(sh, n0, n1);
-    }
-    if (!WQ || c.chains == 1) return B200FC_ERR_UNSUPPORTED;
-    // One wave but for the number of chains: two halves, each a wave of narrower tiles (4 bits 651 x 7680 x 12160: 159 us in
-    // three chains, 96 in one, 275 through widened blocks)
-    rc = plan_wave<MODE>(c, n1 - n0, 1, &sh, &found);
-    if (rc) return rc;
-    const int mid = (int)(((long long)n0 + n1 + 2 * kRowPad - 1) / (2 * kRowPad)) * kRowPad;
-    if (!found || mid <= n0 || mid >= n1) return B200FC_ERR_UNSUPPORTED;
-    WaveShape half[2];
-    for (int h = 0; h < 2; h++) {
-        rc = plan_wave<MODE>(c, h ? n1 - mid : mid - n0, c.chains, &half[h], &found);
-        if (rc) return rc;
-        if (!found) return B200FC_ERR_UNSUPPORTED;
-    }
-    rc = launch(half[0], n0, mid);
-    return rc ? rc : launch(half[1], mid, n1);
+    if (!found) return B200FC_ERR_UNSUPPORTED;
+    // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256
+    // 46.8 / 42.7, 250 x 2784 x 14928 27.6 / 26.7)
+    if (!WQ && sh.cg == 2 && sh.S == 1 && sh.R == 128 && 4 * sh.tiles_m * sh.tiles_n > num_sms()) return B200FC_ERR_UNSUPPORTED;
+    return sh.cg == 1 ? run_wave<1, MODE>(c, sh, n0, n1) : run_wave<2, MODE>(c, sh, n0, n1);
 }
 
 }  // namespace

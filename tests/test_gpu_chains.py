@@ -18,10 +18,10 @@ pytestmark = pytest.mark.gpu
 SHAPES = [
     ("int8", 35, 6400, 21104),    # more chains than accumulators fit beside 160-column tiles
     ("int8", 153, 6496, 4352),    # pair form; the widened blocks have different numbers of chains
-    ("int8", 256, 4096, 16384),   # 256-column tiles: one accumulator and the sum
+    ("int8", 256, 4096, 16384),   # pair form, two accumulators
     ("int4", 202, 7360, 8320),
-    ("int4", 300, 4096, 11008),   # single-CTA tiles although there are more than 128 rows
-    ("int4", 651, 7680, 12160),   # two halves
+    ("int4", 300, 4096, 11008),   # tiles that leave room for one accumulator
+    ("int4", 651, 7680, 12160),   # ... of 512 columns
     ("int4", 60, 11008, 16384),   # the cluster's parts of K have several chains each
     ("bf16", 256, 4096, 4096),
 ]

@@ -101,3 +101,28 @@ def test_pair_form_repeats_bit_for_bit(kind, M, K, N):
         first = C if first is None else first
         assert torch.equal(C, first), i
     capi.sync_check()
+
+
+def test_folded_parts_on_a_capturing_stream():
+    """the sums of folded parts need a workspace, which a stream that is being captured does not have: the graph owns one"""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    M, K, N = 300, 4096, 11008
+    A = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    B = (torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    w = capi.Weight(B.data_ptr(), capi.BF16, K, N, 2 * K, True, capi.PACK_INT4_GROUP)
+    C = torch.zeros((M, N), device="cuda")
+    ep = capi.make_epilogue(C.data_ptr(), 4 * N, capi.F32, capi.STEP_DEQUANT)
+    w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep)
+    capi.sync_check()
+    want = C.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(2):
+            w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep, stream=torch.cuda.current_stream().cuda_stream)
+    for _ in range(3):
+        C.zero_()
+        graph.replay()
+        assert torch.equal(C, want)
+    capi.sync_check()
