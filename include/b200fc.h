@@ -71,6 +71,10 @@ const char* b200fc_version(void);
 /* number of this library's kernels launched by the calling process so far (bench bookkeeping) */
 int64_t b200fc_launch_count(void);
 
+/* diagnostics: the tile of the calling thread's last one-wave GEMM launch, as {CTAs per tile, weight rows per CTA, CTAs that share K,
+ * accumulators, folded parts of K, tiles}, and forgets it (all 0: none since) */
+int b200fc_last_wave_tile(int tile[6]);
+
 /* Limits the persistent GEMM kernels to `sms` SMs (0 = all).  A tensor-parallel caller that overlaps an NCCL
  * all-reduce with the GEMMs leaves the collective a few SMs this way; otherwise its CTAs queue behind the GEMM's. */
 int b200fc_set_sm_limit(int sms);

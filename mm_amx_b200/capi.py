@@ -47,6 +47,7 @@ SIGNATURES = {
                                             ctypes.POINTER(ctypes.c_int)]),
     "b200fc_sync_check": (c_int, [c_void_p]),
     "b200fc_set_wait_limit_ns": (c_int, [ctypes.c_uint64]),
+    "b200fc_last_wave_tile": (c_int, [ctypes.POINTER(ctypes.c_int)]),
     "b200fc_set_sm_limit": (c_int, [c_int]),
     "b200fc_set_decode_ctas_per_sm": (c_int, [c_int]),
     "b200fc_weight_pack": (c_int, [c_void_p, c_int, c_int, c_int, c_i64, c_int, c_int, c_void_p,
@@ -126,6 +127,14 @@ def last_error():
 
 def launch_count():
     return lib().b200fc_launch_count()
+
+
+def last_wave_tile():
+    """(CTAs per tile, weight rows per CTA, CTAs sharing K, accumulators, folded parts, tiles) of this thread's last one-wave GEMM; None
+    if there was none since the last call"""
+    tile = (ctypes.c_int * 6)()
+    check(lib().b200fc_last_wave_tile(tile))
+    return tuple(tile) if tile[0] else None
 
 
 def set_sm_limit(sms):

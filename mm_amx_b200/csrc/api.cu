@@ -383,6 +383,13 @@ const char* b200fc_last_error(void) { return g_err; }
 const char* b200fc_version(void) { return "b200fc 0.1 (sm_100a)"; }
 int64_t b200fc_launch_count(void) { return (int64_t)g_launches.load(); }
 
+int b200fc_last_wave_tile(int tile[6]) {
+    if (!tile) { set_error("last_wave_tile: null pointer"); return B200FC_ERR_INVALID; }
+    int* last = last_wave_tile();
+    for (int i = 0; i < 6; i++) { tile[i] = last[i]; last[i] = 0; }
+    return B200FC_OK;
+}
+
 int b200fc_set_sm_limit(int sms) {
     if (sms < 0) { set_error("set_sm_limit: negative"); return B200FC_ERR_INVALID; }
     g_sm_limit = sms;

@@ -166,6 +166,7 @@ int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, co
                    int64_t lda, int n0, int n1, const Epilogue& ep, cudaStream_t s);
 // 0 = choose by shape, 1 = force the 1-CTA kernel, 2 = force the 2-CTA kernel (B200FC_GEMM_CTAS, for experiments)
 int gemm_forced_ctas();
+int* last_wave_tile();   // six ints of the calling thread, see b200fc_last_wave_tile
 // parts of K that launch_gemm_tc sums one after the other for a bf16 call of nspan columns: chains of fp32 sums
 int gemm_tc_chains(int M, int K, int nspan);
 // rows of compressed weights that are widened to bf16 at a time in front of launch_gemm_tc: 32 MB of them

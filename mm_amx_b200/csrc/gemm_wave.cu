@@ -756,6 +756,8 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
         if (own_sums) B200FC_CUDA(cudaFreeAsync(p.sums, call.s));
     }
     count_launch();
+    const int tile[6] = {CG, p.R, p.S, p.sets, p.parts, sh.tiles_m * sh.tiles_n};
+    for (int i = 0; i < 6; i++) last_wave_tile()[i] = tile[i];
     return B200FC_OK;
 }
 
@@ -796,6 +798,11 @@ int run_wave(WaveCall& c, int n0, int n1) {
 }
 
 }  // namespace
+
+int* last_wave_tile() {
+    static thread_local int tile[6];
+    return tile;
+}
 
 int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,
                      cudaStream_t s) {

@@ -82,8 +82,9 @@ def test_weight_quantiser_bit_exact_on_normal_data(K, N, transposeB):
 
 @pytest.mark.parametrize("M,K,N,n0,n1", [(40, 256, 1024, 0, 1024), (130, 8192, 2600, 0, 2600), (64, 8192, 2600, 512, 2304)])
 def test_compressed_weights_prefill_blocks(M, K, N, n0, n1):
-    """M > 16 with int8-compressed weights: blocks of weight rows are widened into a scratch and multiplied block by
-    block (K = 8192 makes a block 2048 rows, so N = 2600 takes two); per-channel scales, bias and a column range."""
+    """M > 16 with int8-compressed weights: per-channel scales, bias and a column range.  One wave of tiles by default; without the
+    one-wave kernel (test_gpu_persistent.py) blocks of weight rows are widened into a scratch and multiplied block by block
+    (K = 8192 makes a block 2048 rows, so N = 2600 takes two)."""
     rng = np.random.default_rng(M + K + N + n0)
     A = H.normal_bf16(rng, (M, K))
     Wq = rng.integers(-127, 128, (N, K), dtype=np.int8)
@@ -212,7 +213,8 @@ def test_s8_postops(M):
 
 @pytest.mark.parametrize("M,K,N", [(100, 4096, 512), (256, 4096, 1024), (64, 2304, 300), (17, 8192, 256)])
 def test_split_k_shapes_exact(M, K, N):
-    """few output tiles and a long K: the GEMM splits K over CTA pairs and reduces in a second kernel"""
+    """few output tiles and a long K: K is split over the CTAs of a cluster; without the one-wave kernel (test_gpu_persistent.py) over
+    CTA pairs, and reduced in a second kernel"""
     rng = np.random.default_rng(M + K + N)
     A = H.two_valued_bf16(rng, (M, K)); B = H.two_valued_bf16(rng, (K, N))
     bias = (rng.integers(-8, 9, N) * 0.25).astype(np.float32)
@@ -257,7 +259,8 @@ def test_ragged_last_round_goes_through_a_k_split_launch():
 
 @pytest.mark.parametrize("M,K,N", [(512, 192, 10280), (300, 128, 20000), (1024, 64, 5000), (700, 96, 7177)])
 def test_many_tiles_exact(M, K, N):
-    """more 256 x 256 tiles than CTA pairs: every pair walks several tiles, both accumulator buffers get reused"""
+    """more 256 x 256 tiles than CTA pairs: without the one-wave kernel (test_gpu_persistent.py) every pair walks several tiles and
+    both accumulator buffers get reused"""
     rng = np.random.default_rng(M + K + N)
     A = H.two_valued_bf16(rng, (M, K)); B = H.two_valued_bf16(rng, (K, N))
     bias = (rng.integers(-8, 9, N) * 0.25).astype(np.float32)

@@ -100,7 +100,8 @@ def test_int4_column_range_and_bad_n0():
 
 @pytest.mark.parametrize("M,K,N", [(40, 512, 1024), (130, 8192, 2600)])
 def test_int4_prefill_blocks(M, K, N):
-    """M > 16: blocks of weight rows are widened to bf16 (value * group scale, rounded) and multiplied by the GEMM"""
+    """M > 16: weights are widened to bf16 (value * group scale, rounded), in the one-wave kernel or, without it
+    (test_gpu_persistent.py), in blocks of rows in front of the GEMM"""
     rng = np.random.default_rng(M + K)
     x = H.normal_bf16(rng, (M, K)); W = H.normal_bf16(rng, (N, K), 0.02)
     q, d = port.quantize_weight_int4(W)

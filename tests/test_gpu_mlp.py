@@ -104,7 +104,8 @@ def test_mlp_many_tiles():
 
 
 def test_mlp_long_k_few_tiles():
-    """M just above the decode limit with a long K: both GEMMs take the split-K route (SiLU pairing in the reduction)"""
+    """M just above the decode limit with a long K: both GEMMs split K, inside clusters or, without the one-wave kernel
+    (test_gpu_persistent.py), with the SiLU pairing in the reduction kernel"""
     rng = np.random.default_rng(77)
     M, K, N = 40, 2048, 4096
     x, gate, up, down = make_mlp_inputs(rng, M, K, N)

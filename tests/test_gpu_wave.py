@@ -20,8 +20,8 @@ SHAPES = [
     (129, 2080, 1000),   # the first one of the pair form, its second CTA nearly without rows
     (100, 4096, 2750),   # several columns tiles, split K, ragged last tile
     (256, 1536, 4104),   # pair form with a split of K
-    (300, 200, 9000),    # two row tiles, wide tiles whose columns come from two MMAs
-    (2048, 128, 4096),   # 512-column tiles: all of tensor memory
+    (300, 200, 9000),    # two row tiles (bf16 and int8 x int8 go to the persistent kernel: 256 x 256 tiles without a split of K)
+    (2048, 128, 4096),   # 512-column tiles: all of tensor memory, columns of two MMAs
     (2100, 136, 5000),   # more tiles than one wave: the persistent kernel, with widened blocks for quantised weights
 ]
 
@@ -116,6 +116,7 @@ def test_folded_parts_on_a_capturing_stream():
     ep = capi.make_epilogue(C.data_ptr(), 4 * N, capi.F32, capi.STEP_DEQUANT)
     w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep)
     capi.sync_check()
+    assert capi.last_wave_tile()[4] > 1
     want = C.clone()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
@@ -126,3 +127,63 @@ def test_folded_parts_on_a_capturing_stream():
         graph.replay()
         assert torch.equal(C, want)
     capi.sync_check()
+
+
+# kind, M, K, N, tile as capi.last_wave_tile (148 SMs): more than 128 weight rows per CTA, whose columns come from two MMAs
+TILES = [
+    ("int8", 705, 4096, 7680, (2, 160, 1, 1, 1, 72)),      # halves of 96 and 64 rows
+    ("int4", 705, 4096, 7680, (2, 160, 1, 1, 1, 72)),
+    ("bf16", 705, 2560, 7680, (2, 160, 1, 1, 1, 72)),
+    ("int8", 705, 2560, 10240, (2, 224, 1, 1, 1, 69)),     # 128 and 96 rows; few pieces in the rings
+    ("int4", 705, 2560, 10240, (2, 224, 1, 1, 1, 69)),
+    ("s8", 705, 2560, 10240, (2, 224, 1, 1, 1, 69)),
+    ("int8", 705, 4096, 12288, (2, 256, 1, 1, 1, 72)),     # all of tensor memory, the fewest ring slots
+    ("int4", 705, 4096, 12288, (2, 256, 1, 1, 1, 72)),
+    ("int8", 35, 6400, 21104, (1, 160, 1, 3, 3, 132)),     # folded parts of K, three accumulators
+    ("int8", 256, 4096, 16384, (2, 128, 1, 2, 2, 64)),     # ... in the pair form
+    ("int4", 300, 4096, 11008, (2, 160, 1, 1, 3, 70)),     # ... with tiles that leave room for one accumulator
+    ("int4", 60, 11008, 16384, (1, 224, 2, 2, 2, 74)),     # ... and two CTAs that share K
+]
+
+
+@pytest.mark.parametrize("kind,M,K,N,tile", TILES)
+def test_wide_tiles_exact(kind, M, K, N, tile):
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("tiles for 148 SMs")
+    rng = np.random.default_rng(M + 3 * K + 7 * N)
+    rows = np.unique(np.concatenate([[0, 31, 127, 128, 255, 256, M - 1], rng.integers(0, M, 12)]))      # rows the oracle computes
+    rows = rows[rows < M]
+    B = rng.integers(-7, 8, (N, K), dtype=np.int8)
+    steps = 0
+    if kind == "s8":
+        x = rng.integers(-128, 128, (M, K), dtype=np.int8)
+        w, acc, out = H.pack(B, True), port.gemm_i8(x[rows], B, transposeB=True), capi.S32
+    else:
+        x, out = H.two_valued_bf16(rng, (M, K)), capi.F32
+        if kind == "int8":
+            steps = capi.STEP_DEQUANT
+            w = H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=np.ones(N, np.float32))
+            acc = port.gemm_bf16_w8(x[rows], B, transposeB=True)
+        else:
+            B[:, ::128] = 7                 # (every group of 4-bit weights reaches the full range: the scale is 2^-6 exactly)
+            W = H.bf16_bits(B.astype(np.float32) * np.float32(2.0 ** -6))
+            steps = capi.STEP_DEQUANT if kind == "int4" else 0
+            w = H.pack(W, True, capi.PACK_INT4_GROUP if kind == "int4" else capi.PACK_PLAIN)
+            acc = port.gemm_bf16(x[rows], W, transposeB=True)
+    capi.last_wave_tile()
+    got = H.run_matmul(w, x, out, steps=steps)
+    assert capi.last_wave_tile() == tile
+    assert np.array_equal(got[rows], acc)
+
+
+@pytest.mark.parametrize("sms", [2, 37, 100])
+@pytest.mark.parametrize("M,K,N", [(40, 2080, 1000), (200, 4096, 2750), (9, 4096, 3000)])
+@pytest.mark.parametrize("kind", ["bf16", "int8_compressed", "int4"])
+def test_under_an_sm_limit(kind, M, K, N, sms):
+    """fewer SMs change the tile, the split of K and the number of chains, or hand the call to the persistent kernel"""
+    capi.set_sm_limit(sms)
+    try:
+        test_every_weight_type_exact(kind, M, K, N)
+    finally:
+        capi.set_sm_limit(0)
