@@ -81,16 +81,17 @@ static std::map<ScratchKey, Scratch> g_scratch;
 int get_stream_scratch(size_t bytes, cudaStream_t s, int slot, void** out, bool* own) {
     int dev = 0;
     cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(g_mu);
-    Scratch& sc = g_scratch[ScratchKey{dev, s, slot}];
-    if (own) *own = false;
-    if (sc.bytes < bytes) {
+    if (own) {
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (own && cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive) {
+        *own = cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive;
+        if (*own) {
             B200FC_CUDA(cudaMallocAsync(out, bytes, s));
-            *own = true;
             return B200FC_OK;
         }
+    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    Scratch& sc = g_scratch[ScratchKey{dev, s, slot}];
+    if (sc.bytes < bytes) {
         if (sc.p) { cudaStreamSynchronize(s); cudaFree(sc.p); sc.p = nullptr; sc.bytes = 0; }
         B200FC_CUDA(cudaMalloc(&sc.p, bytes));
         sc.bytes = bytes;

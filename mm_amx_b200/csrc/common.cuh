@@ -100,8 +100,8 @@ int check_kernel_status(cudaStream_t s);  // synchronises and reads it
 // may share it; slot 0 = re-strided activations, slot 1 = split-K partial tiles of the GEMM and sums of folded parts of K, 3 = widened weight
 // rows, 4 = normalised activations of the MLP block, 5 = sub-states of the decode attention, 6 = pre-converted activations
 // of the decode kernel
-// own (optional): where s is being captured and its scratch is too small, stream-ordered memory instead, which becomes part of the
-// graph; *own says so, and the caller frees it with cudaFreeAsync behind its last use
+// own (optional): where s is being captured, stream-ordered memory instead, which becomes part of the graph (the stream's scratch may be
+// re-allocated before a replay); *own says so, and the caller frees it with cudaFreeAsync behind its last use
 int get_stream_scratch(size_t bytes, cudaStream_t s, int slot, void** out, bool* own = nullptr);
 // the decode kernel's scratch for stream s (gemv_scratch_bytes(), counters zero); never re-allocated once handed out
 int get_gemv_scratch(cudaStream_t s, void** out);

@@ -698,8 +698,7 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
     const int grid = CG * sh.S * sh.tiles_m * sh.tiles_n;
     bool own_sums = false;
     if (p.parts > 1) {
-        // the workspace of the split of K in gemm_tc.cu, which this takes the place of; memory of the graph where the stream is being
-        // captured and has none that is large enough
+        // the workspace of the split of K in gemm_tc.cu, which this takes the place of; memory of the graph where the stream is being captured
         int rc = get_stream_scratch((size_t)grid * (CG * sh.R / 32) * CHUNK_BYTES, call.s, 1, (void**)&p.sums, &own_sums);
         if (rc) return rc;
     }

@@ -104,28 +104,43 @@ def test_pair_form_repeats_bit_for_bit(kind, M, K, N):
 
 
 def test_folded_parts_on_a_capturing_stream():
-    """the sums of folded parts need a workspace, which a stream that is being captured does not have: the graph owns one"""
+    """the sums of folded parts need a workspace; a graph owns one of its own, so that a replay does not depend on the stream's, which
+    a larger call re-allocates"""
     import torch
     g = torch.Generator(device="cuda")
     g.manual_seed(1)
-    M, K, N = 300, 4096, 11008
-    A = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
-    B = (torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
-    w = capi.Weight(B.data_ptr(), capi.BF16, K, N, 2 * K, True, capi.PACK_INT4_GROUP)
-    C = torch.zeros((M, N), device="cuda")
-    ep = capi.make_epilogue(C.data_ptr(), 4 * N, capi.F32, capi.STEP_DEQUANT)
-    w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep)
-    capi.sync_check()
-    assert capi.last_wave_tile()[4] > 1
-    want = C.clone()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        for _ in range(2):
-            w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep, stream=torch.cuda.current_stream().cuda_stream)
-    for _ in range(3):
-        C.zero_()
-        graph.replay()
-        assert torch.equal(C, want)
+
+    def make(M, K, N):
+        A = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+        B = (torch.randn((N, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+        w = capi.Weight(B.data_ptr(), capi.BF16, K, N, 2 * K, True, capi.PACK_INT4_GROUP)
+        C = torch.zeros((M, N), device="cuda")
+        ep = capi.make_epilogue(C.data_ptr(), 4 * N, capi.F32, capi.STEP_DEQUANT)
+        return C, lambda stream: w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep, stream=stream.cuda_stream), (A, w, ep)
+
+    C, call, keep = make(300, 4096, 11008)
+    _, larger, keep2 = make(651, 7680, 12160)
+    for warm in (False, True):
+        s = torch.cuda.Stream()
+        call(torch.cuda.default_stream())
+        capi.sync_check()
+        assert capi.last_wave_tile()[4] > 1
+        want = C.clone()
+        torch.cuda.synchronize()
+        if warm:
+            call(s)
+            s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            for _ in range(2):
+                call(torch.cuda.current_stream())
+        for _ in range(3):
+            C.zero_()
+            larger(s)
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(C, want)
     capi.sync_check()
 
 
