@@ -842,8 +842,9 @@ int b200fc_mlp_down_allreduce(b200fc_mlp_t* h, int M, const b200fc_allreduce_t* 
 // so that little of the first copy is exposed) for gate/up, the same sequences reversed and a halving sequence for
 // down (short chunks last), each pair rated by a small model of the three engines — the copy engines at PCIe speed and
 // the GEMMs as whole waves of 256 x 256 tiles over the CTA pairs, which is what makes a chunk of 7 x 256 rows of the
-// Llama-70B down projection (224 tiles on 74 pairs) cost four waves instead of three.  The model only has to rank
-// plans; measured on Llama-70B at M = 4096 its first choices are the measured first choices.
+// Llama-70B down projection (224 tiles on 74 pairs) cost four waves instead of three.  That is launch_gemm_tc; chunks whose
+// output fits one wave of launch_gemm_wave's tiles take less than the model says.  It only has to rank plans; measured on
+// Llama-70B at M = 4096 (with launch_gemm_tc alone) its first choices are the measured first choices.
 // B200FC_HOST_PLAN="a,b,c;d,e,f" (chunks in tiles of 256 rows; the last entry of each list takes what is left)
 // replaces the choice, for experiments.
 namespace {
@@ -855,7 +856,7 @@ struct PlanModel {
     int cols_gu, cols_dn, pairs;
     int slabs_gu, slabs_dn;       // K of the two GEMMs in 64-element slabs
     // rounds of tiles a launch of `rows` row tiles x `cols` column tiles takes; a short ragged last round of a long-K
-    // GEMM is split along K by the launcher (launch_gemm_tc) and costs well under a round
+    // GEMM is split along K by launch_gemm_tc and costs well under a round (a chunk of few tiles: see above)
     double waves(int rows, int cols, int k_slabs) const {
         const long long tiles = (long long)rows * cols;
         const long long full = tiles / pairs, rem = tiles % pairs;

@@ -196,10 +196,46 @@ int launch_decode_attention(const b200fc_attention_t& a, cudaStream_t s);
 // matvec.cu
 int launch_matvec(const void* A, int dtype, int M, int K, int64_t lda, const void* b, void* c, cudaStream_t s);
 
+#ifdef __CUDACC__
+// ---------------------------------------------------------------------------------------------------------------
+// Instructions that several decode and GEMM kernels use (device).
+// ---------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void bulk_load_1d(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// fp32 at shared-memory address `addr` (of this CTA's window) in CTA `rank` of the cluster
+__device__ __forceinline__ float ld_peer_f32(unsigned addr, unsigned rank) {
+    unsigned ra;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+    return v;
+}
+// the fp32 values at shared-memory address `addr` of all S <= 8 CTAs of the cluster, added in rank order; the loads travel together
+__device__ __forceinline__ float cluster_sum(unsigned addr, int S) {
+    float t[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) t[q] = q < S ? ld_peer_f32(addr, (unsigned)q) : 0.0f;
+    float sum = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) sum += t[q];
+    return sum;
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Post-op math shared by all kernels (device).
 // ---------------------------------------------------------------------------------------------------------------
-#ifdef __CUDACC__
 
 // erf-GeLU through the minimax polynomial in x^2 that the reference evaluates (gelu_erf_minmax_approx,
 // include/kernels_amx.hpp:242-289): x < -5 -> 0, |x| > 5 -> x, |x| <= 2^-24 -> x/2, else x/2 * (1 + x * P(x^2)).

@@ -25,7 +25,6 @@ namespace b200fc {
 namespace {
 
 constexpr int NUM_THREADS = 192;
-constexpr int EPI_WARP0 = 2;
 constexpr int EPI_TILE_BYTES = 4 * EPI_TILE_WORDS * 4;
 
 template <int BN> struct Cfg {

@@ -451,8 +451,6 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const int r = cc >= rows;
             return r * p.R + (h ? p.R0 : 0) + cc - (r ? rows : 0);
         };
-        // every load of the ring has landed and every MMA has read it: the ring is free
-        unsigned* stage_tile = (unsigned*)(smem + RING_BYTES - (WORKERS - wi) * WARP_TILE_BYTES);
         // columns [32 c, +32) of this CTA's result: the sums of the folded parts, if any, and the last part's accumulators in order
         const int filled = min(p.sets, n_slabs - n_slabs * (parts - 1) / parts);
         auto load_acc = [&](int c, unsigned (&r)[32]) {

@@ -142,25 +142,6 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// fp32 at shared-memory address `addr` (of this CTA's window) in CTA `rank` of the cluster
-__device__ __forceinline__ float ld_peer_f32(unsigned addr, unsigned rank) {
-    unsigned ra;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
-    return v;
-}
-// the fp32 values at shared-memory address `addr` of all S <= 8 CTAs of the cluster, added in rank order; the loads travel together
-// (Llama-7B MLP block at M = 1: 54.64 -> 54.56 us)
-__device__ __forceinline__ float cluster_sum(unsigned addr, int S) {
-    float t[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) t[q] = q < S ? ld_peer_f32(addr, (unsigned)q) : 0.0f;
-    float sum = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 8; q++) sum += t[q];
-    return sum;
-}
 // strong (coherent at GPU scope) 16-byte load: partial sums written by other SMs during this launch
 __device__ __forceinline__ float4 ld_gpu_f4(const float4* p) {
     float4 v;
@@ -196,11 +177,6 @@ __device__ __forceinline__ unsigned u8x2_to_f16x2(unsigned w, unsigned sel) {
 
 __device__ __forceinline__ void cp_async16(unsigned dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void bulk_load_1d(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
 }
 // (w & mask) | 0x64006400: the two nibbles selected by `mask` as the low bits of two fp16 numbers 1024 + ...
 __device__ __forceinline__ unsigned nib_or_magic(unsigned w, unsigned mask) {
@@ -1059,15 +1035,6 @@ __device__ __forceinline__ unsigned long long tc_smem_desc(unsigned smem_addr) {
     d |= (unsigned long long)1 << 46;
     d |= (unsigned long long)2 << 61;
     return d;
-}
-__device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w,

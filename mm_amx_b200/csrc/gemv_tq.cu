@@ -75,29 +75,6 @@ __device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsi
         ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void bulk_load_1d(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ float ld_peer_f32(unsigned addr, unsigned rank) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_rank(addr, rank)) : "memory");
-    return v;
-}
-
-// the fp32 values at shared-memory address `addr` of all S <= 8 CTAs of the cluster, added in rank order; the loads travel together
-// (int8, 1 x 4096 x 4096: 7.33 -> 7.28 us)
-__device__ __forceinline__ float cluster_sum(unsigned addr, int S) {
-    float t[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) t[q] = q < S ? ld_peer_f32(addr, (unsigned)q) : 0.0f;
-    float sum = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 8; q++) sum += t[q];
-    return sum;
-}
-
 template <int WB>
 __global__ void __launch_bounds__(TQ_THREADS, 2)
 gemv_tq_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TqParams p) {
@@ -400,10 +377,13 @@ int launch_gemv_tq(const Weight& w, const void* A, int M, int K, int64_t lda, in
     TqParams p = {};
     p.spr = (int)(w.ld_bytes() / SLAB_BYTES);
     const int row_blocks = (n1 - n0 + TQ_ROWS - 1) / TQ_ROWS;
-    // More row blocks than SMs, so that a CTA has one to itself and some SMs have two CTAs, others one: with long rows that
-    // imbalance costs more than the faster product gains, and gemv_tma.cu cuts the stream into equal pieces (us, there / here:
-    // int8 1 x 8192 x 20480 36.9 / 47.0, x 28672 46.0 / 47.7; 4 bits 8 x 8192 x 25088 35.6 / 40.6; 16 rows int8 x 20480 45.4 / 48.6,
-    // x 25088 51.5 / 49.4; K = 3328 is level at 1 row and 1.2 to 1.3 times faster here at 16).
+    // More row blocks than half of the places for CTAs (max_ctas): K is not split (S = 1 below) and the places beyond the row blocks
+    // stay empty.  With long rows that imbalance costs more than the faster product gains, and gemv_tma.cu cuts the stream into equal
+    // pieces (us, there / here: int8 1 x 8192 x 20480 36.9 / 47.0, x 28672 46.0 / 47.7; 4 bits 8 x 8192 x 25088 35.6 / 40.6;
+    // 16 rows int8 x 20480 45.4 / 48.6, x 25088 51.5 / 49.4; K = 3328 is level at 1 row and 1.2 to 1.3 times faster here at 16).  The
+    // same with one place per SM, where the line lies at 74 row blocks: int8 1 x 4096 x 10240 22.7 / 24.7, x 12800 25.3 / 25.1,
+    // 1 x 8192 x 12800 38.5 / 46.2; 16 rows 4096 x 12800 33.8 / 27.3.  (Row blocks that fill all places would be faster here: 1 x 4096 x 18944
+    // 24.2 / 18.1.)  The lines between are drawn through these sizes.
     if (2 * row_blocks > max_ctas && (M <= 8 ? K >= 4096 : K >= 8192 && 7 * row_blocks < 4 * max_ctas)) return B200FC_ERR_UNSUPPORTED;
     // as many parts of K per row block as keep all CTAs resident, of two stages and more each
     int S = max_ctas / row_blocks;
