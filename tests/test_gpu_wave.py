@@ -119,7 +119,7 @@ def test_folded_parts_on_a_capturing_stream():
         return C, lambda stream: w.matmul(A.data_ptr(), capi.BF16, M, K, 2 * K, ep, stream=stream.cuda_stream), (A, w, ep)
 
     C, call, keep = make(300, 4096, 11008)
-    _, larger, keep2 = make(651, 7680, 12160)
+    C2, larger, keep2 = make(651, 7680, 12160)
     for warm in (False, True):
         s = torch.cuda.Stream()
         call(torch.cuda.default_stream())
