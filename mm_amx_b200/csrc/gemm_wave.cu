@@ -76,9 +76,10 @@ __device__ __forceinline__ unsigned nib2_to_bf16x2_scaled(unsigned w, float scal
 // FOLD: K in several parts, see below (quantised weights).  A kernel of its own, because the folding code costs the widening loop
 // registers and instruction cache also where it does not run (int8 705 x 2560 x 10240: 44.8 us with it, 42.3 without).  Calls whose
 // chains do not fit pay for both (us, one chain / as many as asked for / through widened blocks and a split of K): 4 bits
-// 512 x 4096 x 11008 42 / 61 / 127 (two folds), int8 705 x 4096 x 10240 45 / 58 / 126 (one fold, 6.5 of it, of which the workers read
-// tensor memory at 500 clocks per 32 columns), int8 300 x 11008 x 8192 75 / 103 / 249 (13 are the slower loop).  No gain: folding
-// each chain by itself under the next one, adding with red instead of load and store, the fold as a function that is called.
+// 512 x 4096 x 11008 42 / 62 / 127 (two folds), int8 705 x 4096 x 10240 45 / 59 / 126 (one fold, 6.5 of it, of which the workers read
+// tensor memory at 500 clocks per 32 columns), int8 300 x 11008 x 8192 74 / 99 / 249.  Parts that end anywhere, with the check for a
+// fold inside the loop over a piece's slabs: 66 / 59 / 102.  No gain: folding each chain by itself under the next one, adding with
+// red instead of load and store, the fold as a function that is called.
 template <int CG, int MODE, bool FOLD>
 __global__ void __launch_bounds__(WAVE_THREADS, 1)
 gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const WaveParams p) {
@@ -113,7 +114,10 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int n_units = u1 - u0, n_slabs = min(u1 * SPU, p.slabs) - u0 * SPU;
     // K in chains of fp32 sums: the slabs take the accumulators in turn.  Where tensor memory holds too few of them K is cut into parts
     // as well, after each of which (but the last) the workers add the accumulators to a sum in global memory (L2).
-    const int parts = FOLD ? min(p.parts, n_slabs) : 1, cols = p.sets * W;
+    // Parts end with stored pieces, so that the folding stays out of the loop over a piece's slabs.
+    const int parts = FOLD ? min(p.parts, n_units) : 1, cols = p.sets * W;
+    auto part_unit = [&](int q) { return n_units * q / parts; };
+    auto part_slab = [&](int q) { return FOLD ? min(part_unit(q) * SPU, n_slabs) : q * n_slabs; };
     const unsigned tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
 
     if (threadIdx.x == 0) {
@@ -201,7 +205,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else if (warp == 1) {
         // ---------------- MMA issue ----------------
         if (leader) {
-            int slot = 0, wslot = 0, set = 0, part = 0, start = 0, end = n_slabs / parts;      // slabs of the part
+            int slot = 0, wslot = 0, set = 0, part = 0, start = 0, end = part_slab(1);      // slabs of the part
             unsigned phase = 0, wphase = 0;
             const unsigned ring = smem_u32(smem), wring = smem_u32(wide_ring);
             for (int i = 0; i < n_slabs; i++) {
@@ -209,7 +213,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (!__all_sync(0xffffffffu, mbar_wait<0, CG == 2>(bar_folded, (unsigned)part & 1, abort_flag, p.wait_limit_ns))) break;
                     part++;
                     start = end;
-                    end = n_slabs * (part + 1) / parts;
+                    end = part_slab(part + 1);
                     set = 0;
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * slot, phase, abort_flag, p.wait_limit_ns))) break;
@@ -302,7 +306,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             ok = __all_sync(0xffffffffu, mbar_wait(bar_part, (unsigned)folds & 1, abort_flag, p.wait_limit_ns));
             if (!ok) return;
             tc_fence_after();
-            const int filled = min(p.sets, n_slabs * (folds + 1) / parts - n_slabs * folds / parts);
+            const int filled = min(p.sets, part_slab(folds + 1) - part_slab(folds));
 #pragma unroll 1
             for (int c = third; c < chunks; c += SETS) {
                 unsigned sum[32], x[32];
@@ -350,13 +354,21 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 }
             };
             if constexpr (MODE == W_U4C) load_scales(u0);
-            int slot = 0, rslot = 0, turn = 0, slab = 0;
-            // A part is folded when the ring of widened slabs has been filled behind it: the MMAs of the next one wait for the fold, and
-            // go on at once with the slabs that are there.
-            int fold_at = parts > 1 ? n_slabs / parts + p.wide_slots : n_slabs;
+            int slot = 0, rslot = 0, turn = 0;
+            // A part is folded, where the ring of widened slabs holds a piece, when one has been widened behind it: the MMAs of the
+            // next part wait for the fold, and go on at once with the slabs that are there.
+            constexpr int BEHIND = SPU <= SETS ? 1 : 0;
+            int fold_at = parts > 1 ? part_unit(1) + BEHIND : n_units;
             unsigned phase = 0, rphase = 0;
             for (int j = 0; j < n_units && ok; j++) {
                 const int u = u0 + j;
+                if constexpr (FOLD) {
+                    if (j == fold_at) {
+                        fold_part();
+                        if (!ok) break;
+                        fold_at = folds < parts - 1 ? part_unit(folds + 1) + BEHIND : n_units;
+                    }
+                }
                 if constexpr (MODE == W_U4C) {
 #pragma unroll
                     for (int e = 0; e < 4; e++) { sc[e][0] = sc_next[e][0]; sc[e][1] = sc_next[e][1]; }
@@ -370,13 +382,6 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll 1
                 for (int s = 0; s < SPU; s++) {
                     if (u * SPU + s >= p.slabs) break;          // warp-uniform: the last piece may reach past K
-                    if constexpr (FOLD) {
-                        if (slab++ == fold_at) {
-                            fold_part();
-                            if (!ok) break;
-                            fold_at = folds < parts - 1 ? n_slabs * (folds + 1) / parts + p.wide_slots : n_slabs;
-                        }
-                    }
                     if (turn == set) {
                         constexpr int UNITS = MODE == W_U8C ? 2 : 1;     // 16-byte units of an item's row
                         uint4 v[4][UNITS];
@@ -452,7 +457,7 @@ gemm_wave_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             return r * p.R + (h ? p.R0 : 0) + cc - (r ? rows : 0);
         };
         // columns [32 c, +32) of this CTA's result: the sums of the folded parts, if any, and the last part's accumulators in order
-        const int filled = min(p.sets, n_slabs - n_slabs * (parts - 1) / parts);
+        const int filled = min(p.sets, n_slabs - part_slab(parts - 1));
         auto load_acc = [&](int c, unsigned (&r)[32]) {
             if (FOLD && parts > 1) {
                 load_sums(c, r);
