@@ -114,6 +114,51 @@ unsigned long long wait_limit_ns();
         if (e__ != cudaSuccess) return ::b200fc::cuda_fail(e__, #call);     \
     } while (0)
 
+#ifdef __CUDACC__
+// Largest number of clusters of `size` <= 8 CTAs of so many threads and bytes of shared memory that are resident together; asked once
+// per device.  It is less than places for CTAs / size, because a cluster stays inside a GPC (two CTAs per SM: 296 places, 33 clusters
+// of 8, 37 of 7, 45 of 6).  An empty kernel stands in for the caller's: of a kernel that allocates tensor memory the driver counts one CTA
+// per SM, however little it allocates.
+struct ClusterCounts { std::atomic<int> n[64][9]; };
+static __global__ void cluster_count_kernel() {}
+static inline int resident_clusters(ClusterCounts& counts, int size, int threads, size_t smem, int* out) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::atomic<int>& known = counts.n[dev & 63][size];
+    int n = known.load(std::memory_order_relaxed);
+    if (!n) {
+        B200FC_CUDA(cudaFuncSetAttribute(cluster_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(size * 148), 1, 1);
+        cfg.blockDim = dim3((unsigned)threads, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        B200FC_CUDA(cudaOccupancyMaxActiveClusters(&n, cluster_count_kernel, &cfg));
+        if (n < 1) n = -1;
+        known.store(n, std::memory_order_relaxed);
+    }
+    *out = n < 0 ? 0 : n;
+    return B200FC_OK;
+}
+// Lowers the split *S of K until the row blocks' clusters are all resident: a cluster left over runs as a second round (bf16
+// 4 x 4096 x 4352, 34 row blocks: 15.4 us with S = 8, 9.8 with 7; x 7424, 58 row blocks: 20.9 with 5, 14.1 with 4; int8 4 x 4096 x 4352
+// 10.9 and 8.0).
+static inline int fit_clusters(ClusterCounts& counts, int threads, size_t smem, int row_blocks, int* S) {
+    for (; *S > 1; --*S) {
+        int n = 0;
+        const int rc = resident_clusters(counts, *S, threads, smem, &n);
+        if (rc) return rc;
+        if (n >= row_blocks) break;
+    }
+    return B200FC_OK;
+}
+#endif
+
 // api.cu: gate/up + down of a decode-shaped MLP (1 <= M <= 16) in one launch; B200FC_ERR_UNSUPPORTED without a message =
 // not possible here, launch the two projections separately
 int mlp_decode_fused_device(const Mlp& m, const void* x, int64_t ldx, int M, void* act, void* out, int out_dtype,
@@ -213,6 +258,15 @@ __device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
+}
+// One lane of a converged warp, the same one every time.  The issuing loops below run as whole warps and elect the lane only
+// around the TMA / MMA / commit instructions: these take their operands from uniform registers, which the compiler can keep
+// them in only while the control flow is warp-uniform.  With the loop inside `if (lane == 0)` every MMA cost about 100 clocks of
+// issue and every slab 480 more (880 clocks per 128 bytes of K however few columns a tile has).
+__device__ __forceinline__ bool elect_one() {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
 }
 // fp32 at shared-memory address `addr` (of this CTA's window) in CTA `rank` of the cluster
 __device__ __forceinline__ float ld_peer_f32(unsigned addr, unsigned rank) {

@@ -590,38 +590,11 @@ int allow_smem() {
     });
 }
 
-// Largest number of clusters of `size` CTAs (one CTA per SM) that are resident together; asked once per device.
-template <int CG, int MODE>
-int max_clusters(int size, int* out) {
-    static std::atomic<int> cache[64][9];
-    const int arc = allow_smem<CG, MODE, false>();
-    if (arc) return arc;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int n = cache[dev & 63][size].load(std::memory_order_relaxed);
-    if (!n) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(size * 148), 1, 1);
-        cfg.blockDim = dim3(WAVE_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = WAVE_SMEM;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)size;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        B200FC_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_wave_kernel<CG, MODE, false>, &cfg));
-        if (n < 1) n = -1;
-        cache[dev & 63][size].store(n, std::memory_order_relaxed);
-    }
-    *out = n < 0 ? 0 : n;
-    return B200FC_OK;
-}
-
-template <int CG, int MODE>
+template <int CG>
 int max_tiles(int S, int* out) {
+    static ClusterCounts counts;
     int n = 0;
-    const int rc = max_clusters<CG, MODE>(CG * S, &n);
+    const int rc = resident_clusters(counts, CG * S, WAVE_THREADS, WAVE_SMEM, &n);
     if (rc) return rc;
     const int by_sms = num_sms() / (CG * S);
     *out = n < by_sms ? n : by_sms;
@@ -645,7 +618,7 @@ int pick_shape(int M, int nspan, int slabs, int units, int chains, WaveShape* be
     *found = false;
     for (int S = 1; S * CG <= 8 && S <= units; S++) {
         int cap = 0;
-        const int rc = max_tiles<CG, MODE>(S, &cap);
+        const int rc = max_tiles<CG>(S, &cap);
         if (rc) return rc;
         for (int R = 32; R <= 256; R += 32) {
             const int W = R * CG, tiles_n = (nspan + W - 1) / W;
@@ -750,6 +723,8 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     if (p.parts == 1) {
+        rc = allow_smem<CG, MODE, false>();
+        if (rc) return rc;
         B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_wave_kernel<CG, MODE, false>, ma, mw, p));
     } else if constexpr (WQ) {
         rc = allow_smem<CG, MODE, true>();

@@ -257,7 +257,7 @@ __device__ __forceinline__ float postop_staged(float v, int row, int steps, cons
 // the SiLU*up store, then the down projection over the activation the first job wrote): the producer goes straight on
 // into the second matrix, so its first ring of stages arrives while the consumers finish the first job and wait at a
 // grid-wide barrier (every CTA must have stored its part of the activation before anyone multiplies by it).
-template <int WB, int NT, int NJ>
+template <int WB, int NT, int NJ, bool SHORT>
 __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUtensorMap* map1, const Params* p0, const Params* p1) {
     const Params& p = *p0;            // job 0; the role loops below shadow it with the job they work on
     using L = Layout<WB, NT>;
@@ -378,13 +378,16 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
             return v;
         };
         constexpr int RB = ROWS_PER_WARP / 16;  // 16-row MMA blocks per warp
-        // AS > 1 would give every MMA of a 16-byte weight load its own accumulator set (shorter dependent chains);
-        // measured slower (the extra registers spill), so one set is used.
-        constexpr int AS = 1;
-        float acc[AS][RB][NT][4];
+        // (An accumulator set per MMA of a 16-byte weight load, for shorter dependent chains, spills and is slower.)  The tensor core's
+        // error grows with the length of a chain of sums: with SHORT (row blocks in fewer parts than places for CTAs allow) `total`
+        // takes the sums of four stages, or of a chunk of quantised weights, whose scale may change there.  Else `total` is `acc` itself, and
+        // with 4 bits, whose groups of 128 K are added outside the tensor core.  (SHORT everywhere costs 1 %: Llama-7B MLP at 1 row
+        // 51.9 us, 51.4 without.)
+        float acc[RB][NT][4], chain_sums[RB][NT][4];
+        auto& total = *[&] { if constexpr (W4 || !SHORT) return &acc; else return &chain_sums; }();
         // Compressed weights multiply fp16 x fp16, so every staged chunk is scaled per activation row by the power of two
         // that puts the row's largest magnitude (within the chunk) at 2^13 and converted to fp16: exact, since fp16 keeps
-        // the 8-bit significand of bf16.  The accumulators carry the row's current scale (cur_e) and are rescaled when a
+        // the 8-bit significand of bf16.  The sums carry the row's current scale (cur_e) and are rescaled when a
         // new chunk brings a different one; the scale is undone after the last stage of a piece.
         int cur_e[NT][2];
 
@@ -494,14 +497,12 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
                         pow2_factors(cur_e[nt][0] - e0, a1, a2);
                         pow2_factors(cur_e[nt][1] - e1, b1, b2);
 #pragma unroll
-                        for (int as = 0; as < AS; as++)
-#pragma unroll
-                            for (int rb = 0; rb < RB; rb++) {
-                                acc[as][rb][nt][0] = acc[as][rb][nt][0] * a1 * a2;
-                                acc[as][rb][nt][2] = acc[as][rb][nt][2] * a1 * a2;
-                                acc[as][rb][nt][1] = acc[as][rb][nt][1] * b1 * b2;
-                                acc[as][rb][nt][3] = acc[as][rb][nt][3] * b1 * b2;
-                            }
+                        for (int rb = 0; rb < RB; rb++) {
+                            total[rb][nt][0] = total[rb][nt][0] * a1 * a2;
+                            total[rb][nt][2] = total[rb][nt][2] * a1 * a2;
+                            total[rb][nt][1] = total[rb][nt][1] * b1 * b2;
+                            total[rb][nt][3] = total[rb][nt][3] * b1 * b2;
+                        }
                         cur_e[nt][0] = e0; cur_e[nt][1] = e1;
                     }
                 }
@@ -544,10 +545,10 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
                         pow2_factors(cur_e[nt][1] - e1, b1, b2);
 #pragma unroll
                         for (int rb = 0; rb < RB; rb++) {
-                            acc[0][rb][nt][0] = acc[0][rb][nt][0] * a1 * a2;
-                            acc[0][rb][nt][2] = acc[0][rb][nt][2] * a1 * a2;
-                            acc[0][rb][nt][1] = acc[0][rb][nt][1] * b1 * b2;
-                            acc[0][rb][nt][3] = acc[0][rb][nt][3] * b1 * b2;
+                            total[rb][nt][0] = total[rb][nt][0] * a1 * a2;
+                            total[rb][nt][2] = total[rb][nt][2] * a1 * a2;
+                            total[rb][nt][1] = total[rb][nt][1] * b1 * b2;
+                            total[rb][nt][3] = total[rb][nt][3] * b1 * b2;
                         }
                         cur_e[nt][0] = e0; cur_e[nt][1] = e1;
                     }
@@ -573,13 +574,20 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
             const int ks1 = (long long)(p.spr - ks0) < it_end - it ? p.spr : ks0 + (int)(it_end - it);
             const bool first_piece = it == it_begin;
 #pragma unroll
-            for (int as = 0; as < AS; as++)
+            for (int rb = 0; rb < RB; rb++)
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) acc[rb][nt][i] = total[rb][nt][i] = 0.0f;
+            auto add_chain = [&]() {
+                if constexpr (W4 || !SHORT) return;
 #pragma unroll
                 for (int rb = 0; rb < RB; rb++)
 #pragma unroll
                     for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-                        for (int i = 0; i < 4; i++) acc[as][rb][nt][i] = 0.0f;
+                        for (int i = 0; i < 4; i++) { total[rb][nt][i] += acc[rb][nt][i]; acc[rb][nt][i] = 0.0f; }
+            };
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) cur_e[nt][0] = cur_e[nt][1] = 0;
 
@@ -597,6 +605,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
             for (int ks = ks0; ks < ks1; ks++) {
                 const int it_in_chunk = img ? ks % STAGES_PER_CHUNK : (ks - ks0) % STAGES_PER_CHUNK;
                 if (it_in_chunk == 0 || ks == ks0) {
+                    if constexpr (WQ) add_chain();
                     if (img) {
                         stage_img(ks, ks0, ks1, first_piece);
                     } else {
@@ -610,6 +619,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
                 }
                 if (threadIdx.x == 0 && ks == ks0 && first_piece) TRACE_STAMP(2);   // first activation chunk staged
                 // warp-uniform outcome: either every lane goes on to the MMAs or none does
+                if (!WQ && ((ks - ks0) & 3) == 0) add_chain();
                 ok = __all_sync(0xffffffffu, ok && mbar_wait(bar_full + 8 * stage, phase, abort_flag, limit));
                 if (threadIdx.x == 0 && ks == ks0 && first_piece) TRACE_STAMP(7);   // first stage of weights is there
                 if (!ok) continue;
@@ -662,10 +672,10 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
                         const float s0 = sc[rb * 16], s1 = sc[rb * 16 + 8];
 #pragma unroll
                         for (int nt = 0; nt < NT; nt++) {
-                            acc[0][rb][nt][0] = fmaf(grp[nt][0], s0, acc[0][rb][nt][0]);
-                            acc[0][rb][nt][1] = fmaf(grp[nt][1], s0, acc[0][rb][nt][1]);
-                            acc[0][rb][nt][2] = fmaf(grp[nt][2], s1, acc[0][rb][nt][2]);
-                            acc[0][rb][nt][3] = fmaf(grp[nt][3], s1, acc[0][rb][nt][3]);
+                            acc[rb][nt][0] = fmaf(grp[nt][0], s0, acc[rb][nt][0]);
+                            acc[rb][nt][1] = fmaf(grp[nt][1], s0, acc[rb][nt][1]);
+                            acc[rb][nt][2] = fmaf(grp[nt][2], s1, acc[rb][nt][2]);
+                            acc[rb][nt][3] = fmaf(grp[nt][3], s1, acc[rb][nt][3]);
                         }
                     }
                 } else {
@@ -698,8 +708,8 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
                         }
 #pragma unroll
                         for (int nt = 0; nt < NT; nt++) {
-                            if constexpr (W8) mma_f16(acc[q % AS][rb][nt], a0, a1, a2, a3, xb[nt][2 * q], xb[nt][2 * q + 1]);
-                            else mma_bf16(acc[q % AS][rb][nt], a0, a1, a2, a3, xb[nt][2 * q], xb[nt][2 * q + 1]);
+                            if constexpr (W8) mma_f16(acc[rb][nt], a0, a1, a2, a3, xb[nt][2 * q], xb[nt][2 * q + 1]);
+                            else mma_bf16(acc[rb][nt], a0, a1, a2, a3, xb[nt][2 * q], xb[nt][2 * q + 1]);
                         }
                     }
                 }
@@ -712,24 +722,16 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
             }
             it += ks1 - ks0;
             if (threadIdx.x == 0 && it == it_end) TRACE_STAMP(3);   // last stage multiplied
-            // the accumulator sets are added in a fixed order
-#pragma unroll
-            for (int as = 1; as < AS; as++)
-#pragma unroll
-                for (int rb = 0; rb < RB; rb++)
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-                        for (int i = 0; i < 4; i++) acc[0][rb][nt][i] += acc[as][rb][nt][i];
+            add_chain();
             if constexpr (WQ) {
 #pragma unroll
                 for (int nt = 0; nt < NT; nt++)
 #pragma unroll
                     for (int rb = 0; rb < RB; rb++) {
-                        acc[0][rb][nt][0] = scalbnf(acc[0][rb][nt][0], cur_e[nt][0]);
-                        acc[0][rb][nt][2] = scalbnf(acc[0][rb][nt][2], cur_e[nt][0]);
-                        acc[0][rb][nt][1] = scalbnf(acc[0][rb][nt][1], cur_e[nt][1]);
-                        acc[0][rb][nt][3] = scalbnf(acc[0][rb][nt][3], cur_e[nt][1]);
+                        total[rb][nt][0] = scalbnf(total[rb][nt][0], cur_e[nt][0]);
+                        total[rb][nt][2] = scalbnf(total[rb][nt][2], cur_e[nt][0]);
+                        total[rb][nt][1] = scalbnf(total[rb][nt][1], cur_e[nt][1]);
+                        total[rb][nt][3] = scalbnf(total[rb][nt][3], cur_e[nt][1]);
                     }
             }
 
@@ -741,10 +743,10 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
                 for (int nt = 0; nt < NT; nt++) {
                     const int row = rg * ROWS_PER_WARP + rb * 16 + g, tok = nt * 8 + 2 * t;
                     float* pp = part + kh * PART_HALF;
-                    pp[tok * ROWS_PER_CTA + row] = acc[0][rb][nt][0];
-                    pp[(tok + 1) * ROWS_PER_CTA + row] = acc[0][rb][nt][1];
-                    pp[tok * ROWS_PER_CTA + row + 8] = acc[0][rb][nt][2];
-                    pp[(tok + 1) * ROWS_PER_CTA + row + 8] = acc[0][rb][nt][3];
+                    pp[tok * ROWS_PER_CTA + row] = total[rb][nt][0];
+                    pp[(tok + 1) * ROWS_PER_CTA + row] = total[rb][nt][1];
+                    pp[tok * ROWS_PER_CTA + row + 8] = total[rb][nt][2];
+                    pp[(tok + 1) * ROWS_PER_CTA + row + 8] = total[rb][nt][3];
                 }
             consumer_sync();
 
@@ -904,9 +906,9 @@ __device__ __forceinline__ void decode_body(const CUtensorMap* map0, const CUten
     if (threadIdx.x == 0 && *abort_flag) atomicExch(p.status, 3);
 }
 
-template <int WB, int NT>
+template <int WB, int NT, bool SHORT>
 __global__ void __launch_bounds__(THREADS, 2) gemv_tma_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
-    decode_body<WB, NT, 1>(&map_w, &map_w, &p, &p);
+    decode_body<WB, NT, 1, SHORT>(&map_w, &map_w, &p, &p);
 }
 
 // gate/up (SiLU*up store into the activation) and down projection of a decode-shaped MLP in one launch (bf16 weights)
@@ -914,7 +916,7 @@ template <int NT>
 __global__ void __launch_bounds__(THREADS, 2) mlp_decode_kernel(const __grid_constant__ CUtensorMap map_gate_up,
                                                                 const __grid_constant__ CUtensorMap map_down,
                                                                 const Params p_gate_up, const Params p_down) {
-    decode_body<16, NT, 2>(&map_gate_up, &map_down, &p_gate_up, &p_down);
+    decode_body<16, NT, 2, false>(&map_gate_up, &map_down, &p_gate_up, &p_down);
 }
 
 
@@ -998,9 +1000,12 @@ __global__ void __launch_bounds__(CTHREADS) xstage_kernel(const unsigned char* _
 // swizzle: the canonical operand layout), B = a 16-token x 64 K tile of the activations that travels with the stage
 // (second TMA box, rows >= M zero-filled), D = 128 rows x 16 tokens of fp32 in TMEM.  No register copies of the
 // weights, no activation staging, no barriers between the warps in the loop; sixteen tokens cost what one costs.
-// Roles: warps 0-7 finish pieces (warps 0-3 read the accumulator, one TMEM lane quarter each), warp 8 lane 0 = TMA
-// producer, warp 9 lane 0 = MMA issuer.  Two accumulator buffers (2 x 16 TMEM columns) let the issuer start the next
-// piece while the previous one is reduced.
+// Roles: warps 0-7 finish pieces (warps 0-3 read the accumulators, one TMEM lane quarter each), warp 8 = TMA
+// producer, warp 9 = MMA issuer.  The stages of a piece take four accumulators (16 TMEM columns each) in turn, because the tensor
+// core's error grows with the length of a chain of sums; two sets of them let the issuer start the next piece while the previous one
+// is reduced.
+constexpr int TC_CHAINS = 4;
+constexpr int TC_TMEM = 2 * TC_CHAINS * 16;
 constexpr int TC_THREADS = (CWARPS + 2) * 32;
 constexpr int TC_X_BYTES = 16 * STAGE_K_BYTES;             // activation tile of a stage: 16 tokens x 128 bytes of K
 constexpr int TC_STAGE_BYTES = STAGE_BYTES + TC_X_BYTES;   // 18 KB, a multiple of 1024
@@ -1071,8 +1076,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == CWARPS + 1) {   // the issuer's warp owns the tensor memory: 32 columns = two accumulators of 16
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(32u) : "memory");
+    if (warp == CWARPS + 1) {   // the issuer's warp owns the tensor memory
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"((unsigned)TC_TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -1082,40 +1087,39 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
     const unsigned tmem_base = *tmem_holder;
 
     if (warp == CWARPS) {
-        // ---------------- producer ----------------
-        if (lane == 0) {
-            int stage = 0;
-            unsigned phase = 0;
-            int rb = (int)(it_begin / p.spr), ks = (int)(it_begin - (long long)rb * p.spr);
-            // weights never depend on the previous kernel: the first ring of stages is asked for at once, its activation
-            // tiles only after the previous kernel of the stream has completed
-            const long long n_first = it_end - it_begin < TC_STAGES ? it_end - it_begin : TC_STAGES;
-            {
-                int rb2 = rb, ks2 = ks;
-                for (int i = 0; i < (int)n_first; i++) {
-                    mbar_expect_tx(bar_full + 8 * i, TC_STAGE_BYTES);
-                    tma_load_2d(smem_u32(smem + i * TC_STAGE_BYTES), &map_w, bar_full + 8 * i, ks2 * STAGE_K_BYTES, p.n0 + rb2 * ROWS_PER_CTA);
-                    if (++ks2 == p.spr) { ks2 = 0; rb2++; }
-                }
-            }
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            bool alive = true;
-            for (long long it = it_begin; it < it_end && alive; it++) {
-                const bool pre = it - it_begin < n_first;     // weights already on their way
-                if (!pre) {
-                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, limit)) { alive = false; break; }
-                    mbar_expect_tx(bar_full + 8 * stage, TC_STAGE_BYTES);
-                    tma_load_2d(smem_u32(smem + stage * TC_STAGE_BYTES), &map_w, bar_full + 8 * stage, ks * STAGE_K_BYTES,
-                                p.n0 + rb * ROWS_PER_CTA);
-                }
-                tma_load_2d(smem_u32(smem + stage * TC_STAGE_BYTES + STAGE_BYTES), &map_x, bar_full + 8 * stage, ks * (STAGE_K_BYTES / 2), 0);
-                if (++ks == p.spr) { ks = 0; rb++; }
-                if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
+        // ---------------- producer (the whole warp, see elect_one) ----------------
+        int stage = 0;
+        unsigned phase = 0;
+        int rb = (int)(it_begin / p.spr), ks = (int)(it_begin - (long long)rb * p.spr);
+        auto load_w = [&](int slot, int r, int k) {
+            mbar_expect_tx(bar_full + 8 * slot, TC_STAGE_BYTES);
+            tma_load_2d(smem_u32(smem + slot * TC_STAGE_BYTES), &map_w, bar_full + 8 * slot, k * STAGE_K_BYTES, p.n0 + r * ROWS_PER_CTA);
+        };
+        // weights never depend on the previous kernel: the first ring of stages is asked for at once, its activation
+        // tiles only after the previous kernel of the stream has completed
+        const int n_first = (int)min((long long)TC_STAGES, it_end - it_begin);
+        {
+            int rb2 = rb, ks2 = ks;
+            for (int i = 0; i < n_first; i++) {
+                if (elect_one()) load_w(i, rb2, ks2);
+                if (++ks2 == p.spr) { ks2 = 0; rb2++; }
             }
         }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        for (long long it = it_begin; it < it_end; it++) {
+            const bool pre = it - it_begin < n_first;     // weights already on their way
+            if (!pre && !__all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, limit))) break;
+            if (elect_one()) {
+                if (!pre) load_w(stage, rb, ks);
+                tma_load_2d(smem_u32(smem + stage * TC_STAGE_BYTES + STAGE_BYTES), &map_x, bar_full + 8 * stage, ks * (STAGE_K_BYTES / 2), 0);
+            }
+            if (++ks == p.spr) { ks = 0; rb++; }
+            if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
+        }
+        __syncwarp();
     } else if (warp == CWARPS + 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // ---------------- MMA issuer (the whole warp, see elect_one) ----------------
+        {
             // instruction descriptor: fp32 accumulator, bf16 x bf16, K-major operands, N = 16, M = 128
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
             int stage = 0;
@@ -1128,20 +1132,25 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
                 const int ks0 = (int)(it - (long long)rbk * p.spr);
                 const int ks1 = (long long)(p.spr - ks0) < it_end - it ? p.spr : ks0 + (int)(it_end - it);
                 const int ab = piece & 1;
-                if (!mbar_wait(bar_acc_empty + 8 * ab, ((unsigned)(piece >> 1) & 1) ^ 1, abort_flag, limit)) { alive = false; break; }
+                alive = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty + 8 * ab, ((unsigned)(piece >> 1) & 1) ^ 1, abort_flag, limit));
+                if (!alive) break;
                 tc_fence_after();
-                const unsigned d_tmem = tmem_base + (unsigned)(ab * 16);
                 for (int ks = ks0; ks < ks1; ks++) {
-                    if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, limit)) { alive = false; break; }
+                    alive = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, limit));
+                    if (!alive) break;
                     tc_fence_after();
+                    const int i = ks - ks0;
+                    const unsigned d_tmem = tmem_base + (unsigned)((ab * TC_CHAINS + i % TC_CHAINS) * 16);
                     const unsigned sa = smem_u32(smem + stage * TC_STAGE_BYTES);
                     const unsigned long long adesc = tc_smem_desc(sa), bdesc = tc_smem_desc(sa + STAGE_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++)     // 4 x 16 K per stage, 32 bytes further along the swizzled row each
-                        tc_mma_bf16(d_tmem, adesc + (unsigned long long)(k * 2), bdesc + (unsigned long long)(k * 2), idesc,
-                                    (unsigned)(((ks - ks0) | k) != 0));
-                    tc_commit(bar_empty + 8 * stage);
-                    if (ks == ks1 - 1) tc_commit(bar_acc_full + 8 * ab);
+                        for (int k = 0; k < 4; k++)     // 4 x 16 K per stage, 32 bytes further along the swizzled row each
+                            tc_mma_bf16(d_tmem, adesc + (unsigned long long)(k * 2), bdesc + (unsigned long long)(k * 2), idesc,
+                                        (unsigned)(i >= TC_CHAINS || k != 0));
+                        tc_commit(bar_empty + 8 * stage);
+                        if (ks == ks1 - 1) tc_commit(bar_acc_full + 8 * ab);
+                    }
                     if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
                 }
                 it += ks1 - ks0;
@@ -1180,17 +1189,19 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
             if (warp < 4) {
                 ok = __all_sync(0xffffffffu, ok && mbar_wait(bar_acc_full + 8 * ab, (unsigned)(piece >> 1) & 1, abort_flag, limit));
                 tc_fence_after();
-                unsigned r[16];
-                if (ok) {
-                    tc_ld16(tmem_base + ((unsigned)(warp * 32) << 16) + (unsigned)(ab * 16), r);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                } else {
+                float sum[16];
 #pragma unroll
-                    for (int j = 0; j < 16; j++) r[j] = 0u;
+                for (int j = 0; j < 16; j++) sum[j] = 0.0f;
+                for (int c = 0; ok && c < min(TC_CHAINS, ks1 - ks0); c++) {
+                    unsigned r[16];
+                    tc_ld16(tmem_base + ((unsigned)(warp * 32) << 16) + (unsigned)((ab * TC_CHAINS + c) * 16), r);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 16; j++) sum[j] += __uint_as_float(r[j]);
                 }
                 const int row = warp * 32 + lane;
 #pragma unroll
-                for (int j = 0; j < 16; j++) part[j * ROWS_PER_CTA + row] = __uint_as_float(r[j]);
+                for (int j = 0; j < 16; j++) part[j * ROWS_PER_CTA + row] = sum[j];
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_acc_empty + 8 * ab);
@@ -1299,7 +1310,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
     __syncthreads();
     if (warp == CWARPS + 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(32u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((unsigned)TC_TMEM) : "memory");
     }
     if (threadIdx.x == 0 && *abort_flag) atomicExch(p.status, 3);
 }
@@ -1327,7 +1338,7 @@ int device_sms() {
     return n > 0 ? n : 148;
 }
 
-template <int WB, int NT>
+template <int WB, int NT, bool SHORT>
 int launch_variant(const CUtensorMap& map, const Params& p_in, int grid, cudaStream_t s) {
     const int cluster = p_in.cluster ? p_in.S : 1;
     using L = Layout<WB, NT>;
@@ -1335,7 +1346,7 @@ int launch_variant(const CUtensorMap& map, const Params& p_in, int grid, cudaStr
     static std::atomic<unsigned long long> attr_devices{0};
     {
         const int arc = once_per_device(attr_devices, [] {
-            B200FC_CUDA(cudaFuncSetAttribute(gemv_tma_kernel<WB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM));
+            B200FC_CUDA(cudaFuncSetAttribute(gemv_tma_kernel<WB, NT, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM));
             return (int)B200FC_OK;
         });
         if (arc) return arc;
@@ -1378,7 +1389,7 @@ int launch_variant(const CUtensorMap& map, const Params& p_in, int grid, cudaStr
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemv_tma_kernel<WB, NT>, map, p));
+    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemv_tma_kernel<WB, NT, SHORT>, map, p));
     count_launch();
     return B200FC_OK;
 }
@@ -1524,38 +1535,52 @@ int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, i
     if (rc) return rc;
     p.pf_cap = g_pf_cap;
     const long long gmax = max_ctas();
+    // Measured (Llama-7B MLP, decode): 58.6 against 61.6 us at M = 16, 53.3 against 51.2 us at M = 1 — the tensor-memory
+    // path costs a token column nothing but pays a little for its activation tiles at every stage, so it takes the
+    // calls with more than 8 rows.  B200FC_GEMV_TC=0 never uses it, =2 always.
+    static int use_tc = -1;
+    if (use_tc < 0) { const char* e = getenv("B200FC_GEMV_TC"); use_tc = e ? atoi(e) : 1; }
+    const bool tc = w.dtype == B200FC_BF16 && (((uintptr_t)A | (uintptr_t)lda) & 15) == 0 && (use_tc == 2 || (use_tc == 1 && M > 8));
+    const bool w4 = w.dtype == B200FC_S4, w8 = w.dtype == B200FC_S8;
     // Three ways to cut the work; the cost model counts the stages of the longest CTA plus the time of the reduction
     // that follows, in units of one stage's streaming time.
     //   stream-K: equal pieces whatever the shape; a CTA may hold the end of one row block and the start of the next,
     //             partial sums meet through the global scratch (several round trips to L2, twice for such a CTA);
     //   aligned:  S pieces per row block, one per CTA.  S = 1 needs no reduction; 2 <= S <= 8 runs as clusters of S CTAs
-    //             whose partial sums meet in distributed shared memory (fast, so this wins for small matrices).
+    //             whose partial sums meet in distributed shared memory (fast).  Always taken while there are two places or more per
+    //             row block (bf16, us, stream-K / aligned at 4 rows: 4096 x 9216 20.4 / 16.2, x 12288 24.6 / 21.1, x 18944 27.8 / 27.1,
+    //             11008 x 9216 40.9 / 34.7; above that line the whole row blocks of a gate/up projection slow the next kernel down:
+    //             Llama-7B block at 1 row 55 / 61).
     long long grid = gmax < p.total / 2 ? gmax : p.total / 2;
     if (grid < 1) grid = 1;
-    long long best = (p.total + grid - 1) / grid + 6;
+    const long long best = (p.total + grid - 1) / grid + 6;
+    bool short_chains = false;
     if (!g_force_stream && row_blocks <= gmax) {
         int S = (int)(gmax / row_blocks);
         if (S > 8) S = 8;
         if (S > p.spr / 2) S = p.spr / 2;
         if (S < 1) S = 1;
+        const int places_S = S;
+        static ClusterCounts counts;        // (every variant takes two places per SM)
+        rc = fit_clusters(counts, THREADS, Layout<16, 1>::SMEM, row_blocks, &S);
+        if (rc) return rc;
         const long long cost = (p.spr + S - 1) / S + (S > 1 ? 1 : 0);
-        if (cost <= best || g_force_aligned) { best = cost; p.S = S; p.cluster = S > 1 ? 1 : 0; grid = (long long)row_blocks * S; }
+        if (2 * row_blocks <= gmax || cost <= best || g_force_aligned) {
+            short_chains = S < places_S || cost > best;
+            p.S = S; p.cluster = S > 1 ? 1 : 0;
+            grid = (long long)row_blocks * S;
+        }
     }
-    if (w.dtype == B200FC_S4) {
+    if (w4) {
         if (!w.scale_grp || (n0 % ROWS_PER_CTA)) { set_error("gemv: 4-bit weights need group scales and n0 %% 128 == 0"); return B200FC_ERR_INVALID; }
-        return M <= 8 ? launch_variant<4, 1>(map, p, (int)grid, s) : launch_variant<4, 2>(map, p, (int)grid, s);
+        return M <= 8 ? launch_variant<4, 1, false>(map, p, (int)grid, s) : launch_variant<4, 2, false>(map, p, (int)grid, s);
     }
-    if (w.dtype == B200FC_BF16 && (((uintptr_t)A | (uintptr_t)lda) & 15) == 0) {
-        // Measured (Llama-7B MLP, decode): 58.6 against 61.6 us at M = 16, 53.3 against 51.2 us at M = 1 — the tensor-memory
-        // path costs a token column nothing but pays a little for its activation tiles at every stage, so it takes the
-        // calls with more than 8 rows.  B200FC_GEMV_TC=0 never uses it, =2 always.
-        static int use_tc = -1;
-        if (use_tc < 0) { const char* e = getenv("B200FC_GEMV_TC"); use_tc = e ? atoi(e) : 1; }
-        if (use_tc == 2 || (use_tc == 1 && M > 8)) return launch_tc(map, p, A, M, K, lda, (int)grid, s);
-    }
-    const bool w8 = w.dtype == B200FC_S8;
-    if (M <= 8) return w8 ? launch_variant<8, 1>(map, p, (int)grid, s) : launch_variant<16, 1>(map, p, (int)grid, s);
-    return w8 ? launch_variant<8, 2>(map, p, (int)grid, s) : launch_variant<16, 2>(map, p, (int)grid, s);
+    if (tc) return launch_tc(map, p, A, M, K, lda, (int)grid, s);
+    auto launch = M <= 8 ? (w8 ? (short_chains ? launch_variant<8, 1, true> : launch_variant<8, 1, false>)
+                               : (short_chains ? launch_variant<16, 1, true> : launch_variant<16, 1, false>))
+                         : (w8 ? (short_chains ? launch_variant<8, 2, true> : launch_variant<8, 2, false>)
+                               : (short_chains ? launch_variant<16, 2, true> : launch_variant<16, 2, false>));
+    return launch(map, p, (int)grid, s);
 }
 
 template <int NT>

@@ -10,7 +10,7 @@
 // ([16 rows] x 64 K tiles that travel with the stage) are the B operand.  Widened weights never touch shared memory, whose
 // bandwidth they would exceed (five bytes per weight instead of two), activations are not converted, and sixteen rows cost
 // what one costs.
-//   int8   : exact in bf16; the stages take four fp32 accumulators in turn, which are added at the end: the tensor core's error
+//   int8   : exact in bf16; the stages take four fp32 accumulators (or eight) in turn, which are added at the end: the tensor core's error
 //            grows with the length of a chain of sums (16 x 4096 x 11008, relative to float64: 1.9e-7 in one chain, 0.8e-7 in
 //            four, 1.1e-7 with mma.sync's chains).
 //   4 bits : the integers are multiplied; every group of 128 K has an accumulator of its own, which the warp of its rows reads
@@ -28,15 +28,18 @@ namespace {
 
 constexpr int TQ_ROWS = 128;
 constexpr int TQ_THREADS = 384;
-constexpr int A_BUFS = 3, A_COLS = 64;            // A buffers: 128 K of bf16 = 64 columns
-constexpr int D_BUFS = 4, D_COLS = 16;
-constexpr int TQ_TMEM = 256;                      // 3 x 64 + 4 x 16; two CTAs share an SM's 512 columns
+constexpr int A_COLS = 64, D_COLS = 16;           // an A buffer: 128 K of bf16; an accumulator: 16 rows of activations
+constexpr int TQ_TMEM = 256;                      // two CTAs share an SM's 512 columns
 constexpr int X_TILE = 16 * SLAB_BYTES;           // 16 rows x 64 K of activations
 constexpr int W_STAGE = TQ_ROWS * SLAB_BYTES;
 
-template <int WB> struct TqLayout {
+// LONG: for calls whose K is split less than the places for CTAs would allow, so that the chains of sums get no longer.  int8: two A
+// buffers and eight accumulators instead of three and four (4 x 4096 x 5032: 10.4 us, 10.2 without).  4 bits: a second level of
+// sums in registers (4 x 4096 x 11008, which is not such a call: 12.5 us, 11.8 without).
+template <int WB, bool LONG = false> struct TqLayout {
     static constexpr int PIECES = WB == 4 ? 2 : 1;                    // pieces of 128 K per stage
     static constexpr int STAGES = WB == 4 ? 4 : 5;
+    static constexpr int A_BUFS = LONG && WB == 8 ? 2 : 3, D_BUFS = (TQ_TMEM - A_BUFS * A_COLS) / D_COLS;
     static constexpr int X_BYTES = PIECES * 2 * X_TILE;
     static constexpr int SC_BYTES = WB == 4 ? 2 * TQ_ROWS * 4 : 0;    // the stage's 2 x 128 group scales
     static constexpr int STAGE = W_STAGE + X_BYTES + SC_BYTES;
@@ -75,11 +78,11 @@ __device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsi
         ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-template <int WB>
+template <int WB, bool LONG>
 __global__ void __launch_bounds__(TQ_THREADS, 2)
 gemv_tq_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TqParams p) {
-    using L = TqLayout<WB>;
-    constexpr int PIECES = L::PIECES, STAGES = L::STAGES;
+    using L = TqLayout<WB, LONG>;
+    constexpr int PIECES = L::PIECES, STAGES = L::STAGES, A_BUFS = L::A_BUFS, D_BUFS = L::D_BUFS;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + (((smem_u32(smem_raw) + 1023u) & ~1023u) - smem_u32(smem_raw));
     float* part = (float*)(smem + L::PART_OFF);
@@ -190,9 +193,9 @@ gemv_tq_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const unsigned lane_base = (unsigned)(quarter * 32) << 16;
         const Epilogue& ep = p.ep;
         bool ok = true;
-        float acc[16];
+        float acc[16], total[16];       // (total: 4 bits and LONG, the sums of eight groups of a set)
 #pragma unroll
-        for (int t = 0; t < 16; t++) acc[t] = 0.0f;
+        for (int t = 0; t < 16; t++) acc[t] = total[t] = 0.0f;
         float sc_prev = 0.0f;
         // 4 bits: group sum of piece g -> acc += sum * scale
         auto take_group = [&](int g, float sc) {
@@ -208,6 +211,10 @@ gemv_tq_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_d_empty + 8 * db);
+            if (LONG && ((g >> 1) & 7) == 7) {
+#pragma unroll
+                for (int t = 0; t < 16; t++) { total[t] += acc[t]; acc[t] = 0.0f; }
+            }
         };
 #pragma unroll 1
         for (int g = set; g < n_pieces && ok; g += 2) {
@@ -275,6 +282,10 @@ gemv_tq_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         if constexpr (WB == 4) {
             const int last = n_pieces - 2 + set;       // (a set's last piece; n_pieces is even)
             if (ok && last >= 0) take_group(last, sc_prev);
+            if constexpr (LONG) {
+#pragma unroll
+                for (int t = 0; t < 16; t++) acc[t] += total[t];
+            }
         } else if (set == 0) {
             ok = __all_sync(0xffffffffu, ok && mbar_wait(bar_d_full, 0, abort_flag, limit));
             tc_fence_after();
@@ -339,12 +350,12 @@ gemv_tq_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     else __syncthreads();
 }
 
-template <int WB>
+template <int WB, bool LONG>
 int run_tq(const CUtensorMap& mw, const CUtensorMap& mx, const TqParams& p, int grid, cudaStream_t s) {
-    using L = TqLayout<WB>;
+    using L = TqLayout<WB, LONG>;
     static std::atomic<unsigned long long> attr_devices{0};
     const int arc = once_per_device(attr_devices, [] {
-        B200FC_CUDA(cudaFuncSetAttribute(gemv_tq_kernel<WB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM));
+        B200FC_CUDA(cudaFuncSetAttribute(gemv_tq_kernel<WB, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM));
         return (int)B200FC_OK;
     });
     if (arc) return arc;
@@ -361,7 +372,7 @@ int run_tq(const CUtensorMap& mw, const CUtensorMap& mx, const TqParams& p, int 
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemv_tq_kernel<WB>, mw, mx, p));
+    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemv_tq_kernel<WB, LONG>, mw, mx, p));
     count_launch();
     return B200FC_OK;
 }
@@ -390,6 +401,10 @@ int launch_gemv_tq(const Weight& w, const void* A, int M, int K, int64_t lda, in
     if (S > 8) S = 8;
     if (S > p.spr / 2) S = p.spr / 2;
     if (S < 1) S = 1;
+    const int places_S = S;
+    static ClusterCounts counts;
+    int rc = fit_clusters(counts, TQ_THREADS, es == 4 ? TqLayout<4>::SMEM : TqLayout<8>::SMEM, row_blocks, &S);   // (two per SM, either)
+    if (rc) return rc;
     p.S = S;
     p.M = M; p.n0 = n0; p.n1 = n1;
     p.ep = ep;
@@ -398,11 +413,13 @@ int launch_gemv_tq(const Weight& w, const void* A, int M, int K, int64_t lda, in
     if (!p.status) { set_error("gemv: no kernel status word on this device"); return B200FC_ERR_CUDA; }
     p.wait_limit_ns = wait_limit_ns();
     CUtensorMap mw, mx;
-    int rc = make_map(&mw, w.data, true, (uint64_t)w.ld_bytes(), (uint64_t)w.N_pad, (uint64_t)w.ld_bytes(), TQ_ROWS);
+    rc = make_map(&mw, w.data, true, (uint64_t)w.ld_bytes(), (uint64_t)w.N_pad, (uint64_t)w.ld_bytes(), TQ_ROWS);
     if (rc) return rc;
     rc = make_map(&mx, A, false, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 16);
     if (rc) return rc;
-    return es == 4 ? run_tq<4>(mw, mx, p, row_blocks * S, s) : run_tq<8>(mw, mx, p, row_blocks * S, s);
+    const int grid = row_blocks * S;
+    if (S < places_S) return es == 4 ? run_tq<4, true>(mw, mx, p, grid, s) : run_tq<8, true>(mw, mx, p, grid, s);
+    return es == 4 ? run_tq<4, false>(mw, mx, p, grid, s) : run_tq<8, false>(mw, mx, p, grid, s);
 }
 
 }  // namespace b200fc

@@ -88,15 +88,6 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
         : "memory");
 }
-// One lane of a converged warp, the same one every time.  The issuing loops below run as whole warps and elect the lane only
-// around the TMA / MMA / commit instructions: these take their operands from uniform registers, which the compiler can keep
-// them in only while the control flow is warp-uniform.  With the loop inside `if (lane == 0)` every MMA cost about 100 clocks of
-// issue and every slab 480 more (880 clocks per 128 bytes of K however few columns a tile has).
-__device__ __forceinline__ bool elect_one() {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
-    return ok != 0;
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(unsigned bar) {

@@ -19,6 +19,10 @@ SHAPES = [
     (1000, 4096),     # odd K in eight parts
     (2048, 20008),    # one part, more row blocks than SMs
     (264, 40000),     # more row blocks than CTAs are resident
+    (2048, 4360),     # 35, 49, 72 and 94 row blocks: one more than the clusters of 8, 6, 4 and 3 CTAs that are resident together can
+    (2048, 6200),     # be given, so K is cut into one part less (int8: with eight accumulators)
+    (2304, 9216),
+    (2304, 12032),
 ]
 
 

@@ -257,6 +257,17 @@ def test_ragged_last_round_goes_through_a_k_split_launch():
     assert np.array_equal(got, port.postops(port.gemm_bf16(A, B), port.BIAS, port.F32, bias=bias))
 
 
+@pytest.mark.parametrize("M", [3, 12])
+@pytest.mark.parametrize("K,N", [(2048, 4360), (2048, 6200), (2304, 9216), (2304, 12032), (1096, 18952)])
+def test_decode_parts_exact(K, N, M):
+    """Decode calls whose row blocks are one more than the clusters of 8, 6, 4 and 3 CTAs that are resident together (K is cut into a part
+    less), and one more than the SMs; chunks of K that end inside a part."""
+    rng = np.random.default_rng(K + N + M)
+    A = H.two_valued_bf16(rng, (M, K)); B = H.two_valued_bf16(rng, (K, N))
+    w = H.pack(B, False)
+    assert np.array_equal(H.run_matmul(w, A, capi.F32), port.gemm_bf16(A, B))
+
+
 @pytest.mark.parametrize("M,K,N", [(512, 192, 10280), (300, 128, 20000), (1024, 64, 5000), (700, 96, 7177)])
 def test_many_tiles_exact(M, K, N):
     """more 256 x 256 tiles than CTA pairs: without the one-wave kernel (test_gpu_persistent.py) every pair walks several tiles and
