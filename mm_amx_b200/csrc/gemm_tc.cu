@@ -686,7 +686,6 @@ int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cuda
     p.splits = splits;
     p.split_stride = 0;
     const Epilogue final_ep = p.ep;
-    const int final_vec = p.vec_ok;
     int pitch = 0;
     if (splits > 1) {
         const int nspan = p.n1 - p.n0;
@@ -728,7 +727,6 @@ int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cuda
                                        (long long)p.M * pitch, pitch, splits, p.M, p.n0, p.n1, p.acc_is_int, final_ep));
         count_launch();
     }
-    (void)final_vec;
     return B200FC_OK;
 }
 
@@ -863,11 +861,7 @@ int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, co
     p.splits = 1; p.split_stride = 0;
     p.ar_world = 0; p.ar_rank = 0; p.ar_phases = 3; p.ar_gemm_pairs = 0; p.ar_work_counter = 0; p.ar_target = 0; p.ar_partial_mc = nullptr; p.ar_out_mc = nullptr;
     for (int i = 0; i < 8; i++) p.ar_flags[i] = nullptr;
-    int es = ep.out_dtype == B200FC_F32 || ep.out_dtype == B200FC_S32 ? 4 : (ep.out_dtype == B200FC_BF16 ? 2 : 1);
-    if (ep.steps & B200FC_STEP_SILU_MUL)
-        p.vec_ok = (((uintptr_t)ep.C & 15) == 0 && (ep.ldc & 15) == 0 && (n0 % 32) == 0) ? 1 : 0;
-    else
-        p.vec_ok = (((uintptr_t)ep.C & 15) == 0 && (ep.ldc & 15) == 0 && ((n0 * es) & 15) == 0) ? 1 : 0;
+    p.vec_ok = output_vec(ep, n0);
     if (ep.out_dtype == B200FC_S32 && !i8) { set_error("raw int32 output needs an 8-bit GEMM"); return B200FC_ERR_INVALID; }
     if (ep.mc_reduce && (ep.steps != 0 || i8 || ((n0 | n1) & 1) || ((uintptr_t)ep.C & 3) || (ep.ldc & 3))) {
         set_error("multicast-reduce output needs a bf16 GEMM without post-ops and an even, 4-byte aligned column range");

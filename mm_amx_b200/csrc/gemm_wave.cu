@@ -699,9 +699,7 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
     p.status = kernel_status_word();
     if (!p.status) { set_error("gemm: no kernel status word on this device"); return B200FC_ERR_CUDA; }
     p.wait_limit_ns = wait_limit_ns();
-    const int es = ep.out_dtype == B200FC_F32 || ep.out_dtype == B200FC_S32 ? 4 : (ep.out_dtype == B200FC_BF16 ? 2 : 1);
-    const bool c_aligned = ((uintptr_t)ep.C & 15) == 0 && (ep.ldc & 15) == 0;
-    p.vec_ok = c_aligned && ((ep.steps & B200FC_STEP_SILU_MUL) ? (n0 % 32) == 0 : ((n0 * es) & 15) == 0) ? 1 : 0;
+    p.vec_ok = output_vec(ep, n0);
 
     CUtensorMap ma, mw;
     int rc = make_map(&ma, call.A, I8, (uint64_t)call.K, (uint64_t)call.M, (uint64_t)call.lda, BM);

@@ -211,6 +211,16 @@ def test_s8_postops(M):
                 assert (ref == 127).any() or (ref == -128).any() or True
 
 
+@pytest.mark.parametrize("M,K,N", [(17, 192, 40), (300, 256, 1240), (2600, 64, 5992)])
+def test_s8_rows_of_8_bytes(M, K, N):
+    """int8 output rows that are 8-byte but not 16-byte aligned, in one tile, in one wave and in many tiles; every value exact"""
+    rng = np.random.default_rng(M + N)
+    A = rng.integers(-128, 128, (M, K), dtype=np.int8); B = rng.integers(-128, 128, (K, N), dtype=np.int8)
+    bias = rng.integers(-512, 513, N).astype(np.float32)
+    got = H.run_matmul(H.pack(B), A, capi.S8, steps=capi.STEP_BIAS | capi.STEP_QUANT, bias=bias, q_scale=2.0 ** -11)
+    assert np.array_equal(got, port.postops(port.gemm_i8(A, B), port.BIAS | port.QUANT, port.S8, bias=bias, q_scale=2.0 ** -11))
+
+
 @pytest.mark.parametrize("M,K,N", [(100, 4096, 512), (256, 4096, 1024), (64, 2304, 300), (17, 8192, 256)])
 def test_split_k_shapes_exact(M, K, N):
     """few output tiles and a long K: K is split over the CTAs of a cluster; without the one-wave kernel (test_gpu_persistent.py) over
