@@ -29,6 +29,10 @@ constexpr int ATT_THREADS = ATT_WARPS * 32;
 constexpr int BLK = 16;            // tokens per block (one k-step of the P V product)
 constexpr int ATT_STAGES = 3;
 constexpr int MAX_SPLITS = 64;
+// Heads of 64 have rings of 48 KB a CTA and half the work per block: two CTAs per SM neither fill the memory system nor hide the
+// chain of a block (scores, softmax, values).  us with two / four: B = 14, 16 kv heads, up to 14313 tokens 174 / 106; B = 20, 4 kv heads,
+// up to 5747 tokens 31.3 / 20.4.  Heads of 128: two fill shared memory.
+template <int D> constexpr int ATT_CTAS_PER_SM = D == 64 ? 4 : 2;
 
 struct AttnParams {
     const unsigned char* q; long long q_bs, q_hs;          // bytes
@@ -82,7 +86,7 @@ template <int D> struct AttnSmem {
 };
 
 template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM<D>) decode_attention_kernel(const AttnParams p) {
     using SM = AttnSmem<D>;
     constexpr int CHUNKS = D / 8;          // 16-byte chunks per token row
     constexpr int KSTEPS = D / 16;
@@ -286,14 +290,37 @@ __global__ void __launch_bounds__(D) attention_combine_kernel(const AttnParams p
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int head = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
     const size_t base = ((size_t)b * p.H + head) * p.splits;
-    float m = -INFINITY;
-    for (int sp = 0; sp < p.splits; sp++) m = fmaxf(m, p.ws_ml[(base + sp) * 2]);
-    float l = 0.0f, acc = 0.0f;
-    for (int sp = 0; sp < p.splits; sp++) {
-        const float ms = p.ws_ml[(base + sp) * 2];
-        const float f = ms == -INFINITY ? 0.0f : exp2f(ms - m);
-        l = fmaf(p.ws_ml[(base + sp) * 2 + 1], f, l);
-        acc = fmaf(p.ws_o[(base + sp) * D + d], f, acc);
+    // a warp's lanes hold the maxima and sums of two splits each; the weights then reach the loop over the splits by shuffles, and its
+    // loads travel eight at a time (B = 1, 8 kv heads of 128, 8192 tokens in 37 splits: 12.3 us for the whole call, 15.2 with a plain loop)
+    const int lane = d & 31;
+    float ms[2], f[2], v[8], m = -INFINITY, l = 0.0f, acc = 0.0f;
+    const float* src = p.ws_o + base * D + d;
+    auto load8 = [&](int s0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = s0 + i < p.splits ? src[(size_t)(s0 + i) * D] : 0.0f;
+    };
+    load8(0);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int sp = h * 32 + lane;
+        ms[h] = sp < p.splits ? p.ws_ml[(base + sp) * 2] : -INFINITY;
+        f[h] = sp < p.splits ? p.ws_ml[(base + sp) * 2 + 1] : 0.0f;
+        m = fmaxf(m, ms[h]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const float w = ms[h] == -INFINITY ? 0.0f : exp2f(ms[h] - m);
+        l = fmaf(f[h], w, l);
+        f[h] = w;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    for (int s0 = 0; s0 < p.splits; s0 += 8) {
+        if (s0) load8(s0);
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc = fmaf(v[i], __shfl_sync(0xffffffffu, s0 < 32 ? f[0] : f[1], (s0 + i) & 31), acc);
     }
     const float r = l > 0.0f ? acc / l : 0.0f;
     char* orow = (char*)p.out + (long long)b * p.o_bs + (long long)head * p.o_hs;
@@ -365,14 +392,24 @@ int launch_decode_attention(const b200fc_attention_t& a, cudaStream_t s) {
     p.scale_log2e = a.scale * 1.4426950408889634f;
     // splits: as many as still give ONE round of two CTAs per SM (measured: a ragged second round costs more than a
     // partly filled first one; 96 KB in flight per CTA saturate HBM from ~130 CTAs on), at least two 16-token blocks per
-    // warp and split
+    // warp and split.  Heads of 64, from 1024 tokens on: four CTAs per SM, and where that leaves one or two splits two and a half rounds
+    // in splits of 512 tokens or more, whose short CTAs even the lengths of the sequences out (us, one round / this: B = 20, 16 kv heads,
+    // up to 8765 tokens 111 / 76; B = 14, up to 14313 tokens 106 / 84; B = 19, up to 2540 tokens 34.8 / 26.1.  Not with shorter sequences,
+    // where the second launch costs more: B = 18, 32 kv heads, up to 600 tokens 13.3 / 17.6; nor with more pairs than places, which are even
+    // enough: B = 32, 32 kv heads, up to 800 tokens 25.1 / 27.4; with one round of 7 splits it gains nothing).
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     static int force_splits = -1;
     if (force_splits < 0) { const char* e = getenv("B200FC_ATTN_SPLITS"); force_splits = e ? atoi(e) : 0; }
     const long long pairs = (long long)a.B * a.Hkv;
-    int splits = (int)(2LL * sms / pairs);
+    const bool deep = a.D == 64 && a.N >= 1024;
+    const long long places = (long long)(deep ? ATT_CTAS_PER_SM<64> : 2) * sms;
+    int splits = (int)(places / pairs);
+    if (deep && splits >= 1 && splits <= 2) {
+        const int rounds = (int)((5 * places + 2 * pairs - 1) / (2 * pairs)), by_len = a.N / 512;
+        splits = max(splits, min(rounds, by_len));
+    }
     const int max_by_len = (a.N + 2 * BLK * ATT_WARPS - 1) / (2 * BLK * ATT_WARPS);
     if (splits > max_by_len) splits = max_by_len;
     if (force_splits > 0) splits = force_splits;

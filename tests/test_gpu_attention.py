@@ -70,6 +70,20 @@ def test_decode_attention_sequence_lengths_and_splits(monkeypatch):
     assert H.rel_to_max(got, ref) < 5e-3
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,N,lens", [
+    (15, 60, 20, 1540, [1540, 0, 1, 512, 513, 770, 771, 1024, 1539, 64, 65, 900, 1100, 1300, 1400]),   # 300 pairs: several rounds of short ranges
+    (1, 3, 1, 8300, [8300]),                 # one pair in 64 ranges: more than the lanes of a combining warp
+    (2, 4, 2, 1024, [1024, 1000]),           # the shortest cache that takes four CTAs per SM
+])
+def test_decode_attention_heads_of_64(B, Hq, Hkv, N, lens):
+    rng = np.random.default_rng(N)
+    q = H.normal_bf16(rng, (B, Hq, 64)); k = H.normal_bf16(rng, (B, Hkv, N, 64)); v = H.normal_bf16(rng, (B, Hkv, N, 64))
+    for b, n in enumerate(lens):
+        k[b, :, n:, :] = 0x7FC0; v[b, :, n:, :] = 0x7FC0        # bf16 NaN
+    got = run(q, k, v, 0.125, seq_lens=lens)
+    assert H.rel_to_max(got, port.decode_attention(q, k, v, 0.125, lens)) < 5e-3      # (probabilities in bf16, as above)
+
+
 def test_decode_attention_repeated_calls_of_mixed_shapes():
     """calls of different shapes follow one another on a stream and share the workspace of the sub-states (it grows and
     is reused); every call must see only its own sub-states"""
