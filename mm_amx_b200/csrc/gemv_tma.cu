@@ -1561,6 +1561,11 @@ int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, i
         if (S > p.spr / 2) S = p.spr / 2;
         if (S < 1) S = 1;
         const int places_S = S;
+        // Long rows: clusters of more than four CTAs keep to four fifths of the places.  Behind a kernel that fills the GPU the last of them
+        // find theirs late, and end by as much later (a gate/up and a down projection at 6 rows, us: hidden 6656, 52 row blocks 131 with
+        // S = 5, 116 with 4; 4608, 36 row blocks 72.7 with 7, 64.5 with 6; 4096 53.9 with 8, 52.9 with 7; the down projection alone
+        // 39.4 / 41.5, 23.0 / 23.3 and 18.7 / 18.8).
+        while (S > 4 && p.spr >= 128 && 5LL * S * row_blocks > 4 * gmax) S--;
         static ClusterCounts counts;        // (every variant takes two places per SM)
         rc = fit_clusters(counts, THREADS, Layout<16, 1>::SMEM, row_blocks, &S);
         if (rc) return rc;
