@@ -861,7 +861,7 @@ int launch_gemm_tc(const void* W_data, int w_dtype, int W_K_pad, int W_N_pad, co
     p.splits = 1; p.split_stride = 0;
     p.ar_world = 0; p.ar_rank = 0; p.ar_phases = 3; p.ar_gemm_pairs = 0; p.ar_work_counter = 0; p.ar_target = 0; p.ar_partial_mc = nullptr; p.ar_out_mc = nullptr;
     for (int i = 0; i < 8; i++) p.ar_flags[i] = nullptr;
-    p.vec_ok = output_vec(ep, n0);
+    p.vec_ok = output_vec(ep, n0, i8);
     if (ep.out_dtype == B200FC_S32 && !i8) { set_error("raw int32 output needs an 8-bit GEMM"); return B200FC_ERR_INVALID; }
     if (ep.mc_reduce && (ep.steps != 0 || i8 || ((n0 | n1) & 1) || ((uintptr_t)ep.C & 3) || (ep.ldc & 3))) {
         set_error("multicast-reduce output needs a bf16 GEMM without post-ops and an even, 4-byte aligned column range");

@@ -699,7 +699,7 @@ int run_wave(const WaveCall& call, const WaveShape& sh, int n0, int n1) {
     p.status = kernel_status_word();
     if (!p.status) { set_error("gemm: no kernel status word on this device"); return B200FC_ERR_CUDA; }
     p.wait_limit_ns = wait_limit_ns();
-    p.vec_ok = output_vec(ep, n0);
+    p.vec_ok = output_vec(ep, n0, I8);
 
     CUtensorMap ma, mw;
     int rc = make_map(&ma, call.A, I8, (uint64_t)call.K, (uint64_t)call.M, (uint64_t)call.lda, BM);
@@ -765,6 +765,20 @@ int run_wave(WaveCall& c, int n0, int n1) {
     const int rc = c.M <= BM ? pick_shape<1, MODE>(c.M, n1 - n0, c.slabs, c.units, c.chains, &sh, &found)
                              : pick_shape<2, MODE>(c.M, n1 - n0, c.slabs, c.units, c.chains, &sh, &found);
     if (rc) return rc;
+    if constexpr (WQ) {
+        // Quantised weights: gemm_qt.cu takes the calls that do not fit one wave (us, through blocks of widened weights / there: int8
+        // 571 x 10624 x 21504 575 / 201, 1071 x 2560 x 22784 210 / 112, 4096 x 4096 x 11008 289 / 239; 4 bits 3526 x 8448 x 10168
+        // 575 / 449), and of the others those of up to 512 rows and those whose K would be split (us, here / there: int8 22 x 3840 x 6016
+        // 26.4 / 11.8, 158 x 3840 x 8576 37.0 / 26.5, 949 x 8704 x 2048 39.8 / 34.3; 4 bits 33 x 2400 x 9824 21.7 / 14.6).  More rows in tiles
+        // of all of K keep up here (int8 705 x 2560 x 10240 35.7 / 42.0, 2017 x 1408 x 4200 25.6 / 30.9, 1689 x 1920 x 1920 19.4 / 21.1).
+        // 4 bits with more than 64 rows and many chains are level (100 x 4096 x 11008 24.8 / 24.8).  Folded calls would be faster there as well (4 bits 300 x 4096 x 11008 59.5 / 40.4), but their tiles are what
+        // b200fc_last_wave_tile reports and stay.  K is summed in no fewer chains than it would be here.
+        if (!found) return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, c.chains, false, c.s);
+        const int W = sh.cg * sh.R, chains = (c.chains + sh.S - 1) / sh.S, parts = parts_of(chains, W);
+        const bool level = MODE == W_U4C && c.M > 64 && sh.S * chains > 4;
+        if (parts == 1 && !level && (c.M <= 512 || sh.S > 1))
+            return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, sh.S * chains, true, c.s);
+    }
     if (!found) return B200FC_ERR_UNSUPPORTED;
     // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256
     // 46.8 / 42.7, 250 x 2784 x 14928 27.6 / 26.7)

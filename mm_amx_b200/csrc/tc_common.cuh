@@ -125,6 +125,27 @@ __device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned (&r)[32]) {
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+__device__ __forceinline__ void tc_st32(unsigned taddr, const unsigned (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+          "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+          "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D (128 rows) += A (128 x 16, tensor memory) x B (columns x 16, shared memory)
+__device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // Shared-memory operand descriptor: K-major tile, rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes
 // apart (stride-dimension byte offset); descriptor version 1 (Blackwell).
 __device__ __forceinline__ unsigned long long make_smem_desc(unsigned smem_addr) {
@@ -277,7 +298,7 @@ __device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi) {
 // all lanes of the warp.  This is the form for everything: chunks at the ragged end, unaligned outputs, residuals, multicast.
 __device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m, int n, const EpiArgs& p, bool row_ok, long long c_offset = 0) {
     const Epilogue& ep = p.ep;
-    const bool staged = p.vec_ok == 1 && n + 32 <= p.n1 && !ep.mc_reduce;   // warp-uniform
+    const bool staged = p.vec_ok && (!p.acc_is_int || p.vec_ok == 1) && n + 32 <= p.n1 && !ep.mc_reduce;   // warp-uniform
     const int lane = threadIdx.x & 31, m0 = m - lane;
     char* Cb = (char*)ep.C + c_offset;
     char* crow = Cb + (long long)m * ep.ldc;
@@ -361,7 +382,7 @@ __device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m,
         } else if (ep.mc_reduce) {
             // Fused all-reduce: C is a multicast mapping of the output on every GPU of the tensor-parallel group; the NVSwitch
             // adds this rank's contribution into all replicas (multimem.red), so no separate collective runs.
-            const bool full = p.vec_ok == 1 && n + 32 <= p.n1;
+            const bool full = p.vec_ok && n + 32 <= p.n1;
             if (ep.out_dtype == B200FC_F32) {
                 float* dst = (float*)(crow + (long long)nq * 4);
                 if (full) {
@@ -409,9 +430,10 @@ __device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m,
 // instantiation, and one branch per post-op and chunk.  (With the choice made inside, per eight columns, a chunk took 2400
 // clocks of a warp for a plain bf16 store.)
 template <int V> struct IntConst { static constexpr int value = V; };
-enum EpiKind { EPI_F32 = 0, EPI_BF16, EPI_S8, EPI_S32, EPI_SILU, EPI_GENERAL };
+enum EpiKind { EPI_F32 = 0, EPI_BF16, EPI_S8, EPI_S32, EPI_SILU, EPI_S8_HALF, EPI_GENERAL };
 __device__ __forceinline__ int epilogue_kind(const Epilogue& ep, int vec_ok) {
     if (!vec_ok || ep.mc_reduce || ep.residual) return EPI_GENERAL;
+    if (vec_ok == 2) return EPI_S8_HALF;
     if (ep.steps & B200FC_STEP_SILU_MUL) return EPI_SILU;
     return ep.out_dtype == B200FC_F32 ? EPI_F32 : (ep.out_dtype == B200FC_BF16 ? EPI_BF16 : (ep.out_dtype == B200FC_S8 ? EPI_S8 : EPI_S32));
 }
@@ -516,8 +538,8 @@ __device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m,
             for (int j = 0; j < 8; j++) o[j] = f32x4_to_s8x4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 #pragma unroll
             for (int h = 0; h < 2; h++) tile[tile_pos<2>(lane, h)] = make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
-            if (p.vec_ok == 1) flush_tile<2>(p.tile, C, ep.ldc, m0, n, p.M);
-            else flush_tile_s8_half(p.tile, C, ep.ldc, m0, n, p.M);
+            if constexpr (KIND == EPI_S8_HALF) flush_tile_s8_half(p.tile, C, ep.ldc, m0, n, p.M);
+            else flush_tile<2>(p.tile, C, ep.ldc, m0, n, p.M);
         }
     }
 }
@@ -531,6 +553,7 @@ __device__ __forceinline__ void for_epilogue_kind(int kind, bool i8, const Body&
         case EPI_S8: body(IntConst<EPI_S8>()); break;
         case EPI_S32: if (i8) body(IntConst<EPI_S32>()); break;
         case EPI_SILU: if (!i8) body(IntConst<EPI_SILU>()); break;
+        case EPI_S8_HALF: if (i8) body(IntConst<EPI_S8_HALF>()); break;
         default: break;
     }
 }
@@ -605,6 +628,13 @@ __device__ __forceinline__ unsigned u8x2_to_bf16x2(unsigned w, unsigned sel) {
     asm("lop3.b32 %0, %1, %2, %3, 0xae;" : "=r"(c) : "r"(p), "r"(0x00800080u), "r"(0x43004300u));   // (~p & m) | k
     return bf16x2_sub(a, c);
 }
+// The same divided by 64, exactly, in two instructions: a byte u alone in a bf16 is the subnormal number u * 2^-133 (from 128 on with exponent
+// field 1, which continues it without a step), and one fused multiply-add makes (u - 128) / 64 of it.
+__device__ __forceinline__ unsigned u8x2_to_bf16x2_64th(unsigned w, unsigned sel) {
+    unsigned r;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(__byte_perm(w, 0u, sel)), "r"(0x7f007f00u), "r"(0xc000c000u));    // * 2^127 - 2
+    return r;
+}
 // nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of n - 8, exactly: (128 + n) - 136
 __device__ __forceinline__ unsigned nib2_to_bf16x2(unsigned w) {
     unsigned a;
@@ -645,14 +675,14 @@ int make_map(CUtensorMap* map, const void* base, bool i8, uint64_t k_elems, uint
     return B200FC_OK;
 }
 
-// How the epilogue may store whole chunks of the output: 1 = 16-byte pieces; 2 = int8 rows in 8-byte pieces (widths that are a multiple
-// of 8 only; single bytes took 28.7 us for int8 1559 x 1408 x 1240, 11.9 in pieces); 0 = element by element.
-int output_vec(const Epilogue& ep, int n0) {
+// How the epilogue may store whole chunks of the output: 1 = 16-byte pieces; 2 = int8 rows of an 8-bit GEMM in 8-byte pieces (widths that are a
+// multiple of 8 only; single bytes took 28.7 us for int8 1559 x 1408 x 1240, 11.9 in pieces); 0 = element by element.
+int output_vec(const Epilogue& ep, int n0, bool i8) {
     const int es = ep.out_dtype == B200FC_F32 || ep.out_dtype == B200FC_S32 ? 4 : (ep.out_dtype == B200FC_BF16 ? 2 : 1);
     const uintptr_t rows = (uintptr_t)ep.C | (uintptr_t)ep.ldc;
     if (ep.steps & B200FC_STEP_SILU_MUL) return (rows & 15) == 0 && n0 % 32 == 0;
     if (((rows | (uintptr_t)(n0 * es)) & 15) == 0) return 1;
-    return ep.out_dtype == B200FC_S8 && ((rows | (uintptr_t)n0) & 7) == 0 ? 2 : 0;
+    return i8 && ep.out_dtype == B200FC_S8 && ((rows | (uintptr_t)n0) & 7) == 0 ? 2 : 0;
 }
 
 // tcgen05 instruction descriptor (dense, K-major A and B, M = 128): accumulator format bits [4,6), A format [7,10),

@@ -1,0 +1,58 @@
+"""GPU: GEMM with quantised weights widened into tensor memory (gemm_qt.cu), where one tile is not enough, against the CPU oracle.
+
+Two-valued activations and integer weights (4 bits: power-of-two scales), so that every partial sum is exact in fp32 and the result must
+equal the oracle bit for bit; the oracle computes a choice of rows.  Small shapes are in test_gpu_wave.py.
+"""
+import numpy as np
+import pytest
+
+import helpers as H
+from mm_amx_b200 import capi
+from oracle import port
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (17, 136, 37000),       # more row blocks than SMs, K that ends inside a piece
+    (65, 1024, 20008),      # two rounds of pairs, ragged last row block
+    (385, 200, 24000),      # several rounds, two accumulators in turn
+    (3000, 520, 2600),      # token tiles with a ragged last one
+    (4100, 264, 1032),      # widest tiles: one accumulator
+    (520, 8192, 12800),     # K summed in parts, tiles of more than 128 tokens
+    (200, 5000, 640),       # parts of K in a cluster, each in several chains
+]
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+@pytest.mark.parametrize("kind", ["int8", "int4"])
+def test_exact(kind, M, K, N):
+    rng = np.random.default_rng(M + 3 * K + 7 * N)
+    rows = np.unique(np.concatenate([[0, 15, 16, M - 1], rng.integers(0, M, 10)]))
+    x = H.two_valued_bf16(rng, (M, K))
+    B = rng.integers(-7, 8, (N, K), dtype=np.int8)
+    if kind == "int8":
+        w = H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=np.ones(N, np.float32))
+        acc = port.gemm_bf16_w8(x[rows], B, transposeB=True)
+    else:
+        B[:, ::128] = 7                     # every group reaches the full range: the scale is 2^-6 exactly
+        W = H.bf16_bits(B.astype(np.float32) * np.float32(2.0 ** -6))
+        w = H.pack(W, True, capi.PACK_INT4_GROUP)
+        acc = port.gemm_bf16(x[rows], W, transposeB=True)
+    bias = rng.integers(-8, 9, N).astype(np.float32)
+    assert np.array_equal(H.run_matmul(w, x, capi.F32, steps=capi.STEP_DEQUANT)[rows], acc)
+    got = H.run_matmul(w, x, capi.BF16, steps=capi.STEP_DEQUANT | capi.STEP_BIAS, bias=bias)[rows]
+    assert np.array_equal(got, port.postops(acc, port.BIAS, port.BF16, bias=bias))
+    got = H.run_matmul(w, x, capi.S8, steps=capi.STEP_DEQUANT | capi.STEP_BIAS | capi.STEP_QUANT, bias=bias, q_scale=0.5)[rows]
+    assert np.array_equal(got, port.postops(acc, port.BIAS | port.QUANT, port.S8, bias=bias, q_scale=0.5))
+
+
+def test_extreme_int8_weights_and_scales():
+    """every byte value through the widening, with the largest and the smallest scales and activations that leave the result finite"""
+    K, N, M = 256, 128, 40
+    B = np.tile(np.arange(-128, 128, dtype=np.int8), (N, 1))
+    x = np.zeros((M, K), np.float32)
+    x[np.arange(M), np.arange(M) * 6] = 1.0
+    for scale, unit in [(2.0 ** 127, 2.0 ** -8), (1.0, 2.0 ** 119), (2.0 ** 60, 2.0 ** -126)]:
+        scales = np.full(N, scale, np.float32)
+        got = H.run_matmul(H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=scales), H.bf16_bits(x * np.float32(unit)), capi.F32, steps=capi.STEP_DEQUANT)
+        assert np.array_equal(got, ((x * np.float32(unit)) @ B.T.astype(np.float32)) * scales)
