@@ -635,6 +635,16 @@ __device__ __forceinline__ unsigned u8x2_to_bf16x2_64th(unsigned w, unsigned sel
     asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(__byte_perm(w, 0u, sel)), "r"(0x7f007f00u), "r"(0xc000c000u));    // * 2^127 - 2
     return r;
 }
+// the eight nibbles n of a word -> four bf16x2 of (n - 8) / 64, exactly: nibbles at bits [4,8) and [20,24) need no shift, as the subnormal
+// numbers 16 n * 2^-133
+__device__ __forceinline__ void nib8_to_bf16x2_64th(unsigned w, unsigned* r) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const unsigned v = w >> (8 * h);
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r[2 * h]) : "r"(v & 0x000f000fu), "r"(0x7f007f00u), "r"(0xbe00be00u));          // * 2^127 - 1/8
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r[2 * h + 1]) : "r"(v & 0x00f000f0u), "r"(0x7d007d00u), "r"(0xbe00be00u));      // * 2^123 - 1/8
+    }
+}
 // nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of n - 8, exactly: (128 + n) - 136
 __device__ __forceinline__ unsigned nib2_to_bf16x2(unsigned w) {
     unsigned a;
