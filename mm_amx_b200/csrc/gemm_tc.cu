@@ -25,6 +25,12 @@ namespace b200fc {
 namespace {
 
 constexpr int NUM_THREADS = 192;
+// The 2-CTA kernel has two epilogue warps per TMEM quarter, which share a tile's 32-column chunks.  One alone takes about 2400 clocks a
+// chunk, most of it latency, so that a 256-column tile of its CTA took longer than the MMAs of 2000 K and the last one of a launch ended late
+// (us, with one / two warps: Llama-style MLP 1585 x 1088 x 3456 62 / 52, block 968 x 1984 x 5120 93.5 / 88, int8 1359 x 6144 x 13056 with
+// GeLU, requantised, 111 / 93.5; long K is level: Llama-70B MLP, 4096 rows 4436 / 4442).
+constexpr int EPI2_WARPS = 8;
+constexpr int NUM_THREADS2 = 64 + 32 * EPI2_WARPS;
 constexpr int EPI_TILE_BYTES = 4 * EPI_TILE_WORDS * 4;
 
 template <int BN> struct Cfg {
@@ -62,7 +68,7 @@ struct GemmParams {
     int ar_phases;              // bit 0: multiply, bit 1: reduce (both set in normal use; single bits for measurements)
     int ar_gemm_pairs;          // pairs that multiply; pairs beyond reduce from the start
     int ar_work_counter;        // index, in this rank's counter array, of the counter that hands out reduction units
-    unsigned ar_target;         // arrivals that mean "every rank has stored these 128 rows of the tile" (world x 4 epilogue warps)
+    unsigned ar_target;         // arrivals that mean "every rank has stored these 128 rows of the tile" (world x epilogue warps)
     unsigned* ar_flags[8];      // ar_flags[r]: arrival counters of rank r (peer-mapped), two per tile (one per CTA of the pair)
     const char* ar_partial_mc;  // multicast address of all replicas of the partial buffer
     char* ar_out_mc;            // multicast address of all replicas of the output buffer
@@ -190,7 +196,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const EpiArgs ea{p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, epi_tile};
             const int kind = epilogue_kind(p.ep, p.vec_ok), n_first = p.n0 + tn * BN;
             const int whole = kind == EPI_GENERAL ? 0 : min(BN, p.n1 - n_first) / 32;
-            for_epilogue_kind(kind, I8, [&](auto k) {
+            for_epilogue_kind<I8>(kind, I8, [&](auto k) {
 #pragma unroll 1
                 for (int c = 0; c < whole; c++) {
                     unsigned r[32];
@@ -241,7 +247,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 //                 the peer's TMA loads complete_tx on the leader's barrier (cta_group::2 loads, no multicast).
 //   empty[s]      one per CTA, released by the leader's tcgen05.commit multicast to both CTAs.
 //   acc_full[b]   one per CTA, same multicast commit after the last K slab.
-//   acc_empty[b]  lives in the leader, 8 arrivals: the four epilogue warps of each CTA (the peer's arrive remotely).
+//   acc_empty[b]  lives in the leader, 16 arrivals: the epilogue warps of both CTAs (the peer's arrive remotely).
 // Cluster barriers bracket the kernel so that neither CTA touches the other's barriers before they exist or
 // after it has exited.  All mbarrier waits are bounded as in the 1-CTA kernel.
 template <int BN> struct Cfg2 {
@@ -250,9 +256,10 @@ template <int BN> struct Cfg2 {
     static constexpr int B_BYTES = (BN / 2) * SLAB_BYTES;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;
-    // per epilogue warp: the tile's per-column vectors (dequantisation scales, bias, quantisation scales)
-    static constexpr int COLVEC_BYTES = 4 * 3 * BN * 4;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + EPI_TILE_BYTES + COLVEC_BYTES;
+    // per epilogue warp: half a staging tile, and the per-column vectors of its chunks (dequantisation scales, bias, quantisation scales)
+    static constexpr int TILES_BYTES = EPI2_WARPS * EPI_TILE_WORDS / 2 * 4;
+    static constexpr int COLVEC_BYTES = EPI2_WARPS * 3 * (BN / 2) * 4;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + TILES_BYTES + COLVEC_BYTES;
 };
 
 // tile index (the order in which the CTA pairs take tiles) -> row tile tm and column tile tn
@@ -266,7 +273,7 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& 
         tm = pi * p.panel_rows + r % ph; tn = r / ph;
     }
 }
-constexpr int AR_UNROLL = 22;  // 192 threads x 22 pieces cover the 4096 pieces of a 128 x 256 bf16 unit
+constexpr int AR_UNROLL = 13;  // 320 threads x 13 pieces cover the 4096 pieces of a 128 x 256 bf16 unit
 
 // All-reduce work of the fused tensor-parallel down projection, run by whole CTAs: the pairs reserved for it from the
 // start of the kernel and every multiplying CTA once its own tiles are done.
@@ -310,11 +317,11 @@ __device__ void allreduce_units(const GemmParams& p, int num_tiles, volatile int
         const int ppr = cols >> 3;  // 16-byte pieces (8 bf16) per row
         const int total = rows * ppr;
         const long long base_off = (long long)r0 * p.ep.ldc + (long long)c0 * 2;
-        for (int base = threadIdx.x; base < total; base += NUM_THREADS * AR_UNROLL) {
+        for (int base = threadIdx.x; base < total; base += NUM_THREADS2 * AR_UNROLL) {
             unsigned v[AR_UNROLL][4];
 #pragma unroll
             for (int k = 0; k < AR_UNROLL; k++) {
-                const int i = base + k * NUM_THREADS;
+                const int i = base + k * NUM_THREADS2;
                 const int row = i / ppr, pc = i - row * ppr;
                 const long long off = base_off + (long long)row * p.ep.ldc + pc * 16;
                 if (i < total)
@@ -325,7 +332,7 @@ __device__ void allreduce_units(const GemmParams& p, int num_tiles, volatile int
             }
 #pragma unroll
             for (int k = 0; k < AR_UNROLL; k++) {
-                const int i = base + k * NUM_THREADS;
+                const int i = base + k * NUM_THREADS2;
                 const int row = i / ppr, pc = i - row * ppr;
                 const long long off = base_off + (long long)row * p.ep.ldc + pc * 16;
                 if (i < total)
@@ -338,7 +345,7 @@ __device__ void allreduce_units(const GemmParams& p, int num_tiles, volatile int
 }
 
 template <int BN, bool I8>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS2, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                 const GemmParams p) {
     using C = Cfg2<BN>;
@@ -370,7 +377,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(bar_acc_full + 8 * i, 1);
-            mbar_init(bar_acc_empty + 8 * i, 8);
+            mbar_init(bar_acc_empty + 8 * i, 2 * EPI2_WARPS);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -463,9 +470,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         __syncwarp();
     } else {
         // ---------------- epilogue warps (both CTAs, own 128 rows) ----------------
-        const int quarter = warp & 3;
-        unsigned* epi_tile = (unsigned*)(smem + C::STAGES * C::STAGE_BYTES + 256) + quarter * EPI_TILE_WORDS;
-        float* colvec = (float*)(smem + C::STAGES * C::STAGE_BYTES + 256 + EPI_TILE_BYTES) + quarter * 3 * BN;
+        const int quarter = warp & 3, half = (warp - 2) >> 2;       // this warp's chunks: half, half + 2, ...
+        unsigned* epi_tile = (unsigned*)(smem + C::STAGES * C::STAGE_BYTES + 256) + (warp - 2) * (EPI_TILE_WORDS / 2);
+        float* colvec = (float*)(smem + C::STAGES * C::STAGE_BYTES + 256 + C::TILES_BYTES) + (warp - 2) * 3 * (BN / 2);
         const bool plain_ep = !(p.ep.steps & B200FC_STEP_SILU_MUL) && !p.ep.mc_reduce && p.ep.out_dtype != B200FC_S32;
         const bool use_deq = plain_ep && (p.ep.steps & B200FC_STEP_DEQUANT) && p.ep.deq_per_oc;
         const bool use_bias = plain_ep && (p.ep.steps & B200FC_STEP_BIAS) && p.ep.bias;
@@ -481,16 +488,16 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const unsigned acc_phase = (unsigned)(it >> 1) & 1;
             int tm, tn;
             tile_coords(p, tile, tm, tn);
-            // while the tile's MMAs run: this warp's copy of the per-column vectors of the tile's BN columns (clamped
-            // to the last valid column), so that no chunk waits for global memory
+            // while the tile's MMAs run: this warp's copy of the per-column vectors of its chunks (clamped to the last valid column),
+            // so that no chunk waits for global memory
             if (any_vec) {
                 const int nb = p.n0 + tn * BN;
 #pragma unroll
-                for (int j = 0; j < BN / 32; j++) {
-                    const int col = min(nb + j * 32 + lane, p.n1 - 1);
+                for (int j = 0; j < BN / 64; j++) {
+                    const int col = min(nb + (2 * j + half) * 32 + lane, p.n1 - 1);
                     if (use_deq) colvec[j * 32 + lane] = __ldg(p.ep.deq_per_oc + col);
-                    if (use_bias) colvec[BN + j * 32 + lane] = __ldg(p.ep.bias + col);
-                    if (use_q) colvec[2 * BN + j * 32 + lane] = __ldg(p.ep.q_per_oc + col);
+                    if (use_bias) colvec[BN / 2 + j * 32 + lane] = __ldg(p.ep.bias + col);
+                    if (use_q) colvec[BN + j * 32 + lane] = __ldg(p.ep.q_per_oc + col);
                 }
                 __syncwarp();
             }
@@ -501,29 +508,29 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(ab * BN);
             EpiArgs ea{p.ep, p.vec_ok, I8 ? 1 : 0, p.n1, p.M, epi_tile};
             auto set_vecs = [&](int c) {
-                if (use_deq) ea.cv_deq = colvec + c * 32;
-                if (use_bias) ea.cv_bias = colvec + BN + c * 32;
-                if (use_q) ea.cv_q = colvec + 2 * BN + c * 32;
+                if (use_deq) ea.cv_deq = colvec + (c >> 1) * 32;
+                if (use_bias) ea.cv_bias = colvec + BN / 2 + (c >> 1) * 32;
+                if (use_q) ea.cv_q = colvec + BN + (c >> 1) * 32;
             };
             const int kind = epilogue_kind(p.ep, p.vec_ok), n_first = p.n0 + tn * BN;
             const int whole = kind == EPI_GENERAL ? 0 : min(BN, p.n1 - n_first) / 32;
-            for_epilogue_kind(kind, I8, [&](auto k) {
+            for_epilogue_kind<I8>(kind, I8, [&](auto k) {
 #pragma unroll 1
-                for (int c = 0; c < whole; c++) {
+                for (int c = half; c < whole; c += 2) {
                     unsigned r[32];
                     tc_ld32(taddr + (unsigned)(c * 32), r);
                     tc_wait_ld();
                     set_vecs(c);
-                    epilogue_whole<decltype(k)::value>(r, m, n_first + c * 32, ea, c_offset);
+                    epilogue_whole<decltype(k)::value, true>(r, m, n_first + c * 32, ea, c_offset);
                 }
             });
 #pragma unroll 1
-            for (int c = whole; c < BN / 32 && n_first + c * 32 < p.n1; c++) {   // (warp-uniform)
+            for (int c = whole + ((whole ^ half) & 1); c < BN / 32 && n_first + c * 32 < p.n1; c += 2) {   // (warp-uniform)
                 unsigned r[32];
                 tc_ld32(taddr + (unsigned)(c * 32), r);
                 tc_wait_ld();
                 set_vecs(c);
-                epilogue_chunk(r, m, n_first + c * 32, ea, row_ok, c_offset);
+                epilogue_chunk<true>(r, m, n_first + c * 32, ea, row_ok, c_offset);
             }
             tc_fence_before();
             if (p.ar_world) __threadfence_system();  // this warp's part of the tile is visible to every GPU ...
@@ -705,7 +712,7 @@ int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cuda
     if (splits > 1) p.item_limit = 0;
     int items = p.item_limit > 0 ? p.item_limit : tiles * splits;
     int pairs = items < max_pairs ? items : max_pairs;
-    gemm_tc2_kernel<BN, I8><<<2 * pairs, NUM_THREADS, C::SMEM_BYTES, s>>>(ma, mw, p);
+    gemm_tc2_kernel<BN, I8><<<2 * pairs, NUM_THREADS2, C::SMEM_BYTES, s>>>(ma, mw, p);
     count_launch();
     B200FC_CUDA(cudaGetLastError());
     if (splits > 1) {
@@ -801,7 +808,7 @@ int launch_gemm_tc_allreduce(const void* W_data, int W_K_pad, int W_N_pad, const
     if (comm_pairs < 1) comm_pairs = 1;
     if (comm_pairs > all_pairs - 1) comm_pairs = all_pairs - 1;
     p.ar_gemm_pairs = all_pairs - comm_pairs;
-    p.ar_target = (unsigned)ar.world * 4u;
+    p.ar_target = (unsigned)ar.world * EPI2_WARPS;
     p.ar_work_counter = ar.max_tiles - 1;
     for (int i = 0; i < 8; i++) p.ar_flags[i] = i < ar.world ? ar.flags[i] : nullptr;
     p.ar_partial_mc = (const char*)ar.partial_mc;
@@ -821,7 +828,7 @@ int launch_gemm_tc_allreduce(const void* W_data, int W_K_pad, int W_N_pad, const
         if (arc) return arc;
     }
     // the whole grid must be resident (reducing pairs wait for multiplying pairs of every GPU): one CTA per SM
-    gemm_tc2_kernel<256, false><<<2 * all_pairs, NUM_THREADS, C::SMEM_BYTES, s>>>(ma, mw, p);
+    gemm_tc2_kernel<256, false><<<2 * all_pairs, NUM_THREADS2, C::SMEM_BYTES, s>>>(ma, mw, p);
     count_launch();
     B200FC_CUDA(cudaGetLastError());
     return B200FC_OK;

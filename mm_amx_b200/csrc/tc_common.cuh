@@ -17,7 +17,7 @@ constexpr int MMA_K_BYTES = 32;          // K extent of one tcgen05.mma (16 bf16
 #endif
 constexpr int EPI_SLEEP_NS = B200FC_EPI_SLEEP_NS;
 
-// staging tile of an epilogue warp: 32 rows x 32 four-byte columns
+// staging tile of an epilogue warp: 32 rows x 32 four-byte columns, or (HALF below) 32 x 16, which four-byte outputs go through twice
 constexpr int EPI_TILE_WORDS = 32 * 32;
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------
@@ -296,6 +296,7 @@ __device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi) {
 }
 // Post-ops and store of 32 consecutive columns [n, n + 32) of one output row per lane, whose accumulators are in `acc`.  Called by
 // all lanes of the warp.  This is the form for everything: chunks at the ragged end, unaligned outputs, residuals, multicast.
+template <bool HALF = false>
 __device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m, int n, const EpiArgs& p, bool row_ok, long long c_offset = 0) {
     const Epilogue& ep = p.ep;
     const bool staged = p.vec_ok && (!p.acc_is_int || p.vec_ok == 1) && n + 32 <= p.n1 && !ep.mc_reduce;   // warp-uniform
@@ -374,6 +375,10 @@ __device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m,
                 tile[tile_pos<4>(lane, q)] = make_uint4(pack_bf16x2(f(0), f(1)), pack_bf16x2(f(2), f(3)), pack_bf16x2(f(4), f(5)), pack_bf16x2(f(6), f(7)));
             } else if (ep.out_dtype == B200FC_S8) {
                 ((uint2*)tile)[2 * tile_pos<2>(lane, q >> 1) + (q & 1)] = make_uint2(f32x4_to_s8x4(f(0), f(1), f(2), f(3)), f32x4_to_s8x4(f(4), f(5), f(6), f(7)));
+            } else if constexpr (HALF) {
+                tile[tile_pos<4>(lane, 2 * (q & 1))] = make_uint4(r[0], r[1], r[2], r[3]);
+                tile[tile_pos<4>(lane, 2 * (q & 1) + 1)] = make_uint4(r[4], r[5], r[6], r[7]);
+                if (q & 1) flush_tile<4>(p.tile, Cb, ep.ldc, m0, (long long)(n + 16 * (q >> 1)) * 4, p.M);
             } else {
                 tile[tile_pos<8>(lane, 2 * q)] = make_uint4(r[0], r[1], r[2], r[3]);
                 tile[tile_pos<8>(lane, 2 * q + 1)] = make_uint4(r[4], r[5], r[6], r[7]);
@@ -423,7 +428,23 @@ __device__ __forceinline__ void epilogue_chunk(const unsigned (&acc)[32], int m,
     if (staged) {
         if (ep.out_dtype == B200FC_BF16) flush_tile<4>(p.tile, Cb, ep.ldc, m0, (long long)n * 2, p.M);
         else if (ep.out_dtype == B200FC_S8) flush_tile<2>(p.tile, Cb, ep.ldc, m0, n, p.M);
-        else flush_tile<8>(p.tile, Cb, ep.ldc, m0, (long long)n * 4, p.M);
+        else if constexpr (!HALF) flush_tile<8>(p.tile, Cb, ep.ldc, m0, (long long)n * 4, p.M);
+    }
+}
+// 32 four-byte columns of a row per lane through the staging tile
+template <bool HALF>
+__device__ __forceinline__ void store_words(const unsigned (&v)[32], unsigned* staging, char* C, long long ldc, int m0, int n, int M) {
+    uint4* tile = (uint4*)staging;
+    const int lane = threadIdx.x & 31;
+    constexpr int UNITS = HALF ? 4 : 8;
+#pragma unroll
+    for (int h = 0; h < 8 / UNITS; h++) {
+#pragma unroll
+        for (int j = 0; j < UNITS; j++) {
+            const int i = 4 * (h * UNITS + j);
+            tile[tile_pos<UNITS>(lane, j)] = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        flush_tile<UNITS>(staging, C, ldc, m0, (long long)(n + 16 * h) * 4, M);
     }
 }
 // The same for whole aligned chunks without residual and multicast, i.e. nearly all of them: one output kind per
@@ -437,7 +458,7 @@ __device__ __forceinline__ int epilogue_kind(const Epilogue& ep, int vec_ok) {
     if (ep.steps & B200FC_STEP_SILU_MUL) return EPI_SILU;
     return ep.out_dtype == B200FC_F32 ? EPI_F32 : (ep.out_dtype == B200FC_BF16 ? EPI_BF16 : (ep.out_dtype == B200FC_S8 ? EPI_S8 : EPI_S32));
 }
-template <int KIND>
+template <int KIND, bool HALF = false>
 __device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m, int n, const EpiArgs& p, long long c_offset = 0) {
     const Epilogue& ep = p.ep;
     const int lane = threadIdx.x & 31, m0 = m - lane;
@@ -460,9 +481,7 @@ __device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m,
         __syncwarp();
         return;
     } else if constexpr (KIND == EPI_S32) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) tile[tile_pos<8>(lane, j)] = make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-        flush_tile<8>(p.tile, C, ep.ldc, m0, (long long)n * 4, p.M);
+        store_words<HALF>(acc, p.tile, C, ep.ldc, m0, n, p.M);
         return;
     } else {
         f32x2 w[16];
@@ -522,10 +541,10 @@ __device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m,
 #pragma unroll
         for (int j = 0; j < 16; j++) unpack2(w[j], v[2 * j], v[2 * j + 1]);
         if constexpr (KIND == EPI_F32) {
+            unsigned o[32];
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                tile[tile_pos<8>(lane, j)] = make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3]));
-            flush_tile<8>(p.tile, C, ep.ldc, m0, (long long)n * 4, p.M);
+            for (int j = 0; j < 32; j++) o[j] = __float_as_uint(v[j]);
+            store_words<HALF>(o, p.tile, C, ep.ldc, m0, n, p.M);
         } else if constexpr (KIND == EPI_BF16) {
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -545,7 +564,7 @@ __device__ __forceinline__ void epilogue_whole(const unsigned (&acc)[32], int m,
 }
 // Runs body(IntConst<KIND>) for the call's output kind: the loop over a tile's whole chunks is instantiated per kind.  The chunks
 // that are not whole (all of them for EPI_GENERAL) are left to the caller, who has one loop of epilogue_chunk for them.
-template <class Body>
+template <bool S8_HALF, class Body>
 __device__ __forceinline__ void for_epilogue_kind(int kind, bool i8, const Body& body) {
     switch (kind) {
         case EPI_F32: body(IntConst<EPI_F32>()); break;
@@ -553,7 +572,7 @@ __device__ __forceinline__ void for_epilogue_kind(int kind, bool i8, const Body&
         case EPI_S8: body(IntConst<EPI_S8>()); break;
         case EPI_S32: if (i8) body(IntConst<EPI_S32>()); break;
         case EPI_SILU: if (!i8) body(IntConst<EPI_SILU>()); break;
-        case EPI_S8_HALF: if (i8) body(IntConst<EPI_S8_HALF>()); break;
+        case EPI_S8_HALF: if constexpr (S8_HALF) body(IntConst<EPI_S8_HALF>()); break;
         default: break;
     }
 }
