@@ -773,8 +773,9 @@ int run_wave(WaveCall& c, int n0, int n1) {
         // 575 / 449), and of the others those of up to 512 rows and those whose K would be split (us, here / there: int8 22 x 3840 x 6016
         // 26.4 / 11.8, 158 x 3840 x 8576 37.0 / 26.5, 949 x 8704 x 2048 39.8 / 34.3; 4 bits 33 x 2400 x 9824 21.7 / 14.6).  More rows in tiles
         // of all of K keep up here (int8 705 x 2560 x 10240 35.7 / 42.0, 2017 x 1408 x 4200 25.6 / 30.9, 1689 x 1920 x 1920 19.4 / 21.1).
-        // 4 bits with more than 64 rows and many chains are level (100 x 4096 x 11008 24.8 / 24.8).  Folded calls would be faster there as well (4 bits 300 x 4096 x 11008 59.5 / 40.4), but their tiles are what
-        // b200fc_last_wave_tile reports and stay.  K is summed in no fewer chains than it would be here.
+        // 4 bits with more than 64 rows and many chains are level (100 x 4096 x 11008 24.8 / 24.8).  Folded calls would be faster there as
+        // well (4 bits 300 x 4096 x 11008 59.5 / 40.4), but their tiles are what b200fc_last_wave_tile reports and stay.  K is summed in
+        // no fewer chains than it would be here.
         if (!found) return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, c.chains, false, c.s);
         const int W = sh.cg * sh.R, chains = (c.chains + sh.S - 1) / sh.S, parts = parts_of(chains, W);
         const bool level = MODE == W_U4C && c.M > 64 && sh.S * chains > 4;
