@@ -53,18 +53,34 @@ int* kernel_status_word() {
     return p;
 }
 
-int check_kernel_status(cudaStream_t s) {
-    int* p = kernel_status_word();
-    if (!p) { set_error("no kernel status word"); return B200FC_ERR_CUDA; }
-    int v = 0;
-    B200FC_CUDA(cudaMemcpyAsync(&v, p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    B200FC_CUDA(cudaStreamSynchronize(s));
+static int kernel_status_result(int v, int* p, cudaStream_t s) {
     if (v != 0) {
         cudaMemsetAsync(p, 0, sizeof(int), s);
         set_error("a kernel gave up on a bounded wait (code %d)", v);
         return B200FC_ERR_KERNEL;
     }
     return B200FC_OK;
+}
+// pinned (optional): memory of the caller's for the word; a copy to pageable memory costs 7 us more
+int check_kernel_status(cudaStream_t s, int* pinned) {
+    int* p = kernel_status_word();
+    if (!p) { set_error("no kernel status word"); return B200FC_ERR_CUDA; }
+    int v = 0, *to = pinned ? pinned : &v;
+    B200FC_CUDA(cudaMemcpyAsync(to, p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    B200FC_CUDA(cudaStreamSynchronize(s));
+    return kernel_status_result(*(volatile int*)to, p, s);
+}
+// the device's address of `bytes` of host memory at p, or null where kernels cannot reach all of it or rows are not 16-byte aligned
+static void* host_on_device(const void* p, int64_t ld, size_t bytes) {
+    cudaPointerAttributes a, z;
+    if ((((uintptr_t)p | (uintptr_t)ld) & 15) != 0) return nullptr;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&z, (const char*)p + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    const bool ok = a.type == cudaMemoryTypeHost && z.type == cudaMemoryTypeHost && a.devicePointer && z.devicePointer &&
+                    (char*)z.devicePointer - (char*)a.devicePointer == (ptrdiff_t)(bytes - 1) && ((uintptr_t)a.devicePointer & 15) == 0;
+    return ok ? a.devicePointer : nullptr;
 }
 
 struct Scratch { void* p = nullptr; size_t bytes = 0; };
@@ -767,6 +783,7 @@ int b200fc_mlp_free(b200fc_mlp_t* h) {
     if (!h) return B200FC_OK;
     free_weight(&h->m.gate_up); free_weight(&h->m.down);
     cudaFree(h->m.act); cudaFree(h->m.stage_x); cudaFree(h->m.stage_o);
+    if (h->m.host_status) cudaFreeHost(h->m.host_status);
     for (int i = 0; i < 3; i++) if (h->m.pipe_streams[i]) cudaStreamDestroy(h->m.pipe_streams[i]);
     if (h->m.ev_fork) cudaEventDestroy(h->m.ev_fork);
     if (h->m.ev_join) cudaEventDestroy(h->m.ev_join);
@@ -1014,12 +1031,29 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
     if (rc) return rc;
     static int pipe_min = -1;
     if (pipe_min < 0) { const char* e = getenv("B200FC_HOST_PIPE_MIN"); pipe_min = e ? atoi(e) : 512; }
+    if (!m.host_status) B200FC_CUDA(cudaHostAlloc((void**)&m.host_status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
     if (M < pipe_min) {
+        // Pinned buffers: kernels of this library copy them, in one chain with the projections (us, copy engines / kernels:
+        // 74 x 1024 x 3232 59 / 51, 283 x 1152 x 2912 115 / 96, 511 x 1024 x 3008 163 / 104, 207 x 4736 x 16960 300 / 213).
+        const size_t x_span = (size_t)(M - 1) * (size_t)ldx + row, o_span = (size_t)(M - 1) * (size_t)ldo + row;
+        const bool rows16 = row % 16 == 0 && ldx >= (int64_t)row && ldo >= (int64_t)row;
+        void* xd = rows16 ? host_on_device(x, ldx, x_span) : nullptr;
+        void* od = xd ? host_on_device(out, ldo, o_span) : nullptr;
+        void* sd = od ? host_on_device(m.host_status, 0, sizeof(int)) : nullptr;
+        int* status = sd ? kernel_status_word() : nullptr;
+        if (status) {
+            rc = launch_host_copy(xd, ldx, m.stage_x, (int64_t)row, M, (int)row, nullptr, nullptr, s);
+            if (!rc) rc = mlp_run_device(m, m.stage_x, (int64_t)row, M, m.stage_o, B200FC_BF16, (int64_t)row, s);
+            if (!rc) rc = launch_host_copy(m.stage_o, (int64_t)row, od, ldo, M, (int)row, status, (int*)sd, s);
+            if (rc) return rc;
+            B200FC_CUDA(cudaStreamSynchronize(s));
+            return kernel_status_result(*(volatile int*)m.host_status, status, s);
+        }
         B200FC_CUDA(cudaMemcpy2DAsync(m.stage_x, row, x, (size_t)ldx, row, (size_t)M, cudaMemcpyHostToDevice, s));
         rc = mlp_run_device(m, m.stage_x, (int64_t)row, M, m.stage_o, B200FC_BF16, (int64_t)row, s);
         if (rc) return rc;
         B200FC_CUDA(cudaMemcpy2DAsync(out, (size_t)ldo, m.stage_o, row, row, (size_t)M, cudaMemcpyDeviceToHost, s));
-        return check_kernel_status(s);
+        return check_kernel_status(s, m.host_status);
     }
     // Large batches: rows are independent, so the batch flows through three streams — host-to-device copy,
     // compute, device-to-host copy — and the PCIe transfers overlap the tensor-core work (the copy engines are full
@@ -1077,7 +1111,7 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
     }
     B200FC_CUDA(cudaEventRecord(m.ev_join, s_out));
     B200FC_CUDA(cudaStreamWaitEvent(s, m.ev_join, 0));
-    return check_kernel_status(s);
+    return check_kernel_status(s, m.host_status);
 }
 
 int b200fc_rmsnorm(const void* x, int64_t ldx, int M, int K, const void* weight, float eps, void* out, int64_t ldo,

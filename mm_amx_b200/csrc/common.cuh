@@ -65,6 +65,7 @@ struct Mlp {
     int act_rows = 0;                               // rows of the last gate_up
     void* stage_x = nullptr; size_t stage_x_bytes = 0;
     void* stage_o = nullptr; size_t stage_o_bytes = 0;
+    int* host_status = nullptr;                     // pinned: the status word as the last host-buffer call left it
     // host-buffer entry point, large batches: copy-in / compute / copy-out streams and their events
     cudaStream_t pipe_streams[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -95,7 +96,7 @@ void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 void count_launch(int n = 1);
 int* kernel_status_word();  // device int, 0 = OK; kernels store a non-zero code when a bounded wait runs out
-int check_kernel_status(cudaStream_t s);  // synchronises and reads it
+int check_kernel_status(cudaStream_t s, int* pinned = nullptr);  // synchronises and reads it
 // growing device scratch owned by (device, stream, slot): work on one stream is ordered, so kernels launched on it
 // may share it; slot 0 = re-strided activations, slot 1 = split-K partial tiles of the GEMM and sums of folded parts of K, 3 = widened weight
 // rows, 4 = normalised activations of the MLP block, 5 = sub-states of the decode attention, 6 = pre-converted activations
@@ -176,6 +177,10 @@ int matmul_device(const Weight& w, Weight* w_mut, const void* A, int dtypeA, int
 int launch_pack(const void* B_dev, int dtypeB, int K, int N, int64_t ldb, int transposeB, Weight& w, bool offset_binary,
                 cudaStream_t s);
 int launch_flip_copy2d(const void* src, int64_t lds, void* dst, int64_t ldd, int rows, int cols, cudaStream_t s);
+// rows between device memory and device-accessible host memory, everything in 16-byte units; host_status (optional, host memory as well)
+// receives *status behind them
+int launch_host_copy(const void* src, int64_t lds, void* dst, int64_t ldd, int rows, int row_bytes, const int* status, int* host_status,
+                     cudaStream_t s);
 int launch_pack_gate_up(const void* gate, const void* up, int64_t ld_bytes, int K, int rows, Weight& w, cudaStream_t s);
 int launch_quant_pack(const void* B_dev, int K, int N, int64_t ldb, int transposeB, Weight& w, float* absmax_dev,
                       cudaStream_t s);

@@ -211,6 +211,30 @@ __global__ void copy2d_kernel(const char* __restrict__ src, long long lds, char*
             dst[(long long)r * ldd + c] = c < row_bytes ? src[(long long)r * lds + c] : (char)0;
 }
 
+// Rows of 16-byte units between pinned host memory and the device, as a programmatic dependent in a chain of kernels; optionally the
+// status word goes to the host with them.  A copy engine hands over to the kernels on either side through a semaphore and took 10 us and
+// more for each small copy.  Bound by PCIe; a warp's requests are whole lines, four per thread travel together.
+__global__ void __launch_bounds__(256) host_copy_kernel(const uint4* __restrict__ src, long long lds, uint4* __restrict__ dst, long long ldd, int rows,
+                                                        int units, const int* status, int* host_status) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int total = rows * units, stride = (int)(gridDim.x * blockDim.x);
+    for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < total; i += 4 * stride) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int u = i + j * stride;
+            if (u < total) v[j] = src[(long long)(u / units) * lds + u % units];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int u = i + j * stride;
+            if (u < total) dst[(long long)(u / units) * ldd + u % units] = v[j];
+        }
+    }
+    if (host_status && blockIdx.x == 0 && threadIdx.x == 0) *host_status = *(const volatile int*)status;
+}
+
 // dst[r, c] = src[r, c] ^ 0x80: offset-binary <-> two's complement, row-wise with independent strides
 __global__ void flip_copy2d_kernel(const unsigned char* __restrict__ src, long long lds, unsigned char* __restrict__ dst,
                                    long long ldd, int rows, int cols) {
@@ -401,6 +425,25 @@ int launch_copy2d(const void* src, int64_t lds, void* dst, int64_t ldd, int rows
     copy2d_kernel<<<grid, 256, 0, s>>>((const char*)src, lds, (char*)dst, ldd, rows, row_bytes, dst_row_bytes);
     count_launch();
     B200FC_CUDA(cudaGetLastError());
+    return B200FC_OK;
+}
+
+int launch_host_copy(const void* src, int64_t lds, void* dst, int64_t ldd, int rows, int row_bytes, const int* status, int* host_status,
+                     cudaStream_t s) {
+    const int units = row_bytes / 16;
+    const long long blocks = ((long long)rows * units + 1023) / 1024;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(blocks < 296 ? blocks : 296), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200FC_CUDA(cudaLaunchKernelEx(&cfg, host_copy_kernel, (const uint4*)src, (long long)(lds / 16), (uint4*)dst, (long long)(ldd / 16), rows, units,
+                                   status, host_status));
+    count_launch();
     return B200FC_OK;
 }
 

@@ -293,3 +293,26 @@ def test_decode_mlp_in_one_launch_subprocess():
     env["PYTHONPATH"] = os.pathsep.join([here, os.path.dirname(here), env.get("PYTHONPATH", "")])
     r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "fused ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("M", [1, 40, 511])
+@pytest.mark.parametrize("pad,shift,pinned", [(0, 0, True), (24, 8, True), (3, 0, True), (0, 1, True), (0, 0, False)])
+def test_host_buffers_are_copied_whole(M, pad, shift, pinned):
+    """pinned rows (copied by kernels), with a pitch and an offset, rows that are not 16-byte aligned and pageable memory (copy engines):
+    the bits of the call on device buffers, and nothing written between the rows"""
+    import torch
+    K, N = 320, 96
+    g = torch.Generator().manual_seed(M)
+    gate, up, down = (torch.randn(shape, generator=g).mul_(0.05).to(torch.bfloat16).cuda() for shape in ((N, K), (N, K), (K, N)))
+    mlp = capi.Mlp(gate.data_ptr(), up.data_ptr(), down.data_ptr(), K, N, 0, 1)
+    ld = K + pad
+    x, out = torch.randn(M * ld + shift, generator=g).to(torch.bfloat16), torch.full((M * ld + shift,), 7.0, dtype=torch.bfloat16)
+    if pinned:
+        x, out = x.pin_memory(), out.pin_memory()
+    xs, os = x[shift:].view(M, ld), out[shift:].view(M, ld)
+    mlp.run_host(xs.data_ptr(), 2 * ld, M, os.data_ptr(), 2 * ld)
+    xd, want = xs[:, :K].contiguous().cuda(), torch.empty((M, K), dtype=torch.bfloat16, device="cuda")
+    mlp.run(xd.data_ptr(), 2 * K, M, want.data_ptr(), 2 * K)
+    capi.sync_check()
+    assert torch.equal(os[:, :K], want.cpu())
+    assert (os[:, K:] == 7.0).all() and (out[:shift] == 7.0).all()
