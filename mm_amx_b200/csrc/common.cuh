@@ -55,6 +55,11 @@ struct Epilogue {
     const void* residual = nullptr;   // [M, N] bf16
     long long ld_res = 0;             // bytes
 };
+// fp32 results behind GeLU.  The reference's polynomial is ill-conditioned in fp32 near |x| = 5 (its error is 4.8e-4 from 4.5 on, and
+// neighbouring inputs can differ by 7e-4 in the result), so another order of the sums in front of it moves outputs by 1e-4 to 7e-4 of
+// their rms, a hundred times what fp32 sums do by themselves.  Such calls keep one fixed split of K and one fixed order of sums per
+// shape, also where another is faster for other calls.  (Not 4-bit weights with more than 16 rows, which are rounded to bf16 first.)
+static inline bool sums_pinned(const Epilogue& ep) { return ep.out_dtype == B200FC_F32 && (ep.steps & B200FC_STEP_GELU); }
 
 // Fused Llama MLP object (b200fc_mlp_t)
 struct Mlp {

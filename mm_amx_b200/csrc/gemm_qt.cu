@@ -510,10 +510,10 @@ int d_bufs(int T) { return 2 * T <= 512 - QT_SETS * A_COLS ? 2 : 1; }       // a
 // other's way: the root of the sum of their squares.  Then HBM, the epilogue (of every tile where tensor memory holds one accumulator
 // only, or where it is longer than a tile's pieces) and the exchange of the parts of K.
 template <int CG, int WB>
-int consider(int M, int nspan, int stages, int chains, bool even, QtShape* best, double* best_cost) {
+int consider(int M, int nspan, int stages, int chains, bool even, bool one_chain, QtShape* best, double* best_cost) {
     constexpr int PIECES = WB == 4 ? 2 : 1;
-    const int tiles_n = (nspan + CG * QT_ROWS - 1) / (CG * QT_ROWS);
-    for (int S = 1; S * CG <= 8 && S <= stages; S++) {
+    const int tiles_n = (nspan + CG * QT_ROWS - 1) / (CG * QT_ROWS), max_S = one_chain ? 1 : 8 / CG;
+    for (int S = 1; S <= max_S && S <= stages; S++) {
         int units = 0;
         const int rc = max_units<CG>(S, &units);
         if (rc) return rc;
@@ -616,9 +616,10 @@ int run_qt(const QtCall& c, int chains, bool even) {
     const int stages = (int)(c.w.ld_bytes() / SLAB_BYTES);
     QtShape sh = {};
     double cost = -1.0;
-    int rc = consider<1, WB>(c.M, c.n1 - c.n0, stages, chains, even, &sh, &cost);
+    const bool one_chain = WB == 8 && sums_pinned(c.ep);      // (the caller sends such calls only with chains = 1)
+    int rc = consider<1, WB>(c.M, c.n1 - c.n0, stages, chains, even, one_chain, &sh, &cost);
     if (rc) return rc;
-    rc = consider<2, WB>(c.M, c.n1 - c.n0, stages, chains, even, &sh, &cost);
+    rc = consider<2, WB>(c.M, c.n1 - c.n0, stages, chains, even, one_chain, &sh, &cost);
     if (rc) return rc;
     // (FOLD: the most tokens whose sums a call keeps.  Those of 192 spill, which costs small tiles: 4 bits 100 x 4096 x 11008 34 us instead of 27;
     // but wider tiles are worth it: 493 x 7680 x 14848 116 us, 132 with 128.)

@@ -776,11 +776,17 @@ int run_wave(WaveCall& c, int n0, int n1) {
         // 4 bits with more than 64 rows and many chains are level (100 x 4096 x 11008 24.8 / 24.8).  Folded calls would be faster there as
         // well (4 bits 300 x 4096 x 11008 59.5 / 40.4), but their tiles are what b200fc_last_wave_tile reports and stay.  K is summed in
         // no fewer chains than it would be here.
-        if (!found) return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, c.chains, false, c.s);
-        const int W = sh.cg * sh.R, chains = (c.chains + sh.S - 1) / sh.S, parts = parts_of(chains, W);
-        const bool level = MODE == W_U4C && c.M > 64 && sh.S * chains > 4;
-        if (parts == 1 && !level && (c.M <= 512 || sh.S > 1))
-            return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, sh.S * chains, true, c.s);
+        // fp32 behind GeLU (sums_pinned): only where K is one chain on either path, which gives the same bits (slabs < 96: a ragged last
+        // round of blocks of widened weights is split along K from there on).
+        const bool pinned = MODE == W_U8C && sums_pinned(c.ep);
+        if (!found && (!pinned || (c.chains == 1 && c.slabs < 96)))
+            return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, c.chains, false, c.s);
+        if (found && !pinned) {
+            const int W = sh.cg * sh.R, chains = (c.chains + sh.S - 1) / sh.S, parts = parts_of(chains, W);
+            const bool level = MODE == W_U4C && c.M > 64 && sh.S * chains > 4;
+            if (parts == 1 && !level && (c.M <= 512 || sh.S > 1))
+                return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, sh.S * chains, true, c.s);
+        }
     }
     if (!found) return B200FC_ERR_UNSUPPORTED;
     // 256 x 256 tiles without a split of K are gemm_tc.cu's own, whose loop is a little better (us, here / there: 150 x 6272 x 14256

@@ -67,6 +67,7 @@ struct Params {
     unsigned long long wait_limit_ns;
     int cluster;          // 1: launched as clusters of S CTAs (S <= 8); the pieces of a row block meet in distributed
                           // shared memory instead of the global scratch
+    int chains;           // gemv_tc_kernel: accumulators that the stages of a piece take in turn (1 or TC_CHAINS)
     int pf_cap;           // stages beyond the ring that the producer prefetches into L2 when the CTA starts
     const float* scales;  // 4-bit weights: [row block][stage][2][128] group scales, row block 0 = packed rows [0, 128)
     const unsigned char* ximg;   // quantised weights, optional: the activations already converted by xstage_kernel, one
@@ -1140,14 +1141,14 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
                     if (!alive) break;
                     tc_fence_after();
                     const int i = ks - ks0;
-                    const unsigned d_tmem = tmem_base + (unsigned)((ab * TC_CHAINS + i % TC_CHAINS) * 16);
+                    const unsigned d_tmem = tmem_base + (unsigned)((ab * TC_CHAINS + (i & (p.chains - 1))) * 16);
                     const unsigned sa = smem_u32(smem + stage * TC_STAGE_BYTES);
                     const unsigned long long adesc = tc_smem_desc(sa), bdesc = tc_smem_desc(sa + STAGE_BYTES);
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < 4; k++)     // 4 x 16 K per stage, 32 bytes further along the swizzled row each
                             tc_mma_bf16(d_tmem, adesc + (unsigned long long)(k * 2), bdesc + (unsigned long long)(k * 2), idesc,
-                                        (unsigned)(i >= TC_CHAINS || k != 0));
+                                        (unsigned)(i >= p.chains || k != 0));
                         tc_commit(bar_empty + 8 * stage);
                         if (ks == ks1 - 1) tc_commit(bar_acc_full + 8 * ab);
                     }
@@ -1192,7 +1193,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
                 float sum[16];
 #pragma unroll
                 for (int j = 0; j < 16; j++) sum[j] = 0.0f;
-                for (int c = 0; ok && c < min(TC_CHAINS, ks1 - ks0); c++) {
+                for (int c = 0; ok && c < min(p.chains, ks1 - ks0); c++) {
                     unsigned r[16];
                     tc_ld16(tmem_base + ((unsigned)(warp * 32) << 16) + (unsigned)((ab * TC_CHAINS + c) * 16), r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -1432,6 +1433,7 @@ static int prepare_job(const Weight& w, const void* A, int M, int K, int64_t lda
     if (!p.status) { set_error("gemv: no kernel status word on this device"); return B200FC_ERR_CUDA; }
     p.wait_limit_ns = wait_limit_ns();
     p.S = 0; p.cluster = 0; p.pf_cap = 0;
+    p.chains = sums_pinned(ep) ? 1 : TC_CHAINS;
     p.ximg = nullptr;
 #ifdef B200FC_TRACE
     {
@@ -1565,13 +1567,14 @@ int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, i
         // find theirs late, and end by as much later (a gate/up and a down projection at 6 rows, us: hidden 6656, 52 row blocks 131 with
         // S = 5, 116 with 4; 4608, 36 row blocks 72.7 with 7, 64.5 with 6; 4096 53.9 with 8, 52.9 with 7; the down projection alone
         // 39.4 / 41.5, 23.0 / 23.3 and 18.7 / 18.8).
-        while (S > 4 && p.spr >= 128 && 5LL * S * row_blocks > 4 * gmax) S--;
+        const bool pinned = sums_pinned(ep);        // (as many parts as places allow, resident together or not)
+        while (!pinned && S > 4 && p.spr >= 128 && 5LL * S * row_blocks > 4 * gmax) S--;
         static ClusterCounts counts;        // (every variant takes two places per SM)
-        rc = fit_clusters(counts, THREADS, Layout<16, 1>::SMEM, row_blocks, &S);
+        rc = pinned ? B200FC_OK : fit_clusters(counts, THREADS, Layout<16, 1>::SMEM, row_blocks, &S);
         if (rc) return rc;
         const long long cost = (p.spr + S - 1) / S + (S > 1 ? 1 : 0);
-        if (2 * row_blocks <= gmax || cost <= best || g_force_aligned) {
-            short_chains = S < places_S || cost > best;
+        if ((!pinned && 2 * row_blocks <= gmax) || cost <= best || g_force_aligned) {
+            short_chains = !pinned && (S < places_S || cost > best);
             p.S = S; p.cluster = S > 1 ? 1 : 0;
             grid = (long long)row_blocks * S;
         }

@@ -383,7 +383,8 @@ int launch_gemv_tq(const Weight& w, const void* A, int M, int K, int64_t lda, in
     if (S < 1) S = 1;
     const int places_S = S;
     static ClusterCounts counts;
-    int rc = fit_clusters(counts, TQ_THREADS, es == 4 ? TqLayout<4>::SMEM : TqLayout<8>::SMEM, row_blocks, &S);   // (two per SM, either)
+    int rc = sums_pinned(ep) ? B200FC_OK       // (two CTAs per SM with either layout)
+                             : fit_clusters(counts, TQ_THREADS, es == 4 ? TqLayout<4>::SMEM : TqLayout<8>::SMEM, row_blocks, &S);
     if (rc) return rc;
     p.S = S;
     p.M = M; p.n0 = n0; p.n1 = n1;
