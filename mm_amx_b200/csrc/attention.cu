@@ -421,15 +421,22 @@ int launch_decode_attention(const b200fc_attention_t& a, cudaStream_t s) {
     splits = a.N > 0 ? (a.N + tps - 1) / tps : 1;
     p.tokens_per_split = tps; p.splits = splits;
     p.ws_o = nullptr; p.ws_ml = nullptr;
+    bool own = false;
     if (splits > 1) {
         const size_t n_sub = (size_t)a.B * a.H * splits;
         void* ws = nullptr;
-        int rc = get_stream_scratch(n_sub * (a.D + 2) * sizeof(float), s, 5, &ws);
+        // (memory of the graph where the stream is being captured: the stream's own may be too small, and a later call may free it)
+        int rc = get_stream_scratch(n_sub * (a.D + 2) * sizeof(float), s, 5, &ws, &own);
         if (rc) return rc;
         p.ws_o = (float*)ws;
         p.ws_ml = p.ws_o + n_sub * a.D;
     }
-    return a.D == 128 ? launch_attention_d<128>(p, a.B, s) : launch_attention_d<64>(p, a.B, s);
+    const int rc = a.D == 128 ? launch_attention_d<128>(p, a.B, s) : launch_attention_d<64>(p, a.B, s);
+    if (own) {
+        const cudaError_t e = cudaFreeAsync(p.ws_o, s);
+        if (!rc && e != cudaSuccess) return cuda_fail(e, "cudaFreeAsync of the sub-states");
+    }
+    return rc;
 }
 
 }  // namespace b200fc

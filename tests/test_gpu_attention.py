@@ -84,6 +84,48 @@ def test_decode_attention_heads_of_64(B, Hq, Hkv, N, lens):
     assert H.rel_to_max(got, port.decode_attention(q, k, v, 0.125, lens)) < 5e-3      # (probabilities in bf16, as above)
 
 
+@pytest.mark.parametrize("B,Hkv,N,D", [(20, 16, 2048, 64), (1, 8, 8192, 128)])
+@pytest.mark.parametrize("warm", [False, True])
+def test_captured_sub_states_belong_to_the_graph(B, Hkv, N, D, warm):
+    """captured on a stream without or with a workspace of its own; a larger call on that stream re-allocates it before the replay"""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N)
+    k, v = (torch.randn((B, Hkv, N, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+
+    def make(heads):
+        q = torch.randn((B, heads, D), generator=g, device="cuda").to(torch.bfloat16)
+        out = torch.zeros((B, heads, D), device="cuda")
+        a = capi.Attention(B, heads, Hkv, N, D, q.data_ptr(), heads * D * 2, D * 2, k.data_ptr(), v.data_ptr(), Hkv * N * D * 2, N * D * 2, D * 2,
+                           out.data_ptr(), heads * D * 4, D * 4, capi.F32, None, D ** -0.5)
+        return out, lambda stream: capi.decode_attention(a, stream=stream.cuda_stream), (q, a)
+
+    out, call, keep = make(Hkv)
+    out2, larger, keep2 = make(8 * Hkv)
+    before = capi.launch_count()
+    call(torch.cuda.default_stream())
+    assert capi.launch_count() - before == 2            # (sub-states and their combination: K is split)
+    capi.sync_check()
+    want = out.clone()
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    if warm:
+        call(s)
+        s.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        for _ in range(2):
+            call(torch.cuda.current_stream())
+    for _ in range(3):
+        out.zero_()
+        larger(s)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    capi.sync_check()
+
+
 def test_decode_attention_repeated_calls_of_mixed_shapes():
     """calls of different shapes follow one another on a stream and share the workspace of the sub-states (it grows and
     is reused); every call must see only its own sub-states"""
