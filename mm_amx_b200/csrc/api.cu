@@ -2,6 +2,7 @@
 // dispatch between the decode (gemv.cu) and prefill (gemm_tc.cu) kernels, host-buffer convenience entry points.
 #include <algorithm>
 #include <atomic>
+#include <cuda.h>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -9,6 +10,7 @@
 #include <mutex>
 #include <new>
 #include "common.cuh"
+#include "host_span.h"
 
 namespace b200fc {
 
@@ -70,17 +72,26 @@ int check_kernel_status(cudaStream_t s, int* pinned) {
     B200FC_CUDA(cudaStreamSynchronize(s));
     return kernel_status_result(*(volatile int*)to, p, s);
 }
-// the device's address of `bytes` of host memory at p, or null where kernels cannot reach all of it or rows are not 16-byte aligned
-static void* host_on_device(const void* p, int64_t ld, size_t bytes) {
-    cudaPointerAttributes a, z;
-    if ((((uintptr_t)p | (uintptr_t)ld) & 15) != 0) return nullptr;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&z, (const char*)p + bytes - 1) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    const bool ok = a.type == cudaMemoryTypeHost && z.type == cudaMemoryTypeHost && a.devicePointer && z.devicePointer &&
-                    (char*)z.devicePointer - (char*)a.devicePointer == (ptrdiff_t)(bytes - 1) && ((uintptr_t)a.devicePointer & 15) == 0;
-    return ok ? a.devicePointer : nullptr;
+// the driver's answer about a host address, for span_on_device
+static bool host_range(const void* p, HostRange* r) {
+    typedef CUresult (*Fn)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Fn fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return ok ? (Fn)sym : (Fn) nullptr;
+    }();
+    CUmemorytype type = (CUmemorytype)0;      // (stays 0, as everything else, for memory that CUDA does not know)
+    CUdeviceptr device = 0, start = 0;
+    size_t size = 0;
+    unsigned managed = 0;
+    int access = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void* to[] = {&type, &device, &start, &size, &managed, &access};
+    if (!fn || fn(6, what, to, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    *r = HostRange{type == CU_MEMORYTYPE_HOST && !managed, (access & 1) != 0, (access & 3) == 3, (uintptr_t)device, (uintptr_t)start, size};
+    return true;
 }
 
 struct Scratch { void* p = nullptr; size_t bytes = 0; };
@@ -1037,9 +1048,9 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
         // 74 x 1024 x 3232 59 / 51, 283 x 1152 x 2912 115 / 96, 511 x 1024 x 3008 163 / 104, 207 x 4736 x 16960 300 / 213).
         const size_t x_span = (size_t)(M - 1) * (size_t)ldx + row, o_span = (size_t)(M - 1) * (size_t)ldo + row;
         const bool rows16 = row % 16 == 0 && ldx >= (int64_t)row && ldo >= (int64_t)row;
-        void* xd = rows16 ? host_on_device(x, ldx, x_span) : nullptr;
-        void* od = xd ? host_on_device(out, ldo, o_span) : nullptr;
-        void* sd = od ? host_on_device(m.host_status, 0, sizeof(int)) : nullptr;
+        void* xd = rows16 ? (void*)span_on_device(x, ldx, x_span, false, host_range) : nullptr;
+        void* od = xd ? (void*)span_on_device(out, ldo, o_span, true, host_range) : nullptr;
+        void* sd = od ? (void*)span_on_device(m.host_status, 0, sizeof(int), true, host_range) : nullptr;
         int* status = sd ? kernel_status_word() : nullptr;
         if (status) {
             rc = launch_host_copy(xd, ldx, m.stage_x, (int64_t)row, M, (int)row, nullptr, nullptr, s);

@@ -316,3 +316,21 @@ def test_host_buffers_are_copied_whole(M, pad, shift, pinned):
     capi.sync_check()
     assert torch.equal(os[:, :K], want.cpu())
     assert (os[:, K:] == 7.0).all() and (out[:shift] == 7.0).all()
+
+
+def test_host_rows_go_through_kernels_only_inside_one_allocation():
+    """parts of one pinned allocation are copied by kernels (two launches more), pageable memory on either side by the copy engines"""
+    import torch
+    K, N, M = 320, 96, 40
+    w = torch.full((N, K), 0.01, dtype=torch.bfloat16, device="cuda")
+    mlp = capi.Mlp(w.data_ptr(), w.data_ptr(), w.view(K, N).data_ptr(), K, N, 0, 1)
+
+    def launches(x, out):
+        before = capi.launch_count()
+        mlp.run_host(x.data_ptr(), 2 * K, M, out.data_ptr(), 2 * K)
+        return capi.launch_count() - before
+
+    pinned, pageable = torch.zeros((4 * M, K), dtype=torch.bfloat16).pin_memory(), torch.zeros((2 * M, K), dtype=torch.bfloat16)
+    plain = launches(pageable, pageable[M:])
+    assert launches(pinned, pinned[M:]) == launches(pinned[2 * M:], pinned[3 * M:]) == plain + 2
+    assert launches(pinned, pageable) == launches(pageable, pinned) == plain
