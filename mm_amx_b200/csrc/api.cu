@@ -783,8 +783,13 @@ int b200fc_mlp_create(const void* gate, const void* up, const void* down, int K,
         if (!rc) rc = alloc_weight(m.down, Ns, K, B200FC_BF16);
         if (!rc) rc = launch_pack_gate_up(sg.p, su.p, sg.ld, K, Ns, m.gate_up, s);
         if (!rc) rc = launch_pack(sd.p, B200FC_BF16, Ns, K, sd.ld, 1, m.down, false, s);
+        if (!rc) {      // (for mlp_run_host, whose first call need not allocate it)
+            const cudaError_t e = cudaHostAlloc((void**)&m.host_status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+            if (e != cudaSuccess) rc = cuda_fail(e, "mlp_create status word");
+        }
         if (!rc && cudaStreamSynchronize(s) != cudaSuccess) { rc = cuda_fail(cudaGetLastError(), "mlp_create sync"); }
     }
+    if (rc && m.host_status) cudaFreeHost(m.host_status);
     if (rc) { free_weight(&m.gate_up); free_weight(&m.down); delete h; return rc; }
     *out = h;
     return B200FC_OK;
@@ -1042,7 +1047,6 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
     if (rc) return rc;
     static int pipe_min = -1;
     if (pipe_min < 0) { const char* e = getenv("B200FC_HOST_PIPE_MIN"); pipe_min = e ? atoi(e) : 512; }
-    if (!m.host_status) B200FC_CUDA(cudaHostAlloc((void**)&m.host_status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
     if (M < pipe_min) {
         // Pinned buffers: kernels of this library copy them, in one chain with the projections (us, copy engines / kernels:
         // 74 x 1024 x 3232 59 / 51, 283 x 1152 x 2912 115 / 96, 511 x 1024 x 3008 163 / 104, 207 x 4736 x 16960 300 / 213).
