@@ -234,7 +234,7 @@ inline int widened_block_rows(int K_pad) {
 int launch_gemm_wave(const Weight& w, const void* A, int dtypeA, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep,
                      cudaStream_t s);
 // gemm_qt.cu: the same for int8-compressed and 4-bit weights and any number of rows; K is summed in `chains` chains of fp32 sums at least,
-// with `even` none longer than K / chains (parts of K end with stored pieces of 128 bytes).  A: 16-byte aligned rows
+// with `even` none longer than K / chains where a CTA sums several (split_k.h; parts of K end with stored pieces of 128 bytes).  A: 16-byte aligned rows
 int launch_gemm_qt(const Weight& w, const void* A, int M, int K, int64_t lda, int n0, int n1, const Epilogue& ep, int chains, bool even,
                    cudaStream_t s);
 // gemm_tc.cu: bf16 GEMM whose output is all-reduced over a tensor-parallel group inside the kernel

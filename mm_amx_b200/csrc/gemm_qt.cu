@@ -20,6 +20,7 @@
 // Barriers: x_full (in the pair's leader) / x_empty per slot of activations, raw_full / raw_empty per slot of stored weights, a_full (in
 // the leader) / a_empty per A buffer in tensor memory, d_full / d_empty (in the leader) per accumulator.  Every wait is bounded as in gemm_tc.cu.
 #include <cmath>
+#include "split_k.h"
 #include "tc_common.cuh"
 
 namespace b200fc {
@@ -517,9 +518,7 @@ int consider(int M, int nspan, int stages, int chains, bool even, bool one_chain
         int units = 0;
         const int rc = max_units<CG>(S, &units);
         if (rc) return rc;
-        const int n_st = stages / S;
-        int parts = (chains + S - 1) / S;
-        while (even && parts > 1 && parts < n_st && (n_st + parts - 1) / parts * chains > stages) parts++;
+        const int parts = parts_of_share(stages, S, chains, even);
         for (int T = 16 * CG; T <= 256; T += 16 * CG) {
             if (T / CG > 128 || (parts > 1 && T > 192)) continue;
             const int tiles_m = (M + T - 1) / T;
