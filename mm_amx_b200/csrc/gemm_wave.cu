@@ -755,6 +755,20 @@ int k_chains(const Weight& w, int M, int K, int n0, int n1) {
     return chains;
 }
 
+// Calls with quantised weights that do not fit one wave and are faster through blocks of widened weights than in gemm_qt.cu: many rows
+// and short K.  Widening costs what K x N does, once; the epilogue of gemm_qt, longer per element than that of gemm_tc, and its
+// conversion per tile grow with the rows.  The line is drawn through 245 timed calls of 600 to 4096 rows, K 1024 to 4096, N 3072 to 21248: it loses
+// 0.4 % on average and 11 % at most against the faster of the two (us, blocks / gemm_qt: int8 4096 x 1024 x 11008 86 / 115,
+// 3000 x 1408 x 21248 144 / 159, 1400 x 1408 x 11008 50.3 / 50.6, 3000 x 2304 x 6016 68.7 / 67.7, 2000 x 1792 x 21248 149 / 124; 4 bits
+// 4096 x 1024 x 11008 81 / 123, 2000 x 1408 x 6016 42.9 / 47.2, 3000 x 2304 x 11008 137 / 125; with GeLU int8 3000 x 1408 x 11008 91 / 117).
+// A capturing stream stays with gemm_qt, which needs no workspace.
+bool faster_in_blocks(const WaveCall& c, bool w4, int nspan) {
+    const bool one_block = nspan <= widened_block_rows(c.w.K_pad);
+    if (c.M < (one_block ? 1.25 : 1.9) * c.K * (w4 ? 0.75 : 1.0) * (c.ep.steps & B200FC_STEP_GELU ? 0.8 : 1.0)) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(c.s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
 template <int MODE>
 int run_wave(WaveCall& c, int n0, int n1) {
     constexpr bool WQ = MODE == W_U8C || MODE == W_U4C;
@@ -768,7 +782,7 @@ int run_wave(WaveCall& c, int n0, int n1) {
                              : pick_shape<2, MODE>(c.M, n1 - n0, c.slabs, c.units, c.chains, &sh, &found);
     if (rc) return rc;
     if constexpr (WQ) {
-        // Quantised weights: gemm_qt.cu takes the calls that do not fit one wave (us, through blocks of widened weights / there: int8
+        // Quantised weights: gemm_qt.cu takes most calls that do not fit one wave (us, through blocks of widened weights / there: int8
         // 571 x 10624 x 21504 575 / 201, 1071 x 2560 x 22784 210 / 112, 4096 x 4096 x 11008 289 / 239; 4 bits 3526 x 8448 x 10168
         // 575 / 449), and of the others those of up to 512 rows and those whose K would be split (us, here / there: int8 22 x 3840 x 6016
         // 26.4 / 11.8, 158 x 3840 x 8576 37.0 / 26.5, 949 x 8704 x 2048 39.8 / 34.3; 4 bits 33 x 2400 x 9824 21.7 / 14.6).  More rows in tiles
@@ -779,7 +793,7 @@ int run_wave(WaveCall& c, int n0, int n1) {
         // fp32 behind GeLU (sums_pinned): only where K is one chain on either path, which gives the same bits (slabs < 96: a ragged last
         // round of blocks of widened weights is split along K from there on).
         const bool pinned = MODE == W_U8C && sums_pinned(c.ep);
-        if (!found && (!pinned || (c.chains == 1 && c.slabs < 96)))
+        if (!found && (!pinned || (c.chains == 1 && c.slabs < 96)) && !faster_in_blocks(c, MODE == W_U4C, n1 - n0))
             return launch_gemm_qt(c.w, c.A, c.M, c.K, c.lda, n0, n1, c.ep, c.chains, false, c.s);
         if (found && !pinned) {
             const int W = sh.cg * sh.R, chains = (c.chains + sh.S - 1) / sh.S, parts = parts_of(chains, W);

@@ -56,3 +56,45 @@ def test_extreme_int8_weights_and_scales():
         scales = np.full(N, scale, np.float32)
         got = H.run_matmul(H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=scales), H.bf16_bits(x * np.float32(unit)), capi.F32, steps=capi.STEP_DEQUANT)
         assert np.array_equal(got, ((x * np.float32(unit)) @ B.T.astype(np.float32)) * scales)
+
+
+@pytest.mark.parametrize("kind,M,K,N,blocks", [
+    ("int8", 1281, 1024, 13000, True), ("int8", 1279, 1024, 13000, False),      # the line at 1.25 K (one block of widened rows)
+    ("int8", 1950, 1024, 17000, True), ("int8", 1940, 1024, 17000, False),      # 1.9 K (two blocks)
+    ("int4", 1540, 2048, 10000, False), ("int4", 2920, 2048, 10000, True),      # three quarters of it
+])
+def test_many_rows_and_short_k(kind, M, K, N, blocks):
+    """either side of the line between gemm_qt.cu (one launch) and blocks of widened weights; exact on both, and a capturing stream, whose
+    workspace cannot grow, takes the former always"""
+    import torch
+    rng = np.random.default_rng(M + N)
+    rows = np.concatenate([[0, M - 1], rng.integers(0, M, 6)])
+    x = H.two_valued_bf16(rng, (M, K))
+    B = rng.integers(-7, 8, (N, K), dtype=np.int8)
+    if kind == "int8":
+        w = H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=np.ones(N, np.float32))
+        want = port.gemm_bf16_w8(x[rows], B, transposeB=True)
+    else:
+        B[:, ::128] = 7
+        W = H.bf16_bits(B.astype(np.float32) * np.float32(2.0 ** -6))
+        w = H.pack(W, True, capi.PACK_INT4_GROUP)
+        want = port.gemm_bf16(x[rows], W, transposeB=True)
+    dx, out = H.Dev(x), H.Dev(shape=(M, N), dtype=np.float32, fill=0xCD)
+    ep = capi.make_epilogue(out.ptr, out.ld, capi.F32, capi.STEP_DEQUANT)
+
+    def launches(stream):
+        before = capi.launch_count()
+        w.matmul(dx.ptr, capi.BF16, M, K, 2 * K, ep, stream=stream.cuda_stream)
+        return capi.launch_count() - before
+
+    assert (launches(torch.cuda.default_stream()) > 1) == blocks
+    capi.sync_check()
+    assert np.array_equal(out.numpy()[rows], want)
+    out.t.zero_()
+    torch.cuda.synchronize()
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=s):
+        assert launches(torch.cuda.current_stream()) == 1
+    graph.replay()
+    capi.sync_check()
+    assert np.array_equal(out.numpy()[rows], want)
