@@ -761,10 +761,11 @@ int k_chains(const Weight& w, int M, int K, int n0, int n1) {
 // 0.4 % on average and 11 % at most against the faster of the two (us, blocks / gemm_qt: int8 4096 x 1024 x 11008 86 / 115,
 // 3000 x 1408 x 21248 144 / 159, 1400 x 1408 x 11008 50.3 / 50.6, 3000 x 2304 x 6016 68.7 / 67.7, 2000 x 1792 x 21248 149 / 124; 4 bits
 // 4096 x 1024 x 11008 81 / 123, 2000 x 1408 x 6016 42.9 / 47.2, 3000 x 2304 x 11008 137 / 125; with GeLU int8 3000 x 1408 x 11008 91 / 117).
+// Fewer than 400 rows are not widened for, however short K: 300 x 128 x 40000 37 / 33, 100 x 64 x 40000 33 / 14, 400 x 256 x 40000 41 / 48.
 // A capturing stream stays with gemm_qt, which needs no workspace.
 bool faster_in_blocks(const WaveCall& c, bool w4, int nspan) {
     const bool one_block = nspan <= widened_block_rows(c.w.K_pad);
-    if (c.M < (one_block ? 1.25 : 1.9) * c.K * (w4 ? 0.75 : 1.0) * (c.ep.steps & B200FC_STEP_GELU ? 0.8 : 1.0)) return false;
+    if (c.M < 400 || c.M < (one_block ? 1.25 : 1.9) * c.K * (w4 ? 0.75 : 1.0) * (c.ep.steps & B200FC_STEP_GELU ? 0.8 : 1.0)) return false;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(c.s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }

@@ -61,6 +61,7 @@ def test_extreme_int8_weights_and_scales():
 @pytest.mark.parametrize("kind,M,K,N,blocks", [
     ("int8", 1281, 1024, 13000, True), ("int8", 1279, 1024, 13000, False),      # the line at 1.25 K (one block of widened rows)
     ("int8", 1950, 1024, 17000, True), ("int8", 1940, 1024, 17000, False),      # 1.9 K (two blocks)
+    ("int8", 400, 200, 40000, True), ("int8", 399, 200, 40000, False),          # 400 rows
     ("int4", 1540, 2048, 10000, False), ("int4", 2920, 2048, 10000, True),      # three quarters of it
 ])
 def test_many_rows_and_short_k(kind, M, K, N, blocks):
