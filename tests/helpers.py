@@ -6,6 +6,12 @@ from oracle._common import bf16_bits, bf16_to_f32
 from mm_amx_b200 import capi
 
 NP_OF = {capi.F32: np.float32, capi.BF16: np.uint16, capi.S8: np.int8, capi.S32: np.int32, capi.U8: np.uint8}
+PORT_OF = {capi.F32: port.F32, capi.BF16: port.BF16, capi.S8: port.S8}      # output types as the oracle counts them
+
+
+def sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
 
 
 def two_valued_bf16(rng, shape):

@@ -1,4 +1,5 @@
 """GPU: the one-wave GEMM (gemm_wave.cu) at the edges of its tiles, for every weight type, against the CPU oracle.
+Quantised weights with up to 512 rows, or with K split, go to gemm_qt.cu from most of SHAPES; test_quantised_weights_ragged has shapes that stay.
 
 Inputs on which every partial sum is exact in fp32 (two-valued activations, integer or power-of-two weights), so the result
 must equal the oracle bit for bit whatever the tile width, the split of K and the order of summation.
@@ -22,7 +23,7 @@ SHAPES = [
     (256, 1536, 4104),   # pair form with a split of K
     (300, 200, 9000),    # two row tiles (bf16 and int8 x int8 go to the persistent kernel: 256 x 256 tiles without a split of K)
     (2048, 128, 4096),   # 512-column tiles: all of tensor memory, columns of two MMAs
-    (2100, 136, 5000),   # more tiles than one wave: the persistent kernel, with widened blocks for quantised weights
+    (2100, 136, 5000),   # more tiles than one wave: the persistent kernel, with widened blocks for quantised weights (many rows, short K)
 ]
 
 
@@ -190,6 +191,38 @@ def test_wide_tiles_exact(kind, M, K, N, tile):
     got = H.run_matmul(w, x, out, steps=steps)
     assert capi.last_wave_tile() == tile
     assert np.array_equal(got[rows], acc)
+
+
+@pytest.mark.parametrize("M,K,N,n0,n1,tile", [
+    (700, 200, 4200, 0, 4200, (2, 96, 1, 1, 1, 66)),       # K that ends inside a stored piece, ragged last tile and column chunk
+    (700, 1416, 4200, 0, 4200, (2, 96, 1, 1, 1, 66)),
+    (2017, 1408, 4200, 0, 4200, (2, 256, 1, 1, 1, 72)),    # columns of two MMAs
+    (700, 1416, 4200, 128, 3977, (2, 96, 1, 1, 1, 63)),    # column ranges
+    (700, 520, 5000, 256, 4100, (2, 96, 1, 1, 1, 63)),
+])
+@pytest.mark.parametrize("kind", ["int8", "int4"])
+def test_quantised_weights_ragged(kind, M, K, N, n0, n1, tile):
+    if H.sms() != 148:
+        pytest.skip("tiles for 148 SMs")
+    rng = np.random.default_rng(M + 3 * K + 7 * N + n0)
+    rows = np.unique(np.concatenate([[0, 127, 128, 255, 256, M - 1], rng.integers(0, M, 8)]))
+    x = H.two_valued_bf16(rng, (M, K))
+    B = rng.integers(-7, 8, (N, K), dtype=np.int8)
+    bias = rng.integers(-8, 9, N).astype(np.float32)
+    if kind == "int8":
+        w = H.pack(B, True, capi.PACK_INT8_CHANNEL, scales=np.ones(N, np.float32))
+        acc = port.gemm_bf16_w8(x[rows], B, transposeB=True)
+    else:
+        B[:, ::128] = 7
+        W = H.bf16_bits(B.astype(np.float32) * np.float32(2.0 ** -6))
+        w = H.pack(W, True, capi.PACK_INT4_GROUP)
+        acc = port.gemm_bf16(x[rows], W, transposeB=True)
+    for steps, out in ((0, capi.F32), (capi.STEP_BIAS, capi.BF16), (capi.STEP_BIAS | capi.STEP_QUANT, capi.S8)):
+        capi.last_wave_tile()
+        got = H.run_matmul(w, x, out, steps=steps | capi.STEP_DEQUANT, bias=bias, q_scale=0.5, n0=n0, n1=n1)
+        assert capi.last_wave_tile() == tile
+        assert np.array_equal(got[rows, n0:n1], port.postops(acc, steps, H.PORT_OF[out], bias=bias, q_scale=0.5)[:, n0:n1])
+        assert (np.delete(got, np.s_[n0:n1], axis=1).view(np.uint8) == 0xCD).all()
 
 
 @pytest.mark.parametrize("sms", [2, 37, 100])
