@@ -313,7 +313,8 @@ int matmul_device(const Weight& w, Weight* w_mut, const void* A, int dtypeA, int
     rc = launch_gemm_wave(w, A_use, dtypeA, M, K, lda_use, n0, n1, ep, s);
     if (rc != B200FC_ERR_UNSUPPORTED) return rc;
     if (w.compressed) {
-        // M > 16 with compressed weights.  The reference decompresses 16 weight rows at a time into a reused
+        // Compressed weights and many rows with short K (see launch_gemm_wave), or a GEMM forced by a switch.  The reference
+        // decompresses 16 weight rows at a time into a reused
         // buffer right before the tile product (kernels_amx.hpp:1443-1514); here a block of weight rows is widened to
         // bf16 (exact for int8; 4-bit values are multiplied by their group scale and rounded to bf16, the one place
         // where the group scale cannot wait for the epilogue) into a per-stream scratch of at most 32 MB — small enough to stay in the 126 MB L2 until the
@@ -1049,7 +1050,9 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
     if (pipe_min < 0) { const char* e = getenv("B200FC_HOST_PIPE_MIN"); pipe_min = e ? atoi(e) : 512; }
     if (M < pipe_min) {
         // Pinned buffers: kernels of this library copy them, in one chain with the projections (us, copy engines / kernels:
-        // 74 x 1024 x 3232 59 / 51, 283 x 1152 x 2912 115 / 96, 511 x 1024 x 3008 163 / 104, 207 x 4736 x 16960 300 / 213).
+        // 74 x 1024 x 3232 59 / 51, 283 x 1152 x 2912 115 / 96, 511 x 1024 x 3008 163 / 104, 207 x 4736 x 16960 300 / 213).  From 512
+        // rows on the pipeline below is faster in wide layers, the kernels still in narrow ones (pipeline / kernels: 512 x 4096 x 11008
+        // 282-327 / 307, 768 x 4096 x 11008 351-364 / 430-438, 1024 x 4096 x 11008 443-466 / 542, 768 x 1024 x 3008 176-186 / 126).
         const size_t x_span = (size_t)(M - 1) * (size_t)ldx + row, o_span = (size_t)(M - 1) * (size_t)ldo + row;
         const bool rows16 = row % 16 == 0 && ldx >= (int64_t)row && ldo >= (int64_t)row;
         void* xd = rows16 ? (void*)span_on_device(x, ldx, x_span, false, host_range) : nullptr;

@@ -55,9 +55,6 @@ struct QtParams {
     unsigned long long wait_limit_ns;
 };
 
-__device__ __forceinline__ void st_cluster_v4(unsigned cluster_addr, float a, float b, float c, float d) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 // D (CG x 128 rows x T columns) += A (rows x 16, tensor memory) x B (T x 16, shared memory of the CTAs)
 template <int CG>
 __device__ __forceinline__ void mma_from_tmem(unsigned d_tmem, unsigned a_tmem, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
@@ -70,11 +67,6 @@ __device__ __forceinline__ void mma_from_tmem(unsigned d_tmem, unsigned a_tmem, 
     } else {
         tc_mma_ts(d_tmem, a_tmem, bdesc, idesc, accumulate);
     }
-}
-// Arrival of a widening warp on the leader's barrier: the default (CTA) scope, as CUTLASS has it for the same hand-over of transformed
-// operands to a two-CTA MMA; the MMA is issued behind the leader's wait, which acquires at cluster scope.
-__device__ __forceinline__ void arrive_leader(unsigned cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of (n - 8) * scale, each product rounded once from fp32
 __device__ __forceinline__ unsigned nib2_to_bf16x2_scaled(unsigned w, f32x2 scale) {
@@ -335,7 +327,7 @@ gemm_qt_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             __syncwarp();
             if (lane == 0) {
                 if (CG == 1 || leader) mbar_arrive(bar_a_full + 8 * ab);
-                else arrive_leader(leader_full + 8 * ab);
+                else mbar_arrive_leader(leader_full + 8 * ab);
             }
             for (int i = 0; i < QT_SETS; i++) advance();
         }
@@ -440,7 +432,9 @@ gemm_qt_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                     each_chunk([&](int c, float (&v)[CHUNK]) {
                         const unsigned dst = mapa_rank(mine + (unsigned)((c / p.S * p.S + split) * CHUNK_BYTES), (unsigned)(c % p.S * CG + rank));
 #pragma unroll
-                        for (int j = 0; j < CHUNK / 4; j++) st_cluster_v4(dst + (unsigned)(j * QT_ROWS * 16), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                        for (int j = 0; j < CHUNK / 4; j++)
+                            st_cluster_v4(dst + (unsigned)(j * QT_ROWS * 16), __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]),
+                                          __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3]));
                     });
                 __syncwarp();
                 cluster_sync_all();

@@ -9,7 +9,7 @@
 //     of 32 / 64 up to 256 / 512 (all of TMEM): the launcher picks W and the split of K so that one wave fills the SMs;
 //   - the S parts of a split K form one cluster and add their accumulators in rank order through distributed shared memory;
 //   - int8-compressed and 4-bit weights cross HBM and L2 as they are stored: twelve warps widen each slab to bf16 in shared
-//     memory between the TMA load and the MMA.
+//     memory between the TMA load and the MMA.  (Most calls with such weights go to gemm_qt.cu, see run_wave.)
 // int8 values are exact in bf16; a 4-bit value is multiplied by its group scale in fp32 and rounded to bf16.
 //
 // Warps: 0 = TMA loads of activations (and of plain weights), 1 = MMA issue (one lane) and TMEM owner, 2 = TMA loads of
@@ -56,18 +56,6 @@ struct WaveParams {
     unsigned long long wait_limit_ns;
 };
 
-// Arrival of a widening warp of the second CTA on the leader's barrier.  The bytes are handed over by the warp's proxy fence, which orders
-// them before what the async proxy reads from then on, and the MMA that reads them is issued behind the leader's wait, which
-// acquires at cluster scope.  The arrival itself has the default (CTA) scope: the form that CUTLASS has for the same hand-over
-// of transformed operands to a two-CTA MMA (ClusterBarrier::arrive(cta_id) behind fence_view_async_shared).  A release at cluster
-// scope is a full memory barrier at every slab: in each widening warp 36.7 us for 4 bits, 100 x 4096 x 11008 (26.6 without); in one
-// forwarding warp of the second CTA 38.1 us for int8, 705 x 2560 x 10240 (32.1) and 157 us for 300 x 11008 x 8192 (100).
-__device__ __forceinline__ void mbar_arrive_leader(unsigned cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void st_cluster_v4(unsigned cluster_addr, unsigned a, unsigned b, unsigned c, unsigned d) {
-    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 // nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of (n - 8) * scale, each product rounded once from fp32
 __device__ __forceinline__ unsigned nib2_to_bf16x2_scaled(unsigned w, float scale) {
     const unsigned a = nib2_to_bf16x2(w);

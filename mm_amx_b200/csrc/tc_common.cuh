@@ -664,6 +664,18 @@ __device__ __forceinline__ void nib8_to_bf16x2_64th(unsigned w, unsigned* r) {
         asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r[2 * h + 1]) : "r"(v & 0x00f000f0u), "r"(0x7d007d00u), "r"(0xbe00be00u));      // * 2^123 - 1/8
     }
 }
+// Arrival of a widening warp of the second CTA on the leader's barrier.  The bytes are handed over by the warp's proxy fence, which orders
+// them before what the async proxy reads from then on, and the MMA that reads them is issued behind the leader's wait, which
+// acquires at cluster scope.  The arrival itself has the default (CTA) scope: the form that CUTLASS has for the same hand-over
+// of transformed operands to a two-CTA MMA (ClusterBarrier::arrive(cta_id) behind fence_view_async_shared).  A release at cluster
+// scope is a full memory barrier at every slab: in each widening warp 36.7 us for 4 bits, 100 x 4096 x 11008 (26.6 without); in one
+// forwarding warp of the second CTA 38.1 us for int8, 705 x 2560 x 10240 (32.1) and 157 us for 300 x 11008 x 8192 (100).
+__device__ __forceinline__ void mbar_arrive_leader(unsigned cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void st_cluster_v4(unsigned cluster_addr, unsigned a, unsigned b, unsigned c, unsigned d) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // nibbles n at bits [0,4) and [16,20) of w -> bf16x2 of n - 8, exactly: (128 + n) - 136
 __device__ __forceinline__ unsigned nib2_to_bf16x2(unsigned w) {
     unsigned a;
