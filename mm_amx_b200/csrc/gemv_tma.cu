@@ -67,7 +67,6 @@ struct Params {
     unsigned long long wait_limit_ns;
     int cluster;          // 1: launched as clusters of S CTAs (S <= 8); the pieces of a row block meet in distributed
                           // shared memory instead of the global scratch
-    int chains;           // gemv_tc_kernel: accumulators that the stages of a piece take in turn (1 or TC_CHAINS)
     int pf_cap;           // stages beyond the ring that the producer prefetches into L2 when the CTA starts
     const float* scales;  // 4-bit weights: [row block][stage][2][128] group scales, row block 0 = packed rows [0, 128)
     const unsigned char* ximg;   // quantised weights, optional: the activations already converted by xstage_kernel, one
@@ -1044,6 +1043,8 @@ __device__ __forceinline__ unsigned long long tc_smem_desc(unsigned smem_addr) {
     return d;
 }
 
+// CHAINS: TC_CHAINS, or 1 (see sums_pinned; as an argument of the kernel it cost 1 %)
+template <int CHAINS>
 __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                 const __grid_constant__ CUtensorMap map_x, const Params p) {
     using L = TcLayout;
@@ -1142,14 +1143,14 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
                     if (!alive) break;
                     tc_fence_after();
                     const int i = ks - ks0;
-                    const unsigned d_tmem = tmem_base + (unsigned)((ab * TC_CHAINS + (i & (p.chains - 1))) * 16);
+                    const unsigned d_tmem = tmem_base + (unsigned)((ab * TC_CHAINS + i % CHAINS) * 16);
                     const unsigned sa = smem_u32(smem + stage * TC_STAGE_BYTES);
                     const unsigned long long adesc = tc_smem_desc(sa), bdesc = tc_smem_desc(sa + STAGE_BYTES);
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < 4; k++)     // 4 x 16 K per stage, 32 bytes further along the swizzled row each
                             tc_mma_bf16(d_tmem, adesc + (unsigned long long)(k * 2), bdesc + (unsigned long long)(k * 2), idesc,
-                                        (unsigned)(i >= p.chains || k != 0));
+                                        (unsigned)(i >= CHAINS || k != 0));
                         tc_commit(bar_empty + 8 * stage);
                         if (ks == ks1 - 1) tc_commit(bar_acc_full + 8 * ab);
                     }
@@ -1194,7 +1195,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemv_tc_kernel(const __grid_con
                 float sum[16];
 #pragma unroll
                 for (int j = 0; j < 16; j++) sum[j] = 0.0f;
-                for (int c = 0; ok && c < min(p.chains, ks1 - ks0); c++) {
+                for (int c = 0; ok && c < min(CHAINS, ks1 - ks0); c++) {
                     unsigned r[16];
                     tc_ld16(tmem_base + ((unsigned)(warp * 32) << 16) + (unsigned)((ab * TC_CHAINS + c) * 16), r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -1434,7 +1435,6 @@ static int prepare_job(const Weight& w, const void* A, int M, int K, int64_t lda
     if (!p.status) { set_error("gemv: no kernel status word on this device"); return B200FC_ERR_CUDA; }
     p.wait_limit_ns = wait_limit_ns();
     p.S = 0; p.cluster = 0; p.pf_cap = 0;
-    p.chains = sums_pinned(ep) ? 1 : TC_CHAINS;
     p.ximg = nullptr;
 #ifdef B200FC_TRACE
     {
@@ -1485,6 +1485,7 @@ static long long max_ctas() {
     return gmax > kGemvMaxCtas - 2 ? kGemvMaxCtas - 2 : gmax;   // the last two counter words serve the two-job barrier
 }
 
+template <int CHAINS>
 static int launch_tc(const CUtensorMap& map_w, const Params& p, const void* A, int M, int K, int64_t lda, int grid, cudaStream_t s) {
     EncodeTiledFn fn = encode_fn();
     // the activations as a bf16 matrix [M, K]; box = 64 K x 16 tokens, rows past M and columns past K read as zeros
@@ -1499,7 +1500,7 @@ static int launch_tc(const CUtensorMap& map_w, const Params& p, const void* A, i
     static std::atomic<unsigned long long> attr_devices{0};
     {
         const int arc = once_per_device(attr_devices, [] {
-            B200FC_CUDA(cudaFuncSetAttribute(gemv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TcLayout::SMEM));
+            B200FC_CUDA(cudaFuncSetAttribute(gemv_tc_kernel<CHAINS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcLayout::SMEM));
             return (int)B200FC_OK;
         });
         if (arc) return arc;
@@ -1518,7 +1519,7 @@ static int launch_tc(const CUtensorMap& map_w, const Params& p, const void* A, i
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemv_tc_kernel, map_w, map_x, p));
+    B200FC_CUDA(cudaLaunchKernelEx(&cfg, gemv_tc_kernel<CHAINS>, map_w, map_x, p));
     count_launch();
     return B200FC_OK;
 }
@@ -1584,7 +1585,7 @@ int launch_gemv_tma(const Weight& w, const void* A, int M, int K, int64_t lda, i
         if (!w.scale_grp || (n0 % ROWS_PER_CTA)) { set_error("gemv: 4-bit weights need group scales and n0 %% 128 == 0"); return B200FC_ERR_INVALID; }
         return M <= 8 ? launch_variant<4, 1, false>(map, p, (int)grid, s) : launch_variant<4, 2, false>(map, p, (int)grid, s);
     }
-    if (tc) return launch_tc(map, p, A, M, K, lda, (int)grid, s);
+    if (tc) return sums_pinned(ep) ? launch_tc<1>(map, p, A, M, K, lda, (int)grid, s) : launch_tc<TC_CHAINS>(map, p, A, M, K, lda, (int)grid, s);
     auto launch = M <= 8 ? (w8 ? (short_chains ? launch_variant<8, 1, true> : launch_variant<8, 1, false>)
                                : (short_chains ? launch_variant<16, 1, true> : launch_variant<16, 1, false>))
                          : (w8 ? (short_chains ? launch_variant<8, 2, true> : launch_variant<8, 2, false>)
