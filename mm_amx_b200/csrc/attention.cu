@@ -396,7 +396,10 @@ int launch_decode_attention(const b200fc_attention_t& a, cudaStream_t s) {
     // in splits of 512 tokens or more, whose short CTAs even the lengths of the sequences out (us, one round / this: B = 20, 16 kv heads,
     // up to 8765 tokens 111 / 76; B = 14, up to 14313 tokens 106 / 84; B = 19, up to 2540 tokens 34.8 / 26.1.  Not with shorter sequences,
     // where the second launch costs more: B = 18, 32 kv heads, up to 600 tokens 13.3 / 17.6; nor with more pairs than places, which are even
-    // enough: B = 32, 32 kv heads, up to 800 tokens 25.1 / 27.4; with one round of 7 splits it gains nothing).
+    // enough: B = 32, 32 kv heads, up to 800 tokens 25.1 / 27.4; with one round of 7 splits it gains nothing).  The fuller one round is,
+    // the longer the sequences must be: the line goes through 127 timed calls of 160 to 592 pairs (one split / several: 592 pairs, up to 1210
+    // tokens 24.0 / 26.7, 2100 38.2 / 39.3, 3200 55.9 / 55.1; 448 pairs, 1210 20.9 / 22.7, 1800 29.2 / 28.7; 384, 1030 17.9 / 18.6, 1500 24.0 / 22.9;
+    // 320, 1030 17.6 / 16.5).  Three splits where two fit one round (200 pairs, 1030 tokens, one / two / three: 13.4 / 14.5 / 12.9).
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -406,8 +409,8 @@ int launch_decode_attention(const b200fc_attention_t& a, cudaStream_t s) {
     const bool deep = a.D == 64 && a.N >= 1024;
     const long long places = (long long)(deep ? ATT_CTAS_PER_SM<64> : 2) * sms;
     int splits = (int)(places / pairs);
-    if (deep && splits >= 1 && splits <= 2) {
-        const int rounds = (int)((5 * places + 2 * pairs - 1) / (2 * pairs)), by_len = a.N / 512;
+    if (deep && splits >= 1 && splits <= 2 && (a.N + 1080LL) * places >= 3670 * pairs) {
+        const int rounds = (int)((5 * places + 2 * pairs - 1) / (2 * pairs)), by_len = max(a.N / 512, splits + 1);
         splits = max(splits, min(rounds, by_len));
     }
     const int max_by_len = (a.N + 2 * BLK * ATT_WARPS - 1) / (2 * BLK * ATT_WARPS);

@@ -126,6 +126,30 @@ def test_captured_sub_states_belong_to_the_graph(B, Hkv, N, D, warm):
     capi.sync_check()
 
 
+@pytest.mark.parametrize("pairs,N,launches", [(592, 2470, 1), (592, 2600, 2), (448, 1640, 1), (448, 1700, 2), (320, 1024, 2), (200, 1030, 2), (593, 4000, 1)])
+def test_heads_of_64_are_split_where_that_is_faster(pairs, N, launches):
+    """either side of the line between one range of tokens per pair, which needs no second launch, and several"""
+    import torch
+    if H.sms() != 148:
+        pytest.skip("the line of 148 SMs")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N)
+    D = 64
+    q = torch.randn((pairs, 1, D), generator=g, device="cuda").to(torch.bfloat16)
+    k, v = (torch.randn((pairs, 1, N, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    lens = torch.randint(1, N + 1, (pairs,), generator=g, device="cuda", dtype=torch.int32)
+    out = torch.zeros((pairs, 1, D), device="cuda")
+    before = capi.launch_count()
+    capi.decode_attention(capi.Attention(pairs, 1, 1, N, D, q.data_ptr(), D * 2, D * 2, k.data_ptr(), v.data_ptr(), N * D * 2, N * D * 2, D * 2,
+                                         out.data_ptr(), D * 4, D * 4, capi.F32, lens.data_ptr(), 0.125))
+    assert capi.launch_count() - before == launches
+    capi.sync_check()
+    s = torch.einsum("bhd,bhnd->bhn", q.double(), k.double()) * 0.125
+    s = s.masked_fill(torch.arange(N, device="cuda")[None, None] >= lens[:, None, None], float("-inf"))
+    ref = torch.einsum("bhn,bhnd->bhd", s.softmax(-1), v.double())
+    assert float((out - ref).abs().max() / ref.abs().max()) < 5e-3          # (probabilities in bf16, as above)
+
+
 def test_decode_attention_repeated_calls_of_mixed_shapes():
     """calls of different shapes follow one another on a stream and share the workspace of the sub-states (it grows and
     is reused); every call must see only its own sub-states"""
