@@ -325,13 +325,13 @@ int matmul_device(const Weight& w, Weight* w_mut, const void* A, int dtypeA, int
         const int blk = widened_block_rows(w.K_pad);
         const int r_lo = n0 / kRowPad * kRowPad;                  // packed rows are padded to kRowPad
         void* wide = nullptr;
-        rc = get_stream_scratch((size_t)blk * row_bytes, s, 3, &wide);
-        if (rc) return rc;
-        for (int r0 = r_lo; r0 < n1; r0 += blk) {
+        bool own = false;       // (memory of the graph that the stream is being captured into)
+        rc = get_stream_scratch((size_t)blk * row_bytes, s, 3, &wide, &own);
+        for (int r0 = r_lo; r0 < n1 && !rc; r0 += blk) {
             const int rows = (w.N_pad - r0 < blk) ? (w.N_pad - r0) : blk;
             const int c0 = r0 > n0 ? r0 : n0, c1 = (r0 + rows < n1) ? (r0 + rows) : n1;
             rc = launch_dequant_bf16(w, r0, rows, wide, w.K_pad, s);
-            if (rc) return rc;
+            if (rc) break;
             // the block is addressed as a weight matrix whose row 0 is packed row r0: shift the column range and the
             // per-column arrays of the epilogue accordingly
             Epilogue e2 = ep;
@@ -341,9 +341,12 @@ int matmul_device(const Weight& w, Weight* w_mut, const void* A, int dtypeA, int
             if (e2.q_per_oc) e2.q_per_oc += r0;
             if (e2.residual) e2.residual = (const char*)e2.residual + (long long)r0 * 2;
             rc = launch_gemm_tc(wide, B200FC_BF16, w.K_pad, rows, A_use, B200FC_BF16, M, K, lda_use, c0 - r0, c1 - r0, e2, s);
-            if (rc) return rc;
         }
-        return B200FC_OK;
+        if (own && wide) {
+            const cudaError_t e = cudaFreeAsync(wide, s);
+            if (!rc && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync of widened weights");
+        }
+        return rc;
     }
     return launch_gemm_tc(w.data, w.dtype, w.K_pad, w.N_pad, A_use, dtypeA, M, K, lda_use, n0, n1, ep, s);
 }

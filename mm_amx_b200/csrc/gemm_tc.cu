@@ -694,12 +694,13 @@ int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cuda
     p.split_stride = 0;
     const Epilogue final_ep = p.ep;
     int pitch = 0;
+    bool own = false;       // (the workspace is memory of the graph that the stream is being captured into)
+    void* ws = nullptr;
     if (splits > 1) {
         const int nspan = p.n1 - p.n0;
         pitch = (nspan + 3) / 4 * 4;
         const size_t slab = (size_t)p.M * pitch * 4;
-        void* ws = nullptr;
-        int rc = get_stream_scratch(slab * splits, s, 1, &ws);
+        int rc = get_stream_scratch(slab * splits, s, 1, &ws, &own);
         if (rc) return rc;
         p.split_stride = (long long)slab;
         p.ep.steps = 0;
@@ -733,6 +734,7 @@ int launch_cfg2(const CUtensorMap& ma, const CUtensorMap& mw, GemmParams p, cuda
         B200FC_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel, (const unsigned*)((char*)p.ep.C + (long long)p.n0 * 4),
                                        (long long)p.M * pitch, pitch, splits, p.M, p.n0, p.n1, p.acc_is_int, final_ep));
         count_launch();
+        if (own) B200FC_CUDA(cudaFreeAsync(ws, s));
     }
     return B200FC_OK;
 }

@@ -62,5 +62,47 @@ def test_bits_are_those_recorded(case):
     assert np.array_equal(outputs(*case), np.load(GOLDEN)[name(case)])
 
 
+def test_captured_calls_give_the_same_bits():
+    """blocks of widened weights and their split of K: workspaces of the graph's own, on a fresh stream and where a larger call
+    re-allocates the stream's before the replay"""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+
+    def make(M, K, N):
+        x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+        B = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+        scales = torch.full((N,), 2.5 / K ** 0.5 / 73.3, device="cuda")
+        w = capi.Weight(B.data_ptr(), capi.S8, K, N, K, True, capi.PACK_INT8_CHANNEL, scales.data_ptr())
+        out = torch.zeros((M, N), device="cuda")
+        ep = capi.make_epilogue(out.data_ptr(), 4 * N, capi.F32, capi.STEP_DEQUANT | capi.STEP_GELU)
+        return out, lambda stream: w.matmul(x.data_ptr(), capi.BF16, M, K, 2 * K, ep, stream=stream.cuda_stream), (x, w, ep)
+
+    out, call, keep = make(266, 3072, 23680)
+    out2, larger, keep2 = make(300, 8192, 23680)
+    before = capi.launch_count()
+    call(torch.cuda.default_stream())
+    assert capi.launch_count() - before > 4             # (widened, multiplied in parts of K, added: block by block)
+    capi.sync_check()
+    want = out.clone()
+    torch.cuda.synchronize()
+    for warm in (False, True):
+        s = torch.cuda.Stream()
+        if warm:
+            call(s)
+            s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            call(torch.cuda.current_stream())
+        for _ in range(2):
+            out.zero_()
+            larger(s)
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(out, want)
+    capi.sync_check()
+
+
 if __name__ == "__main__":
     np.savez_compressed(sys.argv[1], **{name(c): outputs(*c) for c in CASES})
