@@ -775,8 +775,10 @@ int run_wave(WaveCall& c, int n0, int n1) {
         // 571 x 10624 x 21504 575 / 201, 1071 x 2560 x 22784 210 / 112, 4096 x 4096 x 11008 289 / 239; 4 bits 3526 x 8448 x 10168
         // 575 / 449), and of the others those of up to 512 rows and those whose K would be split (us, here / there: int8 22 x 3840 x 6016
         // 26.4 / 11.8, 158 x 3840 x 8576 37.0 / 26.5, 949 x 8704 x 2048 39.8 / 34.3; 4 bits 33 x 2400 x 9824 21.7 / 14.6).  More rows in tiles
-        // of all of K keep up here (int8 705 x 2560 x 10240 35.7 / 42.0, 2017 x 1408 x 4200 25.6 / 30.9, 1689 x 1920 x 1920 19.4 / 21.1).
-        // 4 bits with more than 64 rows and many chains are level (100 x 4096 x 11008 24.8 / 24.8).  Folded calls would be faster there as
+        // of all of K are level or faster here, whatever the post-ops (bias, bf16 / bias, GeLU, bf16 / plain fp32, here : there: int8
+        // 705 x 2560 x 10240 34.4 : 35.0 / 39.4 : 40.7 / 35.8 : 34.5, 2017 x 1408 x 4200 27.5 : 29.8 / 33.2 : 35.7 / 29.1 : 28.8; 4 bits
+        // 705 x 2560 x 10240 38.7 : 43.6 / 43.5 : 47.6 / 39.4 : 42.9; not all: int8 1689 x 1920 x 1920 20.5 : 18.7 / 22.7 : 20.8 / 21.1 : 18.5).
+        // 4 bits with more than 64 rows and many chains are nearly level (100 x 4096 x 11008 26.4 : 25.6 / 27.5 : 26.9 / 26.6 : 25.6).  Folded calls would be faster there as
         // well (4 bits 300 x 4096 x 11008 59.5 / 40.4), but their tiles are what b200fc_last_wave_tile reports and stay.  K is summed in
         // no fewer chains than it would be here.
         // fp32 behind GeLU (sums_pinned): only where K is one chain on either path, which gives the same bits (slabs < 96: a ragged last
