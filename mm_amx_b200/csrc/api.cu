@@ -94,6 +94,38 @@ static bool host_range(const void* p, HostRange* r) {
     return true;
 }
 
+// Pinned words that the host-buffer calls receive the status in, one per MLP object from its first such call until it is freed.  All lie in
+// one 16 KB piece, which the first call of the process allocates and which stays: pinned memory of its own took every MLP 1 to 3 ms to
+// allocate and free.  Null (the status then goes through pageable memory) when a thousand objects have theirs already.
+static std::mutex g_host_status_mu;
+static std::vector<int*>& free_host_status() {
+    static std::vector<int*>& words = *new std::vector<int*>;      // (never destroyed: objects may be freed while the process ends)
+    return words;
+}
+static int* take_host_status() {
+    constexpr int kWords = 1024, kStride = 4;                       // (16 bytes apart)
+    static int* page = nullptr;
+    std::lock_guard<std::mutex> lk(g_host_status_mu);
+    std::vector<int*>& words = free_host_status();
+    if (!page) {
+        if (cudaHostAlloc((void**)&page, kWords * kStride * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            page = nullptr;
+            return nullptr;
+        }
+        for (int i = kWords - 1; i >= 0; i--) words.push_back(page + i * kStride);
+    }
+    if (words.empty()) return nullptr;
+    int* p = words.back();
+    words.pop_back();
+    return p;
+}
+static void give_host_status(int* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_host_status_mu);
+    free_host_status().push_back(p);
+}
+
 struct Scratch { void* p = nullptr; size_t bytes = 0; };
 struct ScratchKey {
     int dev; cudaStream_t s; int slot;
@@ -787,13 +819,8 @@ int b200fc_mlp_create(const void* gate, const void* up, const void* down, int K,
         if (!rc) rc = alloc_weight(m.down, Ns, K, B200FC_BF16);
         if (!rc) rc = launch_pack_gate_up(sg.p, su.p, sg.ld, K, Ns, m.gate_up, s);
         if (!rc) rc = launch_pack(sd.p, B200FC_BF16, Ns, K, sd.ld, 1, m.down, false, s);
-        if (!rc) {      // (for mlp_run_host, whose first call need not allocate it)
-            const cudaError_t e = cudaHostAlloc((void**)&m.host_status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-            if (e != cudaSuccess) rc = cuda_fail(e, "mlp_create status word");
-        }
         if (!rc && cudaStreamSynchronize(s) != cudaSuccess) { rc = cuda_fail(cudaGetLastError(), "mlp_create sync"); }
     }
-    if (rc && m.host_status) cudaFreeHost(m.host_status);
     if (rc) { free_weight(&m.gate_up); free_weight(&m.down); delete h; return rc; }
     *out = h;
     return B200FC_OK;
@@ -803,7 +830,7 @@ int b200fc_mlp_free(b200fc_mlp_t* h) {
     if (!h) return B200FC_OK;
     free_weight(&h->m.gate_up); free_weight(&h->m.down);
     cudaFree(h->m.act); cudaFree(h->m.stage_x); cudaFree(h->m.stage_o);
-    if (h->m.host_status) cudaFreeHost(h->m.host_status);
+    give_host_status(h->m.host_status);
     for (int i = 0; i < 3; i++) if (h->m.pipe_streams[i]) cudaStreamDestroy(h->m.pipe_streams[i]);
     if (h->m.ev_fork) cudaEventDestroy(h->m.ev_fork);
     if (h->m.ev_join) cudaEventDestroy(h->m.ev_join);
@@ -1051,6 +1078,7 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
     if (rc) return rc;
     static int pipe_min = -1;
     if (pipe_min < 0) { const char* e = getenv("B200FC_HOST_PIPE_MIN"); pipe_min = e ? atoi(e) : 512; }
+    if (!m.host_status) m.host_status = take_host_status();
     if (M < pipe_min) {
         // Pinned buffers: kernels of this library copy them, in one chain with the projections (us, copy engines / kernels:
         // 74 x 1024 x 3232 59 / 51, 283 x 1152 x 2912 115 / 96, 511 x 1024 x 3008 163 / 104, 207 x 4736 x 16960 300 / 213).  From 512
@@ -1060,7 +1088,7 @@ int b200fc_mlp_run_host(b200fc_mlp_t* h, const void* x, int64_t ldx, int M, void
         const bool rows16 = row % 16 == 0 && ldx >= (int64_t)row && ldo >= (int64_t)row;
         void* xd = rows16 ? (void*)span_on_device(x, ldx, x_span, false, host_range) : nullptr;
         void* od = xd ? (void*)span_on_device(out, ldo, o_span, true, host_range) : nullptr;
-        void* sd = od ? (void*)span_on_device(m.host_status, 0, sizeof(int), true, host_range) : nullptr;
+        void* sd = od && m.host_status ? (void*)span_on_device(m.host_status, 0, sizeof(int), true, host_range) : nullptr;
         int* status = sd ? kernel_status_word() : nullptr;
         if (status) {
             rc = launch_host_copy(xd, ldx, m.stage_x, (int64_t)row, M, (int)row, nullptr, nullptr, s);

@@ -334,3 +334,21 @@ def test_host_rows_go_through_kernels_only_inside_one_allocation():
     plain = launches(pageable, pageable[M:])
     assert launches(pinned, pinned[M:]) == launches(pinned[2 * M:], pinned[3 * M:]) == plain + 2
     assert launches(pinned, pageable) == launches(pageable, pinned) == plain
+
+
+def test_host_calls_of_more_objects_than_status_words():
+    """the 1024 pinned words run out, and words given back are used again"""
+    import torch
+    K, N = 64, 32
+    g = torch.Generator().manual_seed(3)
+    gate, up, down = (torch.randn(s, generator=g).mul_(0.1).to(torch.bfloat16).cuda() for s in ((N, K), (N, K), (K, N)))
+    x, out = torch.randn((1, K), generator=g).to(torch.bfloat16).pin_memory(), torch.empty((1, K), dtype=torch.bfloat16).pin_memory()
+    kept, want = [], None
+    for i in range(1100):
+        if i == 1050:
+            del kept[:100]
+        kept.append(capi.Mlp(gate.data_ptr(), up.data_ptr(), down.data_ptr(), K, N, 0, 1))
+        out.fill_(float("nan"))
+        kept[-1].run_host(x.data_ptr(), 2 * K, 1, out.data_ptr(), 2 * K)
+        want = out.clone() if want is None else want
+        assert torch.equal(out, want), i
